@@ -54,8 +54,8 @@ __device__ __forceinline__ void tfsf_apply(const PatchSet& ps, const C* tab, int
   const int wi = a == 0 ? 0 : ps.hi[0] - ps.lo[0], wj = a == 1 ? 0 : ps.hi[1] - ps.lo[1], wk = a == 2 ? 0 : ps.hi[2] - ps.lo[2];
   if (ui < 0 || uj < 0 || uk < 0 || ui > wi || uj > wj || uk > wk) return;
   const int off = ui * ps.stride[0] + uj * ps.stride[1] + uk * ps.stride[2];
-  if (h0) d = d + tab[ps.tab + off];
-  if (h1) d = d + tab[ps.tab + ps.plane_len + off];
+  if (h0) d = d + __ldg(tab + ps.tab + off);
+  if (h1) d = d + __ldg(tab + ps.tab + ps.plane_len + off);
 }
 
 // psi = b*psi + c*curl; returns curl/kappa + psi (reference: three_dim_pml.cc:186-188).

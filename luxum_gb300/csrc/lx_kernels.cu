@@ -626,73 +626,29 @@ __global__ void __launch_bounds__(256) e_kernel_2d(const StepParams<T, C> p) {
 // enters E as stored (FP16 storage rounds it first), so the step matches the two-sweep kernels
 // bit for bit.
 
-// New Hx of planar cell (i,k), k < Nz-1: the arithmetic of h2_apply (two_dim_pml.cc:149-152).
-// A null psi_out recomputes a neighbour's value and leaves its psi to the owner.
-template <class T, class C, bool UNI, bool FAST>
-__device__ __forceinline__ C hx2_value(const StepParams<T, C>& p, const C* psi_in, C* psi_out, int i, int k, C ey,
-                                       C ey_k, C hx, bool tf) {
-  C d2 = ey_k - ey;
-  if (!UNI) d2 = mulC(d2, p.rd[2]);
-  if (!FAST && tf) tfsf_apply<C>(p.setsH[0][1], p.tab, i, 0, k, d2);
-  if (!FAST && p.pml) {
-    const int sz = slab_index(p.slab[2], k);
-    if (sz >= 0) {
-      const long long q = (long long)i * p.slab[2].n + sz;
-      const C ps = fmaC(p.bH[2][k], psi_in[q], p.cH[2][k] * d2);
-      if (psi_out) psi_out[q] = ps;
-      d2 = fmaC(d2, p.rkH[2][k], ps);
-    }
-  }
-  return fmaC(p.Dbs, d2, hx);
+// One psi term of a planar cell with its old psi and profile values already loaded:
+// psi = b*psi + c*d, d = d/kappa + psi (pml_term's arithmetic).
+template <class C>
+__device__ __forceinline__ void psi2_term(C b, C c, C rk, C& psi, C& d) {
+  psi = fmaC(b, psi, c * d);
+  d = fmaC(d, rk, psi);
 }
 
-// New Hz of planar cell (i,k), i < Nx-1 (two_dim_pml.cc:155-158).
-template <class T, class C, bool UNI, bool FAST>
-__device__ __forceinline__ C hz2_value(const StepParams<T, C>& p, const C* psi_in, C* psi_out, int i, int k, C ey,
-                                       C ey_i, C hz, bool tf) {
-  C d1 = ey_i - ey;
-  if (!UNI) d1 = mulC(d1, p.rd[0]);
-  if (!FAST && tf) tfsf_apply<C>(p.setsH[2][0], p.tab, i, 0, k, d1);
-  if (!FAST && p.pml) {
-    const int sx = slab_index(p.slab[0], i);
-    if (sx >= 0) {
-      const long long q = (long long)sx * p.Nzp + k;
-      const C ps = fmaC(p.bH[0][i], psi_in[q], p.cH[0][i] * d1);
-      if (psi_out) psi_out[q] = ps;
-      d1 = fmaC(d1, p.rkH[0][i], ps);
-    }
-  }
-  return fmaC(-p.Dbs, d1, hz);
-}
-
-// New Ey of planar cell (i,k), i and k in [1, N-2] (two_dim_pml.cc:164-176): e2_apply's arithmetic.
-template <class T, class C, bool UNI, bool FAST>
-__device__ __forceinline__ C ey2_value(const StepParams<T, C>& p, const C* pz_in, C* pz_out, const C* px_in, C* px_out,
-                                       int i, int k, C ey, C hx, C hx_k, C hz, C hz_i, C cb, bool tf) {
-  C d1 = hx - hx_k;  // dHx/dz (z profile)
-  C d2 = hz - hz_i;  // dHz/dx (x profile)
-  if (!UNI) { d1 = mulC(d1, p.rd[2]); d2 = mulC(d2, p.rd[0]); }
-  if (!FAST && tf) {
-    tfsf_apply<C>(p.setsE[1][0], p.tab, i, 0, k, d1);
-    tfsf_apply<C>(p.setsE[1][1], p.tab, i, 0, k, d2);
-  }
-  if (!FAST && p.pml) {
-    const int sz = slab_index(p.slab[2], k), sx = slab_index(p.slab[0], i);
-    if (sz >= 0) {
-      const long long q = (long long)i * p.slab[2].n + sz;
-      const C ps = fmaC(p.bE[2][k], pz_in[q], p.cE[2][k] * d1);
-      pz_out[q] = ps;
-      d1 = fmaC(d1, p.rkE[2][k], ps);
-    }
-    if (sx >= 0) {
-      const long long q = (long long)sx * p.Nzp + k;
-      const C ps = fmaC(p.bE[0][i], px_in[q], p.cE[0][i] * d2);
-      px_out[q] = ps;
-      d2 = fmaC(d2, p.rkE[0][i], ps);
-    }
-  }
-  return fmaC(cb, d1 - d2, ey);
-}
+// What one row of a run reads, issued as a block ahead of the row before it: with the loads of
+// row i+1 in flight while row i is formed and stored, and none of a row's psi loads behind
+// another psi term's store, a row costs one memory round trip.  (Loading each psi term where it
+// is used cost a warp at the grid's edge six round trips a row: 2048^2 FP32 with CPML and TF/SF
+// 69.7 us a step against 40.0 without either.)
+template <class C>
+struct Row2 {
+  C ey_i;         // Ey of the next row
+  C hx, hz, cb;
+  C ey_k;         // lane 31: Ey of column k0+32
+  C hxh, eyh;     // lane 0: Hx and Ey of column k0-1
+  C phx, pez;     // psi of the z slab: Hx and Ey z parts
+  C phxh;         // lane 0: psi of Hx at column k0-1
+  C phz, pex;     // psi of the x slab: Hz and Ey x parts
+};
 
 // One warp's rows [i0, i1) of the 32 columns from k0; returns the bit pattern of its largest
 // Ey^2 (the max over the whole Ey array, two_dim_pml.cc:181).
@@ -710,58 +666,130 @@ __device__ __forceinline__ typename MaxBits<C>::type step2_rows(const StepParams
   T* hxo = p.H1[0];
   const T* hzi = p.H[2];
   T* hzo = p.H1[2];
-  const C* qhx = p.psiH[0][1];  // Hx, z part
-  C* qhxo = p.psiH1[0][1];
-  const C* qhz = p.psiH[2][0];  // Hz, x part
-  C* qhzo = p.psiH1[2][0];
-  const C* qez = p.psiE[1][0];  // Ey, z part
-  C* qezo = p.psiE1[1][0];
-  const C* qex = p.psiE[1][1];  // Ey, x part
-  C* qexo = p.psiE1[1][1];
   const bool kin = FAST || k < Nz;
   const bool ux = FAST || k < Nz - 1;
   const bool ke = FAST || (k >= 1 && k < Nz - 1);
+  const bool halo = lane == 0 && k0 >= 1;
   const long long si = p.si;
+  // the z slab: psi index and profile values of this column, and (lane 0) of column k0-1
+  const int zn = p.slab[2].n;
+  const bool pml = !FAST && p.pml;
+  const int sz = pml ? slab_index(p.slab[2], k) : -1;
+  const int szh = pml && halo ? slab_index(p.slab[2], k0 - 1) : -1;
+  C bHz = C(0), cHz = C(0), rHz = C(0), bEz = C(0), cEz = C(0), rEz = C(0), bHh = C(0), cHh = C(0), rHh = C(0);
+  if (sz >= 0 && ux) { bHz = __ldg(p.bH[2] + k); cHz = __ldg(p.cH[2] + k); rHz = __ldg(p.rkH[2] + k); }
+  if (sz >= 0 && kin) { bEz = __ldg(p.bE[2] + k); cEz = __ldg(p.cE[2] + k); rEz = __ldg(p.rkE[2] + k); }
+  if (szh >= 0) { bHh = __ldg(p.bH[2] + k0 - 1); cHh = __ldg(p.cH[2] + k0 - 1); rHh = __ldg(p.rkH[2] + k0 - 1); }
+
+  auto load = [&](int i, long long c, Row2<C>& r) {
+    const bool nx = FAST || i + 1 < Nx;
+    const bool ue = ke && (FAST || (i >= 1 && i < Nx - 1));
+    r.ey_i = (kin && nx) ? ld<T, C>(eyi + c + si) : C(0);
+    r.hx = kin ? ld<T, C>(hxi + c) : C(0);
+    r.hz = kin ? ld<T, C>(hzi + c) : C(0);
+    r.cb = (kin && ue) ? p.Cbs[1][c] : C(0);
+    r.ey_k = r.hxh = r.eyh = C(0);
+    if (lane == 31 && (FAST || k + 1 < Nz)) r.ey_k = ld<T, C>(eyi + c + 1);
+    if (halo) {
+      r.hxh = ld<T, C>(hxi + c - 1);
+      r.eyh = ld<T, C>(eyi + c - 1);
+    }
+    if (!FAST) {
+      r.phx = r.pez = r.phxh = r.phz = r.pex = C(0);
+      if (pml) {
+        const int sx = slab_index(p.slab[0], i);
+        if (sz >= 0 && ux) r.phx = p.psiH[0][1][(long long)i * zn + sz];
+        if (sz >= 0 && ue) r.pez = p.psiE[1][0][(long long)i * zn + sz];
+        if (szh >= 0) r.phxh = p.psiH[0][1][(long long)i * zn + szh];
+        if (sx >= 0 && kin && nx) r.phz = p.psiH[2][0][(long long)sx * p.Nzp + k];
+        if (sx >= 0 && kin && ue) r.pex = p.psiE[1][1][(long long)sx * p.Nzp + k];
+      }
+    }
+  };
+  // new Hz of (i, k) from its x difference (two_dim_pml.cc:155-158)
+  auto hz_value = [&](int i, int sx, C ey, C ey_i, C hz, C& psi) -> C {
+    C d1 = ey_i - ey;
+    if (!UNI) d1 = mulC(d1, p.rd[0]);
+    if (!FAST && tfH) tfsf_apply<C>(p.setsH[2][0], p.tab, i, 0, k, d1);
+    if (!FAST && sx >= 0) psi2_term(__ldg(p.bH[0] + i), __ldg(p.cH[0] + i), __ldg(p.rkH[0] + i), psi, d1);
+    return stored<T, C>(fmaC(-p.Dbs, d1, hz));
+  };
+
   long long c = (long long)i0 * si + k;
   C ey = kin ? ld<T, C>(eyi + c) : C(0);
+  Row2<C> cur;
+  load(i0, c, cur);
   C hz_p = C(0);  // new Hz of the row above
   if (i0 >= 1) {
     const C eym = kin ? ld<T, C>(eyi + c - si) : C(0);
     const C hzm = kin ? ld<T, C>(hzi + c - si) : C(0);
-    hz_p = stored<T, C>(hz2_value<T, C, UNI, FAST>(p, qhz, nullptr, i0 - 1, k, eym, ey, hzm, tfH));
+    const int sx = pml ? slab_index(p.slab[0], i0 - 1) : -1;
+    C psi = (!FAST && sx >= 0 && kin) ? p.psiH[2][0][(long long)sx * p.Nzp + k] : C(0);  // its owner stores the new psi
+    hz_p = hz_value(i0 - 1, sx, eym, ey, hzm, psi);
   }
   typename MaxBits<C>::type m = 0;
 #pragma unroll 1
   for (int i = i0; i < i1; ++i, c += si) {
+    Row2<C> nxt = cur;
+    if (i + 1 < i1) load(i + 1, c + si, nxt);
     const bool nx = FAST || i + 1 < Nx;
     const bool ue = ke && (FAST || (i >= 1 && i < Nx - 1));
-    const C eyn = (kin && nx) ? ld<T, C>(eyi + c + si) : C(0);
-    const C hx = kin ? ld<T, C>(hxi + c) : C(0);
-    const C hz = kin ? ld<T, C>(hzi + c) : C(0);
-    const C cb = (kin && ue) ? p.Cbs[1][c] : C(0);
+    const int sx = pml ? slab_index(p.slab[0], i) : -1;
     C ey_k = __shfl_down_sync(0xffffffffu, ey, 1);
-    if (lane == 31) ey_k = (FAST || k + 1 < Nz) ? ld<T, C>(eyi + c + 1) : C(0);
-    C hxh = C(0), eyh = C(0);  // lane 0: Hx and Ey of column k0-1
-    if (lane == 0 && k0 >= 1) {
-      hxh = ld<T, C>(hxi + c - 1);
-      eyh = ld<T, C>(eyi + c - 1);
+    if (lane == 31) ey_k = cur.ey_k;
+    // new Hx of (i, k) from its z difference (two_dim_pml.cc:149-152)
+    C hxn = cur.hx;
+    if (kin && ux) {
+      C d2 = ey_k - ey;
+      if (!UNI) d2 = mulC(d2, p.rd[2]);
+      if (!FAST && tfH) tfsf_apply<C>(p.setsH[0][1], p.tab, i, 0, k, d2);
+      if (!FAST && sz >= 0) psi2_term(bHz, cHz, rHz, cur.phx, d2);
+      hxn = stored<T, C>(fmaC(p.Dbs, d2, cur.hx));
     }
-    const C hxn = (kin && ux) ? stored<T, C>(hx2_value<T, C, UNI, FAST>(p, qhx, qhxo, i, k, ey, ey_k, hx, tfH)) : hx;
-    const C hzn = (kin && nx) ? stored<T, C>(hz2_value<T, C, UNI, FAST>(p, qhz, qhzo, i, k, ey, eyn, hz, tfH)) : hz;
+    const C hzn = (kin && nx) ? hz_value(i, sx, ey, cur.ey_i, cur.hz, cur.phz) : cur.hz;
     C hx_k = __shfl_up_sync(0xffffffffu, hxn, 1);
-    if (lane == 0)
-      hx_k = k0 >= 1 ? stored<T, C>(hx2_value<T, C, UNI, FAST>(p, qhx, nullptr, i, k0 - 1, eyh, ey, hxh, tfH)) : C(0);
-    const C eyw = (kin && ue) ? ey2_value<T, C, UNI, FAST>(p, qez, qezo, qex, qexo, i, k, ey, hxn, hx_k, hzn, hz_p, cb, tfE)
-                              : ey;
+    if (lane == 0) {
+      hx_k = C(0);
+      if (halo) {  // new Hx of column k0-1, recomputed; its owner stores the new psi
+        C d2 = ey - cur.eyh;
+        if (!UNI) d2 = mulC(d2, p.rd[2]);
+        if (!FAST && tfH) tfsf_apply<C>(p.setsH[0][1], p.tab, i, 0, k0 - 1, d2);
+        if (!FAST && szh >= 0) psi2_term(bHh, cHh, rHh, cur.phxh, d2);
+        hx_k = stored<T, C>(fmaC(p.Dbs, d2, cur.hxh));
+      }
+    }
+    // new Ey of (i, k), i and k in [1, N-2] (two_dim_pml.cc:164-176): e2_apply's arithmetic
+    C eyw = ey;
+    if (kin && ue) {
+      C d1 = hxn - hx_k;  // dHx/dz (z profile)
+      C d2 = hzn - hz_p;  // dHz/dx (x profile)
+      if (!UNI) { d1 = mulC(d1, p.rd[2]); d2 = mulC(d2, p.rd[0]); }
+      if (!FAST && tfE) {
+        tfsf_apply<C>(p.setsE[1][0], p.tab, i, 0, k, d1);
+        tfsf_apply<C>(p.setsE[1][1], p.tab, i, 0, k, d2);
+      }
+      if (!FAST) {
+        if (sz >= 0) psi2_term(bEz, cEz, rEz, cur.pez, d1);
+        if (sx >= 0) psi2_term(__ldg(p.bE[0] + i), __ldg(p.cE[0] + i), __ldg(p.rkE[0] + i), cur.pex, d2);
+      }
+      eyw = fmaC(cur.cb, d1 - d2, ey);
+    }
     if (kin) {
       st<T, C>(hxo + c, hxn);
       st<T, C>(hzo + c, hzn);
       st<T, C>(eyo + c, eyw);
+      if (!FAST) {
+        if (sz >= 0 && ux) p.psiH1[0][1][(long long)i * zn + sz] = cur.phx;
+        if (sz >= 0 && ue) p.psiE1[1][0][(long long)i * zn + sz] = cur.pez;
+        if (sx >= 0 && nx) p.psiH1[2][0][(long long)sx * p.Nzp + k] = cur.phz;
+        if (sx >= 0 && ue) p.psiE1[1][1][(long long)sx * p.Nzp + k] = cur.pex;
+      }
       const typename MaxBits<C>::type b = MaxBits<C>::of(eyw * eyw);
       m = b > m ? b : m;
     }
     hz_p = hzn;
-    ey = eyn;
+    ey = cur.ey_i;
+    cur = nxt;
   }
   return m;
 }
@@ -778,12 +806,14 @@ __device__ __forceinline__ typename MaxBits<C>::type step2_warp(const StepParams
   return step2_rows<T, C, UNI, false>(p, i0, i1, k0, tfH, tfE);
 }
 
-// Register cap of the single-sweep kernel: 6 blocks of 256 per SM (40 registers, no spills).
-constexpr int kSweepMinBlocks = 6;
+// Register cap of the single-sweep kernel: 5 blocks of 256 per SM (48 registers; the general path
+// spills 48 bytes).  With 6 it spills 120 (4096^2 with CPML and TF/SF 122.5 us a step against
+// 112.7), with 4 none (118.9).
+constexpr int kSweepMinBlocks = 5;
 
 // One simulation: a block is 32 z columns x 8 warps of R rows.
-template <class T, class C, bool UNI, int R>
-__global__ void __launch_bounds__(256, kSweepMinBlocks) step_kernel_2d(const StepParams<T, C> p) {
+template <class T, class C, bool UNI>
+__global__ void __launch_bounds__(256, kSweepMinBlocks) step_kernel_2d(const StepParams<T, C> p, const int R) {
   const int k0 = blockIdx.x * 32;
   const int i0 = (blockIdx.y * 8 + threadIdx.y) * R;
   typename MaxBits<C>::type m = 0;
@@ -1259,23 +1289,23 @@ cudaError_t launch_step(const StepParams<T, C>& p, bool planar, bool uniform, bo
   return cudaGetLastError();
 }
 
+// Rows per warp of the planar sweep, by the rows each resident warp has to do (U).  Short runs
+// spread a small grid over the SMs and even out the end of the launch; long ones form the row
+// above a run's first less often.  With CPML 16 and TF/SF, us a step at 2, 4, 6, 8 rows: 1024^2
+// (U 5.4) 20.0, 20.6, 22.6, 24.6; 2048^2 (21.6) 43.2, 41.1, 41.3, 42.6; 4096^2 (86) 127.2, 113.6,
+// 111.6, 112.8.
+static int sweep_rows(long long cols, int Nx) {
+  const double U = (double)cols * Nx / (152.0 * 8 * kSweepMinBlocks);
+  return U < 8 ? 2 : (U < 60 ? 4 : 6);
+}
+
 template <class T, class C>
 cudaError_t launch_step_sweep2(const StepParams<T, C>& p, bool uniform, cudaStream_t s) {
-  // rows per warp: 16 where that still gives every SM 32 warps, fewer on small grids
   const long long cols = (p.Nz + 31) / 32;
-  int R = 16;
-  while (R > 2 && cols * ((p.Nx + R - 1) / R) < 152LL * 32) R /= 2;
+  const int R = sweep_rows(cols, p.Nx);
   const dim3 block(32, 8), grid((unsigned)cols, (unsigned)((p.Nx + 8 * R - 1) / (8 * R)));
-  switch (R * 2 + (uniform ? 1 : 0)) {
-    case 32: step_kernel_2d<T, C, false, 16><<<grid, block, 0, s>>>(p); break;
-    case 33: step_kernel_2d<T, C, true, 16><<<grid, block, 0, s>>>(p); break;
-    case 16: step_kernel_2d<T, C, false, 8><<<grid, block, 0, s>>>(p); break;
-    case 17: step_kernel_2d<T, C, true, 8><<<grid, block, 0, s>>>(p); break;
-    case 8: step_kernel_2d<T, C, false, 4><<<grid, block, 0, s>>>(p); break;
-    case 9: step_kernel_2d<T, C, true, 4><<<grid, block, 0, s>>>(p); break;
-    case 4: step_kernel_2d<T, C, false, 2><<<grid, block, 0, s>>>(p); break;
-    default: step_kernel_2d<T, C, true, 2><<<grid, block, 0, s>>>(p); break;
-  }
+  if (uniform) step_kernel_2d<T, C, true><<<grid, block, 0, s>>>(p, R);
+  else step_kernel_2d<T, C, false><<<grid, block, 0, s>>>(p, R);
   return cudaGetLastError();
 }
 
