@@ -36,6 +36,44 @@ __device__ __forceinline__ float fmaC(float a, float b, float c) { return fmaf(a
 __device__ __forceinline__ double mulC(double a, double b) { return __dmul_rn(a, b); }
 __device__ __forceinline__ float mulC(float a, float b) { return __fmul_rn(a, b); }
 
+// Differences and products of the update arithmetic.  On this GPU an FP64 add or multiply, or an
+// FMA with an operand from the constant bank or an immediate, holds an SM's FP64 pipe 18.6 cycles
+// a warp, an FMA with three register operands 15.7 (a loop of independent chains), and that pipe
+// bounds the FP64 kernels.  So their differences are fma(b, -1, a) and their products
+// fma(a, b, -0), the same bits as a - b and a * b for every input, signed zeros included, with
+// -1, -0 and the scalar coefficients in registers: 256^3 with CPML and TF/SF 917 -> 814 us a
+// step, 4096^2 planar 278 -> 249.  The compiler would turn an FMA with a known 1 or 0 back into
+// an add or a multiply and read a kernel parameter from the constant bank, so the values are tied
+// to a cell index: u >> 31 is 0 for u >= 0 (in asm, since a block's interior test tells the
+// compiler as much).
+template <class C>
+struct Fp {
+  __device__ __forceinline__ explicit Fp(int) {}
+  __device__ __forceinline__ C sub(C a, C b) const { return a - b; }
+  __device__ __forceinline__ C mul(C a, C b) const { return mulC(a, b); }
+  __device__ __forceinline__ C reg(C a) const { return a; }
+  __device__ __forceinline__ C neg(C a) const { return -a; }
+};
+template <>
+struct Fp<double> {
+  int z;
+  double m1, m0;
+  __device__ __forceinline__ explicit Fp(int u) {
+    asm("shr.s32 %0, %1, 31;" : "=r"(z) : "r"(u));
+    m1 = reg(-1.0);
+    m0 = reg(-0.0);
+  }
+  __device__ __forceinline__ double sub(double a, double b) const { return fma(b, m1, a); }
+  __device__ __forceinline__ double mul(double a, double b) const { return fma(a, b, m0); }
+  __device__ __forceinline__ double reg(double a) const {
+    return __hiloint2double(__double2hiint(a) | z, __double2loint(a));
+  }
+  // a sign flip of a kernel parameter by the compiler is an FP64 add
+  __device__ __forceinline__ double neg(double a) const {
+    return __hiloint2double((__double2hiint(a) ^ 0x80000000) | z, __double2loint(a));
+  }
+};
+
 // ------------------------------------------------------------------ TF/SF
 
 // Adds the increments of the planes of `ps` that cell (i,j,k) lies on to d (reference:
@@ -60,8 +98,8 @@ __device__ __forceinline__ void tfsf_apply(const PatchSet& ps, const C* tab, int
 
 // psi = b*psi + c*curl; returns curl/kappa + psi (reference: three_dim_pml.cc:186-188).
 template <class C>
-__device__ __forceinline__ C pml_term(C d, C* psi, C b, C cc, C rk) {
-  C ps = fmaC(b, *psi, cc * d);
+__device__ __forceinline__ C pml_term(const Fp<C>& fp, C d, C* psi, C b, C cc, C rk) {
+  C ps = fmaC(b, *psi, fp.mul(cc, d));
   *psi = ps;
   return fmaC(d, rk, ps);
 }

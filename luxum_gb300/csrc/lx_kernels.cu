@@ -12,7 +12,8 @@
 // cell lies on a total-field-box plane (one table load), runs the psi recursion only when
 // the cell lies in a CPML slab, and writes the updated component.  Cells outside the slabs
 // and off the planes do 4 FP64 operations per component (3 differences + 1 FMA), which is
-// the bound on GB300, whose FP64 pipe (~0.6 T lane-ops/s) limits before HBM does.
+// the bound on GB300, whose FP64 pipe (~0.6 T lane-ops/s) limits before HBM does; they are all
+// FMAs with three register operands, the pipe's fastest instruction (Fp in lx_device.cuh).
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
@@ -194,41 +195,43 @@ __device__ __forceinline__ void h_apply(const StepParams<T, C>& p, const int i, 
     sz = slab_index(p.slab[2], k);
   }
   C nhx = hx, nhy = hy, nhz = hz;
+  const Fp<C> fp(k);
+  const C mdb = fp.neg(p.Dbs);
   // Hx: i < Nx, j < Ny-1, k < Nz-1; part 1 = dEz/dy (y profile), part 2 = dEy/dz (z profile)
   if (ux) {
-    C d1 = ez_j - ez, d2 = ey_k - ey;
-    if (!UNI) { d1 = mulC(d1, p.rd[1]); d2 = mulC(d2, p.rd[2]); }
+    C d1 = fp.sub(ez_j, ez), d2 = fp.sub(ey_k, ey);
+    if (!UNI) { d1 = fp.mul(d1, fp.reg(p.rd[1])); d2 = fp.mul(d2, fp.reg(p.rd[2])); }
     if (tf) {
       tfsf_apply<C>(p.setsH[0][0], p.tab, i, j, k, d1);
       tfsf_apply<C>(p.setsH[0][1], p.tab, i, j, k, d2);
     }
-    if (sy >= 0) d1 = pml_term<C>(d1, p.psiH[0][0] + psi_index(1, p.slab[1], sy, i, j, k, p.Ny, p.Nzp), p.bH[1][j], p.cH[1][j], p.rkH[1][j]);
-    if (sz >= 0) d2 = pml_term<C>(d2, p.psiH[0][1] + psi_index(2, p.slab[2], sz, i, j, k, p.Ny, p.Nzp), p.bH[2][k], p.cH[2][k], p.rkH[2][k]);
-    nhx = fmaC(-p.Dbs, d1 - d2, hx);
+    if (sy >= 0) d1 = pml_term<C>(fp, d1, p.psiH[0][0] + psi_index(1, p.slab[1], sy, i, j, k, p.Ny, p.Nzp), p.bH[1][j], p.cH[1][j], p.rkH[1][j]);
+    if (sz >= 0) d2 = pml_term<C>(fp, d2, p.psiH[0][1] + psi_index(2, p.slab[2], sz, i, j, k, p.Ny, p.Nzp), p.bH[2][k], p.cH[2][k], p.rkH[2][k]);
+    nhx = fmaC(mdb, fp.sub(d1, d2), hx);
   }
   // Hy: i < Nx-1, j < Ny, k < Nz-1; part 1 = dEx/dz (z), part 2 = dEz/dx (x)
   if (uy) {
-    C d1 = ex_k - ex, d2 = ez_i - ez;
-    if (!UNI) { d1 = mulC(d1, p.rd[2]); d2 = mulC(d2, p.rd[0]); }
+    C d1 = fp.sub(ex_k, ex), d2 = fp.sub(ez_i, ez);
+    if (!UNI) { d1 = fp.mul(d1, fp.reg(p.rd[2])); d2 = fp.mul(d2, fp.reg(p.rd[0])); }
     if (tf) {
       tfsf_apply<C>(p.setsH[1][0], p.tab, i, j, k, d1);
       tfsf_apply<C>(p.setsH[1][1], p.tab, i, j, k, d2);
     }
-    if (sz >= 0) d1 = pml_term<C>(d1, p.psiH[1][0] + psi_index(2, p.slab[2], sz, i, j, k, p.Ny, p.Nzp), p.bH[2][k], p.cH[2][k], p.rkH[2][k]);
-    if (sx >= 0) d2 = pml_term<C>(d2, p.psiH[1][1] + psi_index(0, p.slab[0], sx, i, j, k, p.Ny, p.Nzp), p.bH[0][i], p.cH[0][i], p.rkH[0][i]);
-    nhy = fmaC(-p.Dbs, d1 - d2, hy);
+    if (sz >= 0) d1 = pml_term<C>(fp, d1, p.psiH[1][0] + psi_index(2, p.slab[2], sz, i, j, k, p.Ny, p.Nzp), p.bH[2][k], p.cH[2][k], p.rkH[2][k]);
+    if (sx >= 0) d2 = pml_term<C>(fp, d2, p.psiH[1][1] + psi_index(0, p.slab[0], sx, i, j, k, p.Ny, p.Nzp), p.bH[0][i], p.cH[0][i], p.rkH[0][i]);
+    nhy = fmaC(mdb, fp.sub(d1, d2), hy);
   }
   // Hz: i < Nx-1, j < Ny-1, k < Nz; part 1 = dEy/dx (x), part 2 = dEx/dy (y)
   if (uz) {
-    C d1 = ey_i - ey, d2 = ex_j - ex;
-    if (!UNI) { d1 = mulC(d1, p.rd[0]); d2 = mulC(d2, p.rd[1]); }
+    C d1 = fp.sub(ey_i, ey), d2 = fp.sub(ex_j, ex);
+    if (!UNI) { d1 = fp.mul(d1, fp.reg(p.rd[0])); d2 = fp.mul(d2, fp.reg(p.rd[1])); }
     if (tf) {
       tfsf_apply<C>(p.setsH[2][0], p.tab, i, j, k, d1);
       tfsf_apply<C>(p.setsH[2][1], p.tab, i, j, k, d2);
     }
-    if (sx >= 0) d1 = pml_term<C>(d1, p.psiH[2][0] + psi_index(0, p.slab[0], sx, i, j, k, p.Ny, p.Nzp), p.bH[0][i], p.cH[0][i], p.rkH[0][i]);
-    if (sy >= 0) d2 = pml_term<C>(d2, p.psiH[2][1] + psi_index(1, p.slab[1], sy, i, j, k, p.Ny, p.Nzp), p.bH[1][j], p.cH[1][j], p.rkH[1][j]);
-    nhz = fmaC(-p.Dbs, d1 - d2, hz);
+    if (sx >= 0) d1 = pml_term<C>(fp, d1, p.psiH[2][0] + psi_index(0, p.slab[0], sx, i, j, k, p.Ny, p.Nzp), p.bH[0][i], p.cH[0][i], p.rkH[0][i]);
+    if (sy >= 0) d2 = pml_term<C>(fp, d2, p.psiH[2][1] + psi_index(1, p.slab[1], sy, i, j, k, p.Ny, p.Nzp), p.bH[1][j], p.cH[1][j], p.rkH[1][j]);
+    nhz = fmaC(mdb, fp.sub(d1, d2), hz);
   }
   if (ux) st<T, C>(p.H[0] + c, nhx);
   if (uy) st<T, C>(p.H[1] + c, nhy);
@@ -371,41 +374,42 @@ __device__ __forceinline__ typename MaxBits<C>::type e_apply(const StepParams<T,
     sz = slab_index(p.slab[2], k);
   }
   C exn = ex, eyn = ey, ezn = ez;
+  const Fp<C> fp(k);
   // Ex: i < Nx-1, j in [1,Ny-2], k in [1,Nz-2]; part 1 = dHz/dy (y), part 2 = dHy/dz (z)
   if (ux) {
-    C d1 = hz - hz_j, d2 = hy - hy_k;
-    if (!UNI) { d1 = mulC(d1, p.rd[1]); d2 = mulC(d2, p.rd[2]); }
+    C d1 = fp.sub(hz, hz_j), d2 = fp.sub(hy, hy_k);
+    if (!UNI) { d1 = fp.mul(d1, fp.reg(p.rd[1])); d2 = fp.mul(d2, fp.reg(p.rd[2])); }
     if (tf) {
       tfsf_apply<C>(p.setsE[0][0], p.tab, i, j, k, d1);
       tfsf_apply<C>(p.setsE[0][1], p.tab, i, j, k, d2);
     }
-    if (sy >= 0) d1 = pml_term<C>(d1, p.psiE[0][0] + psi_index(1, p.slab[1], sy, i, j, k, p.Ny, p.Nzp), p.bE[1][j], p.cE[1][j], p.rkE[1][j]);
-    if (sz >= 0) d2 = pml_term<C>(d2, p.psiE[0][1] + psi_index(2, p.slab[2], sz, i, j, k, p.Ny, p.Nzp), p.bE[2][k], p.cE[2][k], p.rkE[2][k]);
-    exn = fmaC(cbx, d1 - d2, ex);
+    if (sy >= 0) d1 = pml_term<C>(fp, d1, p.psiE[0][0] + psi_index(1, p.slab[1], sy, i, j, k, p.Ny, p.Nzp), p.bE[1][j], p.cE[1][j], p.rkE[1][j]);
+    if (sz >= 0) d2 = pml_term<C>(fp, d2, p.psiE[0][1] + psi_index(2, p.slab[2], sz, i, j, k, p.Ny, p.Nzp), p.bE[2][k], p.cE[2][k], p.rkE[2][k]);
+    exn = fmaC(cbx, fp.sub(d1, d2), ex);
   }
   // Ey: i in [1,Nx-2], j < Ny-1, k in [1,Nz-2]; part 1 = dHx/dz (z), part 2 = dHz/dx (x)
   if (uy) {
-    C d1 = hx - hx_k, d2 = hz - hz_i;
-    if (!UNI) { d1 = mulC(d1, p.rd[2]); d2 = mulC(d2, p.rd[0]); }
+    C d1 = fp.sub(hx, hx_k), d2 = fp.sub(hz, hz_i);
+    if (!UNI) { d1 = fp.mul(d1, fp.reg(p.rd[2])); d2 = fp.mul(d2, fp.reg(p.rd[0])); }
     if (tf) {
       tfsf_apply<C>(p.setsE[1][0], p.tab, i, j, k, d1);
       tfsf_apply<C>(p.setsE[1][1], p.tab, i, j, k, d2);
     }
-    if (sz >= 0) d1 = pml_term<C>(d1, p.psiE[1][0] + psi_index(2, p.slab[2], sz, i, j, k, p.Ny, p.Nzp), p.bE[2][k], p.cE[2][k], p.rkE[2][k]);
-    if (sx >= 0) d2 = pml_term<C>(d2, p.psiE[1][1] + psi_index(0, p.slab[0], sx, i, j, k, p.Ny, p.Nzp), p.bE[0][i], p.cE[0][i], p.rkE[0][i]);
-    eyn = fmaC(cby, d1 - d2, ey);
+    if (sz >= 0) d1 = pml_term<C>(fp, d1, p.psiE[1][0] + psi_index(2, p.slab[2], sz, i, j, k, p.Ny, p.Nzp), p.bE[2][k], p.cE[2][k], p.rkE[2][k]);
+    if (sx >= 0) d2 = pml_term<C>(fp, d2, p.psiE[1][1] + psi_index(0, p.slab[0], sx, i, j, k, p.Ny, p.Nzp), p.bE[0][i], p.cE[0][i], p.rkE[0][i]);
+    eyn = fmaC(cby, fp.sub(d1, d2), ey);
   }
   // Ez: i in [1,Nx-2], j in [1,Ny-2], k < Nz-1; part 1 = dHy/dx (x), part 2 = dHx/dy (y)
   if (uz) {
-    C d1 = hy - hy_i, d2 = hx - hx_j;
-    if (!UNI) { d1 = mulC(d1, p.rd[0]); d2 = mulC(d2, p.rd[1]); }
+    C d1 = fp.sub(hy, hy_i), d2 = fp.sub(hx, hx_j);
+    if (!UNI) { d1 = fp.mul(d1, fp.reg(p.rd[0])); d2 = fp.mul(d2, fp.reg(p.rd[1])); }
     if (tf) {
       tfsf_apply<C>(p.setsE[2][0], p.tab, i, j, k, d1);
       tfsf_apply<C>(p.setsE[2][1], p.tab, i, j, k, d2);
     }
-    if (sx >= 0) d1 = pml_term<C>(d1, p.psiE[2][0] + psi_index(0, p.slab[0], sx, i, j, k, p.Ny, p.Nzp), p.bE[0][i], p.cE[0][i], p.rkE[0][i]);
-    if (sy >= 0) d2 = pml_term<C>(d2, p.psiE[2][1] + psi_index(1, p.slab[1], sy, i, j, k, p.Ny, p.Nzp), p.bE[1][j], p.cE[1][j], p.rkE[1][j]);
-    ezn = fmaC(cbz, d1 - d2, ez);
+    if (sx >= 0) d1 = pml_term<C>(fp, d1, p.psiE[2][0] + psi_index(0, p.slab[0], sx, i, j, k, p.Ny, p.Nzp), p.bE[0][i], p.cE[0][i], p.rkE[0][i]);
+    if (sy >= 0) d2 = pml_term<C>(fp, d2, p.psiE[2][1] + psi_index(1, p.slab[1], sy, i, j, k, p.Ny, p.Nzp), p.bE[1][j], p.cE[1][j], p.rkE[1][j]);
+    ezn = fmaC(cbz, fp.sub(d1, d2), ez);
   }
   if (ux) st<T, C>(p.E[0] + c, exn);
   if (uy) st<T, C>(p.E[1] + c, eyn);
@@ -413,7 +417,7 @@ __device__ __forceinline__ typename MaxBits<C>::type e_apply(const StepParams<T,
   typename MaxBits<C>::type mbits = 0;
   if (mon) {
     // Etotal = Ez*Ez + Ey*Ey + Ex*Ex (three_dim_pml.cc:270), same association order
-    const C e2 = fmaC(exn, exn, fmaC(eyn, eyn, ezn * ezn));
+    const C e2 = fmaC(exn, exn, fmaC(eyn, eyn, fp.mul(ezn, ezn)));
     if (p.etotal) p.etotal[c] = e2;
     mbits = MaxBits<C>::of(e2);
   }
@@ -431,10 +435,11 @@ __device__ __forceinline__ typename MaxBits<C>::type e_cell_3d(const StepParams<
 // Resident blocks per SM asked of the compiler for the 3-D E kernel: FP16 storage takes 8 (32
 // registers, about 30 bytes spilled) together with the interior fast path, 0.3196 -> 0.3116 ms
 // per 256^3 step (each alone was slower: the fast path 0.332, the cap 0.356); FP32 storage runs
-// best at the compiler's own 40 (the cap cost it 4 %), and FP64 is bound by its pipe.
+// best at the compiler's own 40 (the cap cost it 4 %), and FP64 with its FMA forms at 6 blocks
+// (256^3 with CPML and TF/SF 0.431 -> 0.415 ms against the compiler's own 60 registers).
 template <class T>
 struct EMinBlocks {
-  static constexpr int v = sizeof(T) == 2 ? 8 : 0;
+  static constexpr int v = sizeof(T) == 2 ? 8 : (sizeof(T) == 8 ? 6 : 0);
 };
 
 template <class T, class C, bool UNI, bool MON, int ZW>
@@ -446,12 +451,9 @@ __global__ void __launch_bounds__(256, EMinBlocks<T>::v) e_kernel_3d(const StepP
   const int i = blockIdx.z;
   const bool tf = p.tfsf && ztile_meets_planes(p.planesE, i, blockIdx.y * RY, RY, z);
   typename MaxBits<C>::type mbits = 0;
-  // The interior fast path pays for float compute (FP16 storage with the register cap above);
-  // FP64 is bound by its pipe either way.
-  constexpr bool kFast = sizeof(T) < 8;
   if (z.valid && j < p.Ny) {
-    if (kFast && !tf && z.n1 == 0 && tile_is_interior(p.slab, p.pml, p.Nx, p.Ny, p.Nz, i, 1, blockIdx.y * RY, RY, z.lo0, z.n0))
-      mbits = e_cell_3d<T, C, UNI, MON, kFast>(p, i, j, k, false);
+    if (!tf && z.n1 == 0 && tile_is_interior(p.slab, p.pml, p.Nx, p.Ny, p.Nz, i, 1, blockIdx.y * RY, RY, z.lo0, z.n0))
+      mbits = e_cell_3d<T, C, UNI, MON, true>(p, i, j, k, false);
     else
       mbits = e_cell_3d<T, C, UNI, MON>(p, i, j, k, tf);
   }
@@ -491,27 +493,29 @@ __device__ __forceinline__ void h2_apply(const StepParams<T, C>& p, const int i,
   if (FAST) tf = false;
   const C ey = v.ey, ey_k = v.ey_k, ey_i = v.ey_i, hx = v.hx, hz = v.hz;
   C nhx = hx, nhz = hz;
+  const Fp<C> fp(k);
+  const C db = fp.reg(p.Dbs);
   // Hx: k < Nz-1; Hx -= Db*(-curl2/kappa - psi2), curl2 = dEy/dz (z profile)
   if (ux) {
-    C d2 = ey_k - ey;
-    if (!UNI) d2 = mulC(d2, p.rd[2]);
+    C d2 = fp.sub(ey_k, ey);
+    if (!UNI) d2 = fp.mul(d2, fp.reg(p.rd[2]));
     if (tf) tfsf_apply<C>(p.setsH[0][1], p.tab, i, 0, k, d2);
     if (!FAST && p.pml) {
       const int sz = slab_index(p.slab[2], k);
-      if (sz >= 0) d2 = pml_term<C>(d2, p.psiH[0][1] + (long long)i * p.slab[2].n + sz, p.bH[2][k], p.cH[2][k], p.rkH[2][k]);
+      if (sz >= 0) d2 = pml_term<C>(fp, d2, p.psiH[0][1] + (long long)i * p.slab[2].n + sz, p.bH[2][k], p.cH[2][k], p.rkH[2][k]);
     }
-    nhx = fmaC(p.Dbs, d2, hx);
+    nhx = fmaC(db, d2, hx);
   }
   // Hz: i < Nx-1; Hz -= Db*(curl1/kappa + psi1), curl1 = dEy/dx (x profile)
   if (uz) {
-    C d1 = ey_i - ey;
-    if (!UNI) d1 = mulC(d1, p.rd[0]);
+    C d1 = fp.sub(ey_i, ey);
+    if (!UNI) d1 = fp.mul(d1, fp.reg(p.rd[0]));
     if (tf) tfsf_apply<C>(p.setsH[2][0], p.tab, i, 0, k, d1);
     if (!FAST && p.pml) {
       const int sx = slab_index(p.slab[0], i);
-      if (sx >= 0) d1 = pml_term<C>(d1, p.psiH[2][0] + (long long)sx * p.Nzp + k, p.bH[0][i], p.cH[0][i], p.rkH[0][i]);
+      if (sx >= 0) d1 = pml_term<C>(fp, d1, p.psiH[2][0] + (long long)sx * p.Nzp + k, p.bH[0][i], p.cH[0][i], p.rkH[0][i]);
     }
-    nhz = fmaC(-p.Dbs, d1, hz);
+    nhz = fmaC(fp.neg(p.Dbs), d1, hz);
   }
   if (ux) st<T, C>(p.H[0] + c, nhx);
   if (uz) st<T, C>(p.H[2] + c, nhz);
@@ -567,25 +571,26 @@ __device__ __forceinline__ typename MaxBits<C>::type e2_apply(const StepParams<T
   const long long c = v.c;
   const C ey = v.ey;
   C eyn = ey;
+  const Fp<C> fp(k);
   if (FAST) tf = false;
   if (FAST || v.u) {
-    C d1 = v.hx - v.hx_k;  // dHx/dz (z profile)
-    C d2 = v.hz - v.hz_i;  // dHz/dx (x profile)
-    if (!UNI) { d1 = mulC(d1, p.rd[2]); d2 = mulC(d2, p.rd[0]); }
+    C d1 = fp.sub(v.hx, v.hx_k);  // dHx/dz (z profile)
+    C d2 = fp.sub(v.hz, v.hz_i);  // dHz/dx (x profile)
+    if (!UNI) { d1 = fp.mul(d1, fp.reg(p.rd[2])); d2 = fp.mul(d2, fp.reg(p.rd[0])); }
     if (tf) {
       tfsf_apply<C>(p.setsE[1][0], p.tab, i, 0, k, d1);
       tfsf_apply<C>(p.setsE[1][1], p.tab, i, 0, k, d2);
     }
     if (!FAST && p.pml) {
       const int sz = slab_index(p.slab[2], k), sx = slab_index(p.slab[0], i);
-      if (sz >= 0) d1 = pml_term<C>(d1, p.psiE[1][0] + (long long)i * p.slab[2].n + sz, p.bE[2][k], p.cE[2][k], p.rkE[2][k]);
-      if (sx >= 0) d2 = pml_term<C>(d2, p.psiE[1][1] + (long long)sx * p.Nzp + k, p.bE[0][i], p.cE[0][i], p.rkE[0][i]);
+      if (sz >= 0) d1 = pml_term<C>(fp, d1, p.psiE[1][0] + (long long)i * p.slab[2].n + sz, p.bE[2][k], p.cE[2][k], p.rkE[2][k]);
+      if (sx >= 0) d2 = pml_term<C>(fp, d2, p.psiE[1][1] + (long long)sx * p.Nzp + k, p.bE[0][i], p.cE[0][i], p.rkE[0][i]);
     }
-    eyn = fmaC(v.cb, d1 - d2, ey);
+    eyn = fmaC(v.cb, fp.sub(d1, d2), ey);
     st<T, C>(p.E[1] + c, eyn);
   }
   // local_max = max(Ey*Ey) over the whole Ey array (two_dim_pml.cc:181)
-  return MON ? MaxBits<C>::of(eyn * eyn) : typename MaxBits<C>::type(0);
+  return MON ? MaxBits<C>::of(fp.mul(eyn, eyn)) : typename MaxBits<C>::type(0);
 }
 
 template <class T, class C, bool UNI, bool MON, bool FAST = false>
