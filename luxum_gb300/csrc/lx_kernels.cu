@@ -246,6 +246,89 @@ __device__ __forceinline__ void h_cell_3d(const StepParams<T, C>& p, const int i
   h_apply<T, C, UNI, FAST>(p, i, j, k, tf, v);
 }
 
+// The two psi terms of a cell in the slab of one axis AX: both half steps form the derivative
+// along AX in part 1 of component AX+1 and part 0 of component AX+2, with one profile and one
+// index for both.  Loaded with the cell's fields, ahead of every store (see h_load).
+template <class C>
+struct AxisPsi {
+  bool on;
+  long long q;
+  C a, b;         // psi of component AX+1 part 1, AX+2 part 0
+  C pb, pc, prk;  // profile b, c, 1/kappa
+};
+
+template <class T, class C, int AX>
+__device__ __forceinline__ void axis_psi_load(const StepParams<T, C>& p, C* const (&psi)[3][2], const C* pb, const C* pc,
+                                              const C* prk, int i, int j, int k, bool ua, bool ub, AxisPsi<C>& w) {
+  const int u = AX == 0 ? i : (AX == 1 ? j : k);
+  const int s = slab_index(p.slab[AX], u);
+  w.on = s >= 0 && (ua || ub);
+  w.a = w.b = w.pb = w.pc = w.prk = C(0);
+  w.q = 0;
+  if (w.on) {
+    w.q = psi_index(AX, p.slab[AX], s, i, j, k, p.Ny, p.Nzp);
+    if (ua) w.a = psi[(AX + 1) % 3][1][w.q];
+    if (ub) w.b = psi[(AX + 2) % 3][0][w.q];
+    w.pb = __ldg(pb + u);
+    w.pc = __ldg(pc + u);
+    w.prk = __ldg(prk + u);
+  }
+}
+// pml_term's arithmetic on a loaded psi.
+template <class C>
+__device__ __forceinline__ void axis_psi_term(const AxisPsi<C>& w, C& psi, C& d) {
+  psi = fmaC(w.pb, psi, w.pc * d);
+  d = fmaC(d, w.prk, psi);
+}
+
+// H of a cell whose block meets the CPML slab of axis AX only and no TF/SF plane (AX = 3: no
+// slab, a block at the walls): h_apply's arithmetic with the two psi terms' loads issued with
+// the field loads.  In h_apply each psi term's load waits behind the previous term's store (the
+// arrays may alias as far as the compiler knows), one memory round trip per term, and such
+// blocks are a third of a 256^3 grid with 16-cell slabs and most of a 64^3 one.
+template <class T, class C, bool UNI, int AX>
+__device__ __forceinline__ void h_slab_3d(const StepParams<T, C>& p, const int i, const int j, const int k) {
+  HCell<C> v;
+  h_load<T, C>(p, i, j, k, v);
+  const bool u[3] = {v.ux, v.uy, v.uz};
+  AxisPsi<C> w;
+  if constexpr (AX < 3)
+    axis_psi_load<T, C, AX>(p, p.psiH, p.bH[AX], p.cH[AX], p.rkH[AX], i, j, k, u[(AX + 1) % 3], u[(AX + 2) % 3], w);
+  // d[c][part]: Hx: dEz/dy, dEy/dz; Hy: dEx/dz, dEz/dx; Hz: dEy/dx, dEx/dy
+  C d[3][2] = {{v.ez_j - v.ez, v.ey_k - v.ey}, {v.ex_k - v.ex, v.ez_i - v.ez}, {v.ey_i - v.ey, v.ex_j - v.ex}};
+  if (!UNI) {
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      d[c][0] = mulC(d[c][0], p.rd[(c + 1) % 3]);
+      d[c][1] = mulC(d[c][1], p.rd[(c + 2) % 3]);
+    }
+  }
+  if constexpr (AX < 3) {
+    constexpr int A = (AX + 1) % 3, B = (AX + 2) % 3;
+    if (w.on) {
+      if (u[A]) axis_psi_term(w, w.a, d[A][1]);
+      if (u[B]) axis_psi_term(w, w.b, d[B][0]);
+      if (u[A]) p.psiH[A][1][w.q] = w.a;
+      if (u[B]) p.psiH[B][0][w.q] = w.b;
+    }
+  }
+  if (u[0]) st<T, C>(p.H[0] + v.c, fmaC(-p.Dbs, d[0][0] - d[0][1], v.hx));
+  if (u[1]) st<T, C>(p.H[1] + v.c, fmaC(-p.Dbs, d[1][0] - d[1][1], v.hy));
+  if (u[2]) st<T, C>(p.H[2] + v.c, fmaC(-p.Dbs, d[2][0] - d[2][1], v.hz));
+}
+
+// The path of a block that is not interior: kGeneral when it meets a TF/SF plane or the slabs
+// of two axes, else the axis of the one slab it meets, or kNoSlab.
+constexpr int kNoSlab = 3, kGeneral = 4;
+__device__ __forceinline__ int slab_path(const Slab (&sl)[3], bool pml, bool tf, int i0, int ni, int j0, int nj, int k0,
+                                         int nk) {
+  if (tf) return kGeneral;
+  if (!pml) return kNoSlab;
+  const bool x = !axis_free(sl[0], i0, ni), y = !axis_free(sl[1], j0, nj), z = !axis_free(sl[2], k0, nk);
+  if (x + y + z > 1) return kGeneral;
+  return x ? 0 : (y ? 1 : (z ? 2 : kNoSlab));
+}
+
 // Resident blocks per SM asked of the compiler for the H kernel (a register cap): 8 for
 // float compute (32 registers, 12-16 bytes spilled; FP16 storage 14 % faster than at 40
 // registers), 5 for FP64 (its natural 48 registers; an explicit 1 lets the compiler take 54).
@@ -303,7 +386,7 @@ __device__ __forceinline__ bool ztile_meets_planes(const int (&pl)[3][2], int i,
 
 // One cell per thread; a block is ZW (z) x 256/ZW (y) cells of one x plane.  Blocks whose tile
 // is interior take the cell code with every condition decided at compile time.
-template <class T, class C, bool UNI, int ZW>
+template <class T, class C, bool UNI, bool SLAB, int ZW>
 __global__ void __launch_bounds__(256, HMinBlocks<C>::v) h_kernel_3d(const StepParams<T, C> p) {
   constexpr int RY = 256 / ZW;
   const ZTile z = z_tile<ZW>(p.Nz, p.zends);
@@ -314,8 +397,14 @@ __global__ void __launch_bounds__(256, HMinBlocks<C>::v) h_kernel_3d(const StepP
   const bool tf = p.tfsf && ztile_meets_planes(p.planesH, i, blockIdx.y * RY, RY, z);
   if (!tf && z.n1 == 0 && tile_is_interior(p.slab, p.pml, p.Nx, p.Ny, p.Nz, i, 1, blockIdx.y * RY, RY, z.lo0, z.n0))
     h_cell_3d<T, C, UNI, true>(p, i, j, k, false);
-  else
-    h_cell_3d<T, C, UNI>(p, i, j, k, tf);
+  else {
+    const int path = SLAB ? slab_path(p.slab, p.pml, tf, i, 1, blockIdx.y * RY, RY, z.lo0, z.n0) : kGeneral;
+    if (path == 0) h_slab_3d<T, C, UNI, 0>(p, i, j, k);
+    else if (path == 1) h_slab_3d<T, C, UNI, 1>(p, i, j, k);
+    else if (path == 2) h_slab_3d<T, C, UNI, 2>(p, i, j, k);
+    else if (path == kNoSlab) h_slab_3d<T, C, UNI, kNoSlab>(p, i, j, k);
+    else h_cell_3d<T, C, UNI>(p, i, j, k, tf);
+  }
 }
 
 // E half-step over cell (i,j,k) for Ex, Ey, Ez (three_dim_pml.cc:218-276, three_dim.cc:134-189).
@@ -432,17 +521,58 @@ __device__ __forceinline__ typename MaxBits<C>::type e_cell_3d(const StepParams<
   return e_apply<T, C, UNI, MON, FAST>(p, i, j, k, tf, v);
 }
 
+// E of a cell whose block meets the CPML slab of axis AX only and no TF/SF plane (see h_slab_3d):
+// e_apply's arithmetic.
+template <class T, class C, bool UNI, bool MON, int AX>
+__device__ __forceinline__ typename MaxBits<C>::type e_slab_3d(const StepParams<T, C>& p, const int i, const int j,
+                                                               const int k) {
+  ECell<C> v;
+  e_load<T, C, MON>(p, i, j, k, v);
+  const bool u[3] = {v.ux, v.uy, v.uz};
+  AxisPsi<C> w;
+  if constexpr (AX < 3)
+    axis_psi_load<T, C, AX>(p, p.psiE, p.bE[AX], p.cE[AX], p.rkE[AX], i, j, k, u[(AX + 1) % 3], u[(AX + 2) % 3], w);
+  // d[c][part]: Ex: dHz/dy, dHy/dz; Ey: dHx/dz, dHz/dx; Ez: dHy/dx, dHx/dy
+  C d[3][2] = {{v.hz - v.hz_j, v.hy - v.hy_k}, {v.hx - v.hx_k, v.hz - v.hz_i}, {v.hy - v.hy_i, v.hx - v.hx_j}};
+  if (!UNI) {
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      d[c][0] = mulC(d[c][0], p.rd[(c + 1) % 3]);
+      d[c][1] = mulC(d[c][1], p.rd[(c + 2) % 3]);
+    }
+  }
+  if constexpr (AX < 3) {
+    constexpr int A = (AX + 1) % 3, B = (AX + 2) % 3;
+    if (w.on) {
+      if (u[A]) axis_psi_term(w, w.a, d[A][1]);
+      if (u[B]) axis_psi_term(w, w.b, d[B][0]);
+      if (u[A]) p.psiE[A][1][w.q] = w.a;
+      if (u[B]) p.psiE[B][0][w.q] = w.b;
+    }
+  }
+  const C exn = u[0] ? fmaC(v.cbx, d[0][0] - d[0][1], v.ex) : v.ex;
+  const C eyn = u[1] ? fmaC(v.cby, d[1][0] - d[1][1], v.ey) : v.ey;
+  const C ezn = u[2] ? fmaC(v.cbz, d[2][0] - d[2][1], v.ez) : v.ez;
+  if (u[0]) st<T, C>(p.E[0] + v.c, exn);
+  if (u[1]) st<T, C>(p.E[1] + v.c, eyn);
+  if (u[2]) st<T, C>(p.E[2] + v.c, ezn);
+  if (!(MON && v.mon)) return 0;
+  const C e2 = fmaC(exn, exn, fmaC(eyn, eyn, ezn * ezn));
+  if (p.etotal) p.etotal[v.c] = e2;
+  return MaxBits<C>::of(e2);
+}
+
 // Resident blocks per SM asked of the compiler for the 3-D E kernel: FP16 storage takes 8 (32
 // registers, about 30 bytes spilled) together with the interior fast path, 0.3196 -> 0.3116 ms
 // per 256^3 step (each alone was slower: the fast path 0.332, the cap 0.356); FP32 storage runs
-// best at the compiler's own 40 (the cap cost it 4 %), and FP64 with its FMA forms at 6 blocks
-// (256^3 with CPML and TF/SF 0.431 -> 0.415 ms against the compiler's own 60 registers).
+// best at 40 (6 blocks; 8 cost it 4 %), and FP64 with its FMA forms at 6 blocks (256^3 with CPML
+// and TF/SF 0.431 -> 0.415 ms against the compiler's own 60 registers).
 template <class T>
 struct EMinBlocks {
-  static constexpr int v = sizeof(T) == 2 ? 8 : (sizeof(T) == 8 ? 6 : 0);
+  static constexpr int v = sizeof(T) == 2 ? 8 : 6;
 };
 
-template <class T, class C, bool UNI, bool MON, int ZW>
+template <class T, class C, bool UNI, bool MON, bool SLAB, int ZW>
 __global__ void __launch_bounds__(256, EMinBlocks<T>::v) e_kernel_3d(const StepParams<T, C> p) {
   constexpr int RY = 256 / ZW;
   const ZTile z = z_tile<ZW>(p.Nz, p.zends);
@@ -454,8 +584,14 @@ __global__ void __launch_bounds__(256, EMinBlocks<T>::v) e_kernel_3d(const StepP
   if (z.valid && j < p.Ny) {
     if (!tf && z.n1 == 0 && tile_is_interior(p.slab, p.pml, p.Nx, p.Ny, p.Nz, i, 1, blockIdx.y * RY, RY, z.lo0, z.n0))
       mbits = e_cell_3d<T, C, UNI, MON, true>(p, i, j, k, false);
-    else
-      mbits = e_cell_3d<T, C, UNI, MON>(p, i, j, k, tf);
+    else {
+      const int path = SLAB ? slab_path(p.slab, p.pml, tf, i, 1, blockIdx.y * RY, RY, z.lo0, z.n0) : kGeneral;
+      if (path == 0) mbits = e_slab_3d<T, C, UNI, MON, 0>(p, i, j, k);
+      else if (path == 1) mbits = e_slab_3d<T, C, UNI, MON, 1>(p, i, j, k);
+      else if (path == 2) mbits = e_slab_3d<T, C, UNI, MON, 2>(p, i, j, k);
+      else if (path == kNoSlab) mbits = e_slab_3d<T, C, UNI, MON, kNoSlab>(p, i, j, k);
+      else mbits = e_cell_3d<T, C, UNI, MON>(p, i, j, k, tf);
+    }
   }
   if (MON && p.max_slot) block_max_atomic(mbits, p.max_slot);
 }
@@ -1242,6 +1378,22 @@ static bool z16_tiles() {
   return on;
 }
 
+template <class T, class C, bool UNI, bool SLAB>
+static void launch_step_3d(const StepParams<T, C>& q, bool mon, bool h_half, cudaStream_t s) {
+  if constexpr (sizeof(T) < 8) {
+    if (!h_half && z16_tiles()) {
+      const dim3 block(16, 16), grid((q.Nz + 15) / 16, (q.Ny + 15) / 16, q.Nx);
+      if (mon) e_kernel_3d<T, C, UNI, true, SLAB, 16><<<grid, block, 0, s>>>(q);
+      else e_kernel_3d<T, C, UNI, false, SLAB, 16><<<grid, block, 0, s>>>(q);
+      return;
+    }
+  }
+  const dim3 block(32, 8), grid(q.zends ? 1 + (q.Nz - 32 + 31) / 32 : (q.Nz + 31) / 32, (q.Ny + 7) / 8, q.Nx);
+  if (h_half) h_kernel_3d<T, C, UNI, SLAB, 32><<<grid, block, 0, s>>>(q);
+  else if (mon) e_kernel_3d<T, C, UNI, true, SLAB, 32><<<grid, block, 0, s>>>(q);
+  else e_kernel_3d<T, C, UNI, false, SLAB, 32><<<grid, block, 0, s>>>(q);
+}
+
 template <class T, class C>
 cudaError_t launch_step(const StepParams<T, C>& p, bool planar, bool uniform, bool h_half, cudaStream_t s) {
   // single simulations: one cell per thread (their parameters sit in the constant bank, and
@@ -1268,28 +1420,20 @@ cudaError_t launch_step(const StepParams<T, C>& p, bool planar, bool uniform, bo
     StepParams<T, C> q = p;
     q.zends = sizeof(T) == 8 && p.pml && p.slab[2].n > 0 && p.slab[2].lo <= 16 && p.Nz - p.slab[2].hi0 <= 16 &&
               p.Nz >= 48;
-    if (sizeof(T) < 8 && !h_half && z16_tiles()) {
-      const dim3 block16(16, 16), grid16((p.Nz + 15) / 16, (p.Ny + 15) / 16, p.Nx);
-      if (mon) {
-        if (uniform) e_kernel_3d<T, C, true, true, 16><<<grid16, block16, 0, s>>>(q);
-        else e_kernel_3d<T, C, false, true, 16><<<grid16, block16, 0, s>>>(q);
-      } else {
-        if (uniform) e_kernel_3d<T, C, true, false, 16><<<grid16, block16, 0, s>>>(q);
-        else e_kernel_3d<T, C, false, false, 16><<<grid16, block16, 0, s>>>(q);
+    // Float grids of 2^22 cells or more give blocks in the slab of one axis their own path
+    // (h_slab_3d): us a step with and without it, 512x512x128 (CPML 20) 602 and 654, 256^3
+    // (CPML 16, TF/SF) 308 and 324, 128^3 57.0 and 57.5, 100^3 (CPML 12) 41.0 and 39.4 (the
+    // longer code costs a short launch more than the path saves).  FP64 is bound by its pipe.
+    bool slab = false;
+    if constexpr (sizeof(C) == 4) slab = p.pml && (long long)p.Nx * p.Ny * p.Nz >= (1LL << 22);
+    if constexpr (sizeof(C) == 4)
+      if (slab) {
+        if (uniform) launch_step_3d<T, C, true, true>(q, mon, h_half, s);
+        else launch_step_3d<T, C, false, true>(q, mon, h_half, s);
+        return cudaGetLastError();
       }
-      return cudaGetLastError();
-    }
-    dim3 grid(q.zends ? 1 + (p.Nz - 32 + 31) / 32 : (p.Nz + 31) / 32, (p.Ny + 7) / 8, p.Nx);
-    if (h_half) {
-      if (uniform) h_kernel_3d<T, C, true, 32><<<grid, block, 0, s>>>(q);
-      else h_kernel_3d<T, C, false, 32><<<grid, block, 0, s>>>(q);
-    } else if (mon) {
-      if (uniform) e_kernel_3d<T, C, true, true, 32><<<grid, block, 0, s>>>(q);
-      else e_kernel_3d<T, C, false, true, 32><<<grid, block, 0, s>>>(q);
-    } else {
-      if (uniform) e_kernel_3d<T, C, true, false, 32><<<grid, block, 0, s>>>(q);
-      else e_kernel_3d<T, C, false, false, 32><<<grid, block, 0, s>>>(q);
-    }
+    if (uniform) launch_step_3d<T, C, true, false>(q, mon, h_half, s);
+    else launch_step_3d<T, C, false, false>(q, mon, h_half, s);
   }
   return cudaGetLastError();
 }
