@@ -396,6 +396,14 @@ static size_t ext_n(const lx_sim* s, int c) { return (size_t)s->ext[c][0] * s->e
 
 static void stop_writer(lx_sim* s);
 
+// Drops the handle's captured step sequence: something its launches were given changed.
+static void drop_graph(lx_sim* s) {
+  if (s->graph) cudaGraphExecDestroy(s->graph);
+  s->graph = nullptr;
+  s->graph_steps = 0;
+  s->alone_steps = 0;
+}
+
 // Completes a batch chunk in flight that this handle is a member of, before the handle's
 // own state is read, written or stepped.  A blow-up is reported by the batch's own wait and
 // shows in this handle's max|E|^2; only CUDA errors are returned here.
@@ -415,6 +423,7 @@ extern "C" LX_API void lx_sim_destroy(lx_sim* s) {
   stop_writer(s);
   if (s->stream) cudaStreamSynchronize(s->stream);
   if (s->side) cudaStreamSynchronize(s->side);
+  drop_graph(s);
   cudaStream_t fs = s->own;
   for (int c = 0; c < 3; c++) {
     dfree(s->E[c], fs); dfree(s->H[c], fs); dfree(s->Cbs[c], fs);
@@ -423,7 +432,7 @@ extern "C" LX_API void lx_sim_destroy(lx_sim* s) {
     for (int q = 0; q < 2; q++) { dfree(s->psiH[c][q], fs); dfree(s->psiE[c][q], fs); }
     for (int q = 0; q < 2; q++) { dfree(s->psiH1[c][q], fs); dfree(s->psiE1[c][q], fs); }
   }
-  dfree(s->tab, fs); dfree(s->d_max, fs); dfree(s->d_series, fs); dfree(s->etotal, fs); dfree(s->xfer, fs);
+  dfree(s->tab, fs); dfree(s->tabs, fs); dfree(s->d_max, fs); dfree(s->d_series, fs); dfree(s->etotal, fs); dfree(s->xfer, fs);
   dfree(s->d_probe_ijk, fs); dfree(s->d_probe, fs);
   for (auto& sl : s->slots) {
     dfree(sl.dev, fs);
@@ -529,9 +538,14 @@ static lx_status create_typed(lx_sim* s) {
     build_sets(s);
     CK(cudaMallocAsync(&s->tab, (size_t)(s->tab_total > 0 ? s->tab_total : 1) * sizeof(C), s->own));
   }
-  CK(cudaMallocAsync(&s->d_max, 64, s->own));
-  CK(cudaMemsetAsync(s->d_max, 0, 64, s->own));
-  s->d_fault = reinterpret_cast<unsigned*>(s->d_max + 1);
+  const size_t words = 1 + 2 * lx::kAhead;
+  const size_t state = words * sizeof(unsigned long long) + sizeof(lx::StepCtl);
+  CK(cudaMallocAsync(&s->d_max, state, s->own));
+  CK(cudaMemsetAsync(s->d_max, 0, state, s->own));
+  s->d_fault = reinterpret_cast<unsigned*>(s->d_max);
+  s->d_ring = s->d_max + 1;
+  s->d_srcv = reinterpret_cast<double*>(s->d_ring + lx::kAhead);
+  s->d_ctl = reinterpret_cast<lx::StepCtl*>(s->d_srcv + lx::kAhead);
   return LX_OK;
 }
 
@@ -1122,6 +1136,7 @@ extern "C" LX_API lx_status lx_sim_set_probes(lx_sim* s, const int* ijk, int npr
     return fail(s, LX_ERR_STATE, "remove the handle from its batch first: batched members keep no snapshot outputs or probes");
   if (nprobes < 0 || nprobes > lx::kMaxProbes || cap < 0) return fail(s, LX_ERR_INVALID, "0..64 probes, capacity >= 0");
   CK(cudaStreamSynchronize(s->stream));
+  drop_graph(s);
   dfree(s->d_probe_ijk, s->own);
   dfree(s->d_probe, s->own);
   s->d_probe_ijk = nullptr;
@@ -1185,6 +1200,7 @@ extern "C" LX_API lx_status lx_sim_add_dft_plane(lx_sim* s, int axis, int index,
   CK(cudaStreamSynchronize(s->own));
   s->n_h2d += nfreq * sizeof(double);
   s->dfts.push_back(d);
+  drop_graph(s);
   *id = (int)s->dfts.size() - 1;
   if (s->batch) batch_member_changed(s->batch);  // the batch samples the new plane from its next step
   return LX_OK;
@@ -1528,15 +1544,57 @@ static lx::PrologueParams make_prologue(lx_sim* s) {
   return pp;
 }
 
+// The tables a handle stepped alone keeps ahead: as many steps as fit kAheadBytes, up to kAhead.
+static lx_status ensure_ahead(lx_sim* s) {
+  constexpr size_t kAheadBytes = 1 << 20;
+  if (s->ahead) return LX_OK;
+  const size_t tab = s->tfsf ? (size_t)s->tab_total * s->csize : 0;
+  int n = lx::kAhead;
+  if (tab) n = (int)std::max<size_t>(1, std::min<size_t>(n, kAheadBytes / tab));
+  if (tab && n > 1) CK(cudaMallocAsync(&s->tabs, tab * n, s->stream));
+  s->ahead = n;
+  return LX_OK;
+}
+
+// Steps per captured sequence, 0 when the handle's steps are launched one by one.  A sequence
+// holds whole periods of everything that does not happen at every step.
+static int sequence_steps(const lx_sim* s) {
+  // Replayed kernels follow each other in 0.55 us, launched ones in 2.05 (empty kernels): worth
+  // the capture (3.5 us a launch, once) where a step takes tens of microseconds.
+  const long long cells = (long long)s->Nx * s->Ny * s->Nz;
+  if (s->stream != s->own || s->batch || cells > (s->planar ? 1LL << 22 : 1LL << 21)) return 0;
+  auto lcm = [](int a, int b) {
+    int x = a, y = b;
+    while (y) { const int r = x % y; x = y; y = r; }
+    return a / x * b;
+  };
+  int L = s->pp ? 2 : 1;
+  for (auto& d : s->dfts) {
+    if (d.every > lx::kAhead) return 0;
+    L = lcm(L, d.every);
+    if (L > lx::kAhead) return 0;
+  }
+  if (s->p.monitor_every > 0) {
+    if (s->p.monitor_every > lx::kAhead) return 0;
+    L = lcm(L, s->p.monitor_every);
+  }
+  if (L > s->ahead) return 0;
+  return L * std::max(1, std::min(8, s->ahead) / L);
+}
+
 template <class T, class C>
 static lx_status run_steps(lx_sim* s, int nsteps, KernelTimer* kt = nullptr) {
   if (!s->batch) {  // stepped alone: single-sweep handles take the ping-pong kernel
     const lx_status st = set_pp(s, true);
     if (st) return st;
   }
+  lx_status st = ensure_ahead(s);
+  if (st) return st;
+  if (s->graph && s->graph_pp != s->pp) drop_graph(s);
   lx::StepParams<T, C> sp = step_params<T, C>(s);
   sp.fault = s->d_fault;
   lx::PrologueParams pp = make_prologue(s);
+  C* const tabs = (C*)(s->tabs ? s->tabs : s->tab);
   T* pf[6];  // the components after the current step (buffer (t+1) & 1 in ping-pong mode)
   auto post_step = [&](int t) {
     const bool b1 = s->pp && ((t + 1) & 1);
@@ -1548,6 +1606,7 @@ static lx_status run_steps(lx_sim* s, int nsteps, KernelTimer* kt = nullptr) {
   lx::ProbeParams prb;
   std::memset(&prb, 0, sizeof prb);
   prb.nprobes = s->nprobes;
+  prb.cap = s->probe_cap;
   prb.Ny = s->Ny;
   prb.Nzp = s->Nzp;
   for (int c = 0; c < 6; c++)
@@ -1555,44 +1614,48 @@ static lx_status run_steps(lx_sim* s, int nsteps, KernelTimer* kt = nullptr) {
   prb.ijk = s->d_probe_ijk;
   prb.hmul = 1.0 / s->hscale;
 
-  unsigned long long* last_slot = s->d_max;
-  for (int q = 0; q < nsteps; q++) {
-    const int t = s->t;
-    bool mon = (q == nsteps - 1) || (s->p.monitor_every > 0 && (t + 1) % s->p.monitor_every == 0);
+  auto tic = [&]() -> lx_status {
+    if (kt) CK(cudaEventRecord(kt->ev[0], s->stream));
+    return LX_OK;
+  };
+  auto toc = [&](int which) -> lx_status {
+    if (!kt) return LX_OK;
+    CK(cudaEventRecord(kt->ev[1], s->stream));
+    CK(cudaEventSynchronize(kt->ev[1]));
+    float ms = 0.f;
+    CK(cudaEventElapsedTime(&ms, kt->ev[0], kt->ev[1]));
+    kt->sum[which] += ms;
+    kt->cnt[which]++;
+    return LX_OK;
+  };
+  auto due = [&](int t) { return s->p.monitor_every > 0 && (t + 1) % s->p.monitor_every == 0; };
+  auto snapshots = [&](int t) {
     unsigned snap = 0;
     for (auto& o : s->outputs)
       if (o.every > 0 && t >= o.first && t % o.every == 0) snap |= o.mask;
-    auto tic = [&]() -> lx_status {
-      if (kt) CK(cudaEventRecord(kt->ev[0], s->stream));
-      return LX_OK;
-    };
-    auto toc = [&](int which) -> lx_status {
-      if (!kt) return LX_OK;
-      CK(cudaEventRecord(kt->ev[1], s->stream));
-      CK(cudaEventSynchronize(kt->ev[1]));
-      float ms = 0.f;
-      CK(cudaEventElapsedTime(&ms, kt->ev[0], kt->ev[1]));
-      kt->sum[which] += ms;
-      kt->cnt[which]++;
-      return LX_OK;
-    };
+    return snap;
+  };
+  // The launches that form a sequence's tables, amplitudes and cleared slots.
+  auto ahead = [&](int t, int n, bool any, const lx::StepCtl* ctl) -> lx_status {
+    if (!any) return LX_OK;
+    pp.t = t;
     lx_status st;
-    unsigned long long* slot = s->d_max;
-    if (mon && s->d_series && (int)s->series_t.size() < s->series_cap) {
-      slot = s->d_series + s->series_t.size();
-      s->series_t.push_back(t);
-    }
-    if (mon) last_slot = slot;
-    if (pp.tab_total > 0 || s->src_kind >= 0 || mon) {
-      pp.t = t;
-      pp.max_slot = mon ? slot : nullptr;
-      if ((st = tic())) return st;
-      if (s->csize == 8) CK(lx::launch_prologue<double>(pp, s->stream));
-      else CK(lx::launch_prologue<float>(pp, s->stream));
-      if ((st = toc(0))) return st;
+    if ((st = tic())) return st;
+    CK(lx::launch_prologue_ahead<C>(pp, n, ctl, tabs, s->d_srcv, s->d_ring, s->stream));
+    if ((st = toc(0))) return st;
+    s->n_kernels++;
+    return LX_OK;
+  };
+  // The launches of step t, the q-th of its sequence; ctl: as part of a captured sequence.
+  auto one_step = [&](int t, int q, bool mon, unsigned snap, const lx::StepCtl* ctl) -> lx_status {
+    lx_status st;
+    if (s->src_kind >= 0) {
+      T* f = (T*)(s->pp && (t & 1) ? pp.src_field1 : pp.src_field);  // the state step t reads
+      CK(lx::launch_source<T>(f, s->src_idx, s->src_kind, s->d_srcv + q, s->stream));
       s->n_kernels++;
     }
-    sp.max_slot = mon ? slot : nullptr;
+    sp.tab = tabs + (size_t)(s->tabs ? q : 0) * s->tab_total;
+    sp.max_slot = mon ? s->d_ring + q : nullptr;
     sp.etotal = (snap & (1u << LX_ETOTAL)) ? (C*)s->etotal : nullptr;
     bool swept = false;
     if constexpr (sizeof(C) == 4) {
@@ -1622,42 +1685,121 @@ static lx_status run_steps(lx_sim* s, int nsteps, KernelTimer* kt = nullptr) {
       lx::DftParams dp;
       std::memset(&dp, 0, sizeof dp);
       dp.axis = d.axis; dp.index = d.index; dp.na = d.na; dp.nb = d.nb; dp.Ny = s->Ny; dp.Nzp = s->Nzp;
-      dp.nfreq = d.nfreq; dp.t = t; dp.dt = s->k.dt; dp.weight = (double)d.every;
+      dp.nfreq = d.nfreq; dp.t = t; dp.ctl = ctl; dp.k = q; dp.dt = s->k.dt; dp.weight = (double)d.every;
       dp.omega = d.d_omega; dp.acc = d.d_acc; dp.phase = d.d_phase; dp.hmul = 1.0 / s->hscale;
       T* f4[4];
-      for (int q = 0; q < 4; q++) {
-        f4[q] = pf[d.comps[q]];
-        for (int a = 0; a < 3; a++) dp.ext[q][a] = s->ext[d.comps[q]][a];
+      for (int c = 0; c < 4; c++) {
+        f4[c] = pf[d.comps[c]];
+        for (int a = 0; a < 3; a++) dp.ext[c][a] = s->ext[d.comps[c]][a];
       }
       CK(lx::launch_dft<T>(dp, f4, s->stream));
       s->n_kernels += 2;  // phase factors, accumulation
     }
-    if (s->nprobes > 0 && s->probe_rows < s->probe_cap) {
-      prb.row = s->probe_rows++;
+    if (s->nprobes > 0 && (ctl || s->probe_rows < s->probe_cap)) {
+      prb.row = s->probe_rows;
+      prb.ctl = ctl;
+      prb.k = q;
+      if (!ctl) s->probe_rows++;
       if ((st = tic())) return st;
       CK(lx::launch_probes<T>(prb, pf, s->d_probe, s->stream));
       if ((st = toc(3))) return st;
       s->n_kernels++;
     }
-    s->t++;
-    if (snap) {
-      lx_status st = snapshot(s, t, snap);
-      if (st) return st;
+    return LX_OK;
+  };
+  // Host record of the series entries of steps t .. t+n-1 given by mask; returns the first index.
+  auto record = [&](int t, unsigned mask) {
+    const int at = (int)s->series_t.size();
+    for (int q = 0; q < lx::kAhead; q++)
+      if ((mask >> q) & 1u)
+        if (s->d_series && (int)s->series_t.size() < s->series_cap) s->series_t.push_back(t + q);
+    return at;
+  };
+
+  const int K = kt ? 0 : sequence_steps(s);
+  unsigned long long* last_slot = s->d_ring;
+  for (int done = 0; done < nsteps;) {
+    const int t = s->t, left = nsteps - done;
+    bool seq = K > 0 && left >= K && t % K == 0 && (s->graph || s->alone_steps + left >= 3 * K);
+    for (int q = 0; seq && q < K; q++) seq = !snapshots(t + q);
+    if (seq) {
+      unsigned mask = 0;
+      for (int q = 0; q < K; q++)
+        if (due(t + q)) mask |= 1u << q;
+      if (!s->graph) {
+        const uint64_t before = s->n_kernels;
+        cudaGraph_t g = nullptr;
+        CK(cudaStreamBeginCapture(s->own, cudaStreamCaptureModeThreadLocal));
+        // a sequence may end a call, so its last step is always monitored
+        st = ahead(t, K, true, s->d_ctl);
+        for (int q = 0; q < K && !st; q++) st = one_step(t + q, q, ((mask >> q) & 1u) || q == K - 1, 0, s->d_ctl);
+        if (!st && lx::launch_finish(s->d_ring, s->d_series ? mask : 0u, s->d_series, 0, s->series_cap, s->d_ctl, K,
+                                     s->probe_cap, s->own) != cudaSuccess)
+          st = fail(s, LX_ERR_CUDA, "launch_finish failed");
+        s->graph_kernels = s->n_kernels - before + 1;
+        s->n_kernels = before;
+        cudaError_t e = cudaStreamEndCapture(s->own, &g);
+        if (!st && e == cudaSuccess) e = cudaGraphInstantiate(&s->graph, g, 0);
+        if (g) cudaGraphDestroy(g);
+        if (st) return st;
+        CK(e);
+        s->graph_steps = K;
+        s->graph_pp = s->pp;
+      }
+      const lx::StepCtl want = {t, s->probe_rows, (int)s->series_t.size()};
+      if (std::memcmp(&want, &s->ctl, sizeof want) != 0) {
+        CK(lx::launch_set_ctl(s->d_ctl, want, s->stream));
+        s->n_kernels++;
+      }
+      CK(cudaGraphLaunch(s->graph, s->stream));
+      s->n_kernels += s->graph_kernels;
+      record(t, s->d_series ? mask : 0u);
+      if (s->nprobes > 0) s->probe_rows = std::min(s->probe_rows + K, s->probe_cap);
+      s->ctl = {t + K, std::min(want.row + K, s->probe_cap), (int)s->series_t.size()};
+      last_slot = s->d_ring + K - 1;
+      s->t += K;
+      s->alone_steps += K;
+      done += K;
+      if (done == nsteps && s->d_series && !((mask >> (K - 1)) & 1u)) {  // a call's last step joins the series
+        const int at = record(t, 1u << (K - 1));
+        CK(lx::launch_finish(s->d_ring, 1u << (K - 1), s->d_series, at, s->series_cap, nullptr, 0, 0, s->stream));
+        s->n_kernels++;
+      }
+      continue;
     }
+    int n = std::min(left, kt ? 1 : s->ahead);
+    if (K > 0 && t % K) n = std::min(n, K - t % K);  // up to the start of a sequence
+    unsigned mask = 0;
+    for (int q = 0; q < n; q++)
+      if (due(t + q) || done + q == nsteps - 1) mask |= 1u << q;
+    if ((st = ahead(t, n, pp.tab_total > 0 || s->src_kind >= 0 || mask, nullptr))) return st;
+    for (int q = 0; q < n; q++) {
+      const unsigned snap = snapshots(t + q);
+      if ((st = one_step(t + q, q, (mask >> q) & 1u, snap, nullptr))) return st;
+      s->t++;
+      if (snap && (st = snapshot(s, t + q, snap))) return st;
+    }
+    for (int q = 0; q < n; q++)
+      if ((mask >> q) & 1u) last_slot = s->d_ring + q;
+    if (s->d_series && mask) {
+      const int at = record(t, mask);
+      CK(lx::launch_finish(s->d_ring, mask, s->d_series, at, s->series_cap, nullptr, 0, 0, s->stream));
+      s->n_kernels++;
+    }
+    s->alone_steps += n;
+    done += n;
   }
   if (nsteps > 0) {
-    unsigned long long bits = 0;
-    unsigned fault = 0;
-    CK(cudaMemcpyAsync(&bits, last_slot, sizeof bits, cudaMemcpyDeviceToHost, s->stream));
-    CK(cudaMemcpyAsync(&fault, s->d_fault, sizeof fault, cudaMemcpyDeviceToHost, s->stream));
+    unsigned long long back[1 + lx::kAhead];  // the fault word and the slots
+    CK(cudaMemcpyAsync(back, s->d_max, sizeof back, cudaMemcpyDeviceToHost, s->stream));
     CK(cudaStreamSynchronize(s->stream));
-    s->n_d2h += sizeof bits + sizeof fault;
-    if (fault) {
-      CK(cudaMemsetAsync(s->d_fault, 0, sizeof fault, s->stream));
+    s->n_d2h += sizeof back;
+    if ((unsigned)back[0]) {
+      CK(cudaMemsetAsync(s->d_fault, 0, sizeof(unsigned), s->stream));
       return fail(s, LX_ERR_CUDA, "a sweep kernel's bounded wait for a staged plane ran out; the step's fields are not valid");
     }
     double v;
-    std::memcpy(&v, &bits, sizeof v);
+    std::memcpy(&v, &back[last_slot - s->d_max], sizeof v);
     s->last_max = v;
     if (!std::isfinite(v)) {
       char b[128];
@@ -1712,6 +1854,7 @@ extern "C" LX_API lx_status lx_sim_set_max_series(lx_sim* s, int capacity) {
   if (s->batch) return fail(s, LX_ERR_STATE, "batched members keep no max series");
   lx_status st = lx_sim_sync(s);
   if (st) return st;
+  drop_graph(s);
   dfree(s->d_series, s->own);
   s->d_series = nullptr;
   s->series_cap = 0;
@@ -1758,6 +1901,7 @@ extern "C" LX_API lx_status lx_sim_set_stream(lx_sim* s, void* stream) {
   lx::DeviceGuard dg_(s->device);
   lx_status st = lx_sim_sync(s);
   if (st) return st;
+  drop_graph(s);
   s->stream = stream ? (cudaStream_t)stream : s->own;
   return LX_OK;
 }
@@ -1778,7 +1922,7 @@ extern "C" LX_API lx_status lx_sim_info(const lx_sim* s, lx_info* info) {
   }
   b += (s->sweep ? 2 : 1) * (info->psi_h_entries + info->psi_e_entries) * s->csize;
   if (s->etotal) b += s->ncell * s->csize;
-  b += s->xfer_cap * sizeof(double) + (size_t)s->tab_total * s->csize;
+  b += s->xfer_cap * sizeof(double) + (size_t)s->tab_total * s->csize * (s->tabs ? 1 + s->ahead : 1);
   for (auto& sl : s->slots) b += sl.cap * sizeof(double);
   for (auto& d : s->dfts) b += d.n_acc * sizeof(double);
   b += (size_t)s->probe_cap * s->nprobes * 6 * sizeof(double);

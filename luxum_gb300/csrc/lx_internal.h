@@ -24,6 +24,17 @@ namespace lx {
 
 constexpr int kMaxProbes = 64;
 constexpr int kMaxDftFreq = 256;
+// Steps whose field-independent values (TF/SF tables, source amplitude) one launch forms ahead
+// for a handle stepped alone.
+constexpr int kAhead = 16;
+
+// Where a handle's replayed step sequence stands (device memory; launches issued one by one take
+// the values from their parameters instead).
+struct StepCtl {
+  int t;       // step of the sequence's first step
+  int row;     // probe rows recorded
+  int series;  // max|E|^2 series entries recorded
+};
 // Default cells each thread of a batched update kernel walks through along x: planar rows 8
 // apart, and 3-D planes (the autotuner's picks on the lens and 3-D cube workloads);
 // lx_batch_autotune picks per batch among 1, 2, 4 and 8.
@@ -165,7 +176,9 @@ __host__ __device__ inline bool tile_is_interior_2d(const Slab (&sl)[3], bool pm
 
 // Probe sampling of one step row.
 struct ProbeParams {
-  int nprobes, row, Ny, Nzp;
+  int nprobes, row, cap, Ny, Nzp;
+  const StepCtl* ctl;  // when non-null, the row is ctl->row + k
+  int k;
   double hmul;      // 1/hscale: stored H -> H
   int ext[6][3];    // staggered extents of the six components (0 for absent ones)
   const int* ijk;   // device array [nprobes][3]
@@ -174,6 +187,8 @@ struct ProbeParams {
 // One DFT plane monitor (see lx_sim_add_dft_plane).
 struct DftParams {
   int axis, index, na, nb, Ny, Nzp, nfreq, t;
+  const StepCtl* ctl;     // single launches: when non-null, the step is ctl->t + k
+  int k;
   int sim;                // batched launches: index of the simulation's step counter
   const void* f[4];       // batched launches: the four sampled components
   const void* f1[4];      // ... in buffer 1, for members stepped in two buffers (null otherwise):

@@ -1,6 +1,7 @@
 // lx_kernels.cu -- sm_103a kernels of the Yee time step.
 //
-// One step = prologue (TF/SF incident tables for this step, point source, monitor reset)
+// One step = prologue (TF/SF incident tables, point source, monitor reset; handles stepped alone
+//             form the tables of several steps in one launch)
 //          -> H kernel (curl E + TF/SF + CPML psi_H + H update, fused)
 //          -> E kernel (curl H + TF/SF + CPML psi_E + E update + max|E|^2, fused)
 // This is the order of every reference driver (e.g. three_dim_pml.cc:158-276): point source,
@@ -66,30 +67,31 @@ __device__ C incident_value(const PrologueParams& p, const PatchSet& ps, int pla
   else return __dmul_rn(exp(a), ps.factor);
 }
 
-template <class C>
-__device__ __forceinline__ void prologue_body(const PrologueParams& p, const int t, C* tab_out, const int gid,
-                                              const int gstride) {
-  if (gid == 0) {
-    if (p.max_slot) *p.max_slot = 0ull;
-    void* const src_field = ((t & 1) && p.src_field1) ? p.src_field1 : p.src_field;  // the state step t reads
-    if (p.src_kind == 0) {
-      // amp_source*sin(omega_source*t*dt), int members (maxwell.h:203,206; three_dim_pml.cc:163)
-      const int wt = (int)((unsigned)p.src_omega_i * (unsigned)t);
-      const double v = (double)p.src_amp_i * sin((double)wt * p.dt);
-      if (p.prec == 0) ((double*)src_field)[p.src_idx] = v;
-      else if (p.prec == 1) ((float*)src_field)[p.src_idx] = (float)v;
-      else ((__half*)src_field)[p.src_idx] = __double2half(v);
-    } else if (p.src_kind == 1) {
-      const double u = (t - p.src_t0) / p.src_tw;
-      const double v = p.src_amp * exp(-(u * u)) * sin(p.src_omega * t * p.dt);
-      if (p.prec == 0) ((double*)src_field)[p.src_idx] += v;
-      else if (p.prec == 1) ((float*)src_field)[p.src_idx] += (float)v;
-      else {
-        __half* f = (__half*)src_field;
-        f[p.src_idx] = __float2half_rn(__half2float(f[p.src_idx]) + (float)v);
-      }
-    }
+// The point source's value at step t (three_dim_pml.cc:163; the pulse is an extension).
+__device__ __forceinline__ double source_value(const PrologueParams& p, const int t) {
+  if (p.src_kind == 0) {
+    // amp_source*sin(omega_source*t*dt), int members (maxwell.h:203,206; three_dim_pml.cc:163)
+    const int wt = (int)((unsigned)p.src_omega_i * (unsigned)t);
+    return (double)p.src_amp_i * sin((double)wt * p.dt);
   }
+  const double u = (t - p.src_t0) / p.src_tw;
+  return p.src_amp * exp(-(u * u)) * sin(p.src_omega * t * p.dt);
+}
+template <class T>
+__device__ __forceinline__ void source_apply(T* f, int kind, double v) {
+  if constexpr (sizeof(T) == 2) {
+    if (kind == 0) *f = __double2half(v);
+    else *f = __float2half_rn(__half2float(*f) + (float)v);
+  } else {
+    if (kind == 0) *f = (T)v;
+    else *f += (T)v;
+  }
+}
+
+// The TF/SF tables of step t.
+template <class C>
+__device__ __forceinline__ void tables_body(const PrologueParams& p, const int t, C* tab_out, const int gid,
+                                            const int gstride) {
   // Work items: one per entry, except that a set whose planes are normal to an axis k has no
   // component along shares its values between the two planes (the normal position is
   // multiplied by 0 in X), so one item writes both.  The sets' work ranges are staged in
@@ -123,10 +125,41 @@ __device__ __forceinline__ void prologue_body(const PrologueParams& p, const int
   }
 }
 
+// Steps ahead of a handle stepped alone: blockIdx.y is the step of the sequence.  The launch's own
+// latency (positions, exponentials and set walk in a few dependent chains, 6-7 us however small
+// the tables) is paid once for up to kAhead steps instead of before every H update.
 template <class C>
-__global__ void prologue_kernel(const PrologueParams p, C* tab_out) {
-  prologue_body<C>(p, p.t, tab_out, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
+__global__ void prologue_ahead_kernel(const PrologueParams p, const StepCtl* ctl, C* tab, double* srcv,
+                                      unsigned long long* ring) {
+  const int q = blockIdx.y, t = (ctl ? ctl->t : p.t) + q;
+  const int gid = blockIdx.x * blockDim.x + threadIdx.x;
+  if (gid == 0) {
+    ring[q] = 0ull;
+    if (p.src_kind >= 0) srcv[q] = source_value(p, t);
+  }
+  tables_body<C>(p, t, tab + (long long)q * p.tab_total, gid, gridDim.x * blockDim.x);
 }
+
+template <class T>
+__global__ void source_kernel(T* field, long long idx, int kind, const double* v) {
+  source_apply<T>(field + idx, kind, *v);
+}
+
+__global__ void finish_kernel(const unsigned long long* ring, unsigned mask, unsigned long long* series, int at, int cap,
+                              StepCtl* ctl, int steps, int rows) {
+  const int q = threadIdx.x;
+  const int base = ctl ? ctl->series : at;
+  const int n = base + __popc(mask & ((1u << q) - 1u));
+  if (((mask >> q) & 1u) && n < cap) series[n] = ring[q];
+  __syncwarp();
+  if (q == 0 && ctl) {
+    ctl->t += steps;
+    ctl->row = min(ctl->row + steps, rows);
+    ctl->series = min(base + __popc(mask), cap);
+  }
+}
+
+__global__ void set_ctl_kernel(StepCtl* ctl, const StepCtl v) { *ctl = v; }
 
 // Batched prologue: blockIdx.y selects the simulation.  Its step counter lives on the device
 // and advances once per chunk, so that a captured chunk can be replayed: step k of a chunk
@@ -134,7 +167,18 @@ __global__ void prologue_kernel(const PrologueParams p, C* tab_out) {
 template <class C>
 __global__ void prologue_batch_kernel(const PrologueParams* __restrict__ pps, const int* __restrict__ ts, int k) {
   const PrologueParams& p = pps[blockIdx.y];
-  prologue_body<C>(p, ts[blockIdx.y] + k, (C*)p.tab, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
+  const int t = ts[blockIdx.y] + k, gid = blockIdx.x * blockDim.x + threadIdx.x;
+  if (gid == 0) {
+    if (p.max_slot) *p.max_slot = 0ull;
+    void* const f = ((t & 1) && p.src_field1) ? p.src_field1 : p.src_field;  // the state step t reads
+    if (p.src_kind >= 0) {
+      const double v = source_value(p, t);
+      if (p.prec == 0) source_apply((double*)f + p.src_idx, p.src_kind, v);
+      else if (p.prec == 1) source_apply((float*)f + p.src_idx, p.src_kind, v);
+      else source_apply((__half*)f + p.src_idx, p.src_kind, v);
+    }
+  }
+  tables_body<C>(p, t, (C*)p.tab, gid, gridDim.x * blockDim.x);
 }
 
 __global__ void tick_kernel(int* ts, int n, int steps) {
@@ -1204,6 +1248,8 @@ __global__ void probe_kernel(const ProbeParams pp, const T* f0, const T* f1, con
                              const T* f5, double* out) {
   const int q = blockIdx.x * blockDim.x + threadIdx.x;
   if (q >= pp.nprobes * 6) return;
+  const int row = pp.ctl ? pp.ctl->row + pp.k : pp.row;
+  if (row >= pp.cap) return;
   const int probe = q / 6, comp = q % 6;
   const T* f[6] = {f0, f1, f2, f3, f4, f5};
   const int i = pp.ijk[3 * probe], j = pp.ijk[3 * probe + 1], k = pp.ijk[3 * probe + 2];
@@ -1214,7 +1260,7 @@ __global__ void probe_kernel(const ProbeParams pp, const T* f0, const T* f1, con
     else v = (double)*src;
     if (comp >= 3 && pp.hmul != 1.0) v *= pp.hmul;
   }
-  out[(long long)pp.row * pp.nprobes * 6 + q] = v;
+  out[(long long)row * pp.nprobes * 6 + q] = v;
 }
 
 // Phase factors of one sample of a DFT plane: cos/sin of omega*(t+1)*dt for the E
@@ -1234,7 +1280,7 @@ __device__ __forceinline__ void dft_phase_body(const DftParams& d, const int t) 
   }
 }
 
-__global__ void dft_phase_kernel(const DftParams d) { dft_phase_body(d, d.t); }
+__global__ void dft_phase_kernel(const DftParams d) { dft_phase_body(d, d.ctl ? d.ctl->t + d.k : d.t); }
 
 // Batched: one block per plane of a sampling class.
 __global__ void dft_phase_batch_kernel(const DftParams* __restrict__ ds, const int* __restrict__ ts, int k) {
@@ -1362,9 +1408,28 @@ static inline unsigned grid1d(long long n, int bs) {
 }
 
 template <class C>
-cudaError_t launch_prologue(const PrologueParams& p, cudaStream_t s) {
+cudaError_t launch_prologue_ahead(const PrologueParams& p, int steps, const StepCtl* ctl, C* tab, double* srcv,
+                                  unsigned long long* ring, cudaStream_t s) {
+  if (steps < 1 || steps > kAhead) return cudaErrorInvalidValue;
   const int bs = 256;
-  prologue_kernel<C><<<grid1d(p.tab_total > 0 ? p.tab_total : 1, bs), bs, 0, s>>>(p, (C*)p.tab);
+  prologue_ahead_kernel<C><<<dim3(grid1d(p.tab_total > 0 ? p.tab_total : 1, bs), steps), bs, 0, s>>>(p, ctl, tab, srcv, ring);
+  return cudaGetLastError();
+}
+
+template <class T>
+cudaError_t launch_source(T* field, long long idx, int kind, const double* v, cudaStream_t s) {
+  source_kernel<T><<<1, 1, 0, s>>>(field, idx, kind, v);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_finish(const unsigned long long* ring, unsigned mask, unsigned long long* series, int at, int cap,
+                          StepCtl* ctl, int steps, int rows, cudaStream_t s) {
+  finish_kernel<<<1, 32, 0, s>>>(ring, mask, series, at, cap, ctl, steps, rows);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_set_ctl(StepCtl* ctl, StepCtl v, cudaStream_t s) {
+  set_ctl_kernel<<<1, 1, 0, s>>>(ctl, v);
   return cudaGetLastError();
 }
 
@@ -1596,6 +1661,7 @@ cudaError_t launch_dft_flux(const double* acc, int nfreq, long long ncell, doubl
   template cudaError_t launch_gather<T>(const T*, double*, const int[3], int, int, double, cudaStream_t);                     \
   template cudaError_t launch_scatter<T>(const double*, T*, const int[3], int, int, int, double, double, double,      \
                                          double, cudaStream_t);                                                        \
+  template cudaError_t launch_source<T>(T*, long long, int, const double*, cudaStream_t);                              \
   template cudaError_t launch_probes<T>(const ProbeParams&, T* const[6], double*, cudaStream_t);                   \
   template cudaError_t launch_dft<T>(const DftParams&, T* const[4], cudaStream_t);                                 \
   template cudaError_t launch_batch_tiles<T, C>(const StepParams<T, C>*, const int*, int, int, bool, int, int4*,    \
@@ -1608,8 +1674,10 @@ LX_INST(float, float)
 LX_INST(__half, float)
 template cudaError_t launch_step_sweep2<float, float>(const StepParams<float, float>&, bool, cudaStream_t);
 template cudaError_t launch_step_sweep2<__half, float>(const StepParams<__half, float>&, bool, cudaStream_t);
-template cudaError_t launch_prologue<double>(const PrologueParams&, cudaStream_t);
-template cudaError_t launch_prologue<float>(const PrologueParams&, cudaStream_t);
+template cudaError_t launch_prologue_ahead<double>(const PrologueParams&, int, const StepCtl*, double*, double*,
+                                                   unsigned long long*, cudaStream_t);
+template cudaError_t launch_prologue_ahead<float>(const PrologueParams&, int, const StepCtl*, float*, double*,
+                                                  unsigned long long*, cudaStream_t);
 template cudaError_t launch_prologue_batch<double>(const PrologueParams*, const int*, int, int, int, cudaStream_t);
 template cudaError_t launch_prologue_batch<float>(const PrologueParams*, const int*, int, int, int, cudaStream_t);
 template cudaError_t launch_eps_box<double>(double*, const int[3], int, int, const int[3], const int[3], double,

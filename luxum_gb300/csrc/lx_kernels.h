@@ -6,8 +6,20 @@
 
 namespace lx {
 
+// What the next `steps` (<= kAhead) steps of a handle stepped alone need that does not depend on
+// its fields: step q's TF/SF tables at tab + q * p.tab_total, its source amplitude in srcv[q], its
+// max|E|^2 slot ring[q] zeroed.  Step q is ctl->t + q, or p.t + q when ctl is null.
 template <class C>
-cudaError_t launch_prologue(const PrologueParams& p, cudaStream_t s);
+cudaError_t launch_prologue_ahead(const PrologueParams& p, int steps, const StepCtl* ctl, C* tab, double* srcv,
+                                  unsigned long long* ring, cudaStream_t s);
+// The point source of one step (its amplitude formed ahead), before the step's H update.
+template <class T>
+cudaError_t launch_source(T* field, long long idx, int kind, const double* v, cudaStream_t s);
+// ring[q] of the steps q in `mask` appended to the max|E|^2 series from entry `at` (ctl: from
+// ctl->series, up to cap); with ctl, the counters then advance by `steps`.
+cudaError_t launch_finish(const unsigned long long* ring, unsigned mask, unsigned long long* series, int at, int cap,
+                          StepCtl* ctl, int steps, int rows, cudaStream_t s);
+cudaError_t launch_set_ctl(StepCtl* ctl, StepCtl v, cudaStream_t s);
 template <class T, class C>
 cudaError_t launch_step(const StepParams<T, C>& p, bool planar, bool uniform, bool h_half, cudaStream_t s);
 // Single-sweep planar step (float compute, two state buffers): reads the buffers named in

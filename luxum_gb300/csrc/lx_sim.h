@@ -116,8 +116,24 @@ struct lx_sim {
   void* tab = nullptr;
   int tab_total = 0;
   lx::PatchSet setsH[3][2] = {}, setsE[3][2] = {};
+  // One allocation: the fault word (set by a kernel whose bounded wait ran out), then for the
+  // steps of a sequence their max|E|^2 slots and source amplitudes, and the replay counters.
   unsigned long long* d_max = nullptr;
-  unsigned* d_fault = nullptr;  // in d_max's allocation: set by a kernel whose bounded wait ran out
+  unsigned* d_fault = nullptr;
+  unsigned long long* d_ring = nullptr;
+  double* d_srcv = nullptr;
+  lx::StepCtl* d_ctl = nullptr;
+  // Stepped alone: TF/SF tables of `ahead` steps (the handle's own table when ahead is 1), formed
+  // by one launch.
+  int ahead = 0;
+  void* tabs = nullptr;
+  // A captured sequence of graph_steps steps (short steps are bound by their launches); dropped
+  // when anything its launches were given changes.  `ctl` is what d_ctl holds.
+  cudaGraphExec_t graph = nullptr;
+  int graph_steps = 0, graph_pp = 0;
+  unsigned long long graph_kernels = 0;
+  long long alone_steps = 0;  // steps taken since the last such change
+  lx::StepCtl ctl = {-1, -1, -1};
   // max|E|^2 series: one slot per monitored step (device), the step of each slot (host)
   unsigned long long* d_series = nullptr;
   int series_cap = 0;
