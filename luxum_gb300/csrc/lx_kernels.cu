@@ -494,7 +494,8 @@ __device__ __forceinline__ void e_load(const StepParams<T, C>& p, const int i, c
 
 template <class T, class C, bool UNI, bool MON, bool FAST = false>
 __device__ __forceinline__ typename MaxBits<C>::type e_apply(const StepParams<T, C>& p, const int i, const int j,
-                                                             const int k, bool tf, const ECell<C>& v) {
+                                                             const int k, bool tf, const ECell<C>& v,
+                                                             const MaxScreen<C>& scr) {
   const long long c = v.c;
   const bool ux = FAST || v.ux, uy = FAST || v.uy, uz = FAST || v.uz, mon = MON && (FAST || v.mon);
   if (FAST) tf = false;
@@ -548,7 +549,7 @@ __device__ __forceinline__ typename MaxBits<C>::type e_apply(const StepParams<T,
   if (uy) st<T, C>(p.E[1] + c, eyn);
   if (uz) st<T, C>(p.E[2] + c, ezn);
   typename MaxBits<C>::type mbits = 0;
-  if (mon) {
+  if (mon && (p.etotal || scr.may(exn, eyn, ezn))) {
     // Etotal = Ez*Ez + Ey*Ey + Ex*Ex (three_dim_pml.cc:270), same association order
     const C e2 = fmaC(exn, exn, fmaC(eyn, eyn, fp.mul(ezn, ezn)));
     if (p.etotal) p.etotal[c] = e2;
@@ -561,8 +562,9 @@ template <class T, class C, bool UNI, bool MON, bool FAST = false>
 __device__ __forceinline__ typename MaxBits<C>::type e_cell_3d(const StepParams<T, C>& p, const int i, const int j,
                                                                const int k, const bool tf) {
   ECell<C> v;
+  const MaxScreen<C> scr(MON ? p.max_slot : nullptr);
   e_load<T, C, MON, FAST>(p, i, j, k, v);
-  return e_apply<T, C, UNI, MON, FAST>(p, i, j, k, tf, v);
+  return e_apply<T, C, UNI, MON, FAST>(p, i, j, k, tf, v, scr);
 }
 
 // E of a cell whose block meets the CPML slab of axis AX only and no TF/SF plane (see h_slab_3d):
@@ -747,7 +749,7 @@ __device__ __forceinline__ void e2_load(const StepParams<T, C>& p, const int i, 
 
 template <class T, class C, bool UNI, bool MON, bool FAST = false>
 __device__ __forceinline__ typename MaxBits<C>::type e2_apply(const StepParams<T, C>& p, const int i, const int k,
-                                                              bool tf, const ECell2<C>& v) {
+                                                              bool tf, const ECell2<C>& v, const MaxScreen<C>& scr) {
   const long long c = v.c;
   const C ey = v.ey;
   C eyn = ey;
@@ -770,15 +772,16 @@ __device__ __forceinline__ typename MaxBits<C>::type e2_apply(const StepParams<T
     st<T, C>(p.E[1] + c, eyn);
   }
   // local_max = max(Ey*Ey) over the whole Ey array (two_dim_pml.cc:181)
-  return MON ? MaxBits<C>::of(fp.mul(eyn, eyn)) : typename MaxBits<C>::type(0);
+  return MON && scr.may(eyn) ? MaxBits<C>::of(fp.mul(eyn, eyn)) : typename MaxBits<C>::type(0);
 }
 
 template <class T, class C, bool UNI, bool MON, bool FAST = false>
 __device__ __forceinline__ typename MaxBits<C>::type e_cell_2d(const StepParams<T, C>& p, const int i, const int k,
                                                                const bool tf) {
   ECell2<C> v;
+  const MaxScreen<C> scr(MON ? p.max_slot : nullptr);
   e2_load<T, C, MON, FAST>(p, i, k, v);
-  return e2_apply<T, C, UNI, MON, FAST>(p, i, k, tf, v);
+  return e2_apply<T, C, UNI, MON, FAST>(p, i, k, tf, v, scr);
 }
 
 template <class T, class C, bool UNI, bool MON>
@@ -1149,11 +1152,12 @@ __global__ void __launch_bounds__(256, E2BatchMinBlocks<C>::v) e_batch_2d(const 
   if (fast && k < p.Nz) {  // interior tile: the next row's loads first (see h_batch_2d)
     const int i0 = tl.y + threadIdx.y;
     ECell2<C> v[2];
+    const MaxScreen<C> scr(p.max_slot);
     e2_load<T, C, true, true>(p, i0, k, v[0]);
 #pragma unroll
     for (int r = 0; r < M; ++r) {
       if (r + 1 < M) e2_load<T, C, true, true>(p, i0 + 8 * (r + 1), k, v[(r + 1) & 1]);
-      const typename MaxBits<C>::type b = e2_apply<T, C, UNI, true, true>(p, i0 + 8 * r, k, false, v[r & 1]);
+      const typename MaxBits<C>::type b = e2_apply<T, C, UNI, true, true>(p, i0 + 8 * r, k, false, v[r & 1], scr);
       mbits = b > mbits ? b : mbits;
     }
   } else if (k < p.Nz) {
