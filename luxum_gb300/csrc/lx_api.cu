@@ -1685,7 +1685,7 @@ static lx_status run_steps(lx_sim* s, int nsteps, KernelTimer* kt = nullptr) {
       lx::DftParams dp;
       std::memset(&dp, 0, sizeof dp);
       dp.axis = d.axis; dp.index = d.index; dp.na = d.na; dp.nb = d.nb; dp.Ny = s->Ny; dp.Nzp = s->Nzp;
-      dp.nfreq = d.nfreq; dp.t = t; dp.ctl = ctl; dp.k = q; dp.dt = s->k.dt; dp.weight = (double)d.every;
+      dp.nfreq = d.nfreq; dp.t = t; dp.t_at = ctl ? &ctl->t : nullptr; dp.k = q; dp.dt = s->k.dt; dp.weight = (double)d.every;
       dp.omega = d.d_omega; dp.acc = d.d_acc; dp.phase = d.d_phase; dp.hmul = 1.0 / s->hscale;
       T* f4[4];
       for (int c = 0; c < 4; c++) {
@@ -1964,27 +1964,33 @@ struct lx_batch {
   // 3-D members of at least kSoloCells cells take one kernel pair each, with their parameter
   // block passed by value (the constant bank, as for a handle stepped alone), spread over the
   // batch stream and kLanes - 1 more so that the members' kernels overlap.  Planar members with
-  // float compute of at least kSoloCells2 cells take the single-sweep kernel the same way, in
-  // their two buffers (ping-pong mode); smaller members share the batched launches in place.
+  // float compute step in their two buffers (ping-pong mode): of at least kSoloCells2 cells one
+  // by one like these, smaller ones together in the batched sweep.  Planar FP64 members and
+  // smaller 3-D ones share the batched half-step launches in place.
   static constexpr long long kSoloCells = 1LL << 18;
-  // (2^21 cells: a member's sweep takes ~15 us; at 2^18 the launches of the 256-lens batch's
-  // larger half cost more than the single sweep saves, 103 -> 96 Gcell/s)
-  static constexpr long long kSoloCells2 = 1LL << 21;
+  // (us a step of 48 lenses of side 128-1024, 12 and 96 of them, 16 of side 1000, one by one from
+  // 2^21, 2^20 and 2^19 cells: 142, 138, 135; 43, 39, 38; 226, 222, 211; 140, 134, 143.  Launched
+  // directly a member's step costs the host 2 us.)
+  static constexpr long long kSoloCells2 = 1LL << 20;
   static constexpr int kLanes = 4;
   cudaStream_t lanes[kLanes - 1] = {};
   cudaEvent_t lane_ev[kLanes] = {};  // [0] fork, [1..] joins
-  struct Group {  // members sharing (planar, uniform, solo): one update launch per half step
+  struct Group {  // members sharing (planar, uniform, solo, sweep): one update launch per (half) step
     bool planar = false, uniform = false;
     bool solo = false;              // members launched one by one (kSoloCells / kSoloCells2 and larger)
-    std::vector<char> host_params;  // solo groups: the members' parameter blocks
-    int march = lx::kMarch3;   // cells each thread walks along x
+    bool sweep = false;             // planar members in two buffers
+    std::vector<char> host_params;  // solo groups: the members' parameter blocks; sweep groups: their
+                                    // SweepParams at their parity when built, then at the other
+    int march = lx::kMarch3;   // cells each thread walks along x (0 while it is still to be chosen)
     std::vector<int> members;  // batch-global indices
     void* d_params = nullptr;
     int* d_first = nullptr;
     int4* d_tiles = nullptr;
     int nblocks = 0;
+    std::vector<int> first;  // sweep groups: the members' first blocks
   };
   int march2d = lx::kMarch2, march3d = lx::kMarch3;  // per dimension (lx_batch_set_march / autotune)
+  bool march_set = false;            // set by a caller or the tuner: not adapted to the batch's size
   std::vector<lx_tune_entry> table;  // march per member class (lx_batch_set_tune_table / autotune)
   struct DftClass {  // DFT planes that sample at the same batch steps
     int every = 1, phase = 0;
@@ -1998,7 +2004,14 @@ struct lx_batch {
   lx::PrologueParams* d_pps = nullptr;
   int max_entries = 0;
   int* d_ts = nullptr;
+  // Steps formed ahead by one prologue launch, their tables, [row][member] slots and amplitudes.
+  int ahead = 1;
+  void* d_tabs = nullptr;
   unsigned long long* d_slots = nullptr;
+  double* d_srcv = nullptr;
+  bool sources = false;
+  int last_row = 0;        // row of the last step enqueued
+  long long built_at = 0;  // batch step of the last rebuild (sweep groups' parity)
   long long step = 0;  // batch steps taken (DFT sampling classes are phases of it)
   cudaGraphExec_t exec = nullptr;
   int exec_steps = 0;
@@ -2047,12 +2060,21 @@ static void table_put(lx_batch* b, const lx_tune_entry& e) {
   b->table.push_back(e);
 }
 
-// The march of a batched member: its class's table entry, else the per-dimension march.
+// The march of a batched member: its class's table entry, else the per-dimension march if one was
+// set, else 0.
 static int batch_march(const lx_batch* b, const lx_sim* s) {
   const lx_tune_entry k = tune_class_of(s);
   for (const auto& x : b->table)
     if (same_class(x, k)) return x.march;
-  return s->planar ? b->march2d : b->march3d;
+  return b->march_set ? (s->planar ? b->march2d : b->march3d) : 0;
+}
+
+// The march of a group nobody chose one for: the dimension's default, halved while the group has
+// fewer blocks than fill the GPU twice.
+template <class F>
+static int adapted_march(int march, F count) {
+  while (march > 1 && count(march) < 152LL * 5 * 2) march /= 2;
+  return march;
 }
 
 static void batch_free_device(lx_batch* b) {
@@ -2071,9 +2093,13 @@ static void batch_free_device(lx_batch* b) {
   dfree(b->d_pps, b->stream);
   dfree(b->d_ts, b->stream);
   dfree(b->d_slots, b->stream);
+  dfree(b->d_srcv, b->stream);
+  dfree(b->d_tabs, b->stream);
   b->d_pps = nullptr;
   b->d_ts = nullptr;
   b->d_slots = nullptr;
+  b->d_srcv = nullptr;
+  b->d_tabs = nullptr;
   if (b->exec) cudaGraphExecDestroy(b->exec);
   b->exec = nullptr;
   b->exec_steps = 0;
@@ -2134,6 +2160,7 @@ extern "C" LX_API lx_status lx_batch_set_chunk(lx_batch* b, int steps) {
   if (!b || steps < 0) return fail(nullptr, LX_ERR_INVALID, "chunk must be >= 0");
   lx::DeviceGuard dg_(b->device);
   b->chunk = steps;
+  b->dirty = true;  // whether the members' steps can be captured depends on it
   if (b->exec) cudaGraphExecDestroy(b->exec);
   b->exec = nullptr;
   b->exec_steps = 0;
@@ -2184,25 +2211,43 @@ static lx_status batch_rebuild(lx_batch* b) {
   b->max_entries = 0;
   b->host_ts.resize(n);
   b->graphable = true;
-  BCK(cudaMallocAsync(&b->d_slots, sizeof(unsigned long long) * (n > 0 ? n : 1), b->stream));
+  b->sources = false;
+  b->built_at = b->step;
+  // Steps ahead: as many as keep the members' tables within 32 MB.
+  size_t entries = 0;
+  for (auto* s : b->sims) entries += s->tfsf ? s->tab_total : 0;
+  constexpr size_t kTabBytes = 32 << 20;
+  b->ahead = entries ? (int)std::max<size_t>(1, std::min<size_t>(lx::kAhead, kTabBytes / (entries * sizeof(C)))) : lx::kAhead;
+  if (entries) BCK(cudaMallocAsync(&b->d_tabs, entries * b->ahead * sizeof(C), b->stream));
+  BCK(cudaMallocAsync(&b->d_slots, sizeof(unsigned long long) * lx::kAhead * (n > 0 ? n : 1), b->stream));
+  BCK(cudaMallocAsync(&b->d_srcv, sizeof(double) * lx::kAhead * (n > 0 ? n : 1), b->stream));
   std::vector<std::vector<lx::DftParams>> dft_planes;
-  // Large planar single-sweep members step in their two buffers, the others in place in buffer 0;
-  // a member whose mode changes at an odd step moves its state (one device copy).
+  // Planar float members step in their two buffers, the others in place in buffer 0; a member
+  // whose mode changes at an odd step moves its state (one device copy).
   for (int q = 0; q < n; q++) {
     lx_sim* s = b->sims[q];
-    const bool two = s->planar && batch_alone(s);
     lx_status st;
-    if ((st = set_pp(s, two))) return st;
+    if ((st = set_pp(s, s->planar && s->sweep))) return st;
     BCK(cudaStreamSynchronize(s->stream));
   }
+  std::vector<C*> tabs(n, nullptr);
+  size_t at = 0;
   for (int q = 0; q < n; q++) {
     lx_sim* s = b->sims[q];
     pps[q] = make_prologue(s);
-    pps[q].max_slot = b->d_slots + q;
+    if (s->tfsf) {
+      tabs[q] = (C*)b->d_tabs + at;
+      pps[q].tab = tabs[q];
+      at += (size_t)s->tab_total * b->ahead;
+    }
+    b->sources |= s->src_kind >= 0;
     b->max_entries = std::max(b->max_entries, pps[q].tab_total);
     b->host_ts[q] = s->t;
+    const bool solo = batch_alone(s);
     T* pf[6] = {(T*)s->E[0], (T*)s->E[1], (T*)s->E[2], (T*)s->H[0], (T*)s->H[1], (T*)s->H[2]};
     for (auto& d : s->dfts) {
+      if (b->chunk > 0 && b->chunk % d.every != 0) b->graphable = false;
+      if (solo) continue;  // sampled in the member's own lane
       lx::DftParams dp;
       std::memset(&dp, 0, sizeof dp);
       dp.axis = d.axis; dp.index = d.index; dp.na = d.na; dp.nb = d.nb; dp.Ny = s->Ny; dp.Nzp = s->Nzp;
@@ -2227,22 +2272,22 @@ static lx_status batch_rebuild(lx_batch* b) {
         ci = (int)b->dft.size() - 1;
       }
       dft_planes[ci].push_back(dp);
-      if (b->chunk > 0 && b->chunk % d.every != 0) b->graphable = false;
     }
-    const bool solo = s->pp || (!s->planar && batch_alone(s));
     if (s->pp && b->chunk % 2) b->graphable = false;  // a captured chunk must keep each member's parity
-    // batched members share a launch only with members of the same march (their classes' picks)
-    const int march = solo ? (s->planar ? b->march2d : b->march3d) : batch_march(b, s);
+    // batched members share a launch only with members of the same march (their classes' picks; 0:
+    // chosen by the group's size)
+    const int march = solo ? lx::kMarch3 : batch_march(b, s);
     int gi = -1;
     for (size_t g = 0; g < b->groups.size(); g++)
       if (b->groups[g].planar == (bool)s->planar && b->groups[g].uniform == (bool)s->uniform &&
-          b->groups[g].solo == solo && (solo || b->groups[g].march == march))
+          b->groups[g].solo == solo && b->groups[g].sweep == (bool)s->pp && (solo || b->groups[g].march == march))
         gi = (int)g;
     if (gi < 0) {
       b->groups.emplace_back();
       b->groups.back().planar = s->planar;
       b->groups.back().uniform = s->uniform;
       b->groups.back().solo = solo;
+      b->groups.back().sweep = s->pp;
       b->groups.back().march = march;
       gi = (int)b->groups.size() - 1;
     }
@@ -2268,21 +2313,53 @@ static lx_status batch_rebuild(lx_batch* b) {
   }
   for (auto& g : b->groups) {
     std::vector<lx::StepParams<T, C>> ps;
-    std::vector<int> first(1, 0);
     for (int q : g.members) {
-      lx_sim* s = b->sims[q];
-      lx::StepParams<T, C> sp = step_params<T, C>(s);
+      lx::StepParams<T, C> sp = step_params<T, C>(b->sims[q]);
+      sp.tab = tabs[q];
+      sp.tab_stride = b->sims[q]->tab_total;
       sp.max_slot = b->d_slots + q;
+      sp.slot_stride = n;
       sp.etotal = nullptr;
       ps.push_back(sp);
-      const long long nb = (long long)first.back() + lx::batch_blocks(s->Nx, s->Ny, s->Nz, s->planar, g.march);
-      if (nb > 0x7fffffffLL) return bfail(b, LX_ERR_INVALID, "batch too large for one launch");
-      first.push_back((int)nb);
     }
     if (g.solo) {  // launched by value from the host copy: no device blocks or tile map
       g.host_params.assign((const char*)ps.data(), (const char*)(ps.data() + ps.size()));
       g.nblocks = 0;
       continue;
+    }
+    auto count = [&](int march) {
+      long long nb = 0;
+      for (int q : g.members) {
+        const lx_sim* s = b->sims[q];
+        nb += lx::batch_blocks(s->Nx, s->Ny, s->Nz, s->planar, march);
+      }
+      return nb;
+    };
+    if (g.march == 0) g.march = adapted_march(g.planar ? b->march2d : b->march3d, count);
+    std::vector<int> first(1, 0);
+    for (int q : g.members) {
+      const lx_sim* s = b->sims[q];
+      const long long nb = (long long)first.back() + lx::batch_blocks(s->Nx, s->Ny, s->Nz, s->planar, g.march);
+      if (nb > 0x7fffffffLL) return bfail(b, LX_ERR_INVALID, "batch too large for one launch");
+      first.push_back((int)nb);
+    }
+    if constexpr (sizeof(C) == 4) {
+      if (g.sweep) {  // passed by value: no device blocks or tile map
+        std::vector<lx::SweepParams<T, C>> sw;
+        for (int par = 0; par < 2; par++)
+          for (size_t m = 0; m < ps.size(); m++) {
+            lx::StepParams<T, C> sp = ps[m];
+            if ((b->sims[g.members[m]]->t + par) & 1) swap_buffers(sp);
+            sw.push_back(lx::sweep_params(sp));
+          }
+        g.host_params.assign((const char*)sw.data(), (const char*)(sw.data() + sw.size()));
+        std::vector<int4> tiles;
+        lx::sweep_tiles(sw.data(), (int)ps.size(), g.march, g.first, tiles);
+        g.nblocks = (int)tiles.size();
+        BCK(cudaMallocAsync(&g.d_tiles, sizeof(int4) * std::max<size_t>(tiles.size(), 1), b->stream));
+        BCK(cudaMemcpyAsync(g.d_tiles, tiles.data(), sizeof(int4) * tiles.size(), cudaMemcpyHostToDevice, b->stream));
+        continue;
+      }
     }
     g.nblocks = first.back();
     BCK(cudaMallocAsync(&g.d_params, sizeof(lx::StepParams<T, C>) * ps.size(), b->stream));
@@ -2297,48 +2374,125 @@ static lx_status batch_rebuild(lx_batch* b) {
   return LX_OK;
 }
 
+// Step q of a chunk for member m, launched by value on `st`; row: its place in the sequence.
+template <class T, class C>
+static lx_status solo_step(lx_batch* b, const lx_batch::Group& g, size_t m, int q, int row, cudaStream_t st) {
+  const int id = g.members[m];
+  lx_sim* s = b->sims[id];
+  const int t = b->host_ts[id] + q;
+  lx::StepParams<T, C> sp = ((const lx::StepParams<T, C>*)g.host_params.data())[m];
+  sp.tab += (size_t)row * sp.tab_stride;
+  sp.max_slot += (size_t)row * sp.slot_stride;
+  bool swept = false;
+  if constexpr (sizeof(C) == 4) {
+    if (g.sweep) {  // single sweep, state t & 1 -> (t+1) & 1
+      if (t & 1) swap_buffers(sp);
+      BCK(lx::launch_step_sweep2<T, C>(sp, g.uniform, st));
+      swept = true;
+    }
+  }
+  if (!swept) {
+    BCK(lx::launch_step<T, C>(sp, g.planar, g.uniform, true, st));
+    BCK(lx::launch_step<T, C>(sp, g.planar, g.uniform, false, st));
+  }
+  for (auto& d : s->dfts) {
+    if (t % d.every != 0) continue;
+    lx::DftParams dp;
+    std::memset(&dp, 0, sizeof dp);
+    dp.axis = d.axis; dp.index = d.index; dp.na = d.na; dp.nb = d.nb; dp.Ny = s->Ny; dp.Nzp = s->Nzp;
+    dp.nfreq = d.nfreq; dp.t_at = b->d_ts + id; dp.k = q; dp.dt = s->k.dt; dp.weight = (double)d.every;
+    dp.omega = d.d_omega; dp.acc = d.d_acc; dp.phase = d.d_phase; dp.hmul = 1.0 / s->hscale;
+    const bool b1 = g.sweep && ((t + 1) & 1);
+    T* f4[4];
+    for (int c = 0; c < 4; c++) {
+      const int k = d.comps[c];
+      f4[c] = (T*)(k < 3 ? (b1 ? s->E1[k] : s->E[k]) : (b1 ? s->H1[k - 3] : s->H[k - 3]));
+      for (int a = 0; a < 3; a++) dp.ext[c][a] = s->ext[k][a];
+    }
+    BCK(lx::launch_dft<T>(dp, f4, st));
+  }
+  return LX_OK;
+}
+
 template <class T, class C>
 static lx_status batch_enqueue(lx_batch* b, long long step0, int nsteps) {
   const int n = (int)b->sims.size();
-  // the members' device step counters advance once, after the chunk; step q runs at ts + q
-  for (int q = 0; q < nsteps; q++) {
-    BCK(lx::launch_prologue_batch<C>(b->d_pps, b->d_ts, q, n, b->max_entries, b->stream));
-    for (auto& g : b->groups) {
-      if (g.solo) {  // each member's H and E on one of the lanes; members are independent
-        const auto* hp = (const lx::StepParams<T, C>*)g.host_params.data();
-        const int L = std::min<int>(lx_batch::kLanes, (int)g.members.size());
-        BCK(cudaEventRecord(b->lane_ev[0], b->stream));
-        for (int l = 0; l < L - 1; l++) BCK(cudaStreamWaitEvent(b->lanes[l], b->lane_ev[0], 0));
-        for (size_t m = 0; m < g.members.size(); m++) {
-          cudaStream_t st = (m % L) ? b->lanes[m % L - 1] : b->stream;
-          if constexpr (sizeof(C) == 4) {
-            if (g.planar) {  // single sweep, state t & 1 -> (t+1) & 1
-              lx::StepParams<T, C> sw = hp[m];
-              if ((b->host_ts[g.members[m]] + q) & 1) swap_buffers(sw);
-              BCK(lx::launch_step_sweep2<T, C>(sw, g.uniform, st));
-              continue;
-            }
-          }
-          BCK(lx::launch_step<T, C>(hp[m], g.planar, g.uniform, true, st));
-          BCK(lx::launch_step<T, C>(hp[m], g.planar, g.uniform, false, st));
-        }
-        for (int l = 0; l < L - 1; l++) {
-          BCK(cudaEventRecord(b->lane_ev[1 + l], b->lanes[l]));
-          BCK(cudaStreamWaitEvent(b->stream, b->lane_ev[1 + l], 0));
-        }
-        continue;
-      }
-      BCK(lx::launch_batch_step<T, C>((const lx::StepParams<T, C>*)g.d_params, g.d_tiles, g.nblocks, g.planar,
-                                      g.uniform, g.march, true, b->stream));
+  // members launched one by one, largest first, each to the lane with the least work
+  struct Solo { const lx_batch::Group* g; size_t m; double cells; };
+  std::vector<Solo> solo;
+  bool grouped = false;
+  for (auto& g : b->groups) {
+    grouped |= !g.solo;
+    for (size_t m = 0; g.solo && m < g.members.size(); m++) {
+      const lx_sim* s = b->sims[g.members[m]];
+      solo.push_back({&g, m, (double)s->Nx * s->Ny * s->Nz});
     }
-    for (auto& g : b->groups)
-      if (!g.solo)
-        BCK(lx::launch_batch_step<T, C>((const lx::StepParams<T, C>*)g.d_params, g.d_tiles, g.nblocks, g.planar,
-                                        g.uniform, g.march, false, b->stream));
-    const long long bs = step0 + q;
-    for (auto& cl : b->dft)
-      if (bs % cl.every == cl.phase)
-        BCK(lx::launch_dft_batch<T>(cl.d_planes, cl.d_map, cl.nplanes, cl.nblocks, b->d_ts, q, b->stream));
+  }
+  std::stable_sort(solo.begin(), solo.end(), [](const Solo& x, const Solo& y) { return x.cells > y.cells; });
+  std::vector<Solo> lane[lx_batch::kLanes];  // lane 0 is the batch stream: the grouped launches' when there are any
+  double load[lx_batch::kLanes] = {};
+  const int l0 = grouped ? 1 : 0;
+  for (const Solo& x : solo) {
+    int best = l0;
+    for (int l = l0; l < lx_batch::kLanes; l++)
+      if (load[l] < load[best]) best = l;
+    lane[best].push_back(x);
+    load[best] += x.cells;
+  }
+  // The members' device step counters advance once, after the chunk; step q runs at ts + q.  The
+  // lanes meet only where a prologue forms the next rows.
+  for (int q0 = 0; q0 < nsteps; q0 += b->ahead) {
+    const int kn = std::min(b->ahead, nsteps - q0);
+    BCK(lx::launch_prologue_batch<C>(b->d_pps, b->d_ts, q0, kn, n, b->max_entries, b->d_srcv, b->d_slots, b->stream));
+    b->last_row = kn - 1;
+    const int sub = b->sources ? 1 : kn;  // steps between sources: the members' amplitudes go in together
+    for (int r0 = 0; r0 < kn; r0 += sub) {
+      if (b->sources) BCK(lx::launch_source_batch(b->d_pps, b->d_ts, q0 + r0, n, b->d_srcv + (size_t)r0 * n, b->stream));
+      bool fork = false;
+      for (int l = 1; l < lx_batch::kLanes; l++) fork |= !lane[l].empty();
+      if (fork) {
+        BCK(cudaEventRecord(b->lane_ev[0], b->stream));
+        for (int l = 1; l < lx_batch::kLanes; l++)
+          if (!lane[l].empty()) BCK(cudaStreamWaitEvent(b->lanes[l - 1], b->lane_ev[0], 0));
+      }
+      size_t deep = 0;
+      for (auto& v : lane) deep = std::max(deep, v.size());
+      // a lane takes its members in turn, each through the rows: a member's state stays in L2
+      for (size_t pos = 0; pos < deep; pos++)
+        for (int r = r0; r < r0 + sub; r++)
+          for (int l = l0; l < lx_batch::kLanes; l++)
+            if (pos < lane[l].size()) {
+              const lx_status st = solo_step<T, C>(b, *lane[l][pos].g, lane[l][pos].m, q0 + r, r,
+                                                   l ? b->lanes[l - 1] : b->stream);
+              if (st) return st;
+            }
+      for (int r = r0; grouped && r < r0 + sub; r++) {
+        const long long bs = step0 + q0 + r;
+        for (int half = 0; half < 2; half++)
+          for (auto& g : b->groups) {
+            if (g.solo) continue;
+            const auto* ps = (const lx::StepParams<T, C>*)g.d_params;
+            if constexpr (sizeof(C) == 4) {
+              if (g.sweep) {
+                const auto* sw = (const lx::SweepParams<T, C>*)g.host_params.data();
+                if (half == 0)
+                  BCK(lx::launch_batch_sweep<T, C>(sw + ((bs - b->built_at) & 1) * g.members.size(), (int)g.members.size(),
+                                                   g.first.data(), g.d_tiles, g.uniform, g.march, r, b->stream));
+                continue;
+              }
+            }
+            BCK(lx::launch_batch_step<T, C>(ps, g.d_tiles, g.nblocks, g.planar, g.uniform, g.march, half == 0, r, b->stream));
+          }
+        for (auto& cl : b->dft)
+          if (bs % cl.every == cl.phase)
+            BCK(lx::launch_dft_batch<T>(cl.d_planes, cl.d_map, cl.nplanes, cl.nblocks, b->d_ts, q0 + r, b->stream));
+      }
+      for (int l = 1; l < lx_batch::kLanes; l++)
+        if (!lane[l].empty()) {
+          BCK(cudaEventRecord(b->lane_ev[l], b->lanes[l - 1]));
+          BCK(cudaStreamWaitEvent(b->stream, b->lane_ev[l], 0));
+        }
+    }
   }
   if (nsteps > 0) BCK(lx::launch_tick(b->d_ts, n, nsteps, b->stream));
   return LX_OK;
@@ -2385,6 +2539,7 @@ static lx_status batch_run_async(lx_batch* b, int nsteps) {
         b->exec_base_mod = base_mod;
       }
       BCK(cudaGraphLaunch(b->exec, b->stream));
+      b->last_row = (b->chunk - 1) % b->ahead;
       b->step += b->chunk;
       done += b->chunk;
     }
@@ -2418,7 +2573,7 @@ extern "C" LX_API lx_status lx_batch_wait(lx_batch* b) {
   if (b->pending == 0) return LX_OK;
   const int n = (int)b->sims.size();
   std::vector<unsigned long long> slots(n);
-  if (n) BCK(cudaMemcpyAsync(slots.data(), b->d_slots, sizeof(unsigned long long) * n, cudaMemcpyDeviceToHost, b->stream));
+  if (n) BCK(cudaMemcpyAsync(slots.data(), b->d_slots + (size_t)b->last_row * n, sizeof(unsigned long long) * n, cudaMemcpyDeviceToHost, b->stream));
   BCK(cudaStreamSynchronize(b->stream));
   b->pending = 0;
   std::string bad;
@@ -2447,6 +2602,7 @@ extern "C" LX_API lx_status lx_batch_set_march(lx_batch* b, int planar_rows, int
   if (st) return st;
   b->march2d = planar_rows;
   b->march3d = planes_3d;
+  b->march_set = true;
   b->dirty = true;
   if (b->exec) cudaGraphExecDestroy(b->exec);
   b->exec = nullptr;

@@ -79,7 +79,7 @@ struct Fp<double> {
 // Adds the increments of the planes of `ps` that cell (i,j,k) lies on to d (reference:
 // curl = curl +/- exp(...) * dir / d..., one line of plane_wave_execute per plane).
 template <class C>
-__device__ __forceinline__ void tfsf_apply(const PatchSet& ps, const C* tab, int i, int j, int k, C& d) {
+__device__ __forceinline__ void tfsf_apply(const PlaneSet& ps, const C* tab, int i, int j, int k, C& d) {
   if (!ps.active) return;
   const int a = ps.axis;
   const int n = a == 0 ? i : (a == 1 ? j : k);

@@ -55,15 +55,17 @@ __host__ __device__ inline int slab_index(const Slab& s, int u) {
 // One TF/SF correction set: the two planes (low and high face of the total-field box)
 // that feed one curl part of one component, with the in-plane index ranges of the
 // reference loops (maxwell.cc:512-812) and the layout of its incident-value table.
-struct PatchSet {
+struct PlaneSet {  // what the update kernels read of it
   int active;
   int axis;        // normal axis of the planes (0 = x, 1 = y, 2 = z)
   int plane[2];    // cell index along `axis` of the low and high plane
   int lo[3], hi[3];  // inclusive in-plane ranges (entry `axis` unused)
-  int n[3];        // table extent per axis (1 on `axis` and on axes the wave does not vary along)
   int stride[3];   // table stride per axis (0 on collapsed axes)
   int tab;         // offset of the low plane's table in the table buffer
   int plane_len;   // entries per plane table (high plane at tab + plane_len)
+};
+struct PatchSet : PlaneSet {
+  int n[3];        // table extent per axis (1 on `axis` and on axes the wave does not vary along)
   // incident-value expression of the table entries
   double pos_n[2];   // wave position along `axis` of each plane (e.g. p1, p2, p1-0.5, p2+0.5)
   double off[3];     // in-plane position offsets (0 or 0.5)
@@ -97,7 +99,6 @@ struct PrologueParams {
   int src_amp_i, src_omega_i;
   double src_amp, src_omega, src_t0, src_tw;
   int prec;           // storage precision of src_field
-  unsigned long long* max_slot;  // reset to 0 when non-null
 };
 
 // Device pointers and constants of one 3-D or planar simulation, passed by value.
@@ -125,11 +126,14 @@ struct StepParams {
   int tfsf;
   int planesH[3][2];     // per axis, the planes any H-update set uses (-2 when none): block skip test
   int planesE[3][2];
-  PatchSet setsH[3][2];  // [component][part]
-  PatchSet setsE[3][2];
+  PlaneSet setsH[3][2];  // [component][part]
+  PlaneSet setsE[3][2];
   const C* tab;
   // monitor / |E|^2 snapshot (E kernel)
   unsigned long long* max_slot;  // atomicMax of the bit pattern of max|E|^2 (non-negative)
+  // Batched members: tab and max_slot are those of a sequence's first step, these the distances to
+  // the next step's.
+  int tab_stride, slot_stride;
   C* etotal;                     // when non-null, |E|^2 into the Ez-shaped array (3D)
   // Second copy of the state, held by planar float-compute handles (null for the others; the
   // in-place kernels ignore it).  For the single-sweep kernel, E, H, psiH, psiE name the copy
@@ -143,6 +147,33 @@ struct StepParams {
   int zends;
   // Set to nonzero by a kernel whose bounded wait for staged data ran out (null: not reported).
   unsigned* fault;
+};
+
+// What the planar sweep reads of a simulation: the buffers of one step's parity.
+template <class T, class C>
+struct SweepParams {
+  const T *ey, *hx, *hz;  // state n
+  T *ey1, *hx1, *hz1;     // state n + 1
+  const C* cb;
+  const C *qhx, *qhz, *qez, *qex;  // psi of Hx (z part), Hz (x part), Ey (z and x parts)
+  C *qhx1, *qhz1, *qez1, *qex1;
+  const C *bHx, *cHx, *rHx, *bHz, *cHz, *rHz;  // profiles along x and z
+  const C *bEx, *cEx, *rEx, *bEz, *cEz, *rEz;
+  const C* tab;
+  unsigned long long* max_slot;
+  int Nx, Nz, si;  // si: the row stride (Nzp)
+  int pml, tfsf;
+  Slab slab[3];
+  C Dbs, rd[3];
+  int tab_stride, slot_stride;
+  int planesH[3][2], planesE[3][2];
+  PlaneSet setHx, setHz, setEz, setEx;  // Hx z part, Hz x part, Ey z and x parts
+};
+// Members of one batched sweep launch: as many as the parameter space of a launch takes.
+constexpr int kSweepMembers = 48;
+template <class T, class C>
+struct SweepBatch {
+  SweepParams<T, C> m[kSweepMembers];
 };
 
 // Whether a block's tile [i0,i0+ni) x [j0,j0+nj) x [k0,k0+nk) meets any TF/SF plane of the
@@ -187,7 +218,7 @@ struct ProbeParams {
 // One DFT plane monitor (see lx_sim_add_dft_plane).
 struct DftParams {
   int axis, index, na, nb, Ny, Nzp, nfreq, t;
-  const StepCtl* ctl;     // single launches: when non-null, the step is ctl->t + k
+  const int* t_at;        // single launches: when non-null, the step is *t_at + k
   int k;
   int sim;                // batched launches: index of the simulation's step counter
   const void* f[4];       // batched launches: the four sampled components

@@ -20,6 +20,7 @@
 
 #include <cstdlib>
 #include <cstring>
+#include <vector>
 
 #include "lx_device.cuh"
 #include "lx_internal.h"
@@ -161,24 +162,31 @@ __global__ void finish_kernel(const unsigned long long* ring, unsigned mask, uns
 
 __global__ void set_ctl_kernel(StepCtl* ctl, const StepCtl v) { *ctl = v; }
 
-// Batched prologue: blockIdx.y selects the simulation.  Its step counter lives on the device
-// and advances once per chunk, so that a captured chunk can be replayed: step k of a chunk
-// runs at ts[sim] + k.
+// Batched: blockIdx.y selects the simulation, blockIdx.z the step of the sequence.  A simulation's
+// step counter lives on the device and advances once per chunk, so that a captured chunk can be
+// replayed: step k of a chunk runs at ts[sim] + k.
 template <class C>
-__global__ void prologue_batch_kernel(const PrologueParams* __restrict__ pps, const int* __restrict__ ts, int k) {
+__global__ void prologue_batch_kernel(const PrologueParams* __restrict__ pps, const int* __restrict__ ts, int k,
+                                      double* srcv, unsigned long long* slots) {
   const PrologueParams& p = pps[blockIdx.y];
-  const int t = ts[blockIdx.y] + k, gid = blockIdx.x * blockDim.x + threadIdx.x;
+  const int q = blockIdx.z, t = ts[blockIdx.y] + k + q, gid = blockIdx.x * blockDim.x + threadIdx.x;
   if (gid == 0) {
-    if (p.max_slot) *p.max_slot = 0ull;
-    void* const f = ((t & 1) && p.src_field1) ? p.src_field1 : p.src_field;  // the state step t reads
-    if (p.src_kind >= 0) {
-      const double v = source_value(p, t);
-      if (p.prec == 0) source_apply((double*)f + p.src_idx, p.src_kind, v);
-      else if (p.prec == 1) source_apply((float*)f + p.src_idx, p.src_kind, v);
-      else source_apply((__half*)f + p.src_idx, p.src_kind, v);
-    }
+    slots[q * gridDim.y + blockIdx.y] = 0ull;
+    if (p.src_kind >= 0) srcv[q * gridDim.y + blockIdx.y] = source_value(p, t);
   }
-  tables_body<C>(p, t, (C*)p.tab, gid, gridDim.x * blockDim.x);
+  tables_body<C>(p, t, (C*)p.tab + (long long)q * p.tab_total, gid, gridDim.x * blockDim.x);
+}
+
+__global__ void source_batch_kernel(const PrologueParams* __restrict__ pps, const int* __restrict__ ts, int k, int nsims,
+                                    const double* __restrict__ v) {
+  const int s = blockIdx.x * blockDim.x + threadIdx.x;
+  if (s >= nsims) return;
+  const PrologueParams& p = pps[s];
+  if (p.src_kind < 0) return;
+  void* const f = (((ts[s] + k) & 1) && p.src_field1) ? p.src_field1 : p.src_field;  // the state the step reads
+  if (p.prec == 0) source_apply((double*)f + p.src_idx, p.src_kind, v[s]);
+  else if (p.prec == 1) source_apply((float*)f + p.src_idx, p.src_kind, v[s]);
+  else source_apply((__half*)f + p.src_idx, p.src_kind, v[s]);
 }
 
 __global__ void tick_kernel(int* ts, int n, int steps) {
@@ -840,20 +848,14 @@ struct Row2 {
 
 // One warp's rows [i0, i1) of the 32 columns from k0; returns the bit pattern of its largest
 // Ey^2 (the max over the whole Ey array, two_dim_pml.cc:181).
-// The parameter block names the buffer read in E, H, psiH, psiE and the one written in E1,
-// H1, psiH1, psiE1 (the host swaps them on odd steps).
 template <class T, class C, bool UNI, bool FAST>
-__device__ __forceinline__ typename MaxBits<C>::type step2_rows(const StepParams<T, C>& p, const int i0, const int i1,
-                                                                const int k0, const bool tfH, const bool tfE) {
+__device__ __forceinline__ typename MaxBits<C>::type step2_rows(const SweepParams<T, C>& p, const int i0, const int i1,
+                                                                const int k0, const bool tfH, const bool tfE,
+                                                                const C* tab) {
   const int lane = threadIdx.x;
   const int k = k0 + lane;
   const int Nx = p.Nx, Nz = p.Nz;
-  const T* eyi = p.E[1];
-  T* eyo = p.E1[1];
-  const T* hxi = p.H[0];
-  T* hxo = p.H1[0];
-  const T* hzi = p.H[2];
-  T* hzo = p.H1[2];
+  const T *eyi = p.ey, *hxi = p.hx, *hzi = p.hz;
   const bool kin = FAST || k < Nz;
   const bool ux = FAST || k < Nz - 1;
   const bool ke = FAST || (k >= 1 && k < Nz - 1);
@@ -865,9 +867,9 @@ __device__ __forceinline__ typename MaxBits<C>::type step2_rows(const StepParams
   const int sz = pml ? slab_index(p.slab[2], k) : -1;
   const int szh = pml && halo ? slab_index(p.slab[2], k0 - 1) : -1;
   C bHz = C(0), cHz = C(0), rHz = C(0), bEz = C(0), cEz = C(0), rEz = C(0), bHh = C(0), cHh = C(0), rHh = C(0);
-  if (sz >= 0 && ux) { bHz = __ldg(p.bH[2] + k); cHz = __ldg(p.cH[2] + k); rHz = __ldg(p.rkH[2] + k); }
-  if (sz >= 0 && kin) { bEz = __ldg(p.bE[2] + k); cEz = __ldg(p.cE[2] + k); rEz = __ldg(p.rkE[2] + k); }
-  if (szh >= 0) { bHh = __ldg(p.bH[2] + k0 - 1); cHh = __ldg(p.cH[2] + k0 - 1); rHh = __ldg(p.rkH[2] + k0 - 1); }
+  if (sz >= 0 && ux) { bHz = __ldg(p.bHz + k); cHz = __ldg(p.cHz + k); rHz = __ldg(p.rHz + k); }
+  if (sz >= 0 && kin) { bEz = __ldg(p.bEz + k); cEz = __ldg(p.cEz + k); rEz = __ldg(p.rEz + k); }
+  if (szh >= 0) { bHh = __ldg(p.bHz + k0 - 1); cHh = __ldg(p.cHz + k0 - 1); rHh = __ldg(p.rHz + k0 - 1); }
 
   auto load = [&](int i, long long c, Row2<C>& r) {
     const bool nx = FAST || i + 1 < Nx;
@@ -875,7 +877,7 @@ __device__ __forceinline__ typename MaxBits<C>::type step2_rows(const StepParams
     r.ey_i = (kin && nx) ? ld<T, C>(eyi + c + si) : C(0);
     r.hx = kin ? ld<T, C>(hxi + c) : C(0);
     r.hz = kin ? ld<T, C>(hzi + c) : C(0);
-    r.cb = (kin && ue) ? p.Cbs[1][c] : C(0);
+    r.cb = (kin && ue) ? p.cb[c] : C(0);
     r.ey_k = r.hxh = r.eyh = C(0);
     if (lane == 31 && (FAST || k + 1 < Nz)) r.ey_k = ld<T, C>(eyi + c + 1);
     if (halo) {
@@ -886,11 +888,11 @@ __device__ __forceinline__ typename MaxBits<C>::type step2_rows(const StepParams
       r.phx = r.pez = r.phxh = r.phz = r.pex = C(0);
       if (pml) {
         const int sx = slab_index(p.slab[0], i);
-        if (sz >= 0 && ux) r.phx = p.psiH[0][1][(long long)i * zn + sz];
-        if (sz >= 0 && ue) r.pez = p.psiE[1][0][(long long)i * zn + sz];
-        if (szh >= 0) r.phxh = p.psiH[0][1][(long long)i * zn + szh];
-        if (sx >= 0 && kin && nx) r.phz = p.psiH[2][0][(long long)sx * p.Nzp + k];
-        if (sx >= 0 && kin && ue) r.pex = p.psiE[1][1][(long long)sx * p.Nzp + k];
+        if (sz >= 0 && ux) r.phx = p.qhx[(long long)i * zn + sz];
+        if (sz >= 0 && ue) r.pez = p.qez[(long long)i * zn + sz];
+        if (szh >= 0) r.phxh = p.qhx[(long long)i * zn + szh];
+        if (sx >= 0 && kin && nx) r.phz = p.qhz[(long long)sx * si + k];
+        if (sx >= 0 && kin && ue) r.pex = p.qex[(long long)sx * si + k];
       }
     }
   };
@@ -898,8 +900,8 @@ __device__ __forceinline__ typename MaxBits<C>::type step2_rows(const StepParams
   auto hz_value = [&](int i, int sx, C ey, C ey_i, C hz, C& psi) -> C {
     C d1 = ey_i - ey;
     if (!UNI) d1 = mulC(d1, p.rd[0]);
-    if (!FAST && tfH) tfsf_apply<C>(p.setsH[2][0], p.tab, i, 0, k, d1);
-    if (!FAST && sx >= 0) psi2_term(__ldg(p.bH[0] + i), __ldg(p.cH[0] + i), __ldg(p.rkH[0] + i), psi, d1);
+    if (!FAST && tfH) tfsf_apply<C>(p.setHz, tab, i, 0, k, d1);
+    if (!FAST && sx >= 0) psi2_term(__ldg(p.bHx + i), __ldg(p.cHx + i), __ldg(p.rHx + i), psi, d1);
     return stored<T, C>(fmaC(-p.Dbs, d1, hz));
   };
 
@@ -912,7 +914,7 @@ __device__ __forceinline__ typename MaxBits<C>::type step2_rows(const StepParams
     const C eym = kin ? ld<T, C>(eyi + c - si) : C(0);
     const C hzm = kin ? ld<T, C>(hzi + c - si) : C(0);
     const int sx = pml ? slab_index(p.slab[0], i0 - 1) : -1;
-    C psi = (!FAST && sx >= 0 && kin) ? p.psiH[2][0][(long long)sx * p.Nzp + k] : C(0);  // its owner stores the new psi
+    C psi = (!FAST && sx >= 0 && kin) ? p.qhz[(long long)sx * si + k] : C(0);  // its owner stores the new psi
     hz_p = hz_value(i0 - 1, sx, eym, ey, hzm, psi);
   }
   typename MaxBits<C>::type m = 0;
@@ -930,7 +932,7 @@ __device__ __forceinline__ typename MaxBits<C>::type step2_rows(const StepParams
     if (kin && ux) {
       C d2 = ey_k - ey;
       if (!UNI) d2 = mulC(d2, p.rd[2]);
-      if (!FAST && tfH) tfsf_apply<C>(p.setsH[0][1], p.tab, i, 0, k, d2);
+      if (!FAST && tfH) tfsf_apply<C>(p.setHx, tab, i, 0, k, d2);
       if (!FAST && sz >= 0) psi2_term(bHz, cHz, rHz, cur.phx, d2);
       hxn = stored<T, C>(fmaC(p.Dbs, d2, cur.hx));
     }
@@ -941,7 +943,7 @@ __device__ __forceinline__ typename MaxBits<C>::type step2_rows(const StepParams
       if (halo) {  // new Hx of column k0-1, recomputed; its owner stores the new psi
         C d2 = ey - cur.eyh;
         if (!UNI) d2 = mulC(d2, p.rd[2]);
-        if (!FAST && tfH) tfsf_apply<C>(p.setsH[0][1], p.tab, i, 0, k0 - 1, d2);
+        if (!FAST && tfH) tfsf_apply<C>(p.setHx, tab, i, 0, k0 - 1, d2);
         if (!FAST && szh >= 0) psi2_term(bHh, cHh, rHh, cur.phxh, d2);
         hx_k = stored<T, C>(fmaC(p.Dbs, d2, cur.hxh));
       }
@@ -953,24 +955,24 @@ __device__ __forceinline__ typename MaxBits<C>::type step2_rows(const StepParams
       C d2 = hzn - hz_p;  // dHz/dx (x profile)
       if (!UNI) { d1 = mulC(d1, p.rd[2]); d2 = mulC(d2, p.rd[0]); }
       if (!FAST && tfE) {
-        tfsf_apply<C>(p.setsE[1][0], p.tab, i, 0, k, d1);
-        tfsf_apply<C>(p.setsE[1][1], p.tab, i, 0, k, d2);
+        tfsf_apply<C>(p.setEz, tab, i, 0, k, d1);
+        tfsf_apply<C>(p.setEx, tab, i, 0, k, d2);
       }
       if (!FAST) {
         if (sz >= 0) psi2_term(bEz, cEz, rEz, cur.pez, d1);
-        if (sx >= 0) psi2_term(__ldg(p.bE[0] + i), __ldg(p.cE[0] + i), __ldg(p.rkE[0] + i), cur.pex, d2);
+        if (sx >= 0) psi2_term(__ldg(p.bEx + i), __ldg(p.cEx + i), __ldg(p.rEx + i), cur.pex, d2);
       }
       eyw = fmaC(cur.cb, d1 - d2, ey);
     }
     if (kin) {
-      st<T, C>(hxo + c, hxn);
-      st<T, C>(hzo + c, hzn);
-      st<T, C>(eyo + c, eyw);
+      st<T, C>(p.hx1 + c, hxn);
+      st<T, C>(p.hz1 + c, hzn);
+      st<T, C>(p.ey1 + c, eyw);
       if (!FAST) {
-        if (sz >= 0 && ux) p.psiH1[0][1][(long long)i * zn + sz] = cur.phx;
-        if (sz >= 0 && ue) p.psiE1[1][0][(long long)i * zn + sz] = cur.pez;
-        if (sx >= 0 && nx) p.psiH1[2][0][(long long)sx * p.Nzp + k] = cur.phz;
-        if (sx >= 0 && ue) p.psiE1[1][1][(long long)sx * p.Nzp + k] = cur.pex;
+        if (sz >= 0 && ux) p.qhx1[(long long)i * zn + sz] = cur.phx;
+        if (sz >= 0 && ue) p.qez1[(long long)i * zn + sz] = cur.pez;
+        if (sx >= 0 && nx) p.qhz1[(long long)sx * si + k] = cur.phz;
+        if (sx >= 0 && ue) p.qex1[(long long)sx * si + k] = cur.pex;
       }
       const typename MaxBits<C>::type b = MaxBits<C>::of(eyw * eyw);
       m = b > m ? b : m;
@@ -985,13 +987,13 @@ __device__ __forceinline__ typename MaxBits<C>::type step2_rows(const StepParams
 // A warp's run with its TF/SF and interior tests: H is formed on rows [i0-1, i1) and columns
 // [k0-1, k0+32), E on rows [i0, i1) and columns [k0, k0+32).
 template <class T, class C, bool UNI>
-__device__ __forceinline__ typename MaxBits<C>::type step2_warp(const StepParams<T, C>& p, const int i0, const int i1,
-                                                                const int k0) {
+__device__ __forceinline__ typename MaxBits<C>::type step2_warp(const SweepParams<T, C>& p, const int i0, const int i1,
+                                                                const int k0, const C* tab) {
   const bool tfH = p.tfsf && tile_meets_planes(p.planesH, i0 - 1, i1 - i0 + 1, 0, 1, k0 - 1, 34);
   const bool tfE = p.tfsf && tile_meets_planes(p.planesE, i0, i1 - i0, 0, 1, k0, 32);
   if (!tfH && !tfE && tile_is_interior_2d(p.slab, p.pml, p.Nx, p.Nz, i0 - 1, i1 - i0 + 2, k0 - 1, 34))
-    return step2_rows<T, C, UNI, true>(p, i0, i1, k0, false, false);
-  return step2_rows<T, C, UNI, false>(p, i0, i1, k0, tfH, tfE);
+    return step2_rows<T, C, UNI, true>(p, i0, i1, k0, false, false, tab);
+  return step2_rows<T, C, UNI, false>(p, i0, i1, k0, tfH, tfE, tab);
 }
 
 // Register cap of the single-sweep kernel: 5 blocks of 256 per SM (48 registers; the general path
@@ -1001,15 +1003,59 @@ constexpr int kSweepMinBlocks = 5;
 
 // One simulation: a block is 32 z columns x 8 warps of R rows.
 template <class T, class C, bool UNI>
-__global__ void __launch_bounds__(256, kSweepMinBlocks) step_kernel_2d(const StepParams<T, C> p, const int R) {
+__global__ void __launch_bounds__(256, kSweepMinBlocks) step_kernel_2d(const SweepParams<T, C> p, const int R) {
   const int k0 = blockIdx.x * 32;
   const int i0 = (blockIdx.y * 8 + threadIdx.y) * R;
   typename MaxBits<C>::type m = 0;
-  if (i0 < p.Nx) m = step2_warp<T, C, UNI>(p, i0, min(i0 + R, p.Nx), k0);
+  if (i0 < p.Nx) m = step2_warp<T, C, UNI>(p, i0, min(i0 + R, p.Nx), k0, p.tab);
   if (p.max_slot) block_max_atomic(m, p.max_slot);
 }
 
+// Members of a batch: a block is 32 z columns x 8 warps of R rows of one member, `row` the step's
+// place in its sequence.  The members' blocks come by value in the launch's parameters, and a
+// block finds its member, tile and path (interior: every warp's run) in one 16-byte entry.  At 4
+// blocks per SM (64 registers: the pointers of a member that only the entry names take a pair
+// each) 48 lenses of side 128-1024 take 142 us a step, at 5 with spills 158; parameters copied to
+// shared memory took 168, and the half-step kernels h_batch_2d and e_batch_2d, which move 40
+// bytes a cell where this moves 28, 166.
+template <class T, class C, bool UNI>
+__global__ void __launch_bounds__(256, 4) step_batch_2d(const __grid_constant__ SweepBatch<T, C> b,
+                                                                       const int4* __restrict__ tiles, const int R,
+                                                                       const int row) {
+  const int4 tl = __ldg(tiles + blockIdx.x);
+  const SweepParams<T, C>& g = b.m[tl.x];
+  const int k0 = tl.w, i0 = tl.y + threadIdx.y * R;
+  if (i0 >= g.Nx) return;
+  const int i1 = min(i0 + R, g.Nx);
+  const C* tab = g.tab + (long long)row * g.tab_stride;
+  const typename MaxBits<C>::type v =
+      warp_max(tl.z ? step2_rows<T, C, UNI, true>(g, i0, i1, k0, false, false, tab) : step2_warp<T, C, UNI>(g, i0, i1, k0, tab));
+  if (threadIdx.x == 0) {  // (a warp's maximum straight to the slot: a block's warps end at different times)
+    unsigned long long* slot = g.max_slot + (long long)row * g.slot_stride;
+    const unsigned long long bits = as_slot_bits(v);
+    if (bits > *reinterpret_cast<volatile unsigned long long*>(slot)) atomicMax(slot, bits);
+  }
+}
+
 // ------------------------------------------------------------------ batched update kernels
+
+// The parameter block of a block's member, in shared memory, with the tables and the slot of step
+// `row` of the sequence.  Read through a global pointer instead, the block is held in registers
+// or loaded again behind every store.
+template <class T, class C>
+__device__ __forceinline__ void member_params(StepParams<T, C>& sp, const StepParams<T, C>* __restrict__ g, const int row) {
+  static_assert(sizeof(StepParams<T, C>) % 4 == 0, "copied in words");
+  const unsigned* src = reinterpret_cast<const unsigned*>(g);
+  unsigned* dst = reinterpret_cast<unsigned*>(&sp);
+  const int tid = threadIdx.y * blockDim.x + threadIdx.x;
+  for (int w = tid; w < (int)(sizeof(StepParams<T, C>) / 4); w += 256) dst[w] = __ldg(src + w);
+  __syncthreads();
+  if (tid == 0) {
+    sp.tab += (long long)row * sp.tab_stride;
+    sp.max_slot += (long long)row * sp.slot_stride;
+  }
+  __syncthreads();
+}
 
 __device__ __forceinline__ int find_member(const int* __restrict__ first, int n, int t) {
   int lo = 0, hi = n;  // first[lo] <= t < first[hi]
@@ -1060,9 +1106,10 @@ struct B3MinBlocks {
 
 // 3-D members: a block is 32 z x 8 y cells over M consecutive x planes.
 template <class T, class C, bool UNI, int M>
-__global__ void __launch_bounds__(256, B3MinBlocks<C>::v) h_batch_3d(const StepParams<T, C>* __restrict__ ps, const int4* __restrict__ tiles) {
+__global__ void __launch_bounds__(256, B3MinBlocks<C>::v) h_batch_3d(const StepParams<T, C>* __restrict__ ps, const int4* __restrict__ tiles, int row) {
+  __shared__ StepParams<T, C> p;
   const int4 tl = tiles[blockIdx.x];
-  const StepParams<T, C>& p = ps[tl.x];
+  member_params(p, ps + tl.x, row);
   const int k = tl.w + threadIdx.x, j = tl.z + threadIdx.y, i0 = tl.y;
   if (k >= p.Nz || j >= p.Ny) return;
   const bool tf = p.tfsf && tile_meets_planes(p.planesH, i0, M, tl.z, 8, tl.w, 32);
@@ -1077,9 +1124,10 @@ __global__ void __launch_bounds__(256, B3MinBlocks<C>::v) h_batch_3d(const StepP
 }
 
 template <class T, class C, bool UNI, int M>
-__global__ void __launch_bounds__(256, B3MinBlocks<C>::v) e_batch_3d(const StepParams<T, C>* __restrict__ ps, const int4* __restrict__ tiles) {
+__global__ void __launch_bounds__(256, B3MinBlocks<C>::v) e_batch_3d(const StepParams<T, C>* __restrict__ ps, const int4* __restrict__ tiles, int row) {
+  __shared__ StepParams<T, C> p;
   const int4 tl = tiles[blockIdx.x];
-  const StepParams<T, C>& p = ps[tl.x];
+  member_params(p, ps + tl.x, row);
   const int k = tl.w + threadIdx.x, j = tl.z + threadIdx.y, i0 = tl.y;
   const bool tf = p.tfsf && tile_meets_planes(p.planesE, i0, M, tl.z, 8, tl.w, 32);
   typename MaxBits<C>::type mbits = 0;
@@ -1109,9 +1157,10 @@ __global__ void __launch_bounds__(256, B3MinBlocks<C>::v) e_batch_3d(const StepP
 // written only by their own thread, and the rows are 8 apart); the 256-lens batch ran 103 ->
 // 111 Gcell/s.  The same in the general tiles took 46-48 registers and ran 90.
 template <class T, class C, bool UNI, int M>
-__global__ void __launch_bounds__(256) h_batch_2d(const StepParams<T, C>* __restrict__ ps, const int4* __restrict__ tiles) {
+__global__ void __launch_bounds__(256) h_batch_2d(const StepParams<T, C>* __restrict__ ps, const int4* __restrict__ tiles, int row) {
+  __shared__ StepParams<T, C> p;
   const int4 tl = tiles[blockIdx.x];
-  const StepParams<T, C>& p = ps[tl.x];
+  member_params(p, ps + tl.x, row);
   const int k = tl.w + threadIdx.x;
   if (k >= p.Nz) return;
   const bool tf = p.tfsf && tile_meets_planes(p.planesH, tl.y, 8 * M, 0, 1, tl.w, 32);
@@ -1142,9 +1191,10 @@ struct E2BatchMinBlocks {
   static constexpr int v = sizeof(C) == 4 ? 8 : 1;
 };
 template <class T, class C, bool UNI, int M>
-__global__ void __launch_bounds__(256, E2BatchMinBlocks<C>::v) e_batch_2d(const StepParams<T, C>* __restrict__ ps, const int4* __restrict__ tiles) {
+__global__ void __launch_bounds__(256, E2BatchMinBlocks<C>::v) e_batch_2d(const StepParams<T, C>* __restrict__ ps, const int4* __restrict__ tiles, int row) {
+  __shared__ StepParams<T, C> p;
   const int4 tl = tiles[blockIdx.x];
-  const StepParams<T, C>& p = ps[tl.x];
+  member_params(p, ps + tl.x, row);
   const int k = tl.w + threadIdx.x;
   const bool tf = p.tfsf && tile_meets_planes(p.planesE, tl.y, 8 * M, 0, 1, tl.w, 32);
   const bool fast = !tf && tile_is_interior_2d(p.slab, p.pml, p.Nx, p.Nz, tl.y, 8 * M, tl.w, 32);
@@ -1284,7 +1334,7 @@ __device__ __forceinline__ void dft_phase_body(const DftParams& d, const int t) 
   }
 }
 
-__global__ void dft_phase_kernel(const DftParams d) { dft_phase_body(d, d.ctl ? d.ctl->t + d.k : d.t); }
+__global__ void dft_phase_kernel(const DftParams d) { dft_phase_body(d, d.t_at ? *d.t_at + d.k : d.t); }
 
 // Batched: one block per plane of a sampling class.
 __global__ void dft_phase_batch_kernel(const DftParams* __restrict__ ds, const int* __restrict__ ts, int k) {
@@ -1518,13 +1568,81 @@ static int sweep_rows(long long cols, int Nx) {
 }
 
 template <class T, class C>
+SweepParams<T, C> sweep_params(const StepParams<T, C>& p) {
+  SweepParams<T, C> q;
+  std::memset(&q, 0, sizeof q);
+  q.ey = p.E[1]; q.hx = p.H[0]; q.hz = p.H[2];
+  q.ey1 = p.E1[1]; q.hx1 = p.H1[0]; q.hz1 = p.H1[2];
+  q.cb = p.Cbs[1];
+  q.qhx = p.psiH[0][1]; q.qhz = p.psiH[2][0]; q.qez = p.psiE[1][0]; q.qex = p.psiE[1][1];
+  q.qhx1 = p.psiH1[0][1]; q.qhz1 = p.psiH1[2][0]; q.qez1 = p.psiE1[1][0]; q.qex1 = p.psiE1[1][1];
+  q.bHx = p.bH[0]; q.cHx = p.cH[0]; q.rHx = p.rkH[0]; q.bHz = p.bH[2]; q.cHz = p.cH[2]; q.rHz = p.rkH[2];
+  q.bEx = p.bE[0]; q.cEx = p.cE[0]; q.rEx = p.rkE[0]; q.bEz = p.bE[2]; q.cEz = p.cE[2]; q.rEz = p.rkE[2];
+  q.tab = p.tab;
+  q.max_slot = p.max_slot;
+  q.Nx = p.Nx; q.Nz = p.Nz; q.si = p.Nzp;
+  q.pml = p.pml; q.tfsf = p.tfsf;
+  q.Dbs = p.Dbs;
+  q.tab_stride = p.tab_stride; q.slot_stride = p.slot_stride;
+  for (int a = 0; a < 3; ++a) {
+    q.slab[a] = p.slab[a];
+    q.rd[a] = p.rd[a];
+    for (int e = 0; e < 2; ++e) {
+      q.planesH[a][e] = p.planesH[a][e];
+      q.planesE[a][e] = p.planesE[a][e];
+    }
+  }
+  q.setHx = p.setsH[0][1]; q.setHz = p.setsH[2][0]; q.setEz = p.setsE[1][0]; q.setEx = p.setsE[1][1];
+  return q;
+}
+
+template <class T, class C>
 cudaError_t launch_step_sweep2(const StepParams<T, C>& p, bool uniform, cudaStream_t s) {
   const long long cols = (p.Nz + 31) / 32;
   const int R = sweep_rows(cols, p.Nx);
   const dim3 block(32, 8), grid((unsigned)cols, (unsigned)((p.Nx + 8 * R - 1) / (8 * R)));
-  if (uniform) step_kernel_2d<T, C, true><<<grid, block, 0, s>>>(p, R);
-  else step_kernel_2d<T, C, false><<<grid, block, 0, s>>>(p, R);
+  const SweepParams<T, C> q = sweep_params(p);
+  if (uniform) step_kernel_2d<T, C, true><<<grid, block, 0, s>>>(q, R);
+  else step_kernel_2d<T, C, false><<<grid, block, 0, s>>>(q, R);
   return cudaGetLastError();
+}
+
+template <class T, class C>
+cudaError_t launch_batch_sweep(const SweepParams<T, C>* m, int n, const int* first, const int4* tiles, bool uniform, int R,
+                               int row, cudaStream_t s) {
+  SweepBatch<T, C> b;
+  static_assert(sizeof(b) + 16 <= 32764, "a launch's parameter space");
+  const dim3 block(32, 8);
+  for (int at = 0; at < n; at += kSweepMembers) {
+    const int k = n - at < kSweepMembers ? n - at : kSweepMembers;
+    std::memcpy(b.m, m + at, k * sizeof(SweepParams<T, C>));
+    const int nb = first[at + k] - first[at];
+    if (uniform) step_batch_2d<T, C, true><<<nb, block, 0, s>>>(b, tiles + first[at], R, row);
+    else step_batch_2d<T, C, false><<<nb, block, 0, s>>>(b, tiles + first[at], R, row);
+    const cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+  }
+  return cudaSuccess;
+}
+
+// {member of its launch, first row, interior, first column} of each block of the members' sweeps.
+template <class T, class C>
+void sweep_tiles(const SweepParams<T, C>* m, int n, int R, std::vector<int>& first, std::vector<int4>& tiles) {
+  first.assign(1, 0);
+  tiles.clear();
+  for (int q = 0; q < n; ++q) {
+    const SweepParams<T, C>& p = m[q];
+    for (int i = 0; i < p.Nx; i += 8 * R)
+      for (int k = 0; k < p.Nz; k += 32) {
+        // as step2_warp decides for each of the block's runs
+        const int i1 = i + 8 * R;
+        const bool tf = p.tfsf && (tile_meets_planes(p.planesH, i - 1, i1 - i + 1, 0, 1, k - 1, 34) ||
+                                   tile_meets_planes(p.planesE, i, i1 - i, 0, 1, k, 32));
+        const bool in = !tf && tile_is_interior_2d(p.slab, p.pml, p.Nx, p.Nz, i - 1, i1 - i + 2, k - 1, 34);
+        tiles.push_back(make_int4(q % kSweepMembers, i, in ? 1 : 0, k));
+      }
+    first.push_back((int)tiles.size());
+  }
 }
 
 template <class T>
@@ -1580,36 +1698,36 @@ cudaError_t launch_batch_tiles(const StepParams<T, C>* ps, const int* first, int
 
 template <class T, class C, int M>
 static void batch_step_m(const StepParams<T, C>* ps, const int4* tiles, int nblocks, bool planar, bool uniform,
-                         bool h_half, cudaStream_t s) {
+                         bool h_half, int row, cudaStream_t s) {
   dim3 block(32, 8);
   if (planar) {
     if (h_half) {
-      if (uniform) h_batch_2d<T, C, true, M><<<nblocks, block, 0, s>>>(ps, tiles);
-      else h_batch_2d<T, C, false, M><<<nblocks, block, 0, s>>>(ps, tiles);
+      if (uniform) h_batch_2d<T, C, true, M><<<nblocks, block, 0, s>>>(ps, tiles, row);
+      else h_batch_2d<T, C, false, M><<<nblocks, block, 0, s>>>(ps, tiles, row);
     } else {
-      if (uniform) e_batch_2d<T, C, true, M><<<nblocks, block, 0, s>>>(ps, tiles);
-      else e_batch_2d<T, C, false, M><<<nblocks, block, 0, s>>>(ps, tiles);
+      if (uniform) e_batch_2d<T, C, true, M><<<nblocks, block, 0, s>>>(ps, tiles, row);
+      else e_batch_2d<T, C, false, M><<<nblocks, block, 0, s>>>(ps, tiles, row);
     }
   } else {
     if (h_half) {
-      if (uniform) h_batch_3d<T, C, true, M><<<nblocks, block, 0, s>>>(ps, tiles);
-      else h_batch_3d<T, C, false, M><<<nblocks, block, 0, s>>>(ps, tiles);
+      if (uniform) h_batch_3d<T, C, true, M><<<nblocks, block, 0, s>>>(ps, tiles, row);
+      else h_batch_3d<T, C, false, M><<<nblocks, block, 0, s>>>(ps, tiles, row);
     } else {
-      if (uniform) e_batch_3d<T, C, true, M><<<nblocks, block, 0, s>>>(ps, tiles);
-      else e_batch_3d<T, C, false, M><<<nblocks, block, 0, s>>>(ps, tiles);
+      if (uniform) e_batch_3d<T, C, true, M><<<nblocks, block, 0, s>>>(ps, tiles, row);
+      else e_batch_3d<T, C, false, M><<<nblocks, block, 0, s>>>(ps, tiles, row);
     }
   }
 }
 
 template <class T, class C>
 cudaError_t launch_batch_step(const StepParams<T, C>* ps, const int4* tiles, int nblocks, bool planar, bool uniform,
-                              int march, bool h_half, cudaStream_t s) {
+                              int march, bool h_half, int row, cudaStream_t s) {
   if (nblocks <= 0) return cudaSuccess;
   switch (march) {
-    case 1: batch_step_m<T, C, 1>(ps, tiles, nblocks, planar, uniform, h_half, s); break;
-    case 2: batch_step_m<T, C, 2>(ps, tiles, nblocks, planar, uniform, h_half, s); break;
-    case 4: batch_step_m<T, C, 4>(ps, tiles, nblocks, planar, uniform, h_half, s); break;
-    case 8: batch_step_m<T, C, 8>(ps, tiles, nblocks, planar, uniform, h_half, s); break;
+    case 1: batch_step_m<T, C, 1>(ps, tiles, nblocks, planar, uniform, h_half, row, s); break;
+    case 2: batch_step_m<T, C, 2>(ps, tiles, nblocks, planar, uniform, h_half, row, s); break;
+    case 4: batch_step_m<T, C, 4>(ps, tiles, nblocks, planar, uniform, h_half, row, s); break;
+    case 8: batch_step_m<T, C, 8>(ps, tiles, nblocks, planar, uniform, h_half, row, s); break;
     default: return cudaErrorInvalidValue;
   }
   return cudaGetLastError();
@@ -1627,13 +1745,19 @@ cudaError_t launch_block_map(const int* first, int n, int nblocks, int2* map, cu
 }
 
 template <class C>
-cudaError_t launch_prologue_batch(const PrologueParams* pps, const int* ts, int k, int nsims, int max_entries,
-                                  cudaStream_t s) {
-  if (nsims <= 0) return cudaSuccess;
+cudaError_t launch_prologue_batch(const PrologueParams* pps, const int* ts, int k, int steps, int nsims, int max_entries,
+                                  double* srcv, unsigned long long* slots, cudaStream_t s) {
+  if (nsims <= 0 || steps <= 0) return cudaSuccess;
   long long gx = (max_entries + 255) / 256;
   if (gx < 1) gx = 1;
   if (gx > 1024) gx = 1024;
-  prologue_batch_kernel<C><<<dim3((unsigned)gx, (unsigned)nsims), 256, 0, s>>>(pps, ts, k);
+  prologue_batch_kernel<C><<<dim3((unsigned)gx, (unsigned)nsims, (unsigned)steps), 256, 0, s>>>(pps, ts, k, srcv, slots);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_source_batch(const PrologueParams* pps, const int* ts, int k, int nsims, const double* v, cudaStream_t s) {
+  if (nsims <= 0) return cudaSuccess;
+  source_batch_kernel<<<(nsims + 127) / 128, 128, 0, s>>>(pps, ts, k, nsims, v);
   return cudaGetLastError();
 }
 
@@ -1670,7 +1794,7 @@ cudaError_t launch_dft_flux(const double* acc, int nfreq, long long ncell, doubl
   template cudaError_t launch_dft<T>(const DftParams&, T* const[4], cudaStream_t);                                 \
   template cudaError_t launch_batch_tiles<T, C>(const StepParams<T, C>*, const int*, int, int, bool, int, int4*,    \
                                                 cudaStream_t);                                                     \
-  template cudaError_t launch_batch_step<T, C>(const StepParams<T, C>*, const int4*, int, bool, bool, int, bool,     \
+  template cudaError_t launch_batch_step<T, C>(const StepParams<T, C>*, const int4*, int, bool, bool, int, bool, int, \
                                                cudaStream_t);                                                          \
   template cudaError_t launch_dft_batch<T>(const DftParams*, const int2*, int, int, const int*, int, cudaStream_t);
 LX_INST(double, double)
@@ -1682,8 +1806,19 @@ template cudaError_t launch_prologue_ahead<double>(const PrologueParams&, int, c
                                                    unsigned long long*, cudaStream_t);
 template cudaError_t launch_prologue_ahead<float>(const PrologueParams&, int, const StepCtl*, float*, double*,
                                                   unsigned long long*, cudaStream_t);
-template cudaError_t launch_prologue_batch<double>(const PrologueParams*, const int*, int, int, int, cudaStream_t);
-template cudaError_t launch_prologue_batch<float>(const PrologueParams*, const int*, int, int, int, cudaStream_t);
+template SweepParams<float, float> sweep_params<float, float>(const StepParams<float, float>&);
+template SweepParams<__half, float> sweep_params<__half, float>(const StepParams<__half, float>&);
+template cudaError_t launch_batch_sweep<float, float>(const SweepParams<float, float>*, int, const int*, const int4*, bool,
+                                                      int, int, cudaStream_t);
+template cudaError_t launch_batch_sweep<__half, float>(const SweepParams<__half, float>*, int, const int*, const int4*, bool,
+                                                       int, int, cudaStream_t);
+template void sweep_tiles<float, float>(const SweepParams<float, float>*, int, int, std::vector<int>&, std::vector<int4>&);
+template void sweep_tiles<__half, float>(const SweepParams<__half, float>*, int, int, std::vector<int>&,
+                                         std::vector<int4>&);
+template cudaError_t launch_prologue_batch<double>(const PrologueParams*, const int*, int, int, int, int, double*,
+                                                   unsigned long long*, cudaStream_t);
+template cudaError_t launch_prologue_batch<float>(const PrologueParams*, const int*, int, int, int, int, double*,
+                                                  unsigned long long*, cudaStream_t);
 template cudaError_t launch_eps_box<double>(double*, const int[3], int, int, const int[3], const int[3], double,
                                             cudaStream_t);
 template cudaError_t launch_eps_box<float>(float*, const int[3], int, int, const int[3], const int[3], double,

@@ -2,6 +2,8 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <vector>
+
 #include "lx_internal.h"
 
 namespace lx {
@@ -49,18 +51,31 @@ cudaError_t launch_dft(const DftParams& d, T* const f[4], cudaStream_t s);
 template <class T, class C>
 cudaError_t launch_batch_tiles(const StepParams<T, C>* ps, const int* first, int n, int nblocks, bool planar, int march,
                                int4* tiles, cudaStream_t s);
+// row: the step's place in its sequence (the members' tables and slots of that row)
 template <class T, class C>
 cudaError_t launch_batch_step(const StepParams<T, C>* ps, const int4* tiles, int nblocks, bool planar, bool uniform,
-                              int march, bool h_half, cudaStream_t s);
+                              int march, bool h_half, int row, cudaStream_t s);
+// Planar members in two buffers: H and E of a step, kSweepMembers members a launch, R rows a warp.
+template <class T, class C>
+SweepParams<T, C> sweep_params(const StepParams<T, C>& p);
+template <class T, class C>
+cudaError_t launch_batch_sweep(const SweepParams<T, C>* m, int n, const int* first, const int4* tiles, bool uniform, int R,
+                               int row, cudaStream_t s);
+// The members' first blocks (n + 1) and the blocks' tiles for it.
+template <class T, class C>
+void sweep_tiles(const SweepParams<T, C>* m, int n, int R, std::vector<int>& first, std::vector<int4>& tiles);
 // blocks one member occupies in a batched update launch; march = cells each thread walks
 // along x (planar: rows 8 apart; 3-D: planes), one of 1, 2, 4, 8
 int batch_blocks(int Nx, int Ny, int Nz, bool planar, int march);
 // block -> {member, block within the member} for a prefix `first` of n members
 cudaError_t launch_block_map(const int* first, int n, int nblocks, int2* map, cudaStream_t s);
+// The fields-independent part of steps k .. k+steps-1 of every member (step k runs at ts[sim] + k;
+// launch_tick advances ts): row q of the members' tables, of srcv and of slots ([row][sim]).
 template <class C>
-// step k of a chunk runs at ts[sim] + k; launch_tick advances ts by the chunk's steps
-cudaError_t launch_prologue_batch(const PrologueParams* pps, const int* ts, int k, int nsims, int max_entries,
-                                  cudaStream_t s);
+cudaError_t launch_prologue_batch(const PrologueParams* pps, const int* ts, int k, int steps, int nsims, int max_entries,
+                                  double* srcv, unsigned long long* slots, cudaStream_t s);
+// The members' point sources of step k, before its H updates (amplitudes v[sim]).
+cudaError_t launch_source_batch(const PrologueParams* pps, const int* ts, int k, int nsims, const double* v, cudaStream_t s);
 cudaError_t launch_tick(int* ts, int n, int steps, cudaStream_t s);
 template <class T>
 cudaError_t launch_dft_batch(const DftParams* ds, const int2* map, int nplanes, int nblocks, const int* ts, int k,

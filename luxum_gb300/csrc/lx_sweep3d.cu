@@ -193,7 +193,7 @@ __device__ __forceinline__ C tile_at(const unsigned char* st, int off, int strid
 // rows j0-1 .. j0+kTY-1 and columns k0-1 .. k0+31: y and z once per block, x per plane (a few
 // comparisons: a per-plane pass over the twelve sets cost as much as the rest of the plane)
 
-__device__ __forceinline__ bool set_reaches_yz(const PatchSet& ps, int jlo, int jhi, int klo, int khi) {
+__device__ __forceinline__ bool set_reaches_yz(const PlaneSet& ps, int jlo, int jhi, int klo, int khi) {
   if (!ps.active) return false;
   const bool y = ps.axis == 1 ? ((ps.plane[0] >= jlo && ps.plane[0] <= jhi) || (ps.plane[1] >= jlo && ps.plane[1] <= jhi))
                               : (ps.lo[1] <= jhi && ps.hi[1] >= jlo);
@@ -221,7 +221,7 @@ __device__ __forceinline__ BlockSets block_sets(const StepParams<T, C>& p, int j
   if (p.tfsf) {
 #pragma unroll
     for (int b = 0; b < 12; ++b) {
-      const PatchSet& ps = b < 6 ? p.setsH[b >> 1][b & 1] : p.setsE[(b - 6) >> 1][(b - 6) & 1];
+      const PlaneSet& ps = b < 6 ? p.setsH[b >> 1][b & 1] : p.setsE[(b - 6) >> 1][(b - 6) & 1];
       if (!set_reaches_yz(ps, j0 - 1, j0 + kTY - 1, k0 - 1, k0 + 31)) continue;
       if (ps.axis == 0) {
         bs.xn |= 1u << b;
