@@ -1468,6 +1468,13 @@ static lx::StepParams<T, C> step_params(lx_sim* s) {
     p.rkH[a] = (const C*)s->prof[a][5];
   }
   if (s->planar) { p.slab[1].lo = 0; p.slab[1].hi0 = 1 << 30; p.slab[1].n = 0; }
+  const int N[3] = {s->Nx, s->Ny, s->Nz};
+  for (int a = 0; a < 3; a++) {
+    p.free0[a] = p.slab[a].n ? p.slab[a].lo : 0;
+    p.free1[a] = p.slab[a].n ? p.slab[a].hi0 : N[a];
+    p.in0[a] = std::max(1, p.free0[a]);
+    p.in1[a] = std::min(N[a] - 1, p.free1[a]);
+  }
   for (int c = 0; c < 3; c++)
     for (int q = 0; q < 2; q++) {
       p.psiH[c][q] = (C*)s->psiH[c][q];

@@ -96,6 +96,20 @@ __device__ __forceinline__ void tfsf_apply(const PlaneSet& ps, const C* tab, int
   if (h1) d = d + __ldg(tab + ps.tab + ps.plane_len + off);
 }
 
+// The same for a set whose planes are normal to axis A (the sets of one curl part are).
+template <int A, class C>
+__device__ __forceinline__ void tfsf_axis(const PlaneSet& ps, const C* tab, int i, int j, int k, C& d) {
+  const int n = A == 0 ? i : (A == 1 ? j : k);
+  const bool h0 = n == ps.plane[0], h1 = n == ps.plane[1];
+  if (!ps.active || !(h0 || h1)) return;
+  constexpr int U = A == 0 ? 1 : 0, V = A == 2 ? 1 : 2;  // the in-plane axes
+  const int u = (A == 0 ? j : i) - ps.lo[U], v = (A == 2 ? j : k) - ps.lo[V];
+  if (u < 0 || v < 0 || u > ps.hi[U] - ps.lo[U] || v > ps.hi[V] - ps.lo[V]) return;
+  const C* e = tab + ps.tab + u * ps.stride[U] + v * ps.stride[V];
+  if (h0) d = d + __ldg(e);
+  if (h1) d = d + __ldg(e + ps.plane_len);
+}
+
 // psi = b*psi + c*curl; returns curl/kappa + psi (reference: three_dim_pml.cc:186-188).
 template <class C>
 __device__ __forceinline__ C pml_term(const Fp<C>& fp, C d, C* psi, C b, C cc, C rk) {

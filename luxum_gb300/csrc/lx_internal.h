@@ -142,6 +142,9 @@ struct StepParams {
   T* H1[3];
   C* psiH1[3][2];
   C* psiE1[3][2];
+  // Per axis, the indices [free0, free1) no CPML slab reaches, and of them [in0, in1) where every
+  // component of both half steps updates.
+  int free0[3], free1[3], in0[3], in1[3];
   // Set by the single-simulation 3-D launch: 1 when a block's z tile 0 is the row's two
   // 16-cell ends (see ZTile in lx_kernels.cu), 0 for plain 32-cell tiles.
   int zends;
@@ -184,6 +187,18 @@ __host__ __device__ inline bool tile_meets_planes(const int (&pl)[3][2], int i0,
     t |= (unsigned)(pl[0][q] - i0) < (unsigned)ni;
     t |= (unsigned)(pl[1][q] - j0) < (unsigned)nj;
     t |= (unsigned)(pl[2][q] - k0) < (unsigned)nk;
+  }
+  return t;
+}
+
+// The same per axis: bit a is set when the tile meets a plane normal to axis a (only the sets of
+// those axes can apply to the tile's cells).
+__host__ __device__ inline unsigned tile_plane_axes(const int (&pl)[3][2], int i0, int ni, int j0, int nj, int k0, int nk) {
+  unsigned t = 0;
+  for (int q = 0; q < 2; ++q) {
+    t |= (unsigned)(pl[0][q] - i0) < (unsigned)ni ? 1u : 0u;
+    t |= (unsigned)(pl[1][q] - j0) < (unsigned)nj ? 2u : 0u;
+    t |= (unsigned)(pl[2][q] - k0) < (unsigned)nk ? 4u : 0u;
   }
   return t;
 }

@@ -20,6 +20,7 @@
 
 #include <cstdlib>
 #include <cstring>
+#include <type_traits>
 #include <vector>
 
 #include "lx_device.cuh"
@@ -298,6 +299,12 @@ __device__ __forceinline__ void h_cell_3d(const StepParams<T, C>& p, const int i
   h_apply<T, C, UNI, FAST>(p, i, j, k, tf, v);
 }
 
+// Whether the slab paths also take blocks that meet TF/SF planes: FP16 storage, bound by
+// instructions (201x187x259 193 -> 189 us a step).  FP32 is bound by memory and lost to the longer
+// code more than it gained (512x512x128 598 -> 611).
+template <class T>
+constexpr bool kSlabTf = sizeof(T) == 2;
+
 // The two psi terms of a cell in the slab of one axis AX: both half steps form the derivative
 // along AX in part 1 of component AX+1 and part 0 of component AX+2, with one profile and one
 // index for both.  Loaded with the cell's fields, ahead of every store (see h_load).
@@ -305,61 +312,122 @@ template <class C>
 struct AxisPsi {
   bool on;
   long long q;
-  C a, b;         // psi of component AX+1 part 1, AX+2 part 0
-  C pb, pc, prk;  // profile b, c, 1/kappa
+  C a, b;        // psi of component AX+1 part 1, AX+2 part 0
+  C fb, fc, rk;  // profile b, c, 1/kappa
 };
 
 template <class T, class C, int AX>
-__device__ __forceinline__ void axis_psi_load(const StepParams<T, C>& p, C* const (&psi)[3][2], const C* pb, const C* pc,
-                                              const C* prk, int i, int j, int k, bool ua, bool ub, AxisPsi<C>& w) {
+__device__ __forceinline__ void axis_psi_load(const StepParams<T, C>& p, C* const (&psi)[3][2], const C* fb, const C* fc,
+                                              const C* rk, int i, int j, int k, unsigned o, AxisPsi<C>& w) {
   const int u = AX == 0 ? i : (AX == 1 ? j : k);
-  const int s = slab_index(p.slab[AX], u);
-  w.on = s >= 0 && (ua || ub);
-  w.a = w.b = w.pb = w.pc = w.prk = C(0);
-  w.q = 0;
+  const int s = u < p.free0[AX] ? u : u - p.free1[AX] + p.free0[AX];
+  w.on = AX == 0 || u < p.free0[AX] || u >= p.free1[AX];
   if (w.on) {
-    w.q = psi_index(AX, p.slab[AX], s, i, j, k, p.Ny, p.Nzp);
-    if (ua) w.a = psi[(AX + 1) % 3][1][w.q];
-    if (ub) w.b = psi[(AX + 2) % 3][0][w.q];
-    w.pb = __ldg(pb + u);
-    w.pc = __ldg(pc + u);
-    w.prk = __ldg(prk + u);
+    // the offset of the block's plane (or slab plane) is uniform, the rest 32 bits
+    const unsigned n = p.slab[AX].n;
+    const long long base = AX == 0 ? (long long)s * p.si : (AX == 1 ? (long long)i * n * p.Nzp : (long long)i * p.Ny * n);
+    const unsigned q = AX == 0 ? o : (AX == 1 ? (unsigned)s * p.Nzp + k : (unsigned)j * n + s);
+    w.q = base + q;
+    w.a = psi[(AX + 1) % 3][1][w.q];
+    w.b = psi[(AX + 2) % 3][0][w.q];
+    w.fb = __ldg(fb + u);
+    w.fc = __ldg(fc + u);
+    w.rk = __ldg(rk + u);
   }
 }
 // pml_term's arithmetic on a loaded psi.
 template <class C>
 __device__ __forceinline__ void axis_psi_term(const AxisPsi<C>& w, C& psi, C& d) {
-  psi = fmaC(w.pb, psi, w.pc * d);
-  d = fmaC(d, w.prk, psi);
+  psi = fmaC(w.fb, psi, w.fc * d);
+  d = fmaC(d, w.rk, psi);
 }
 
-// H of a cell whose block meets the CPML slab of axis AX only and no TF/SF plane (AX = 3: no
-// slab, a block at the walls): h_apply's arithmetic with the two psi terms' loads issued with
-// the field loads.  In h_apply each psi term's load waits behind the previous term's store (the
-// arrays may alias as far as the compiler knows), one memory round trip per term, and such
-// blocks are a third of a 256^3 grid with 16-cell slabs and most of a 64^3 one.
+// H of a cell on planes 1 .. Nx-2 whose block meets the CPML slab of axis AX only
+// (AX = 3: no slab, a block at the y or z walls): h_apply's arithmetic.  In h_apply each psi
+// term's load waits behind the previous term's store (the arrays may alias as far as the compiler
+// knows), and its conditions and 64-bit offsets double a cell's instructions.  Here every load is
+// issued first and unconditionally (off these planes' walls a neighbour is memory of the same
+// array, whatever it holds), and only the stores ask whether the cell updates.
 template <class T, class C, bool UNI, int AX>
-__device__ __forceinline__ void h_slab_3d(const StepParams<T, C>& p, const int i, const int j, const int k) {
+__device__ __forceinline__ void h_slab_3d(const StepParams<T, C>& p, const int i, const int j, const int k,
+                                          const unsigned tf) {
+  // FP32 keeps h_load's conditions: with the plain loads the kernel spills 12-36 bytes at its 32
+  // registers, on the way of every block (512x512x128 H 265 us a launch against 269-282), which
+  // FP16 storage, bound by instructions, makes up for (256^3 H 135 -> 124).
+  constexpr bool kPlain = sizeof(T) == 2;
   HCell<C> v;
-  h_load<T, C>(p, i, j, k, v);
+  const unsigned o = (unsigned)j * (unsigned)p.Nzp + (unsigned)k;
+  if constexpr (kPlain) {
+    const long long c = (long long)i * p.si + o;
+    const bool jn = j < p.Ny - 1, kn = k < p.Nz - 1;
+    v.c = c;
+    v.ux = jn && kn;
+    v.uy = kn;
+    v.uz = jn;
+    v.ex = ld<T, C>(p.E[0] + c);
+    v.ey = ld<T, C>(p.E[1] + c);
+    v.ez = ld<T, C>(p.E[2] + c);
+    v.ez_j = ld<T, C>(p.E[2] + c + p.Nzp);
+    v.ex_j = ld<T, C>(p.E[0] + c + p.Nzp);
+    v.ey_k = ld<T, C>(p.E[1] + c + 1);
+    v.ex_k = ld<T, C>(p.E[0] + c + 1);
+    v.ez_i = ld<T, C>(p.E[2] + c + p.si);
+    v.ey_i = ld<T, C>(p.E[1] + c + p.si);
+    v.hx = ld<T, C>(p.H[0] + c);
+    v.hy = ld<T, C>(p.H[1] + c);
+    v.hz = ld<T, C>(p.H[2] + c);
+  } else {
+    h_load<T, C>(p, i, j, k, v);
+  }
   const bool u[3] = {v.ux, v.uy, v.uz};
+  constexpr int A = (AX + 1) % 3, B = (AX + 2) % 3;
   AxisPsi<C> w;
-  if constexpr (AX < 3)
-    axis_psi_load<T, C, AX>(p, p.psiH, p.bH[AX], p.cH[AX], p.rkH[AX], i, j, k, u[(AX + 1) % 3], u[(AX + 2) % 3], w);
+  if constexpr (AX < 3) {
+    if constexpr (kPlain) {
+      axis_psi_load<T, C, AX>(p, p.psiH, p.bH[AX], p.cH[AX], p.rkH[AX], i, j, k, o, w);
+    } else {
+      const int n = AX == 0 ? i : (AX == 1 ? j : k);
+      const int sl = slab_index(p.slab[AX], n);
+      w.on = sl >= 0 && (u[A] || u[B]);
+      w.a = w.b = w.fb = w.fc = w.rk = C(0);
+      w.q = 0;
+      if (w.on) {
+        w.q = psi_index(AX, p.slab[AX], sl, i, j, k, p.Ny, p.Nzp);
+        if (u[A]) w.a = p.psiH[A][1][w.q];
+        if (u[B]) w.b = p.psiH[B][0][w.q];
+        w.fb = __ldg(p.bH[AX] + n);
+        w.fc = __ldg(p.cH[AX] + n);
+        w.rk = __ldg(p.rkH[AX] + n);
+      }
+    }
+  }
   // d[c][part]: Hx: dEz/dy, dEy/dz; Hy: dEx/dz, dEz/dx; Hz: dEy/dx, dEx/dy
   C d[3][2] = {{v.ez_j - v.ez, v.ey_k - v.ey}, {v.ex_k - v.ex, v.ez_i - v.ez}, {v.ey_i - v.ey, v.ex_j - v.ex}};
   if (!UNI) {
 #pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      d[c][0] = mulC(d[c][0], p.rd[(c + 1) % 3]);
-      d[c][1] = mulC(d[c][1], p.rd[(c + 2) % 3]);
+    for (int m = 0; m < 3; ++m) {
+      d[m][0] = mulC(d[m][0], p.rd[(m + 1) % 3]);
+      d[m][1] = mulC(d[m][1], p.rd[(m + 2) % 3]);
+    }
+  }
+  if (kSlabTf<T> && tf) {
+    if (tf & 1u) {
+      tfsf_axis<0, C>(p.setsH[1][1], p.tab, i, j, k, d[1][1]);
+      tfsf_axis<0, C>(p.setsH[2][0], p.tab, i, j, k, d[2][0]);
+    }
+    if (tf & 2u) {
+      tfsf_axis<1, C>(p.setsH[0][0], p.tab, i, j, k, d[0][0]);
+      tfsf_axis<1, C>(p.setsH[2][1], p.tab, i, j, k, d[2][1]);
+    }
+    if (tf & 4u) {
+      tfsf_axis<2, C>(p.setsH[0][1], p.tab, i, j, k, d[0][1]);
+      tfsf_axis<2, C>(p.setsH[1][0], p.tab, i, j, k, d[1][0]);
     }
   }
   if constexpr (AX < 3) {
-    constexpr int A = (AX + 1) % 3, B = (AX + 2) % 3;
     if (w.on) {
-      if (u[A]) axis_psi_term(w, w.a, d[A][1]);
-      if (u[B]) axis_psi_term(w, w.b, d[B][0]);
+      if (kPlain || u[A]) axis_psi_term(w, w.a, d[A][1]);
+      if (kPlain || u[B]) axis_psi_term(w, w.b, d[B][0]);
       if (u[A]) p.psiH[A][1][w.q] = w.a;
       if (u[B]) p.psiH[B][0][w.q] = w.b;
     }
@@ -369,15 +437,22 @@ __device__ __forceinline__ void h_slab_3d(const StepParams<T, C>& p, const int i
   if (u[2]) st<T, C>(p.H[2] + v.c, fmaC(-p.Dbs, d[2][0] - d[2][1], v.hz));
 }
 
-// The path of a block that is not interior: kGeneral when it meets a TF/SF plane or the slabs
-// of two axes, else the axis of the one slab it meets, or kNoSlab.
+// Whether a tile lies where every component updates and no slab reaches.
+template <class T, class C>
+__device__ __forceinline__ bool tile_in(const StepParams<T, C>& p, int i, int j0, int nj, int k0, int nk) {
+  return i >= p.in0[0] && i < p.in1[0] && j0 >= p.in0[1] && j0 + nj <= p.in1[1] && k0 >= p.in0[2] && k0 + nk <= p.in1[2];
+}
+
+// The path of a block that is not interior: kGeneral when it meets the slabs of two axes, an x wall or
+// (FP32) a TF/SF plane, else the axis of the one slab it meets, or kNoSlab.
 constexpr int kNoSlab = 3, kGeneral = 4;
-__device__ __forceinline__ int slab_path(const Slab (&sl)[3], bool pml, bool tf, int i0, int ni, int j0, int nj, int k0,
-                                         int nk) {
-  if (tf) return kGeneral;
-  if (!pml) return kNoSlab;
-  const bool x = !axis_free(sl[0], i0, ni), y = !axis_free(sl[1], j0, nj), z = !axis_free(sl[2], k0, nk);
-  if (x + y + z > 1) return kGeneral;
+template <class T, class C>
+__device__ __forceinline__ int slab_path(const StepParams<T, C>& p, unsigned tf, int i, int j0, int nj, int k0, int nk) {
+  if (i < 1 || i > p.Nx - 2) return kGeneral;
+  const bool x = i < p.free0[0] || i >= p.free1[0];
+  const bool y = j0 < p.free0[1] || min(j0 + nj, p.Ny) > p.free1[1];
+  const bool z = k0 < p.free0[2] || min(k0 + nk, p.Nz) > p.free1[2];
+  if (x + y + z > 1 || (!kSlabTf<T> && tf)) return kGeneral;
   return x ? 0 : (y ? 1 : (z ? 2 : kNoSlab));
 }
 
@@ -435,6 +510,12 @@ __device__ __forceinline__ ZTile z_tile(int Nz, bool ends) {
 __device__ __forceinline__ bool ztile_meets_planes(const int (&pl)[3][2], int i, int j0, int nj, const ZTile& z) {
   return tile_meets_planes(pl, i, 1, j0, nj, z.lo0, z.n0) || (z.n1 > 0 && tile_meets_planes(pl, i, 1, j0, nj, z.lo1, z.n1));
 }
+// The axes whose planes it meets, as bits.
+__device__ __forceinline__ unsigned ztile_plane_axes(const int (&pl)[3][2], int i, int j0, int nj, const ZTile& z) {
+  unsigned t = tile_plane_axes(pl, i, 1, j0, nj, z.lo0, z.n0);
+  if (z.n1 > 0) t |= tile_plane_axes(pl, i, 1, j0, nj, z.lo1, z.n1);
+  return t;
+}
 
 // One cell per thread; a block is ZW (z) x 256/ZW (y) cells of one x plane.  Blocks whose tile
 // is interior take the cell code with every condition decided at compile time.
@@ -446,16 +527,18 @@ __global__ void __launch_bounds__(256, HMinBlocks<C>::v) h_kernel_3d(const StepP
   const int j = blockIdx.y * RY + threadIdx.y;
   const int i = blockIdx.z;
   if (!z.valid || j >= p.Ny) return;
-  const bool tf = p.tfsf && ztile_meets_planes(p.planesH, i, blockIdx.y * RY, RY, z);
+  std::conditional_t<SLAB && kSlabTf<T>, unsigned, bool> tf = 0;
+  if constexpr (SLAB && kSlabTf<T>) tf = p.tfsf ? ztile_plane_axes(p.planesH, i, blockIdx.y * RY, RY, z) : 0u;
+  else tf = p.tfsf && ztile_meets_planes(p.planesH, i, blockIdx.y * RY, RY, z);
   if (!tf && z.n1 == 0 && tile_is_interior(p.slab, p.pml, p.Nx, p.Ny, p.Nz, i, 1, blockIdx.y * RY, RY, z.lo0, z.n0))
     h_cell_3d<T, C, UNI, true>(p, i, j, k, false);
   else {
-    const int path = SLAB ? slab_path(p.slab, p.pml, tf, i, 1, blockIdx.y * RY, RY, z.lo0, z.n0) : kGeneral;
-    if (path == 0) h_slab_3d<T, C, UNI, 0>(p, i, j, k);
-    else if (path == 1) h_slab_3d<T, C, UNI, 1>(p, i, j, k);
-    else if (path == 2) h_slab_3d<T, C, UNI, 2>(p, i, j, k);
-    else if (path == kNoSlab) h_slab_3d<T, C, UNI, kNoSlab>(p, i, j, k);
-    else h_cell_3d<T, C, UNI>(p, i, j, k, tf);
+    const int path = SLAB ? slab_path(p, tf, i, blockIdx.y * RY, RY, z.lo0, z.n0) : kGeneral;
+    if (path == 0) h_slab_3d<T, C, UNI, 0>(p, i, j, k, tf);
+    else if (path == 1) h_slab_3d<T, C, UNI, 1>(p, i, j, k, tf);
+    else if (path == 2) h_slab_3d<T, C, UNI, 2>(p, i, j, k, tf);
+    else if (path == kNoSlab) h_slab_3d<T, C, UNI, kNoSlab>(p, i, j, k, tf);
+    else h_cell_3d<T, C, UNI>(p, i, j, k, tf != 0);
   }
 }
 
@@ -575,44 +658,64 @@ __device__ __forceinline__ typename MaxBits<C>::type e_cell_3d(const StepParams<
   return e_apply<T, C, UNI, MON, FAST>(p, i, j, k, tf, v, scr);
 }
 
-// E of a cell whose block meets the CPML slab of axis AX only and no TF/SF plane (see h_slab_3d):
-// e_apply's arithmetic.
+// E of a cell on planes 1 .. Nx-2 whose block meets the CPML slab of axis AX only
+// (see h_slab_3d): e_apply's arithmetic.
 template <class T, class C, bool UNI, bool MON, int AX>
 __device__ __forceinline__ typename MaxBits<C>::type e_slab_3d(const StepParams<T, C>& p, const int i, const int j,
-                                                               const int k) {
-  ECell<C> v;
-  e_load<T, C, MON>(p, i, j, k, v);
-  const bool u[3] = {v.ux, v.uy, v.uz};
+                                                               const int k, const unsigned tf) {
+  const unsigned o = (unsigned)j * (unsigned)p.Nzp + (unsigned)k;
+  const long long c = (long long)i * p.si + o;
+  const C hx = ld<T, C>(p.H[0] + c), hy = ld<T, C>(p.H[1] + c), hz = ld<T, C>(p.H[2] + c);
+  const C hz_j = ld<T, C>(p.H[2] + c - p.Nzp), hx_j = ld<T, C>(p.H[0] + c - p.Nzp);
+  const C hy_k = ld<T, C>(p.H[1] + c - 1), hx_k = ld<T, C>(p.H[0] + c - 1);
+  const C hz_i = ld<T, C>(p.H[2] + c - p.si), hy_i = ld<T, C>(p.H[1] + c - p.si);
+  const C ex = ld<T, C>(p.E[0] + c), ey = ld<T, C>(p.E[1] + c), ez = ld<T, C>(p.E[2] + c);
+  const C cb[3] = {p.Cbs[0][c], p.Cbs[1][c], p.Cbs[2][c]};
   AxisPsi<C> w;
-  if constexpr (AX < 3)
-    axis_psi_load<T, C, AX>(p, p.psiE, p.bE[AX], p.cE[AX], p.rkE[AX], i, j, k, u[(AX + 1) % 3], u[(AX + 2) % 3], w);
+  if constexpr (AX < 3) axis_psi_load<T, C, AX>(p, p.psiE, p.bE[AX], p.cE[AX], p.rkE[AX], i, j, k, o, w);
+  const bool jn = j < p.Ny - 1, kn = k < p.Nz - 1, jj = j >= 1 && jn, kk = k >= 1 && kn;
+  const bool u[3] = {jj && kk, jn && kk, jj && kn};
   // d[c][part]: Ex: dHz/dy, dHy/dz; Ey: dHx/dz, dHz/dx; Ez: dHy/dx, dHx/dy
-  C d[3][2] = {{v.hz - v.hz_j, v.hy - v.hy_k}, {v.hx - v.hx_k, v.hz - v.hz_i}, {v.hy - v.hy_i, v.hx - v.hx_j}};
+  C d[3][2] = {{hz - hz_j, hy - hy_k}, {hx - hx_k, hz - hz_i}, {hy - hy_i, hx - hx_j}};
   if (!UNI) {
 #pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      d[c][0] = mulC(d[c][0], p.rd[(c + 1) % 3]);
-      d[c][1] = mulC(d[c][1], p.rd[(c + 2) % 3]);
+    for (int m = 0; m < 3; ++m) {
+      d[m][0] = mulC(d[m][0], p.rd[(m + 1) % 3]);
+      d[m][1] = mulC(d[m][1], p.rd[(m + 2) % 3]);
+    }
+  }
+  if (kSlabTf<T> && tf) {
+    if (tf & 1u) {
+      tfsf_axis<0, C>(p.setsE[1][1], p.tab, i, j, k, d[1][1]);
+      tfsf_axis<0, C>(p.setsE[2][0], p.tab, i, j, k, d[2][0]);
+    }
+    if (tf & 2u) {
+      tfsf_axis<1, C>(p.setsE[0][0], p.tab, i, j, k, d[0][0]);
+      tfsf_axis<1, C>(p.setsE[2][1], p.tab, i, j, k, d[2][1]);
+    }
+    if (tf & 4u) {
+      tfsf_axis<2, C>(p.setsE[0][1], p.tab, i, j, k, d[0][1]);
+      tfsf_axis<2, C>(p.setsE[1][0], p.tab, i, j, k, d[1][0]);
     }
   }
   if constexpr (AX < 3) {
     constexpr int A = (AX + 1) % 3, B = (AX + 2) % 3;
     if (w.on) {
-      if (u[A]) axis_psi_term(w, w.a, d[A][1]);
-      if (u[B]) axis_psi_term(w, w.b, d[B][0]);
+      axis_psi_term(w, w.a, d[A][1]);
+      axis_psi_term(w, w.b, d[B][0]);
       if (u[A]) p.psiE[A][1][w.q] = w.a;
       if (u[B]) p.psiE[B][0][w.q] = w.b;
     }
   }
-  const C exn = u[0] ? fmaC(v.cbx, d[0][0] - d[0][1], v.ex) : v.ex;
-  const C eyn = u[1] ? fmaC(v.cby, d[1][0] - d[1][1], v.ey) : v.ey;
-  const C ezn = u[2] ? fmaC(v.cbz, d[2][0] - d[2][1], v.ez) : v.ez;
-  if (u[0]) st<T, C>(p.E[0] + v.c, exn);
-  if (u[1]) st<T, C>(p.E[1] + v.c, eyn);
-  if (u[2]) st<T, C>(p.E[2] + v.c, ezn);
-  if (!(MON && v.mon)) return 0;
+  const C exn = u[0] ? fmaC(cb[0], d[0][0] - d[0][1], ex) : ex;
+  const C eyn = u[1] ? fmaC(cb[1], d[1][0] - d[1][1], ey) : ey;
+  const C ezn = u[2] ? fmaC(cb[2], d[2][0] - d[2][1], ez) : ez;
+  if (u[0]) st<T, C>(p.E[0] + c, exn);
+  if (u[1]) st<T, C>(p.E[1] + c, eyn);
+  if (u[2]) st<T, C>(p.E[2] + c, ezn);
+  if (!(MON && jn && kn)) return 0;
   const C e2 = fmaC(exn, exn, fmaC(eyn, eyn, ezn * ezn));
-  if (p.etotal) p.etotal[v.c] = e2;
+  if (p.etotal) p.etotal[c] = e2;
   return MaxBits<C>::of(e2);
 }
 
@@ -633,18 +736,20 @@ __global__ void __launch_bounds__(256, EMinBlocks<T>::v) e_kernel_3d(const StepP
   const int k = z.k;
   const int j = blockIdx.y * RY + threadIdx.y;
   const int i = blockIdx.z;
-  const bool tf = p.tfsf && ztile_meets_planes(p.planesE, i, blockIdx.y * RY, RY, z);
+  std::conditional_t<SLAB && kSlabTf<T>, unsigned, bool> tf = 0;
+  if constexpr (SLAB && kSlabTf<T>) tf = p.tfsf ? ztile_plane_axes(p.planesE, i, blockIdx.y * RY, RY, z) : 0u;
+  else tf = p.tfsf && ztile_meets_planes(p.planesE, i, blockIdx.y * RY, RY, z);
   typename MaxBits<C>::type mbits = 0;
   if (z.valid && j < p.Ny) {
-    if (!tf && z.n1 == 0 && tile_is_interior(p.slab, p.pml, p.Nx, p.Ny, p.Nz, i, 1, blockIdx.y * RY, RY, z.lo0, z.n0))
+    if (!tf && z.n1 == 0 && tile_in(p, i, blockIdx.y * RY, RY, z.lo0, z.n0))
       mbits = e_cell_3d<T, C, UNI, MON, true>(p, i, j, k, false);
     else {
-      const int path = SLAB ? slab_path(p.slab, p.pml, tf, i, 1, blockIdx.y * RY, RY, z.lo0, z.n0) : kGeneral;
-      if (path == 0) mbits = e_slab_3d<T, C, UNI, MON, 0>(p, i, j, k);
-      else if (path == 1) mbits = e_slab_3d<T, C, UNI, MON, 1>(p, i, j, k);
-      else if (path == 2) mbits = e_slab_3d<T, C, UNI, MON, 2>(p, i, j, k);
-      else if (path == kNoSlab) mbits = e_slab_3d<T, C, UNI, MON, kNoSlab>(p, i, j, k);
-      else mbits = e_cell_3d<T, C, UNI, MON>(p, i, j, k, tf);
+      const int path = SLAB ? slab_path(p, tf, i, blockIdx.y * RY, RY, z.lo0, z.n0) : kGeneral;
+      if (path == 0) mbits = e_slab_3d<T, C, UNI, MON, 0>(p, i, j, k, tf);
+      else if (path == 1) mbits = e_slab_3d<T, C, UNI, MON, 1>(p, i, j, k, tf);
+      else if (path == 2) mbits = e_slab_3d<T, C, UNI, MON, 2>(p, i, j, k, tf);
+      else if (path == kNoSlab) mbits = e_slab_3d<T, C, UNI, MON, kNoSlab>(p, i, j, k, tf);
+      else mbits = e_cell_3d<T, C, UNI, MON>(p, i, j, k, tf != 0);
     }
   }
   if (MON && p.max_slot) block_max_atomic(mbits, p.max_slot);
@@ -689,7 +794,7 @@ __device__ __forceinline__ void h2_apply(const StepParams<T, C>& p, const int i,
   if (ux) {
     C d2 = fp.sub(ey_k, ey);
     if (!UNI) d2 = fp.mul(d2, fp.reg(p.rd[2]));
-    if (tf) tfsf_apply<C>(p.setsH[0][1], p.tab, i, 0, k, d2);
+    if (tf) tfsf_axis<2, C>(p.setsH[0][1], p.tab, i, 0, k, d2);
     if (!FAST && p.pml) {
       const int sz = slab_index(p.slab[2], k);
       if (sz >= 0) d2 = pml_term<C>(fp, d2, p.psiH[0][1] + (long long)i * p.slab[2].n + sz, p.bH[2][k], p.cH[2][k], p.rkH[2][k]);
@@ -700,7 +805,7 @@ __device__ __forceinline__ void h2_apply(const StepParams<T, C>& p, const int i,
   if (uz) {
     C d1 = fp.sub(ey_i, ey);
     if (!UNI) d1 = fp.mul(d1, fp.reg(p.rd[0]));
-    if (tf) tfsf_apply<C>(p.setsH[2][0], p.tab, i, 0, k, d1);
+    if (tf) tfsf_axis<0, C>(p.setsH[2][0], p.tab, i, 0, k, d1);
     if (!FAST && p.pml) {
       const int sx = slab_index(p.slab[0], i);
       if (sx >= 0) d1 = pml_term<C>(fp, d1, p.psiH[2][0] + (long long)sx * p.Nzp + k, p.bH[0][i], p.cH[0][i], p.rkH[0][i]);
@@ -768,8 +873,8 @@ __device__ __forceinline__ typename MaxBits<C>::type e2_apply(const StepParams<T
     C d2 = fp.sub(v.hz, v.hz_i);  // dHz/dx (x profile)
     if (!UNI) { d1 = fp.mul(d1, fp.reg(p.rd[2])); d2 = fp.mul(d2, fp.reg(p.rd[0])); }
     if (tf) {
-      tfsf_apply<C>(p.setsE[1][0], p.tab, i, 0, k, d1);
-      tfsf_apply<C>(p.setsE[1][1], p.tab, i, 0, k, d2);
+      tfsf_axis<2, C>(p.setsE[1][0], p.tab, i, 0, k, d1);
+      tfsf_axis<0, C>(p.setsE[1][1], p.tab, i, 0, k, d2);
     }
     if (!FAST && p.pml) {
       const int sz = slab_index(p.slab[2], k), sx = slab_index(p.slab[0], i);
@@ -900,7 +1005,7 @@ __device__ __forceinline__ typename MaxBits<C>::type step2_rows(const SweepParam
   auto hz_value = [&](int i, int sx, C ey, C ey_i, C hz, C& psi) -> C {
     C d1 = ey_i - ey;
     if (!UNI) d1 = mulC(d1, p.rd[0]);
-    if (!FAST && tfH) tfsf_apply<C>(p.setHz, tab, i, 0, k, d1);
+    if (!FAST && tfH) tfsf_axis<0, C>(p.setHz, tab, i, 0, k, d1);
     if (!FAST && sx >= 0) psi2_term(__ldg(p.bHx + i), __ldg(p.cHx + i), __ldg(p.rHx + i), psi, d1);
     return stored<T, C>(fmaC(-p.Dbs, d1, hz));
   };
@@ -932,7 +1037,7 @@ __device__ __forceinline__ typename MaxBits<C>::type step2_rows(const SweepParam
     if (kin && ux) {
       C d2 = ey_k - ey;
       if (!UNI) d2 = mulC(d2, p.rd[2]);
-      if (!FAST && tfH) tfsf_apply<C>(p.setHx, tab, i, 0, k, d2);
+      if (!FAST && tfH) tfsf_axis<2, C>(p.setHx, tab, i, 0, k, d2);
       if (!FAST && sz >= 0) psi2_term(bHz, cHz, rHz, cur.phx, d2);
       hxn = stored<T, C>(fmaC(p.Dbs, d2, cur.hx));
     }
@@ -943,7 +1048,7 @@ __device__ __forceinline__ typename MaxBits<C>::type step2_rows(const SweepParam
       if (halo) {  // new Hx of column k0-1, recomputed; its owner stores the new psi
         C d2 = ey - cur.eyh;
         if (!UNI) d2 = mulC(d2, p.rd[2]);
-        if (!FAST && tfH) tfsf_apply<C>(p.setHx, tab, i, 0, k0 - 1, d2);
+        if (!FAST && tfH) tfsf_axis<2, C>(p.setHx, tab, i, 0, k0 - 1, d2);
         if (!FAST && szh >= 0) psi2_term(bHh, cHh, rHh, cur.phxh, d2);
         hx_k = stored<T, C>(fmaC(p.Dbs, d2, cur.hxh));
       }
@@ -955,8 +1060,8 @@ __device__ __forceinline__ typename MaxBits<C>::type step2_rows(const SweepParam
       C d2 = hzn - hz_p;  // dHz/dx (x profile)
       if (!UNI) { d1 = mulC(d1, p.rd[2]); d2 = mulC(d2, p.rd[0]); }
       if (!FAST && tfE) {
-        tfsf_apply<C>(p.setEz, tab, i, 0, k, d1);
-        tfsf_apply<C>(p.setEx, tab, i, 0, k, d2);
+        tfsf_axis<2, C>(p.setEz, tab, i, 0, k, d1);
+        tfsf_axis<0, C>(p.setEx, tab, i, 0, k, d2);
       }
       if (!FAST) {
         if (sz >= 0) psi2_term(bEz, cEz, rEz, cur.pez, d1);
@@ -1539,12 +1644,13 @@ cudaError_t launch_step(const StepParams<T, C>& p, bool planar, bool uniform, bo
     StepParams<T, C> q = p;
     q.zends = sizeof(T) == 8 && p.pml && p.slab[2].n > 0 && p.slab[2].lo <= 16 && p.Nz - p.slab[2].hi0 <= 16 &&
               p.Nz >= 48;
-    // Float grids of 2^22 cells or more give blocks in the slab of one axis their own path
-    // (h_slab_3d): us a step with and without it, 512x512x128 (CPML 20) 602 and 654, 256^3
-    // (CPML 16, TF/SF) 308 and 324, 128^3 57.0 and 57.5, 100^3 (CPML 12) 41.0 and 39.4 (the
-    // longer code costs a short launch more than the path saves).  FP64 is bound by its pipe.
+    // Float grids of 2^20 cells or more give blocks in the slab of one axis their own path
+    // (h_slab_3d): us a step with and without it, 512x512x128 FP32 (CPML 20) 592 and 654, 256^3
+    // (CPML 16, TF/SF) 299 and 324, in FP16 storage 268 and 299, 150^3 (CPML 12) 82.9 and 88.4,
+    // 100^3 30.7 and 30.8, 73^3 16.9 and 16.6 (the longer code costs a short launch more than the
+    // path saves).  FP64 is bound by its pipe.
     bool slab = false;
-    if constexpr (sizeof(C) == 4) slab = p.pml && (long long)p.Nx * p.Ny * p.Nz >= (1LL << 22);
+    if constexpr (sizeof(C) == 4) slab = p.pml && (long long)p.Nx * p.Ny * p.Nz >= (1LL << 20);
     if constexpr (sizeof(C) == 4)
       if (slab) {
         if (uniform) launch_step_3d<T, C, true, true>(q, mon, h_half, s);
