@@ -5,6 +5,8 @@
 // the same way on x86-64 and aarch64 hosts.
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
+#include <sys/mman.h>
+#include <unistd.h>
 
 #include <algorithm>
 #include <cmath>
@@ -851,6 +853,44 @@ extern "C" LX_API lx_status lx_sim_field_shape(const lx_sim* s, int comp, int sh
   return LX_OK;
 }
 
+#ifndef MADV_POPULATE_WRITE
+#define MADV_POPULATE_WRITE 23
+#endif
+
+// Has the kernel back a caller's buffer with pages before a device-to-host copy into it.  A
+// buffer fresh from the allocator has none, and a copy that takes the page faults itself runs at
+// 10-20 GB/s (2 MB 230 us, 134 MB 6.5 ms, against 31 us and 0.8 ms into resident pages);
+// populating costs 36 us and, on four threads, 1.8 ms, and runs beside the gather kernel.
+// Advice only: a kernel that does not know it, or memory it does not apply to, is left to fault.
+static void populate(void* host, size_t bytes) {
+  constexpr size_t kLeast = 256 << 10, kPerThread = 4 << 20;
+  if (bytes < kLeast) return;
+  const size_t page = (size_t)sysconf(_SC_PAGESIZE);
+  const size_t a = ((size_t)host + page - 1) / page * page, e = ((size_t)host + bytes) / page * page;
+  if (e <= a) return;
+  // a buffer used before is resident: three of its pages tell
+  bool resident = true;
+  for (size_t at : {a, a + (e - a) / page / 2 * page, e - page}) {
+    unsigned char in = 0;
+    resident = resident && mincore((void*)at, page, &in) == 0 && (in & 1);
+  }
+  if (resident) return;
+  const size_t parts = std::max<size_t>(1, std::min<size_t>(4, (e - a) / kPerThread));
+  const size_t step = ((e - a) / parts + page - 1) / page * page;
+  auto part = [=](size_t q) {
+    const size_t from = a + q * step, to = std::min(e, from + step);
+    if (from < to) madvise((void*)from, to - from, MADV_POPULATE_WRITE);
+  };
+  std::thread th[3];
+  size_t made = 0;
+  try {
+    for (; made + 1 < parts; made++) th[made] = std::thread(part, made + 1);
+  } catch (const std::exception&) {  // no thread to be had: the copy faults those pages in
+  }
+  part(0);
+  for (size_t q = 0; q < made; q++) th[q].join();
+}
+
 extern "C" LX_API lx_status lx_sim_read_field(lx_sim* s, int comp, double* host, size_t n) {
   if (!s) return fail(nullptr, LX_ERR_INVALID, "null handle");
   lx::DeviceGuard dg_(s->device);
@@ -863,6 +903,7 @@ extern "C" LX_API lx_status lx_sim_read_field(lx_sim* s, int comp, double* host,
   lx_status st = ensure_xfer(s);
   if (st) return st;
   if ((st = gather(s, comp, s->xfer))) return st;
+  populate(host, m * sizeof(double));
   CK(cudaMemcpyAsync(host, s->xfer, m * sizeof(double), cudaMemcpyDeviceToHost, s->stream));
   CK(cudaStreamSynchronize(s->stream));
   s->n_d2h += m * sizeof(double);
@@ -1213,6 +1254,7 @@ extern "C" LX_API lx_status lx_sim_read_dft(lx_sim* s, int id, double* host, siz
   if (id < 0 || id >= (int)s->dfts.size()) return fail(s, LX_ERR_INVALID, "no such DFT plane");
   const lx::DftPlane& d = s->dfts[id];
   if (n != d.n_acc) return fail(s, LX_ERR_INVALID, "buffer size must be nfreq*4*na*nb*2");
+  populate(host, n * sizeof(double));
   CK(cudaMemcpyAsync(host, d.d_acc, n * sizeof(double), cudaMemcpyDeviceToHost, s->stream));
   CK(cudaStreamSynchronize(s->stream));
   s->n_d2h += n * sizeof(double);
