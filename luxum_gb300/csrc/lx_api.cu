@@ -426,6 +426,8 @@ extern "C" LX_API void lx_sim_destroy(lx_sim* s) {
   if (s->stream) cudaStreamSynchronize(s->stream);
   if (s->side) cudaStreamSynchronize(s->side);
   drop_graph(s);
+  for (auto& e : s->seq_ev)
+    if (e) cudaEventDestroy(e);
   cudaStream_t fs = s->own;
   for (int c = 0; c < 3; c++) {
     dfree(s->E[c], fs); dfree(s->H[c], fs); dfree(s->Cbs[c], fs);
@@ -1695,9 +1697,19 @@ static lx_status run_steps(lx_sim* s, int nsteps, KernelTimer* kt = nullptr) {
     s->n_kernels++;
     return LX_OK;
   };
+  // In a captured sequence of a handle in two buffers, what only reads a step's state (DFT planes,
+  // probes) runs beside the next step: that step writes the other buffer, the one after it waits.
+  // A point source writes into the state it would read.
+  bool beside[2] = {false, false};  // readers of the step of this parity not waited for yet
+  auto wait_readers = [&](int par) -> lx_status {
+    if (beside[par]) CK(cudaStreamWaitEvent(s->stream, s->seq_ev[1 + par], 0));
+    beside[par] = false;
+    return LX_OK;
+  };
   // The launches of step t, the q-th of its sequence; ctl: as part of a captured sequence.
   auto one_step = [&](int t, int q, bool mon, unsigned snap, const lx::StepCtl* ctl) -> lx_status {
     lx_status st;
+    if ((st = wait_readers(t & 1))) return st;  // the step before last's
     if (s->src_kind >= 0) {
       T* f = (T*)(s->pp && (t & 1) ? pp.src_field1 : pp.src_field);  // the state step t reads
       CK(lx::launch_source<T>(f, s->src_idx, s->src_kind, s->d_srcv + q, s->stream));
@@ -1729,6 +1741,16 @@ static lx_status run_steps(lx_sim* s, int nsteps, KernelTimer* kt = nullptr) {
       s->n_kernels += 2;
     }
     post_step(t);
+    cudaStream_t rs = s->stream;
+    bool due_dft = false;
+    for (auto& d : s->dfts) due_dft |= t % d.every == 0;
+    if (ctl && s->pp && s->src_kind < 0 && (due_dft || s->nprobes > 0)) {
+      for (auto& e : s->seq_ev)
+        if (!e) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+      rs = s->side;
+      CK(cudaEventRecord(s->seq_ev[0], s->stream));
+      CK(cudaStreamWaitEvent(rs, s->seq_ev[0], 0));
+    }
     for (auto& d : s->dfts) {
       if (t % d.every != 0) continue;
       lx::DftParams dp;
@@ -1741,7 +1763,7 @@ static lx_status run_steps(lx_sim* s, int nsteps, KernelTimer* kt = nullptr) {
         f4[c] = pf[d.comps[c]];
         for (int a = 0; a < 3; a++) dp.ext[c][a] = s->ext[d.comps[c]][a];
       }
-      CK(lx::launch_dft<T>(dp, f4, s->stream));
+      CK(lx::launch_dft<T>(dp, f4, rs));
       s->n_kernels += 2;  // phase factors, accumulation
     }
     if (s->nprobes > 0 && (ctl || s->probe_rows < s->probe_cap)) {
@@ -1750,9 +1772,13 @@ static lx_status run_steps(lx_sim* s, int nsteps, KernelTimer* kt = nullptr) {
       prb.k = q;
       if (!ctl) s->probe_rows++;
       if ((st = tic())) return st;
-      CK(lx::launch_probes<T>(prb, pf, s->d_probe, s->stream));
+      CK(lx::launch_probes<T>(prb, pf, s->d_probe, rs));
       if ((st = toc(3))) return st;
       s->n_kernels++;
+    }
+    if (rs != s->stream) {
+      CK(cudaEventRecord(s->seq_ev[1 + (t & 1)], rs));
+      beside[t & 1] = true;
     }
     return LX_OK;
   };
@@ -1782,6 +1808,7 @@ static lx_status run_steps(lx_sim* s, int nsteps, KernelTimer* kt = nullptr) {
         // a sequence may end a call, so its last step is always monitored
         st = ahead(t, K, true, s->d_ctl);
         for (int q = 0; q < K && !st; q++) st = one_step(t + q, q, ((mask >> q) & 1u) || q == K - 1, 0, s->d_ctl);
+        for (int par = 0; par < 2 && !st; par++) st = wait_readers(par);
         if (!st && lx::launch_finish(s->d_ring, s->d_series ? mask : 0u, s->d_series, 0, s->series_cap, s->d_ctl, K,
                                      s->probe_cap, s->own) != cudaSuccess)
           st = fail(s, LX_ERR_CUDA, "launch_finish failed");

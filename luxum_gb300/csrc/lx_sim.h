@@ -130,6 +130,7 @@ struct lx_sim {
   // A captured sequence of graph_steps steps (short steps are bound by their launches); dropped
   // when anything its launches were given changes.  `ctl` is what d_ctl holds.
   cudaGraphExec_t graph = nullptr;
+  cudaEvent_t seq_ev[3] = {};  // while capturing: a step done, its readers done (by step parity)
   int graph_steps = 0, graph_pp = 0;
   unsigned long long graph_kernels = 0;
   long long alone_steps = 0;  // steps taken since the last such change
