@@ -1794,7 +1794,7 @@ cudaError_t launch_dft(const DftParams& d, T* const f[4], cudaStream_t s) {
   dft_phase_kernel<<<1, 128, 0, s>>>(d);
   // A thread walks its frequencies four at a time, one memory round trip each.  A small plane
   // (a planar grid's line: 17 blocks at side 1031) splits them over blocks instead: 32
-  // frequencies 11.5 -> 4.0 us; a plane that fills the GPU reads its fields once.
+  // frequencies 11.4 -> 4.9 us; a plane that fills the GPU reads its fields once.
   const long long nb = (n + 255) / 256;
   const int per = nb < 152 * 2 ? 4 : d.nfreq;
   dft_kernel<T><<<dim3((unsigned)nb, (unsigned)((d.nfreq + per - 1) / per)), 256, 0, s>>>(d, f[0], f[1], f[2], f[3], per);
