@@ -755,6 +755,182 @@ __global__ void __launch_bounds__(256, EMinBlocks<T>::v) e_kernel_3d(const StepP
   if (MON && p.max_slot) block_max_atomic(mbits, p.max_slot);
 }
 
+// ------------------------------------------------------------------ small 3-D grids
+
+// The half steps of a grid whose cells are all resident at once.  Such a launch is one chain from
+// its first load to its last store, so a cell issues every load it may need, psi of all three
+// slabs and their profile values included, before anything waits (the general path, built for many
+// warps at few registers, waits for a psi load behind every psi store).  Blocks are small, to reach
+// more SMs.
+template <class C>
+struct SlabPsi {
+  bool on;
+  long long q;
+  C a, b;        // psi of component AX+1 part 1, AX+2 part 0
+  C fb, fc, rk;  // profile b, c, 1/kappa
+};
+template <int AX, class T, class C>
+__device__ __forceinline__ void slab_psi_load(const StepParams<T, C>& p, C* const (&psi)[3][2], const C* fb, const C* fc,
+                                              const C* rk, int i, int j, int k, const bool (&u)[3], SlabPsi<C>& w) {
+  const int n = AX == 0 ? i : (AX == 1 ? j : k);
+  const int s = p.pml ? slab_index(p.slab[AX], n) : -1;
+  const bool ua = u[(AX + 1) % 3], ub = u[(AX + 2) % 3];
+  w.on = s >= 0 && (ua || ub);
+  w.a = w.b = w.fb = w.fc = w.rk = C(0);
+  w.q = w.on ? psi_index(AX, p.slab[AX], s, i, j, k, p.Ny, p.Nzp) : 0;
+  if (w.on) {
+    if (ua) w.a = psi[(AX + 1) % 3][1][w.q];
+    if (ub) w.b = psi[(AX + 2) % 3][0][w.q];
+    w.fb = __ldg(fb + n);
+    w.fc = __ldg(fc + n);
+    w.rk = __ldg(rk + n);
+  }
+}
+// Both psi terms of the slab (pml_term's arithmetic) and their stores.
+template <int AX, class C>
+__device__ __forceinline__ void slab_psi_apply(const Fp<C>& fp, SlabPsi<C>& w, C (&d)[3][2]) {
+  constexpr int A = (AX + 1) % 3, B = (AX + 2) % 3;
+  if (!w.on) return;
+  w.a = fmaC(w.fb, w.a, fp.mul(w.fc, d[A][1]));
+  d[A][1] = fmaC(d[A][1], w.rk, w.a);
+  w.b = fmaC(w.fb, w.b, fp.mul(w.fc, d[B][0]));
+  d[B][0] = fmaC(d[B][0], w.rk, w.b);
+}
+template <int AX, class C>
+__device__ __forceinline__ void slab_psi_store(C* const (&psi)[3][2], const SlabPsi<C>& w, const bool (&u)[3]) {
+  constexpr int A = (AX + 1) % 3, B = (AX + 2) % 3;
+  if (w.on && u[A]) psi[A][1][w.q] = w.a;
+  if (w.on && u[B]) psi[B][0][w.q] = w.b;
+}
+template <class C>
+__device__ __forceinline__ void tfsf_all(const PlaneSet (&sets)[3][2], const C* tab, unsigned tf, int i, int j, int k,
+                                         const bool (&u)[3], C (&d)[3][2]) {
+  if (tf & 1u) {
+    if (u[1]) tfsf_axis<0, C>(sets[1][1], tab, i, j, k, d[1][1]);
+    if (u[2]) tfsf_axis<0, C>(sets[2][0], tab, i, j, k, d[2][0]);
+  }
+  if (tf & 2u) {
+    if (u[0]) tfsf_axis<1, C>(sets[0][0], tab, i, j, k, d[0][0]);
+    if (u[2]) tfsf_axis<1, C>(sets[2][1], tab, i, j, k, d[2][1]);
+  }
+  if (tf & 4u) {
+    if (u[0]) tfsf_axis<2, C>(sets[0][1], tab, i, j, k, d[0][1]);
+    if (u[1]) tfsf_axis<2, C>(sets[1][0], tab, i, j, k, d[1][0]);
+  }
+}
+
+// A block is NT consecutive cells (y, z) of one x plane (PACK), or 32 z x NT/32 y cells of it.
+template <class C>
+struct SmallCells {
+  static constexpr int v = sizeof(C) == 8 ? 64 : 128;
+};
+template <int NT, bool PACK>
+__device__ __forceinline__ void small_cell(int Nz, int& i, int& j, int& k) {
+  i = blockIdx.z;
+  if (PACK) {
+    const int c = blockIdx.x * NT + threadIdx.x;
+    j = c / Nz;
+    k = c - j * Nz;
+  } else {
+    j = blockIdx.y * (NT / 32) + (threadIdx.x >> 5);
+    k = blockIdx.x * 32 + (threadIdx.x & 31);
+  }
+}
+// Axes of the TF/SF planes that the block may touch.
+template <int NT, bool PACK>
+__device__ __forceinline__ unsigned small_plane_axes(const int (&planes)[3][2], int Nz) {
+  if (!PACK) return tile_plane_axes(planes, blockIdx.z, 1, blockIdx.y * (NT / 32), NT / 32, blockIdx.x * 32, 32);
+  const int c0 = blockIdx.x * NT, j0 = c0 / Nz, j1 = (c0 + NT - 1) / Nz;
+  const bool row = j0 == j1;
+  return tile_plane_axes(planes, blockIdx.z, 1, j0, j1 - j0 + 1, row ? c0 - j0 * Nz : 0, row ? NT : Nz);
+}
+
+template <class T, class C, bool UNI, bool PACK>
+__global__ void __launch_bounds__(SmallCells<C>::v) h_small_3d(const StepParams<T, C> p) {
+  int i, j, k;
+  small_cell<SmallCells<C>::v, PACK>(p.Nz, i, j, k);
+  if (j >= p.Ny || (!PACK && k >= p.Nz)) return;
+  HCell<C> v;
+  h_load<T, C>(p, i, j, k, v);
+  const bool u[3] = {v.ux, v.uy, v.uz};
+  SlabPsi<C> x, y, z;
+  slab_psi_load<0>(p, p.psiH, p.bH[0], p.cH[0], p.rkH[0], i, j, k, u, x);
+  slab_psi_load<1>(p, p.psiH, p.bH[1], p.cH[1], p.rkH[1], i, j, k, u, y);
+  slab_psi_load<2>(p, p.psiH, p.bH[2], p.cH[2], p.rkH[2], i, j, k, u, z);
+  const unsigned tf = p.tfsf ? small_plane_axes<SmallCells<C>::v, PACK>(p.planesH, p.Nz) : 0u;
+  const Fp<C> fp(k);
+  // d[c][part]: Hx: dEz/dy, dEy/dz; Hy: dEx/dz, dEz/dx; Hz: dEy/dx, dEx/dy
+  C d[3][2] = {{fp.sub(v.ez_j, v.ez), fp.sub(v.ey_k, v.ey)},
+               {fp.sub(v.ex_k, v.ex), fp.sub(v.ez_i, v.ez)},
+               {fp.sub(v.ey_i, v.ey), fp.sub(v.ex_j, v.ex)}};
+  if (!UNI) {
+#pragma unroll
+    for (int m = 0; m < 3; ++m) {
+      d[m][0] = fp.mul(d[m][0], fp.reg(p.rd[(m + 1) % 3]));
+      d[m][1] = fp.mul(d[m][1], fp.reg(p.rd[(m + 2) % 3]));
+    }
+  }
+  if (tf) tfsf_all<C>(p.setsH, p.tab, tf, i, j, k, u, d);
+  slab_psi_apply<0>(fp, x, d);
+  slab_psi_apply<1>(fp, y, d);
+  slab_psi_apply<2>(fp, z, d);
+  const C mdb = fp.neg(p.Dbs);
+  if (u[0]) st<T, C>(p.H[0] + v.c, fmaC(mdb, fp.sub(d[0][0], d[0][1]), v.hx));
+  if (u[1]) st<T, C>(p.H[1] + v.c, fmaC(mdb, fp.sub(d[1][0], d[1][1]), v.hy));
+  if (u[2]) st<T, C>(p.H[2] + v.c, fmaC(mdb, fp.sub(d[2][0], d[2][1]), v.hz));
+  slab_psi_store<0>(p.psiH, x, u);
+  slab_psi_store<1>(p.psiH, y, u);
+  slab_psi_store<2>(p.psiH, z, u);
+}
+
+template <class T, class C, bool UNI, bool MON, bool PACK>
+__global__ void __launch_bounds__(SmallCells<C>::v) e_small_3d(const StepParams<T, C> p) {
+  int i, j, k;
+  small_cell<SmallCells<C>::v, PACK>(p.Nz, i, j, k);
+  typename MaxBits<C>::type mbits = 0;
+  if (j < p.Ny && (PACK || k < p.Nz)) {
+    ECell<C> v;
+    e_load<T, C, MON>(p, i, j, k, v);
+    const bool u[3] = {v.ux, v.uy, v.uz};
+    SlabPsi<C> x, y, z;
+    slab_psi_load<0>(p, p.psiE, p.bE[0], p.cE[0], p.rkE[0], i, j, k, u, x);
+    slab_psi_load<1>(p, p.psiE, p.bE[1], p.cE[1], p.rkE[1], i, j, k, u, y);
+    slab_psi_load<2>(p, p.psiE, p.bE[2], p.cE[2], p.rkE[2], i, j, k, u, z);
+    const unsigned tf = p.tfsf ? small_plane_axes<SmallCells<C>::v, PACK>(p.planesE, p.Nz) : 0u;
+    const Fp<C> fp(k);
+    // d[c][part]: Ex: dHz/dy, dHy/dz; Ey: dHx/dz, dHz/dx; Ez: dHy/dx, dHx/dy
+    C d[3][2] = {{fp.sub(v.hz, v.hz_j), fp.sub(v.hy, v.hy_k)},
+                 {fp.sub(v.hx, v.hx_k), fp.sub(v.hz, v.hz_i)},
+                 {fp.sub(v.hy, v.hy_i), fp.sub(v.hx, v.hx_j)}};
+    if (!UNI) {
+#pragma unroll
+      for (int m = 0; m < 3; ++m) {
+        d[m][0] = fp.mul(d[m][0], fp.reg(p.rd[(m + 1) % 3]));
+        d[m][1] = fp.mul(d[m][1], fp.reg(p.rd[(m + 2) % 3]));
+      }
+    }
+    if (tf) tfsf_all<C>(p.setsE, p.tab, tf, i, j, k, u, d);
+    slab_psi_apply<0>(fp, x, d);
+    slab_psi_apply<1>(fp, y, d);
+    slab_psi_apply<2>(fp, z, d);
+    const C exn = u[0] ? fmaC(v.cbx, fp.sub(d[0][0], d[0][1]), v.ex) : v.ex;
+    const C eyn = u[1] ? fmaC(v.cby, fp.sub(d[1][0], d[1][1]), v.ey) : v.ey;
+    const C ezn = u[2] ? fmaC(v.cbz, fp.sub(d[2][0], d[2][1]), v.ez) : v.ez;
+    if (u[0]) st<T, C>(p.E[0] + v.c, exn);
+    if (u[1]) st<T, C>(p.E[1] + v.c, eyn);
+    if (u[2]) st<T, C>(p.E[2] + v.c, ezn);
+    slab_psi_store<0>(p.psiE, x, u);
+    slab_psi_store<1>(p.psiE, y, u);
+    slab_psi_store<2>(p.psiE, z, u);
+    if (MON && v.mon) {
+      const C e2 = fmaC(exn, exn, fmaC(eyn, eyn, fp.mul(ezn, ezn)));
+      if (p.etotal) p.etotal[v.c] = e2;
+      mbits = MaxBits<C>::of(e2);
+    }
+  }
+  if (MON && p.max_slot) block_max_atomic(mbits, p.max_slot);
+}
+
 // ------------------------------------------------------------------ planar kernels
 
 // Planar H half-step (x-z plane, Ny = 1): Hx and Hz (two_dim_pml.cc:144-162, two_dim.cc:95-111).
@@ -1620,6 +1796,44 @@ static void launch_step_3d(const StepParams<T, C>& q, bool mon, bool h_half, cud
   else e_kernel_3d<T, C, UNI, false, SLAB, 32><<<grid, block, 0, s>>>(q);
 }
 
+// Grids that take the kernels of one cell a thread with every load ahead (h_small_3d).  Us a step
+// with them and without:
+// - FP64 with CPML, while all blocks are resident (10 of 64 threads an SM at 96 registers): 20^3
+//   7.5 and 11.0, 34x30x36 10.0 and 12.4, 44^3 14.6 and 16.3; beyond, the loads a second wave
+//   could overlap wait, 48^3 18.7 and 17.1.  Without CPML the general path has nothing to wait
+//   for: 34^3 9.5 and 9.1.
+// - Float with CPML, up to where the slab paths begin: 34^3 6.2 and 9.2, 64^3 9.4 and 12.0, 100^3
+//   27.3 and 30.4, in FP16 storage 29.1 and 32.2; 128^3 with 6 and 12 cells of CPML 37.0 and
+//   35.4, 43.1 and 45.8, in FP16 storage 41.0 and 35.8, 45.8 and 42.9.
+// - Float without CPML: 26^3 3.9 and 4.6, 64^3 6.9 and 6.9, 100^3 19.1 and 16.0.
+template <class T, class C>
+static bool small_grid(const StepParams<T, C>& p) {
+  const long long cells = (long long)p.Nx * p.Ny * p.Nz;
+  if (sizeof(C) == 8) return p.pml && cells <= 152 * 10 * SmallCells<C>::v;
+  return cells < (p.pml ? 1LL << 20 : 1LL << 18);
+}
+
+// Float rows that fill less than 4/5 of their 32-cell tiles are packed (73^3 FP32 13.5 us a step,
+// in tiles 14.0; 200x200x25 23.1 and 25.3), longer ones keep the rows of a tile together (64^3
+// 9.9, packed 10.9; 90^3 19.1 and 21.3).  FP64 pays a pipe slot for each idle lane and is always
+// packed (34^3 10.0, in tiles 14.2).
+template <class T, class C, bool PACK>
+static void launch_small_3d(const StepParams<T, C>& p, bool uniform, bool mon, bool h_half, cudaStream_t s) {
+  constexpr int NT = SmallCells<C>::v;
+  const dim3 grid = PACK ? dim3((unsigned)(((long long)p.Ny * p.Nz + NT - 1) / NT), 1, p.Nx)
+                         : dim3((p.Nz + 31) / 32, (p.Ny + NT / 32 - 1) / (NT / 32), p.Nx);
+  if (h_half) {
+    if (uniform) h_small_3d<T, C, true, PACK><<<grid, NT, 0, s>>>(p);
+    else h_small_3d<T, C, false, PACK><<<grid, NT, 0, s>>>(p);
+  } else if (mon) {
+    if (uniform) e_small_3d<T, C, true, true, PACK><<<grid, NT, 0, s>>>(p);
+    else e_small_3d<T, C, false, true, PACK><<<grid, NT, 0, s>>>(p);
+  } else {
+    if (uniform) e_small_3d<T, C, true, false, PACK><<<grid, NT, 0, s>>>(p);
+    else e_small_3d<T, C, false, false, PACK><<<grid, NT, 0, s>>>(p);
+  }
+}
+
 template <class T, class C>
 cudaError_t launch_step(const StepParams<T, C>& p, bool planar, bool uniform, bool h_half, cudaStream_t s) {
   // single simulations: one cell per thread (their parameters sit in the constant bank, and
@@ -1643,6 +1857,12 @@ cudaError_t launch_step(const StepParams<T, C>& p, bool planar, bool uniform, bo
     // The E kernel with float storage takes 16-cell z tiles (LUXUM_ZTILE=32 keeps 32): on the
     // 256^3 drop-in grid E 0.2035 -> 0.189 ms (FP32), 0.200 -> 0.187 (FP16 storage), from its
     // CPML and TF/SF tiles; the H kernel ran 0.015 ms slower with them, CPML or not.
+    if (small_grid<T, C>(p)) {
+      const bool pack = sizeof(C) == 8 || 5LL * p.Nz <= 4LL * ((p.Nz + 31) & ~31);
+      if (pack) launch_small_3d<T, C, true>(p, uniform, mon, h_half, s);
+      else if constexpr (sizeof(C) == 4) launch_small_3d<T, C, false>(p, uniform, mon, h_half, s);
+      return cudaGetLastError();
+    }
     StepParams<T, C> q = p;
     q.zends = sizeof(T) == 8 && p.pml && p.slab[2].n > 0 && p.slab[2].lo <= 16 && p.Nz - p.slab[2].hi0 <= 16 &&
               p.Nz >= 48;
