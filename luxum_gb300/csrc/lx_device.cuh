@@ -11,6 +11,15 @@ namespace lx {
 
 // ------------------------------------------------------------------ storage access
 
+// First statement of a step's kernels: their blocks may be on the SMs before the kernel ahead of
+// them in the stream is complete, and go on when it is and its stores are visible.  Every thread
+// passes here, so that a kernel is complete only after the one ahead of it.
+__device__ __forceinline__ void step_behind() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+// From here the next kernel's blocks may take the places that this one's leave (without it, from
+// when the last of this one's blocks ends).
+__device__ __forceinline__ void step_open() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 template <class T, class C>
 __device__ __forceinline__ C ld(const T* p) {
   return static_cast<C>(*p);

@@ -144,6 +144,7 @@ __global__ void prologue_ahead_kernel(const PrologueParams p, const StepCtl* ctl
 
 template <class T>
 __global__ void source_kernel(T* field, long long idx, int kind, const double* v) {
+  step_behind();
   source_apply<T>(field + idx, kind, *v);
 }
 
@@ -521,6 +522,8 @@ __device__ __forceinline__ unsigned ztile_plane_axes(const int (&pl)[3][2], int 
 // is interior take the cell code with every condition decided at compile time.
 template <class T, class C, bool UNI, bool SLAB, int ZW>
 __global__ void __launch_bounds__(256, HMinBlocks<C>::v) h_kernel_3d(const StepParams<T, C> p) {
+  step_behind();
+  step_open();
   constexpr int RY = 256 / ZW;
   const ZTile z = z_tile<ZW>(p.Nz, p.zends);
   const int k = z.k;
@@ -731,6 +734,8 @@ struct EMinBlocks {
 
 template <class T, class C, bool UNI, bool MON, bool SLAB, int ZW>
 __global__ void __launch_bounds__(256, EMinBlocks<T>::v) e_kernel_3d(const StepParams<T, C> p) {
+  step_behind();
+  step_open();
   constexpr int RY = 256 / ZW;
   const ZTile z = z_tile<ZW>(p.Nz, p.zends);
   const int k = z.k;
@@ -847,6 +852,7 @@ __device__ __forceinline__ unsigned small_plane_axes(const int (&planes)[3][2], 
 
 template <class T, class C, bool UNI, bool PACK>
 __global__ void __launch_bounds__(SmallCells<C>::v) h_small_3d(const StepParams<T, C> p) {
+  step_behind();
   int i, j, k;
   small_cell<SmallCells<C>::v, PACK>(p.Nz, i, j, k);
   if (j >= p.Ny || (!PACK && k >= p.Nz)) return;
@@ -885,6 +891,7 @@ __global__ void __launch_bounds__(SmallCells<C>::v) h_small_3d(const StepParams<
 
 template <class T, class C, bool UNI, bool MON, bool PACK>
 __global__ void __launch_bounds__(SmallCells<C>::v) e_small_3d(const StepParams<T, C> p) {
+  step_behind();
   int i, j, k;
   small_cell<SmallCells<C>::v, PACK>(p.Nz, i, j, k);
   typename MaxBits<C>::type mbits = 0;
@@ -1002,6 +1009,7 @@ __device__ __forceinline__ void h_cell_2d(const StepParams<T, C>& p, const int i
 // One cell per thread; a block is 32 (z) x 8 (x) cells.
 template <class T, class C, bool UNI>
 __global__ void __launch_bounds__(256) h_kernel_2d(const StepParams<T, C> p) {
+  step_behind();
   const int k = blockIdx.x * 32 + threadIdx.x;
   const int ib = blockIdx.y * 8, i = ib + threadIdx.y;
   if (k >= p.Nz || i >= p.Nx) return;
@@ -1075,6 +1083,7 @@ __device__ __forceinline__ typename MaxBits<C>::type e_cell_2d(const StepParams<
 
 template <class T, class C, bool UNI, bool MON>
 __global__ void __launch_bounds__(256) e_kernel_2d(const StepParams<T, C> p) {
+  step_behind();
   const int k = blockIdx.x * 32 + threadIdx.x;
   const int ib = blockIdx.y * 8, i = ib + threadIdx.y;
   const bool tf = p.tfsf && tile_meets_planes(p.planesE, ib, 8, 0, 1, blockIdx.x * 32, 32);
@@ -1285,6 +1294,8 @@ constexpr int kSweepMinBlocks = 5;
 // One simulation: a block is 32 z columns x 8 warps of R rows.
 template <class T, class C, bool UNI>
 __global__ void __launch_bounds__(256, kSweepMinBlocks) step_kernel_2d(const SweepParams<T, C> p, const int R) {
+  step_behind();
+  step_open();
   const int k0 = blockIdx.x * 32;
   const int i0 = (blockIdx.y * 8 + threadIdx.y) * R;
   typename MaxBits<C>::type m = 0;
@@ -1581,6 +1592,7 @@ __global__ void __launch_bounds__(256) eps_box_kernel(C* dst, int n0, int n1, in
 template <class T>
 __global__ void probe_kernel(const ProbeParams pp, const T* f0, const T* f1, const T* f2, const T* f3, const T* f4,
                              const T* f5, double* out) {
+  step_behind();
   const int q = blockIdx.x * blockDim.x + threadIdx.x;
   if (q >= pp.nprobes * 6) return;
   const int row = pp.ctl ? pp.ctl->row + pp.k : pp.row;
@@ -1753,9 +1765,25 @@ cudaError_t launch_prologue_ahead(const PrologueParams& p, int steps, const Step
   return cudaGetLastError();
 }
 
+// Launches a kernel of a step; behind: after another step kernel, whose last blocks it may start
+// beside (step_behind).
+template <class... P, class... A>
+static void start(void (*kernel)(P...), dim3 grid, dim3 block, bool behind, cudaStream_t s, A... a) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.stream = s;
+  cudaLaunchAttribute at = {};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = behind ? 1 : 0;
+  (void)cudaLaunchKernelEx(&cfg, kernel, a...);  // the caller reads the error
+}
+
 template <class T>
-cudaError_t launch_source(T* field, long long idx, int kind, const double* v, cudaStream_t s) {
-  source_kernel<T><<<1, 1, 0, s>>>(field, idx, kind, v);
+cudaError_t launch_source(T* field, long long idx, int kind, const double* v, bool behind, cudaStream_t s) {
+  start(source_kernel<T>, 1, 1, behind, s, field, idx, kind, v);
   return cudaGetLastError();
 }
 
@@ -1781,19 +1809,19 @@ static bool z16_tiles() {
 }
 
 template <class T, class C, bool UNI, bool SLAB>
-static void launch_step_3d(const StepParams<T, C>& q, bool mon, bool h_half, cudaStream_t s) {
+static void launch_step_3d(const StepParams<T, C>& q, bool mon, bool h_half, bool behind, cudaStream_t s) {
   if constexpr (sizeof(T) < 8) {
     if (!h_half && z16_tiles()) {
       const dim3 block(16, 16), grid((q.Nz + 15) / 16, (q.Ny + 15) / 16, q.Nx);
-      if (mon) e_kernel_3d<T, C, UNI, true, SLAB, 16><<<grid, block, 0, s>>>(q);
-      else e_kernel_3d<T, C, UNI, false, SLAB, 16><<<grid, block, 0, s>>>(q);
+      if (mon) start(e_kernel_3d<T, C, UNI, true, SLAB, 16>, grid, block, behind, s, q);
+      else start(e_kernel_3d<T, C, UNI, false, SLAB, 16>, grid, block, behind, s, q);
       return;
     }
   }
   const dim3 block(32, 8), grid(q.zends ? 1 + (q.Nz - 32 + 31) / 32 : (q.Nz + 31) / 32, (q.Ny + 7) / 8, q.Nx);
-  if (h_half) h_kernel_3d<T, C, UNI, SLAB, 32><<<grid, block, 0, s>>>(q);
-  else if (mon) e_kernel_3d<T, C, UNI, true, SLAB, 32><<<grid, block, 0, s>>>(q);
-  else e_kernel_3d<T, C, UNI, false, SLAB, 32><<<grid, block, 0, s>>>(q);
+  if (h_half) start(h_kernel_3d<T, C, UNI, SLAB, 32>, grid, block, behind, s, q);
+  else if (mon) start(e_kernel_3d<T, C, UNI, true, SLAB, 32>, grid, block, behind, s, q);
+  else start(e_kernel_3d<T, C, UNI, false, SLAB, 32>, grid, block, behind, s, q);
 }
 
 // Grids that take the kernels of one cell a thread with every load ahead (h_small_3d).  Us a step
@@ -1818,24 +1846,24 @@ static bool small_grid(const StepParams<T, C>& p) {
 // 9.9, packed 10.9; 90^3 19.1 and 21.3).  FP64 pays a pipe slot for each idle lane and is always
 // packed (34^3 10.0, in tiles 14.2).
 template <class T, class C, bool PACK>
-static void launch_small_3d(const StepParams<T, C>& p, bool uniform, bool mon, bool h_half, cudaStream_t s) {
+static void launch_small_3d(const StepParams<T, C>& p, bool uniform, bool mon, bool h_half, bool behind, cudaStream_t s) {
   constexpr int NT = SmallCells<C>::v;
   const dim3 grid = PACK ? dim3((unsigned)(((long long)p.Ny * p.Nz + NT - 1) / NT), 1, p.Nx)
                          : dim3((p.Nz + 31) / 32, (p.Ny + NT / 32 - 1) / (NT / 32), p.Nx);
   if (h_half) {
-    if (uniform) h_small_3d<T, C, true, PACK><<<grid, NT, 0, s>>>(p);
-    else h_small_3d<T, C, false, PACK><<<grid, NT, 0, s>>>(p);
+    if (uniform) start(h_small_3d<T, C, true, PACK>, grid, NT, behind, s, p);
+    else start(h_small_3d<T, C, false, PACK>, grid, NT, behind, s, p);
   } else if (mon) {
-    if (uniform) e_small_3d<T, C, true, true, PACK><<<grid, NT, 0, s>>>(p);
-    else e_small_3d<T, C, false, true, PACK><<<grid, NT, 0, s>>>(p);
+    if (uniform) start(e_small_3d<T, C, true, true, PACK>, grid, NT, behind, s, p);
+    else start(e_small_3d<T, C, false, true, PACK>, grid, NT, behind, s, p);
   } else {
-    if (uniform) e_small_3d<T, C, true, false, PACK><<<grid, NT, 0, s>>>(p);
-    else e_small_3d<T, C, false, false, PACK><<<grid, NT, 0, s>>>(p);
+    if (uniform) start(e_small_3d<T, C, true, false, PACK>, grid, NT, behind, s, p);
+    else start(e_small_3d<T, C, false, false, PACK>, grid, NT, behind, s, p);
   }
 }
 
 template <class T, class C>
-cudaError_t launch_step(const StepParams<T, C>& p, bool planar, bool uniform, bool h_half, cudaStream_t s) {
+cudaError_t launch_step(const StepParams<T, C>& p, bool planar, bool uniform, bool h_half, bool behind, cudaStream_t s) {
   // single simulations: one cell per thread (their parameters sit in the constant bank, and
   // walking several cells raises register use past what pays off)
   dim3 block(32, 8);
@@ -1843,14 +1871,14 @@ cudaError_t launch_step(const StepParams<T, C>& p, bool planar, bool uniform, bo
   if (planar) {
     dim3 grid((p.Nz + 31) / 32, (p.Nx + 7) / 8, 1);
     if (h_half) {
-      if (uniform) h_kernel_2d<T, C, true><<<grid, block, 0, s>>>(p);
-      else h_kernel_2d<T, C, false><<<grid, block, 0, s>>>(p);
+      if (uniform) start(h_kernel_2d<T, C, true>, grid, block, behind, s, p);
+      else start(h_kernel_2d<T, C, false>, grid, block, behind, s, p);
     } else if (mon) {
-      if (uniform) e_kernel_2d<T, C, true, true><<<grid, block, 0, s>>>(p);
-      else e_kernel_2d<T, C, false, true><<<grid, block, 0, s>>>(p);
+      if (uniform) start(e_kernel_2d<T, C, true, true>, grid, block, behind, s, p);
+      else start(e_kernel_2d<T, C, false, true>, grid, block, behind, s, p);
     } else {
-      if (uniform) e_kernel_2d<T, C, true, false><<<grid, block, 0, s>>>(p);
-      else e_kernel_2d<T, C, false, false><<<grid, block, 0, s>>>(p);
+      if (uniform) start(e_kernel_2d<T, C, true, false>, grid, block, behind, s, p);
+      else start(e_kernel_2d<T, C, false, false>, grid, block, behind, s, p);
     }
   } else {
     // FP64 with z CPML slabs of at most 16 cells: the rows' two ends share one tile (ZTile).
@@ -1859,8 +1887,8 @@ cudaError_t launch_step(const StepParams<T, C>& p, bool planar, bool uniform, bo
     // CPML and TF/SF tiles; the H kernel ran 0.015 ms slower with them, CPML or not.
     if (small_grid<T, C>(p)) {
       const bool pack = sizeof(C) == 8 || 5LL * p.Nz <= 4LL * ((p.Nz + 31) & ~31);
-      if (pack) launch_small_3d<T, C, true>(p, uniform, mon, h_half, s);
-      else if constexpr (sizeof(C) == 4) launch_small_3d<T, C, false>(p, uniform, mon, h_half, s);
+      if (pack) launch_small_3d<T, C, true>(p, uniform, mon, h_half, behind, s);
+      else if constexpr (sizeof(C) == 4) launch_small_3d<T, C, false>(p, uniform, mon, h_half, behind, s);
       return cudaGetLastError();
     }
     StepParams<T, C> q = p;
@@ -1875,12 +1903,12 @@ cudaError_t launch_step(const StepParams<T, C>& p, bool planar, bool uniform, bo
     if constexpr (sizeof(C) == 4) slab = p.pml && (long long)p.Nx * p.Ny * p.Nz >= (1LL << 20);
     if constexpr (sizeof(C) == 4)
       if (slab) {
-        if (uniform) launch_step_3d<T, C, true, true>(q, mon, h_half, s);
-        else launch_step_3d<T, C, false, true>(q, mon, h_half, s);
+        if (uniform) launch_step_3d<T, C, true, true>(q, mon, h_half, behind, s);
+        else launch_step_3d<T, C, false, true>(q, mon, h_half, behind, s);
         return cudaGetLastError();
       }
-    if (uniform) launch_step_3d<T, C, true, false>(q, mon, h_half, s);
-    else launch_step_3d<T, C, false, false>(q, mon, h_half, s);
+    if (uniform) launch_step_3d<T, C, true, false>(q, mon, h_half, behind, s);
+    else launch_step_3d<T, C, false, false>(q, mon, h_half, behind, s);
   }
   return cudaGetLastError();
 }
@@ -1925,13 +1953,13 @@ SweepParams<T, C> sweep_params(const StepParams<T, C>& p) {
 }
 
 template <class T, class C>
-cudaError_t launch_step_sweep2(const StepParams<T, C>& p, bool uniform, cudaStream_t s) {
+cudaError_t launch_step_sweep2(const StepParams<T, C>& p, bool uniform, bool behind, cudaStream_t s) {
   const long long cols = (p.Nz + 31) / 32;
   const int R = sweep_rows(cols, p.Nx);
   const dim3 block(32, 8), grid((unsigned)cols, (unsigned)((p.Nx + 8 * R - 1) / (8 * R)));
   const SweepParams<T, C> q = sweep_params(p);
-  if (uniform) step_kernel_2d<T, C, true><<<grid, block, 0, s>>>(q, R);
-  else step_kernel_2d<T, C, false><<<grid, block, 0, s>>>(q, R);
+  if (uniform) start(step_kernel_2d<T, C, true>, grid, block, behind, s, q, R);
+  else start(step_kernel_2d<T, C, false>, grid, block, behind, s, q, R);
   return cudaGetLastError();
 }
 
@@ -2002,9 +2030,10 @@ cudaError_t launch_eps_box(C* dst, const int ext[3], int Ny, int Nzp, const int 
 }
 
 template <class T>
-cudaError_t launch_probes(const ProbeParams& pp, T* const f[6], double* out, cudaStream_t s) {
+cudaError_t launch_probes(const ProbeParams& pp, T* const f[6], double* out, bool behind, cudaStream_t s) {
   const int n = pp.nprobes * 6;
-  probe_kernel<T><<<(n + 127) / 128, 128, 0, s>>>(pp, f[0], f[1], f[2], f[3], f[4], f[5], out);
+  start(probe_kernel<T>, (n + 127) / 128, 128, behind, s, pp, (const T*)f[0], (const T*)f[1], (const T*)f[2], (const T*)f[3],
+        (const T*)f[4], (const T*)f[5], out);
   return cudaGetLastError();
 }
 
@@ -2118,12 +2147,12 @@ cudaError_t launch_dft_flux(const double* acc, int nfreq, long long ncell, doubl
 }
 
 #define LX_INST(T, C)                                                                                                  \
-  template cudaError_t launch_step<T, C>(const StepParams<T, C>&, bool, bool, bool, cudaStream_t);                   \
+  template cudaError_t launch_step<T, C>(const StepParams<T, C>&, bool, bool, bool, bool, cudaStream_t);                 \
   template cudaError_t launch_gather<T>(const T*, double*, const int[3], int, int, double, cudaStream_t);                     \
   template cudaError_t launch_scatter<T>(const double*, T*, const int[3], int, int, int, double, double, double,      \
                                          double, cudaStream_t);                                                        \
-  template cudaError_t launch_source<T>(T*, long long, int, const double*, cudaStream_t);                              \
-  template cudaError_t launch_probes<T>(const ProbeParams&, T* const[6], double*, cudaStream_t);                   \
+  template cudaError_t launch_source<T>(T*, long long, int, const double*, bool, cudaStream_t);                            \
+  template cudaError_t launch_probes<T>(const ProbeParams&, T* const[6], double*, bool, cudaStream_t);                 \
   template cudaError_t launch_dft<T>(const DftParams&, T* const[4], cudaStream_t);                                 \
   template cudaError_t launch_batch_tiles<T, C>(const StepParams<T, C>*, const int*, int, int, bool, int, int4*,    \
                                                 cudaStream_t);                                                     \
@@ -2133,8 +2162,8 @@ cudaError_t launch_dft_flux(const double* acc, int nfreq, long long ncell, doubl
 LX_INST(double, double)
 LX_INST(float, float)
 LX_INST(__half, float)
-template cudaError_t launch_step_sweep2<float, float>(const StepParams<float, float>&, bool, cudaStream_t);
-template cudaError_t launch_step_sweep2<__half, float>(const StepParams<__half, float>&, bool, cudaStream_t);
+template cudaError_t launch_step_sweep2<float, float>(const StepParams<float, float>&, bool, bool, cudaStream_t);
+template cudaError_t launch_step_sweep2<__half, float>(const StepParams<__half, float>&, bool, bool, cudaStream_t);
 template cudaError_t launch_prologue_ahead<double>(const PrologueParams&, int, const StepCtl*, double*, double*,
                                                    unsigned long long*, cudaStream_t);
 template cudaError_t launch_prologue_ahead<float>(const PrologueParams&, int, const StepCtl*, float*, double*,

@@ -14,20 +14,22 @@ namespace lx {
 template <class C>
 cudaError_t launch_prologue_ahead(const PrologueParams& p, int steps, const StepCtl* ctl, C* tab, double* srcv,
                                   unsigned long long* ring, cudaStream_t s);
+// `behind`, of the launches of a step: the stream's last launch was one too, and this one may start
+// beside its end.
 // The point source of one step (its amplitude formed ahead), before the step's H update.
 template <class T>
-cudaError_t launch_source(T* field, long long idx, int kind, const double* v, cudaStream_t s);
+cudaError_t launch_source(T* field, long long idx, int kind, const double* v, bool behind, cudaStream_t s);
 // ring[q] of the steps q in `mask` appended to the max|E|^2 series from entry `at` (ctl: from
 // ctl->series, up to cap); with ctl, the counters then advance by `steps`.
 cudaError_t launch_finish(const unsigned long long* ring, unsigned mask, unsigned long long* series, int at, int cap,
                           StepCtl* ctl, int steps, int rows, cudaStream_t s);
 cudaError_t launch_set_ctl(StepCtl* ctl, StepCtl v, cudaStream_t s);
 template <class T, class C>
-cudaError_t launch_step(const StepParams<T, C>& p, bool planar, bool uniform, bool h_half, cudaStream_t s);
+cudaError_t launch_step(const StepParams<T, C>& p, bool planar, bool uniform, bool h_half, bool behind, cudaStream_t s);
 // Single-sweep planar step (float compute, two state buffers): reads the buffers named in
 // p.E, p.H, p.psiH, p.psiE and writes those in p.E1, p.H1, p.psiH1, p.psiE1.
 template <class T, class C>
-cudaError_t launch_step_sweep2(const StepParams<T, C>& p, bool uniform, cudaStream_t s);
+cudaError_t launch_step_sweep2(const StepParams<T, C>& p, bool uniform, bool behind, cudaStream_t s);
 // Single-sweep 3-D step (float compute, two state buffers), lx_sweep3d.cu: the same buffer
 // convention as launch_step_sweep2.
 template <class T, class C>
@@ -41,7 +43,7 @@ template <class C>
 cudaError_t launch_eps_box(C* dst, const int ext[3], int Ny, int Nzp, const int lo[3], const int hi[3], double val,
                            cudaStream_t s);
 template <class T>
-cudaError_t launch_probes(const ProbeParams& pp, T* const f[6], double* out, cudaStream_t s);
+cudaError_t launch_probes(const ProbeParams& pp, T* const f[6], double* out, bool behind, cudaStream_t s);
 
 template <class T>
 cudaError_t launch_dft(const DftParams& d, T* const f[4], cudaStream_t s);
