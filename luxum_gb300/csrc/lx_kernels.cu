@@ -760,38 +760,53 @@ __global__ void __launch_bounds__(256, EMinBlocks<T>::v) e_kernel_3d(const StepP
   if (MON && p.max_slot) block_max_atomic(mbits, p.max_slot);
 }
 
-// ------------------------------------------------------------------ small 3-D grids
+// ------------------------------------------------------------------ 3-D cells, loads ahead
 
-// The half steps of a grid whose cells are all resident at once.  Such a launch is one chain from
-// its first load to its last store, so a cell issues every load it may need, psi of all three
-// slabs and their profile values included, before anything waits (the general path, built for many
-// warps at few registers, waits for a psi load behind every psi store).  Blocks are small, to reach
-// more SMs.
+// The half steps of grids bound by latency or by instructions rather than by memory.  On a small
+// grid a launch is one chain from its first load to its last store, and the general path, built
+// for many warps at few registers, waits for a psi load behind every psi store; on a larger one
+// with CPML its conditions and 64-bit offsets cost more than the update (100^3 FP32: 362
+// instructions a warp in H with them, 78 % of the issue slots).  Here a cell issues every load it
+// may need, psi of all three slabs and their profile values included, before anything waits.
+// Fields, psi and coefficients are read at unsigned 32-bit byte offsets from their arrays, which
+// the load instructions add themselves, and unconditionally: a neighbour beyond a wall is the cell
+// itself, and only the stores ask whether the cell updates.  Blocks are small, to reach more SMs
+// (128 threads; with 256 100^3 24.9 us a step against 23.8, 512x512x128 622 against 584).  H
+// is capped at 48 registers (200^3 H 78.8 us against 82.4, E, at 56, 94.3 against 93.7).
+template <class T>
+__device__ __forceinline__ const T* at(const T* p, unsigned o) {
+  return reinterpret_cast<const T*>(reinterpret_cast<const char*>(p) + o);
+}
+template <class T>
+__device__ __forceinline__ T* at(T* p, unsigned o) {
+  return reinterpret_cast<T*>(reinterpret_cast<char*>(p) + o);
+}
 template <class C>
 struct SlabPsi {
   bool on;
-  long long q;
+  unsigned q;
   C a, b;        // psi of component AX+1 part 1, AX+2 part 0
   C fb, fc, rk;  // profile b, c, 1/kappa
 };
 template <int AX, class T, class C>
 __device__ __forceinline__ void slab_psi_load(const StepParams<T, C>& p, C* const (&psi)[3][2], const C* fb, const C* fc,
-                                              const C* rk, int i, int j, int k, const bool (&u)[3], SlabPsi<C>& w) {
+                                              const C* rk, int i, int j, int k, SlabPsi<C>& w) {
   const int n = AX == 0 ? i : (AX == 1 ? j : k);
   const int s = p.pml ? slab_index(p.slab[AX], n) : -1;
-  const bool ua = u[(AX + 1) % 3], ub = u[(AX + 2) % 3];
-  w.on = s >= 0 && (ua || ub);
+  w.on = s >= 0;
   w.a = w.b = w.fb = w.fc = w.rk = C(0);
-  w.q = w.on ? psi_index(AX, p.slab[AX], s, i, j, k, p.Ny, p.Nzp) : 0;
+  w.q = 0;
   if (w.on) {
-    if (ua) w.a = psi[(AX + 1) % 3][1][w.q];
-    if (ub) w.b = psi[(AX + 2) % 3][0][w.q];
+    const unsigned m = p.slab[AX].n;
+    w.q = (AX == 0 ? ((unsigned)s * p.Ny + j) * p.Nzp + k
+                   : (AX == 1 ? ((unsigned)i * m + s) * p.Nzp + k : ((unsigned)i * p.Ny + j) * m + s)) * (unsigned)sizeof(C);
+    w.a = *at(psi[(AX + 1) % 3][1], w.q);
+    w.b = *at(psi[(AX + 2) % 3][0], w.q);
     w.fb = __ldg(fb + n);
     w.fc = __ldg(fc + n);
     w.rk = __ldg(rk + n);
   }
 }
-// Both psi terms of the slab (pml_term's arithmetic) and their stores.
 template <int AX, class C>
 __device__ __forceinline__ void slab_psi_apply(const Fp<C>& fp, SlabPsi<C>& w, C (&d)[3][2]) {
   constexpr int A = (AX + 1) % 3, B = (AX + 2) % 3;
@@ -804,8 +819,8 @@ __device__ __forceinline__ void slab_psi_apply(const Fp<C>& fp, SlabPsi<C>& w, C
 template <int AX, class C>
 __device__ __forceinline__ void slab_psi_store(C* const (&psi)[3][2], const SlabPsi<C>& w, const bool (&u)[3]) {
   constexpr int A = (AX + 1) % 3, B = (AX + 2) % 3;
-  if (w.on && u[A]) psi[A][1][w.q] = w.a;
-  if (w.on && u[B]) psi[B][0][w.q] = w.b;
+  if (w.on && u[A]) *at(psi[A][1], w.q) = w.a;
+  if (w.on && u[B]) *at(psi[B][0], w.q) = w.b;
 }
 template <class C>
 __device__ __forceinline__ void tfsf_all(const PlaneSet (&sets)[3][2], const C* tab, unsigned tf, int i, int j, int k,
@@ -851,18 +866,33 @@ __device__ __forceinline__ unsigned small_plane_axes(const int (&planes)[3][2], 
 }
 
 template <class T, class C, bool UNI, bool PACK>
-__global__ void __launch_bounds__(SmallCells<C>::v) h_small_3d(const StepParams<T, C> p) {
+__global__ void __launch_bounds__(SmallCells<C>::v, sizeof(C) == 4 ? 10 : 1) h_small_3d(const StepParams<T, C> p) {
   step_behind();
   int i, j, k;
   small_cell<SmallCells<C>::v, PACK>(p.Nz, i, j, k);
   if (j >= p.Ny || (!PACK && k >= p.Nz)) return;
+  const unsigned c = ((unsigned)i * p.Ny + j) * p.Nzp + k, b = c * (unsigned)sizeof(T);
+  const bool in = i < p.Nx - 1, jn = j < p.Ny - 1, kn = k < p.Nz - 1;
+  const bool u[3] = {jn && kn, in && kn, in && jn};
+  const unsigned bi = b + (in ? (unsigned)p.si * (unsigned)sizeof(T) : 0u), bj = b + (jn ? p.Nzp * (unsigned)sizeof(T) : 0u),
+                 bk = b + (kn ? (unsigned)sizeof(T) : 0u);
   HCell<C> v;
-  h_load<T, C>(p, i, j, k, v);
-  const bool u[3] = {v.ux, v.uy, v.uz};
+  v.ex = ld<T, C>(at(p.E[0], b));
+  v.ey = ld<T, C>(at(p.E[1], b));
+  v.ez = ld<T, C>(at(p.E[2], b));
+  v.ez_j = ld<T, C>(at(p.E[2], bj));
+  v.ey_k = ld<T, C>(at(p.E[1], bk));
+  v.ex_k = ld<T, C>(at(p.E[0], bk));
+  v.ez_i = ld<T, C>(at(p.E[2], bi));
+  v.ey_i = ld<T, C>(at(p.E[1], bi));
+  v.ex_j = ld<T, C>(at(p.E[0], bj));
+  v.hx = ld<T, C>(at(p.H[0], b));
+  v.hy = ld<T, C>(at(p.H[1], b));
+  v.hz = ld<T, C>(at(p.H[2], b));
   SlabPsi<C> x, y, z;
-  slab_psi_load<0>(p, p.psiH, p.bH[0], p.cH[0], p.rkH[0], i, j, k, u, x);
-  slab_psi_load<1>(p, p.psiH, p.bH[1], p.cH[1], p.rkH[1], i, j, k, u, y);
-  slab_psi_load<2>(p, p.psiH, p.bH[2], p.cH[2], p.rkH[2], i, j, k, u, z);
+  slab_psi_load<0>(p, p.psiH, p.bH[0], p.cH[0], p.rkH[0], i, j, k, x);
+  slab_psi_load<1>(p, p.psiH, p.bH[1], p.cH[1], p.rkH[1], i, j, k, y);
+  slab_psi_load<2>(p, p.psiH, p.bH[2], p.cH[2], p.rkH[2], i, j, k, z);
   const unsigned tf = p.tfsf ? small_plane_axes<SmallCells<C>::v, PACK>(p.planesH, p.Nz) : 0u;
   const Fp<C> fp(k);
   // d[c][part]: Hx: dEz/dy, dEy/dz; Hy: dEx/dz, dEz/dx; Hz: dEy/dx, dEx/dy
@@ -881,9 +911,9 @@ __global__ void __launch_bounds__(SmallCells<C>::v) h_small_3d(const StepParams<
   slab_psi_apply<1>(fp, y, d);
   slab_psi_apply<2>(fp, z, d);
   const C mdb = fp.neg(p.Dbs);
-  if (u[0]) st<T, C>(p.H[0] + v.c, fmaC(mdb, fp.sub(d[0][0], d[0][1]), v.hx));
-  if (u[1]) st<T, C>(p.H[1] + v.c, fmaC(mdb, fp.sub(d[1][0], d[1][1]), v.hy));
-  if (u[2]) st<T, C>(p.H[2] + v.c, fmaC(mdb, fp.sub(d[2][0], d[2][1]), v.hz));
+  if (u[0]) st<T, C>(at(p.H[0], b), fmaC(mdb, fp.sub(d[0][0], d[0][1]), v.hx));
+  if (u[1]) st<T, C>(at(p.H[1], b), fmaC(mdb, fp.sub(d[1][0], d[1][1]), v.hy));
+  if (u[2]) st<T, C>(at(p.H[2], b), fmaC(mdb, fp.sub(d[2][0], d[2][1]), v.hz));
   slab_psi_store<0>(p.psiH, x, u);
   slab_psi_store<1>(p.psiH, y, u);
   slab_psi_store<2>(p.psiH, z, u);
@@ -896,13 +926,32 @@ __global__ void __launch_bounds__(SmallCells<C>::v) e_small_3d(const StepParams<
   small_cell<SmallCells<C>::v, PACK>(p.Nz, i, j, k);
   typename MaxBits<C>::type mbits = 0;
   if (j < p.Ny && (PACK || k < p.Nz)) {
+    const unsigned c = ((unsigned)i * p.Ny + j) * p.Nzp + k, b = c * (unsigned)sizeof(T), cb = c * (unsigned)sizeof(C);
+    const bool in = i < p.Nx - 1, jn = j < p.Ny - 1, kn = k < p.Nz - 1, ii = in && i >= 1, jj = jn && j >= 1,
+               kk = kn && k >= 1;
+    const bool u[3] = {in && jj && kk, ii && jn && kk, ii && jj && kn};
+    const unsigned bi = b - (i >= 1 ? (unsigned)p.si * (unsigned)sizeof(T) : 0u),
+                   bj = b - (j >= 1 ? p.Nzp * (unsigned)sizeof(T) : 0u), bk = b - (k >= 1 ? (unsigned)sizeof(T) : 0u);
     ECell<C> v;
-    e_load<T, C, MON>(p, i, j, k, v);
-    const bool u[3] = {v.ux, v.uy, v.uz};
+    v.hx = ld<T, C>(at(p.H[0], b));
+    v.hy = ld<T, C>(at(p.H[1], b));
+    v.hz = ld<T, C>(at(p.H[2], b));
+    v.hz_j = ld<T, C>(at(p.H[2], bj));
+    v.hy_k = ld<T, C>(at(p.H[1], bk));
+    v.hx_k = ld<T, C>(at(p.H[0], bk));
+    v.hz_i = ld<T, C>(at(p.H[2], bi));
+    v.hy_i = ld<T, C>(at(p.H[1], bi));
+    v.hx_j = ld<T, C>(at(p.H[0], bj));
+    v.ex = ld<T, C>(at(p.E[0], b));
+    v.ey = ld<T, C>(at(p.E[1], b));
+    v.ez = ld<T, C>(at(p.E[2], b));
+    v.cbx = *at(p.Cbs[0], cb);
+    v.cby = *at(p.Cbs[1], cb);
+    v.cbz = *at(p.Cbs[2], cb);
     SlabPsi<C> x, y, z;
-    slab_psi_load<0>(p, p.psiE, p.bE[0], p.cE[0], p.rkE[0], i, j, k, u, x);
-    slab_psi_load<1>(p, p.psiE, p.bE[1], p.cE[1], p.rkE[1], i, j, k, u, y);
-    slab_psi_load<2>(p, p.psiE, p.bE[2], p.cE[2], p.rkE[2], i, j, k, u, z);
+    slab_psi_load<0>(p, p.psiE, p.bE[0], p.cE[0], p.rkE[0], i, j, k, x);
+    slab_psi_load<1>(p, p.psiE, p.bE[1], p.cE[1], p.rkE[1], i, j, k, y);
+    slab_psi_load<2>(p, p.psiE, p.bE[2], p.cE[2], p.rkE[2], i, j, k, z);
     const unsigned tf = p.tfsf ? small_plane_axes<SmallCells<C>::v, PACK>(p.planesE, p.Nz) : 0u;
     const Fp<C> fp(k);
     // d[c][part]: Ex: dHz/dy, dHy/dz; Ey: dHx/dz, dHz/dx; Ez: dHy/dx, dHx/dy
@@ -923,15 +972,15 @@ __global__ void __launch_bounds__(SmallCells<C>::v) e_small_3d(const StepParams<
     const C exn = u[0] ? fmaC(v.cbx, fp.sub(d[0][0], d[0][1]), v.ex) : v.ex;
     const C eyn = u[1] ? fmaC(v.cby, fp.sub(d[1][0], d[1][1]), v.ey) : v.ey;
     const C ezn = u[2] ? fmaC(v.cbz, fp.sub(d[2][0], d[2][1]), v.ez) : v.ez;
-    if (u[0]) st<T, C>(p.E[0] + v.c, exn);
-    if (u[1]) st<T, C>(p.E[1] + v.c, eyn);
-    if (u[2]) st<T, C>(p.E[2] + v.c, ezn);
+    if (u[0]) st<T, C>(at(p.E[0], b), exn);
+    if (u[1]) st<T, C>(at(p.E[1], b), eyn);
+    if (u[2]) st<T, C>(at(p.E[2], b), ezn);
     slab_psi_store<0>(p.psiE, x, u);
     slab_psi_store<1>(p.psiE, y, u);
     slab_psi_store<2>(p.psiE, z, u);
-    if (MON && v.mon) {
+    if (MON && in && jn && kn) {
       const C e2 = fmaC(exn, exn, fmaC(eyn, eyn, fp.mul(ezn, ezn)));
-      if (p.etotal) p.etotal[v.c] = e2;
+      if (p.etotal) p.etotal[c] = e2;
       mbits = MaxBits<C>::of(e2);
     }
   }
@@ -1824,27 +1873,37 @@ static void launch_step_3d(const StepParams<T, C>& q, bool mon, bool h_half, boo
   else start(e_kernel_3d<T, C, UNI, false, SLAB, 32>, grid, block, behind, s, q);
 }
 
-// Grids that take the kernels of one cell a thread with every load ahead (h_small_3d).  Us a step
-// with them and without:
-// - FP64 with CPML, while all blocks are resident (10 of 64 threads an SM at 96 registers): 20^3
-//   7.5 and 11.0, 34x30x36 10.0 and 12.4, 44^3 14.6 and 16.3; beyond, the loads a second wave
-//   could overlap wait, 48^3 18.7 and 17.1.  Without CPML the general path has nothing to wait
-//   for: 34^3 9.5 and 9.1.
-// - Float with CPML, up to where the slab paths begin: 34^3 6.2 and 9.2, 64^3 9.4 and 12.0, 100^3
-//   27.3 and 30.4, in FP16 storage 29.1 and 32.2; 128^3 with 6 and 12 cells of CPML 37.0 and
-//   35.4, 43.1 and 45.8, in FP16 storage 41.0 and 35.8, 45.8 and 42.9.
-// - Float without CPML: 26^3 3.9 and 4.6, 64^3 6.9 and 6.9, 100^3 19.1 and 16.0.
+// Half steps that take h_small_3d / e_small_3d.  Us a step with them and without (a launch each):
+// - FP64 while all blocks are resident (10 of 64 threads an SM at 90 registers): 20^3 with CPML 6.7
+//   and 11.0, 34x30x36 9.0 and 12.4, 44^3 13.9 and 19.1; beyond, idle and diverged lanes of the
+//   FP64 pipe cost more than the loads ahead give, 52^3 23.1 and 19.2.  Without CPML to half of
+//   that: 34^3 9.2 and 10.2, 48^3 16.7 and 12.8.
+// - FP32 with CPML, E: 100^3 24.0 and 30.4 (both halves), 128^3 launches of 24.6 and 27.3, 256^3
+//   with CPML 6 150.6 and 152.8, with 25 169 and 187, 512x512x128 311 and 336 (monitored 636 and
+//   674 a step).  H up to 5 M cells if tiled: 118^3 21.9 and 26, 160^3 with CPML 6 and 12 37.5 and
+//   37.9, 38.3 and 40.0; 200^3 72.0 and 69.5, 75.1 and 77.1; 512x512x128 269 and 262: the general
+//   kernel's 64 warps an SM hide more of the memory's latency than these 40.  Packed rows at any
+//   size: 512x512x100 232 and 260, 800x800x40 249 and 320.
+// - FP16 storage with CPML: H 128^3 with CPML 6 and 12 21.4 and 22.2, 21.7 and 23.7, 150^3 44 and
+//   39; E 150^3 45.8 and 46.7 (with CPML 15 42.5 and 46.7), 200^3 113 and 77 (the slab paths there
+//   have 64 warps an SM).
+// - Float without CPML: 64^3 5.7 and 6.4, 73^3 7.7 and 8.5, 80^3 9.5 and 9.2.
+// 32-bit byte offsets: arrays below 2^31 bytes.
 template <class T, class C>
-static bool small_grid(const StepParams<T, C>& p) {
+static bool loads_ahead(const StepParams<T, C>& p, bool h_half, bool pack) {
   const long long cells = (long long)p.Nx * p.Ny * p.Nz;
-  if (sizeof(C) == 8) return p.pml && cells <= 152 * 10 * SmallCells<C>::v;
-  return cells < (p.pml ? 1LL << 20 : 1LL << 18);
+  if (sizeof(C) == 8) return cells <= 152LL * SmallCells<C>::v * (p.pml ? 10 : 5);
+  if ((long long)p.Nx * p.Ny * p.Nzp >= 1LL << 29 || p.Ny > 4 * 65535) return false;
+  if (!p.pml) return cells <= 3LL << 17;
+  if (sizeof(T) == 2) return cells <= (h_half ? 1LL << 21 : 1LL << 22);
+  return !h_half || pack || cells <= 5LL << 20;
 }
 
-// Float rows that fill less than 4/5 of their 32-cell tiles are packed (73^3 FP32 13.5 us a step,
-// in tiles 14.0; 200x200x25 23.1 and 25.3), longer ones keep the rows of a tile together (64^3
-// 9.9, packed 10.9; 90^3 19.1 and 21.3).  FP64 pays a pipe slot for each idle lane and is always
-// packed (34^3 10.0, in tiles 14.2).
+// Float rows that fill less than 4/5 of their 32-cell tiles are packed (us a step, in tiles:
+// 73^3 9.8 and 10.9 with CPML 8, 60x60x100 9.3 and 10.2, 512x512x100 519 and 541), longer ones keep
+// the rows of a tile together (90^3 19.1, packed 21.3; 128^3 43.2 and 53.3 before the 32-bit
+// offsets).  FP64 pays a pipe slot for each idle lane and is always packed (34^3 10.0, in tiles
+// 14.2).
 template <class T, class C, bool PACK>
 static void launch_small_3d(const StepParams<T, C>& p, bool uniform, bool mon, bool h_half, bool behind, cudaStream_t s) {
   constexpr int NT = SmallCells<C>::v;
@@ -1885,8 +1944,8 @@ cudaError_t launch_step(const StepParams<T, C>& p, bool planar, bool uniform, bo
     // The E kernel with float storage takes 16-cell z tiles (LUXUM_ZTILE=32 keeps 32): on the
     // 256^3 drop-in grid E 0.2035 -> 0.189 ms (FP32), 0.200 -> 0.187 (FP16 storage), from its
     // CPML and TF/SF tiles; the H kernel ran 0.015 ms slower with them, CPML or not.
-    if (small_grid<T, C>(p)) {
-      const bool pack = sizeof(C) == 8 || 5LL * p.Nz <= 4LL * ((p.Nz + 31) & ~31);
+    const bool pack = sizeof(C) == 8 || 5LL * p.Nz <= 4LL * ((p.Nz + 31) & ~31);
+    if (loads_ahead<T, C>(p, h_half, pack)) {
       if (pack) launch_small_3d<T, C, true>(p, uniform, mon, h_half, behind, s);
       else if constexpr (sizeof(C) == 4) launch_small_3d<T, C, false>(p, uniform, mon, h_half, behind, s);
       return cudaGetLastError();
@@ -1894,11 +1953,10 @@ cudaError_t launch_step(const StepParams<T, C>& p, bool planar, bool uniform, bo
     StepParams<T, C> q = p;
     q.zends = sizeof(T) == 8 && p.pml && p.slab[2].n > 0 && p.slab[2].lo <= 16 && p.Nz - p.slab[2].hi0 <= 16 &&
               p.Nz >= 48;
-    // Float grids of 2^20 cells or more give blocks in the slab of one axis their own path
-    // (h_slab_3d): us a step with and without it, 512x512x128 FP32 (CPML 20) 592 and 654, 256^3
-    // (CPML 16, TF/SF) 299 and 324, in FP16 storage 268 and 299, 150^3 (CPML 12) 82.9 and 88.4,
-    // 100^3 30.7 and 30.8, 73^3 16.9 and 16.6 (the longer code costs a short launch more than the
-    // path saves).  FP64 is bound by its pipe.
+    // Float half steps beyond those give blocks in the slab of one axis their own path (h_slab_3d):
+    // us a step of both with and without it, 512x512x128 FP32 (CPML 20) 592 and 654, 256^3 (CPML
+    // 16, TF/SF) 299 and 324, in FP16 storage 268 and 299; from 2^20 cells, as the longer code costs
+    // a short launch more than the path saves.  FP64 is bound by its pipe.
     bool slab = false;
     if constexpr (sizeof(C) == 4) slab = p.pml && (long long)p.Nx * p.Ny * p.Nz >= (1LL << 20);
     if constexpr (sizeof(C) == 4)

@@ -1,10 +1,11 @@
-"""Small 3-D grids, whose kernels issue every load ahead and pack rows that fill their tiles badly:
-the bits of the members of a batch, which march through the general cell code.  DFT planes that
+"""3-D grids whose kernels issue every load ahead and pack rows that fill their tiles badly: the bits
+of the members of a batch, which march through the general cell code, or of the single sweep.  DFT planes that
 split their frequencies over blocks: the bits of a batch's accumulation, which walks them in order."""
 import numpy as np
 import pytest
 
 import cases
+from test_gpu_sweep import _big3, _pair, _same
 
 pytestmark = pytest.mark.gpu
 
@@ -51,6 +52,21 @@ def _march(make, steps=19):
 def test_small_grids_equal_batch_members(engine, precision, n, pml, tf, dy):
     for s in _march(lambda: _sim(n, precision, pml, tf, dy)):
         s.close()
+
+
+# Larger float grids: both halves, E only, packed; against the independently written single sweep.
+@pytest.mark.parametrize("precision", [1, 2])
+@pytest.mark.parametrize("uniform, n", [(True, (101, 103, 105)), (False, (129, 128, 128)), (True, (150, 149, 151)),
+                                        (False, (176, 175, 177)), (True, (260, 259, 65))])
+def test_loads_ahead_equal_single_sweep(engine, precision, uniform, n):
+    p, boxes = _big3(precision, uniform, n)
+    a, b = _pair(p, boxes)
+    a.step(37)
+    b.step(37)
+    _same(a, b)
+    assert a.max_e2() == b.max_e2() > 0
+    a.close()
+    b.close()
 
 
 # 128 x 152 cells fill the 304 blocks from which a plane walks its frequencies in order
