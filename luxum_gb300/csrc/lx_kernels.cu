@@ -300,6 +300,19 @@ __device__ __forceinline__ void h_cell_3d(const StepParams<T, C>& p, const int i
   h_apply<T, C, UNI, FAST>(p, i, j, k, tf, v);
 }
 
+// An array's element at a byte offset (an unsigned 32-bit one is added by the load instruction).
+template <class T, class O>
+__device__ __forceinline__ const T* at(const T* p, O o) {
+  return reinterpret_cast<const T*>(reinterpret_cast<const char*>(p) + o);
+}
+template <class T, class O>
+__device__ __forceinline__ T* at(T* p, O o) {
+  return reinterpret_cast<T*>(reinterpret_cast<char*>(p) + o);
+}
+
+// Paths of a block: the slab of one axis (0, 1, 2), none, the general code, interior.
+constexpr int kNoSlab = 3, kGeneral = 4, kInside = 5;
+
 // Whether the slab paths also take blocks that meet TF/SF planes: FP16 storage, bound by
 // instructions (201x187x259 193 -> 189 us a step).  FP32 is bound by memory and lost to the longer
 // code more than it gained (512x512x128 598 -> 611).
@@ -309,17 +322,17 @@ constexpr bool kSlabTf = sizeof(T) == 2;
 // The two psi terms of a cell in the slab of one axis AX: both half steps form the derivative
 // along AX in part 1 of component AX+1 and part 0 of component AX+2, with one profile and one
 // index for both.  Loaded with the cell's fields, ahead of every store (see h_load).
-template <class C>
+template <class C, class Off>
 struct AxisPsi {
   bool on;
-  long long q;
+  Off q;         // in bytes
   C a, b;        // psi of component AX+1 part 1, AX+2 part 0
   C fb, fc, rk;  // profile b, c, 1/kappa
 };
 
-template <class T, class C, int AX>
+template <class T, class C, int AX, class Off>
 __device__ __forceinline__ void axis_psi_load(const StepParams<T, C>& p, C* const (&psi)[3][2], const C* fb, const C* fc,
-                                              const C* rk, int i, int j, int k, unsigned o, AxisPsi<C>& w) {
+                                              const C* rk, int i, int j, int k, unsigned o, AxisPsi<C, Off>& w) {
   const int u = AX == 0 ? i : (AX == 1 ? j : k);
   const int s = u < p.free0[AX] ? u : u - p.free1[AX] + p.free0[AX];
   w.on = AX == 0 || u < p.free0[AX] || u >= p.free1[AX];
@@ -328,17 +341,17 @@ __device__ __forceinline__ void axis_psi_load(const StepParams<T, C>& p, C* cons
     const unsigned n = p.slab[AX].n;
     const long long base = AX == 0 ? (long long)s * p.si : (AX == 1 ? (long long)i * n * p.Nzp : (long long)i * p.Ny * n);
     const unsigned q = AX == 0 ? o : (AX == 1 ? (unsigned)s * p.Nzp + k : (unsigned)j * n + s);
-    w.q = base + q;
-    w.a = psi[(AX + 1) % 3][1][w.q];
-    w.b = psi[(AX + 2) % 3][0][w.q];
+    w.q = (Off)(base + q) * (Off)sizeof(C);
+    w.a = *at(psi[(AX + 1) % 3][1], w.q);
+    w.b = *at(psi[(AX + 2) % 3][0], w.q);
     w.fb = __ldg(fb + u);
     w.fc = __ldg(fc + u);
     w.rk = __ldg(rk + u);
   }
 }
 // pml_term's arithmetic on a loaded psi.
-template <class C>
-__device__ __forceinline__ void axis_psi_term(const AxisPsi<C>& w, C& psi, C& d) {
+template <class C, class Off>
+__device__ __forceinline__ void axis_psi_term(const AxisPsi<C, Off>& w, C& psi, C& d) {
   psi = fmaC(w.fb, psi, w.fc * d);
   d = fmaC(d, w.rk, psi);
 }
@@ -382,7 +395,7 @@ __device__ __forceinline__ void h_slab_3d(const StepParams<T, C>& p, const int i
   }
   const bool u[3] = {v.ux, v.uy, v.uz};
   constexpr int A = (AX + 1) % 3, B = (AX + 2) % 3;
-  AxisPsi<C> w;
+  AxisPsi<C, long long> w;
   if constexpr (AX < 3) {
     if constexpr (kPlain) {
       axis_psi_load<T, C, AX>(p, p.psiH, p.bH[AX], p.cH[AX], p.rkH[AX], i, j, k, o, w);
@@ -393,9 +406,9 @@ __device__ __forceinline__ void h_slab_3d(const StepParams<T, C>& p, const int i
       w.a = w.b = w.fb = w.fc = w.rk = C(0);
       w.q = 0;
       if (w.on) {
-        w.q = psi_index(AX, p.slab[AX], sl, i, j, k, p.Ny, p.Nzp);
-        if (u[A]) w.a = p.psiH[A][1][w.q];
-        if (u[B]) w.b = p.psiH[B][0][w.q];
+        w.q = psi_index(AX, p.slab[AX], sl, i, j, k, p.Ny, p.Nzp) * (long long)sizeof(C);
+        if (u[A]) w.a = *at(p.psiH[A][1], w.q);
+        if (u[B]) w.b = *at(p.psiH[B][0], w.q);
         w.fb = __ldg(p.bH[AX] + n);
         w.fc = __ldg(p.cH[AX] + n);
         w.rk = __ldg(p.rkH[AX] + n);
@@ -429,8 +442,8 @@ __device__ __forceinline__ void h_slab_3d(const StepParams<T, C>& p, const int i
     if (w.on) {
       if (kPlain || u[A]) axis_psi_term(w, w.a, d[A][1]);
       if (kPlain || u[B]) axis_psi_term(w, w.b, d[B][0]);
-      if (u[A]) p.psiH[A][1][w.q] = w.a;
-      if (u[B]) p.psiH[B][0][w.q] = w.b;
+      if (u[A]) *at(p.psiH[A][1], w.q) = w.a;
+      if (u[B]) *at(p.psiH[B][0], w.q) = w.b;
     }
   }
   if (u[0]) st<T, C>(p.H[0] + v.c, fmaC(-p.Dbs, d[0][0] - d[0][1], v.hx));
@@ -446,7 +459,6 @@ __device__ __forceinline__ bool tile_in(const StepParams<T, C>& p, int i, int j0
 
 // The path of a block that is not interior: kGeneral when it meets the slabs of two axes, an x wall or
 // (FP32) a TF/SF plane, else the axis of the one slab it meets, or kNoSlab.
-constexpr int kNoSlab = 3, kGeneral = 4;
 template <class T, class C>
 __device__ __forceinline__ int slab_path(const StepParams<T, C>& p, unsigned tf, int i, int j0, int nj, int k0, int nk) {
   if (i < 1 || i > p.Nx - 2) return kGeneral;
@@ -662,21 +674,27 @@ __device__ __forceinline__ typename MaxBits<C>::type e_cell_3d(const StepParams<
 }
 
 // E of a cell on planes 1 .. Nx-2 whose block meets the CPML slab of axis AX only
-// (see h_slab_3d): e_apply's arithmetic.
+// (see h_slab_3d): e_apply's arithmetic.  FP16 storage reads at 32-bit byte offsets and takes
+// interior cells too (201x187x259 E 108 -> 104 us a launch, 256^3 monitored 191 -> 165; the same in
+// h_slab_3d cost H 4-8 us of 92 there and 9 of 262 at 512x512x128 FP32); FP32 comes here with
+// arrays that such offsets do not reach.
 template <class T, class C, bool UNI, bool MON, int AX>
 __device__ __forceinline__ typename MaxBits<C>::type e_slab_3d(const StepParams<T, C>& p, const int i, const int j,
                                                                const int k, const unsigned tf) {
+  using Off = std::conditional_t<sizeof(T) == 2, unsigned, long long>;
   const unsigned o = (unsigned)j * (unsigned)p.Nzp + (unsigned)k;
-  const long long c = (long long)i * p.si + o;
-  const C hx = ld<T, C>(p.H[0] + c), hy = ld<T, C>(p.H[1] + c), hz = ld<T, C>(p.H[2] + c);
-  const C hz_j = ld<T, C>(p.H[2] + c - p.Nzp), hx_j = ld<T, C>(p.H[0] + c - p.Nzp);
-  const C hy_k = ld<T, C>(p.H[1] + c - 1), hx_k = ld<T, C>(p.H[0] + c - 1);
-  const C hz_i = ld<T, C>(p.H[2] + c - p.si), hy_i = ld<T, C>(p.H[1] + c - p.si);
-  const C ex = ld<T, C>(p.E[0] + c), ey = ld<T, C>(p.E[1] + c), ez = ld<T, C>(p.E[2] + c);
-  const C cb[3] = {p.Cbs[0][c], p.Cbs[1][c], p.Cbs[2][c]};
-  AxisPsi<C> w;
+  const Off c = (Off)i * (Off)p.si + o, b = c * (Off)sizeof(T), bi = b - (Off)p.si * (Off)sizeof(T),
+            bj = b - p.Nzp * (Off)sizeof(T), bc = c * (Off)sizeof(C);
+  const C hx = ld<T, C>(at(p.H[0], b)), hy = ld<T, C>(at(p.H[1], b)), hz = ld<T, C>(at(p.H[2], b));
+  const C hz_j = ld<T, C>(at(p.H[2], bj)), hx_j = ld<T, C>(at(p.H[0], bj));
+  const C hy_k = ld<T, C>(at(p.H[1], b) - 1), hx_k = ld<T, C>(at(p.H[0], b) - 1);
+  const C hz_i = ld<T, C>(at(p.H[2], bi)), hy_i = ld<T, C>(at(p.H[1], bi));
+  const C ex = ld<T, C>(at(p.E[0], b)), ey = ld<T, C>(at(p.E[1], b)), ez = ld<T, C>(at(p.E[2], b));
+  const C cb[3] = {*at(p.Cbs[0], bc), *at(p.Cbs[1], bc), *at(p.Cbs[2], bc)};
+  AxisPsi<C, Off> w;
   if constexpr (AX < 3) axis_psi_load<T, C, AX>(p, p.psiE, p.bE[AX], p.cE[AX], p.rkE[AX], i, j, k, o, w);
-  const bool jn = j < p.Ny - 1, kn = k < p.Nz - 1, jj = j >= 1 && jn, kk = k >= 1 && kn;
+  constexpr bool in = AX == kInside;
+  const bool jn = in || j < p.Ny - 1, kn = in || k < p.Nz - 1, jj = in || (j >= 1 && jn), kk = in || (k >= 1 && kn);
   const bool u[3] = {jj && kk, jn && kk, jj && kn};
   // d[c][part]: Ex: dHz/dy, dHy/dz; Ey: dHx/dz, dHz/dx; Ez: dHy/dx, dHx/dy
   C d[3][2] = {{hz - hz_j, hy - hy_k}, {hx - hx_k, hz - hz_i}, {hy - hy_i, hx - hx_j}};
@@ -687,7 +705,7 @@ __device__ __forceinline__ typename MaxBits<C>::type e_slab_3d(const StepParams<
       d[m][1] = mulC(d[m][1], p.rd[(m + 2) % 3]);
     }
   }
-  if (kSlabTf<T> && tf) {
+  if (kSlabTf<T> && !in && tf) {
     if (tf & 1u) {
       tfsf_axis<0, C>(p.setsE[1][1], p.tab, i, j, k, d[1][1]);
       tfsf_axis<0, C>(p.setsE[2][0], p.tab, i, j, k, d[2][0]);
@@ -706,34 +724,40 @@ __device__ __forceinline__ typename MaxBits<C>::type e_slab_3d(const StepParams<
     if (w.on) {
       axis_psi_term(w, w.a, d[A][1]);
       axis_psi_term(w, w.b, d[B][0]);
-      if (u[A]) p.psiE[A][1][w.q] = w.a;
-      if (u[B]) p.psiE[B][0][w.q] = w.b;
+      if (u[A]) *at(p.psiE[A][1], w.q) = w.a;
+      if (u[B]) *at(p.psiE[B][0], w.q) = w.b;
     }
   }
   const C exn = u[0] ? fmaC(cb[0], d[0][0] - d[0][1], ex) : ex;
   const C eyn = u[1] ? fmaC(cb[1], d[1][0] - d[1][1], ey) : ey;
   const C ezn = u[2] ? fmaC(cb[2], d[2][0] - d[2][1], ez) : ez;
-  if (u[0]) st<T, C>(p.E[0] + c, exn);
-  if (u[1]) st<T, C>(p.E[1] + c, eyn);
-  if (u[2]) st<T, C>(p.E[2] + c, ezn);
+  if (u[0]) st<T, C>(at(p.E[0], b), exn);
+  if (u[1]) st<T, C>(at(p.E[1], b), eyn);
+  if (u[2]) st<T, C>(at(p.E[2], b), ezn);
   if (!(MON && jn && kn)) return 0;
   const C e2 = fmaC(exn, exn, fmaC(eyn, eyn, ezn * ezn));
   if (p.etotal) p.etotal[c] = e2;
   return MaxBits<C>::of(e2);
 }
 
-// Resident blocks per SM asked of the compiler for the 3-D E kernel: FP16 storage takes 8 (32
-// registers, about 30 bytes spilled) together with the interior fast path, 0.3196 -> 0.3116 ms
-// per 256^3 step (each alone was slower: the fast path 0.332, the cap 0.356); FP32 storage runs
-// best at 40 (6 blocks; 8 cost it 4 %), and FP64 with its FMA forms at 6 blocks (256^3 with CPML
-// and TF/SF 0.431 -> 0.415 ms against the compiler's own 60 registers).
-template <class T>
+template <class T, class C, bool UNI, bool MON, bool SLAB>
+__device__ __forceinline__ typename MaxBits<C>::type e_in_3d(const StepParams<T, C>& p, const int i, const int j, const int k) {
+  if constexpr (SLAB && sizeof(T) == 2) return e_slab_3d<T, C, UNI, MON, kInside>(p, i, j, k, 0u);
+  else return e_cell_3d<T, C, UNI, MON, true>(p, i, j, k, false);
+}
+
+// Resident blocks per SM asked of the compiler for the 3-D E kernel.  FP16 storage with the slab
+// paths' 32-bit offsets and FP32 run best at 40 registers (6 blocks; us an E launch of 201x187x259
+// FP16 104 against 108 with 8, 256^3 145 and 147, monitored 165 and 172), FP16 without CPML at 32
+// with a few spilled (256^3 0.3196 -> 0.3116 ms a step), and FP64 with its FMA forms at 6 blocks
+// (256^3 with CPML and TF/SF 0.431 -> 0.415 ms against the compiler's own 60 registers).
+template <class T, bool SLAB>
 struct EMinBlocks {
-  static constexpr int v = sizeof(T) == 2 ? 8 : 6;
+  static constexpr int v = sizeof(T) == 2 && !SLAB ? 8 : 6;
 };
 
 template <class T, class C, bool UNI, bool MON, bool SLAB, int ZW>
-__global__ void __launch_bounds__(256, EMinBlocks<T>::v) e_kernel_3d(const StepParams<T, C> p) {
+__global__ void __launch_bounds__(256, EMinBlocks<T, SLAB>::v) e_kernel_3d(const StepParams<T, C> p) {
   step_behind();
   step_open();
   constexpr int RY = 256 / ZW;
@@ -747,7 +771,7 @@ __global__ void __launch_bounds__(256, EMinBlocks<T>::v) e_kernel_3d(const StepP
   typename MaxBits<C>::type mbits = 0;
   if (z.valid && j < p.Ny) {
     if (!tf && z.n1 == 0 && tile_in(p, i, blockIdx.y * RY, RY, z.lo0, z.n0))
-      mbits = e_cell_3d<T, C, UNI, MON, true>(p, i, j, k, false);
+      mbits = e_in_3d<T, C, UNI, MON, SLAB>(p, i, j, k);
     else {
       const int path = SLAB ? slab_path(p, tf, i, blockIdx.y * RY, RY, z.lo0, z.n0) : kGeneral;
       if (path == 0) mbits = e_slab_3d<T, C, UNI, MON, 0>(p, i, j, k, tf);
@@ -773,14 +797,6 @@ __global__ void __launch_bounds__(256, EMinBlocks<T>::v) e_kernel_3d(const StepP
 // itself, and only the stores ask whether the cell updates.  Blocks are small, to reach more SMs
 // (128 threads; with 256 100^3 24.9 us a step against 23.8, 512x512x128 622 against 584).  H
 // is capped at 48 registers (200^3 H 78.8 us against 82.4, E, at 56, 94.3 against 93.7).
-template <class T>
-__device__ __forceinline__ const T* at(const T* p, unsigned o) {
-  return reinterpret_cast<const T*>(reinterpret_cast<const char*>(p) + o);
-}
-template <class T>
-__device__ __forceinline__ T* at(T* p, unsigned o) {
-  return reinterpret_cast<T*>(reinterpret_cast<char*>(p) + o);
-}
 template <class C>
 struct SlabPsi {
   bool on;
@@ -1958,7 +1974,8 @@ cudaError_t launch_step(const StepParams<T, C>& p, bool planar, bool uniform, bo
     // 16, TF/SF) 299 and 324, in FP16 storage 268 and 299; from 2^20 cells, as the longer code costs
     // a short launch more than the path saves.  FP64 is bound by its pipe.
     bool slab = false;
-    if constexpr (sizeof(C) == 4) slab = p.pml && (long long)p.Nx * p.Ny * p.Nz >= (1LL << 20);
+    const bool reach = sizeof(T) != 2 || (long long)p.Nx * p.Ny * p.Nzp < (1LL << 30);  // e_slab_3d's offsets
+    if constexpr (sizeof(C) == 4) slab = p.pml && reach && (long long)p.Nx * p.Ny * p.Nz >= (1LL << 20);
     if constexpr (sizeof(C) == 4)
       if (slab) {
         if (uniform) launch_step_3d<T, C, true, true>(q, mon, h_half, behind, s);

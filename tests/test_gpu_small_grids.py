@@ -54,10 +54,11 @@ def test_small_grids_equal_batch_members(engine, precision, n, pml, tf, dy):
         s.close()
 
 
-# Larger float grids: both halves, E only, packed; against the independently written single sweep.
+# Larger float grids: both halves, E only, packed, neither or E only again; against the independently written single sweep.
 @pytest.mark.parametrize("precision", [1, 2])
 @pytest.mark.parametrize("uniform, n", [(True, (101, 103, 105)), (False, (129, 128, 128)), (True, (150, 149, 151)),
-                                        (False, (176, 175, 177)), (True, (260, 259, 65))])
+                                        (False, (176, 175, 177)), (True, (260, 259, 65)), (True, (180, 176, 190)),
+                                        (False, (176, 191, 180))])
 def test_loads_ahead_equal_single_sweep(engine, precision, uniform, n):
     p, boxes = _big3(precision, uniform, n)
     a, b = _pair(p, boxes)
