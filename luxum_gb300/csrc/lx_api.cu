@@ -2053,13 +2053,13 @@ struct lx_batch {
   // block passed by value (the constant bank, as for a handle stepped alone), spread over the
   // batch stream and kLanes - 1 more so that the members' kernels overlap.  Planar members with
   // float compute step in their two buffers (ping-pong mode): of at least kSoloCells2 cells one
-  // by one like these, smaller ones together in the batched sweep.  Planar FP64 members and
-  // smaller 3-D ones share the batched half-step launches in place.
+  // by one like these, a few smaller ones together in the batched sweep (see batch_rebuild).  The
+  // others share the batched half-step launches in place.
   static constexpr long long kSoloCells = 1LL << 18;
   // (us a step of 48 lenses of side 128-1024, 12 and 96 of them, 16 of side 1000, one by one from
-  // 2^21, 2^20 and 2^19 cells: 142, 138, 135; 43, 39, 38; 226, 222, 211; 140, 134, 143.  Launched
-  // directly a member's step costs the host 2 us.)
-  static constexpr long long kSoloCells2 = 1LL << 20;
+  // 2^21, 2^20 and 2^19 cells: 142, 138, 135; 43, 39, 38; 226, 222, 211; 140, 134, 143; 256 of them
+  // 107, 106 and 113 Gcell/s.  Launched directly a member's step costs the host 2 us.)
+  static constexpr long long kSoloCells2 = 1LL << 19;
   static constexpr int kLanes = 4;
   cudaStream_t lanes[kLanes - 1] = {};
   cudaEvent_t lane_ev[kLanes] = {};  // [0] fork, [1..] joins
@@ -2113,11 +2113,17 @@ struct lx_batch {
 
 static void batch_member_changed(lx_batch* b) { b->dirty = true; }
 
-// A member launched one by one, with no tile shape: 3-D members of kSoloCells cells or more,
-// planar single-sweep members of kSoloCells2 cells or more.
+// A member launched one by one: 3-D members of kSoloCells cells or more, planar single-sweep
+// members of kSoloCells2 cells or more.
 static bool batch_alone(const lx_sim* s) {
   return s->planar ? s->sweep && (long long)s->Nx * s->Nz >= lx_batch::kSoloCells2
                    : (long long)s->Nx * s->Ny * s->Nz >= lx_batch::kSoloCells;
+}
+
+// A member the tuner takes no sample of: it never shares a launch.  (Planar members between
+// kSoloCells2 and this keep their entry in the table.)
+static bool batch_untuned(const lx_sim* s) {
+  return s->planar ? s->sweep && (long long)s->Nx * s->Nz >= 1LL << 21 : batch_alone(s);
 }
 
 // The tile-shape class of a handle: dimension, floor(log4(cells)), precision, x slab depth.
@@ -2310,12 +2316,24 @@ static lx_status batch_rebuild(lx_batch* b) {
   BCK(cudaMallocAsync(&b->d_slots, sizeof(unsigned long long) * lx::kAhead * (n > 0 ? n : 1), b->stream));
   BCK(cudaMallocAsync(&b->d_srcv, sizeof(double) * lx::kAhead * (n > 0 ? n : 1), b->stream));
   std::vector<std::vector<lx::DftParams>> dft_planes;
-  // Planar float members step in their two buffers, the others in place in buffer 0; a member
-  // whose mode changes at an odd step moves its state (one device copy).
+  // Planar float members step in their two buffers, one by one or while those that share a launch
+  // are few, the others in place in buffer 0; a member whose mode changes at an odd step moves its
+  // state (one device copy).  The batched sweep has one launch a step and half the latency; many
+  // small members, whose rows are mostly CPML, run faster in the two half-step launches at twice the
+  // warps, FP16 storage sooner.  Gcell/s of the sweep and of those, FP32: 100 lenses of side 128-300
+  // 53 and 77, 256 of 128-400 69 and 85 (48 of 128-256 66 and 47, 128-700 96 and 75 before their
+  // tables were formed ahead); FP16: 48 of 128-700 79 and 107, 100 of 128-300 41 and 79.
+  long long shared = 0, shared_cells = 0;
+  for (auto* s : b->sims)
+    if (s->planar && s->sweep && !batch_alone(s)) {
+      shared++;
+      shared_cells += (long long)s->Nx * s->Nz;
+    }
+  const bool few = shared <= lx::kSweepMembers && (sizeof(T) == 4 || shared_cells <= 1LL << 22);
   for (int q = 0; q < n; q++) {
     lx_sim* s = b->sims[q];
     lx_status st;
-    if ((st = set_pp(s, s->planar && s->sweep))) return st;
+    if ((st = set_pp(s, s->planar && s->sweep && (few || batch_alone(s))))) return st;
     BCK(cudaStreamSynchronize(s->stream));
   }
   std::vector<C*> tabs(n, nullptr);
@@ -2815,7 +2833,7 @@ extern "C" LX_API lx_status lx_batch_autotune(lx_batch* b, int steps, int* plana
   std::vector<const lx_sim*> sample;
   double sampled = 0.0;
   for (auto* s : b->sims) {
-    if (batch_alone(s)) continue;
+    if (batch_untuned(s)) continue;
     const lx_tune_entry k = tune_class_of(s);
     size_t c = 0;
     while (c < classes.size() && !same_class(classes[c], k)) c++;
@@ -2899,7 +2917,7 @@ extern "C" LX_API lx_status lx_batch_tune_member(lx_batch* b, const lx_sim* s, i
   lx::DeviceGuard dg_(b->device);
   lx_status st = lx_batch_wait(b);
   if (st) return st;
-  if (batch_alone(s)) return LX_OK;
+  if (batch_untuned(s)) return LX_OK;
   // Twins of the handle alone, replicated to 2^24 cells or 64 twins: a batch of hundreds of
   // members fills the GPU many times over, and a sample that fills it once or less favours
   // short marches (16 twins of a 300^2 lens picked 2 where the full batch runs best at 8).
