@@ -203,21 +203,20 @@ def kernel_model(sim, p):
     H (3); E kernel reads H (3), E (3), Cb (3) and writes E (3); each stored psi entry is
     read and written once.  FP64 instructions per component: 2 differences, 1 subtraction
     and 1 FMA (4); per psi term: psi = b*psi + c*d (a multiply and an FMA) and d/kappa + psi
-    (an FMA), 3; with the max monitor every step the E kernel also forms
-    |E|^2 = Ex^2 + Ey^2 + Ez^2 per cell (a multiply and two FMAs, 3).  Flops count an FMA as 2.
+    (an FMA), 3.  The max monitor's |E|^2 is not counted: the E kernel screens cells without the
+    FP64 pipe and forms it for few.  Flops count an FMA as 2.
     """
     info = sim.info()
     el = info["field_bytes"]
     cel = 8 if p.precision == 0 else 4
     cells = info["cells"]
     psi_h, psi_e = info["psi_h_entries"], info["psi_e_entries"]
-    mon = p.monitor_every == 1
     h_bytes = cells * 9 * el + psi_h * 2 * cel
     e_bytes = cells * 9 * el + cells * 3 * cel + psi_e * 2 * cel
     h_ops = cells * 12 + psi_h * 3
-    e_ops = cells * 12 + psi_e * 3 + (cells * 3 if mon else 0)
+    e_ops = cells * 12 + psi_e * 3
     h_flops = cells * 15 + psi_h * 5
-    e_flops = cells * 15 + psi_e * 5 + (cells * 5 if mon else 0)
+    e_flops = cells * 15 + psi_e * 5
     return {"h_update": (h_bytes, h_ops, h_flops), "e_update": (e_bytes, e_ops, e_flops)}
 
 

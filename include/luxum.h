@@ -260,12 +260,13 @@ LX_API lx_status lx_hdf5_write(const char* path, int ndatasets, const char* cons
 LX_API lx_status lx_hdf5_read(const char* path, const char* dataset, double* out, size_t n, int shape[3]);
 
 /* ---- batches: many independent simulations stepped together (engine feature) ----
- * Member handles keep their own device state; each step runs one prologue launch, one H and
- * one E launch per group of members sharing (planar, uniform spacing) over a tile table of
- * all of them, one launch for every member's DFT planes and a step-counter tick.  3-D
- * members of 2^18 cells or more instead take one H and one E launch each, spread over four
- * streams so that they overlap.  Members are updated in place (planar FP32/FP16 handles
- * move their state into their first buffer on joining).  From the second chunk
+ * Member handles keep their own device state; a step runs one H and one E launch per group
+ * of members sharing (planar, uniform spacing) over a tile table of all of them (a few planar
+ * FP32/FP16 members one launch for both, from one of their two buffers into the other) and
+ * one launch for the grouped members' DFT planes; a prologue forms several steps' tables at
+ * once and a tick ends a chunk.  3-D members of 2^18 cells or more and planar FP32/FP16
+ * members of 2^19 or more instead take launches of their own, spread over four streams so
+ * that they overlap.  From the second chunk
  * after a change of members on, chunks of steps are captured once as a CUDA graph and replayed
  * (the first is launched directly, so that a batch whose members change every chunk never
  * waits for a capture).  All members share one precision;
@@ -310,7 +311,7 @@ LX_API lx_status lx_batch_set_tune_table(lx_batch* b, const lx_tune_entry* entri
 /* Copies up to cap entries to entries (may be NULL when cap is 0); *n = the table's length. */
 LX_API lx_status lx_batch_get_tune_table(const lx_batch* b, lx_tune_entry* entries, int cap, int* n);
 /* Tunes the class of every batched member (3-D members of 2^18 cells or more and planar
- * single-sweep members are launched one by one and have no tile shape).  Zero-field twins of
+ * single-sweep members of 2^21 are launched one by one and have no tile shape).  Zero-field twins of
  * a sample of the members (up to 1.5e8 cells, at least one per class; created and freed here)
  * are stepped together, `steps` steps per timing: first with one march for every class, then
  * with each class in turn (largest first) moved to each other march, a move kept when the
