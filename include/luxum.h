@@ -265,7 +265,7 @@ LX_API lx_status lx_hdf5_read(const char* path, const char* dataset, double* out
  * FP32/FP16 members one launch for both, from one of their two buffers into the other) and
  * one launch for the grouped members' DFT planes; a prologue forms several steps' tables at
  * once and a tick ends a chunk.  3-D members of 2^18 cells or more and planar FP32/FP16
- * members of 2^19 or more instead take launches of their own, spread over four streams so
+ * members of 2^19-2^20 or more instead take launches of their own, spread over four streams so
  * that they overlap.  From the second chunk
  * after a change of members on, chunks of steps are captured once as a CUDA graph and replayed
  * (the first is launched directly, so that a batch whose members change every chunk never

@@ -2058,8 +2058,11 @@ struct lx_batch {
   static constexpr long long kSoloCells = 1LL << 18;
   // (us a step of 48 lenses of side 128-1024, 12 and 96 of them, 16 of side 1000, one by one from
   // 2^21, 2^20 and 2^19 cells: 142, 138, 135; 43, 39, 38; 226, 222, 211; 140, 134, 143; 256 of them
-  // 107, 106 and 113 Gcell/s.  Launched directly a member's step costs the host 2 us.)
+  // 107, 106 and 113 Gcell/s.  Launched directly a member's step costs the host 2 us: a served burst
+  // of 32 requests 91.1 and 96.3 ms from 2^20 and 2^19.)  Twice that in an FP32 batch whose planar
+  // members all fit one sweep launch.
   static constexpr long long kSoloCells2 = 1LL << 19;
+  long long solo_cells2 = kSoloCells2;
   static constexpr int kLanes = 4;
   cudaStream_t lanes[kLanes - 1] = {};
   cudaEvent_t lane_ev[kLanes] = {};  // [0] fork, [1..] joins
@@ -2114,16 +2117,17 @@ struct lx_batch {
 static void batch_member_changed(lx_batch* b) { b->dirty = true; }
 
 // A member launched one by one: 3-D members of kSoloCells cells or more, planar single-sweep
-// members of kSoloCells2 cells or more.
-static bool batch_alone(const lx_sim* s) {
-  return s->planar ? s->sweep && (long long)s->Nx * s->Nz >= lx_batch::kSoloCells2
+// members of solo_cells2 cells or more.
+static bool batch_alone(const lx_batch* b, const lx_sim* s) {
+  return s->planar ? s->sweep && (long long)s->Nx * s->Nz >= b->solo_cells2
                    : (long long)s->Nx * s->Ny * s->Nz >= lx_batch::kSoloCells;
 }
 
-// A member the tuner takes no sample of: it never shares a launch.  (Planar members between
-// kSoloCells2 and this keep their entry in the table.)
+// A member the tuner takes no sample of: it never shares a launch.  (Smaller planar members
+// keep their entry in the table.)
 static bool batch_untuned(const lx_sim* s) {
-  return s->planar ? s->sweep && (long long)s->Nx * s->Nz >= 1LL << 21 : batch_alone(s);
+  return s->planar ? s->sweep && (long long)s->Nx * s->Nz >= 1LL << 21
+                   : (long long)s->Nx * s->Ny * s->Nz >= lx_batch::kSoloCells;
 }
 
 // The tile-shape class of a handle: dimension, floor(log4(cells)), precision, x slab depth.
@@ -2323,9 +2327,11 @@ static lx_status batch_rebuild(lx_batch* b) {
   // warps, FP16 storage sooner.  Gcell/s of the sweep and of those, FP32: 100 lenses of side 128-300
   // 53 and 77, 256 of 128-400 69 and 85 (48 of 128-256 66 and 47, 128-700 96 and 75 before their
   // tables were formed ahead); FP16: 48 of 128-700 79 and 107, 100 of 128-300 41 and 79.
-  long long shared = 0, shared_cells = 0;
+  long long shared = 0, shared_cells = 0, sweeps = 0;
+  for (auto* s : b->sims) sweeps += s->planar && s->sweep;
+  b->solo_cells2 = lx_batch::kSoloCells2 * (sizeof(T) == 4 && sweeps <= lx::kSweepMembers ? 2 : 1);
   for (auto* s : b->sims)
-    if (s->planar && s->sweep && !batch_alone(s)) {
+    if (s->planar && s->sweep && !batch_alone(b, s)) {
       shared++;
       shared_cells += (long long)s->Nx * s->Nz;
     }
@@ -2333,7 +2339,7 @@ static lx_status batch_rebuild(lx_batch* b) {
   for (int q = 0; q < n; q++) {
     lx_sim* s = b->sims[q];
     lx_status st;
-    if ((st = set_pp(s, s->planar && s->sweep && (few || batch_alone(s))))) return st;
+    if ((st = set_pp(s, s->planar && s->sweep && (few || batch_alone(b, s))))) return st;
     BCK(cudaStreamSynchronize(s->stream));
   }
   std::vector<C*> tabs(n, nullptr);
@@ -2349,7 +2355,7 @@ static lx_status batch_rebuild(lx_batch* b) {
     b->sources |= s->src_kind >= 0;
     b->max_entries = std::max(b->max_entries, pps[q].tab_total);
     b->host_ts[q] = s->t;
-    const bool solo = batch_alone(s);
+    const bool solo = batch_alone(b, s);
     T* pf[6] = {(T*)s->E[0], (T*)s->E[1], (T*)s->E[2], (T*)s->H[0], (T*)s->H[1], (T*)s->H[2]};
     for (auto& d : s->dfts) {
       if (b->chunk > 0 && b->chunk % d.every != 0) b->graphable = false;
