@@ -1995,7 +1995,9 @@ cudaError_t launch_step(const StepParams<T, C>& p, bool planar, bool uniform, bo
 // 111.6, 112.8.
 static int sweep_rows(long long cols, int Nx) {
   const double U = (double)cols * Nx / (152.0 * 8 * kSweepMinBlocks);
-  return U < 8 ? 2 : (U < 60 ? 4 : 6);
+  const int R = U < 8 ? 2 : (U < 60 ? 4 : 6);
+  const int least = (int)(((long long)Nx + 8 * 65535 - 1) / (8 * 65535));  // the grid is at most 65535 blocks high
+  return R < least ? least : R;
 }
 
 template <class T, class C>
