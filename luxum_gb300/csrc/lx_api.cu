@@ -436,7 +436,7 @@ extern "C" LX_API void lx_sim_destroy(lx_sim* s) {
     for (int q = 0; q < 2; q++) { dfree(s->psiH[c][q], fs); dfree(s->psiE[c][q], fs); }
     for (int q = 0; q < 2; q++) { dfree(s->psiH1[c][q], fs); dfree(s->psiE1[c][q], fs); }
   }
-  dfree(s->tab, fs); dfree(s->tabs, fs); dfree(s->d_max, fs); dfree(s->d_series, fs); dfree(s->etotal, fs); dfree(s->xfer, fs);
+  dfree(s->tab, fs); dfree(s->d_max, fs); dfree(s->d_series, fs); dfree(s->etotal, fs); dfree(s->xfer, fs);
   dfree(s->d_probe_ijk, fs); dfree(s->d_probe, fs);
   for (auto& sl : s->slots) {
     dfree(sl.dev, fs);
@@ -1595,14 +1595,28 @@ static lx::PrologueParams make_prologue(lx_sim* s) {
   return pp;
 }
 
-// The tables a handle stepped alone keeps ahead: as many steps as fit kAheadBytes, up to kAhead.
+// The tables a handle stepped alone keeps ahead: as many steps as fit kAheadBytes, up to kAhead,
+// in place of the one step's that it was created with.  Without the memory for them it steps with
+// those.
 static lx_status ensure_ahead(lx_sim* s) {
   constexpr size_t kAheadBytes = 1 << 20;
   if (s->ahead) return LX_OK;
   const size_t tab = s->tfsf ? (size_t)s->tab_total * s->csize : 0;
   int n = lx::kAhead;
   if (tab) n = (int)std::max<size_t>(1, std::min<size_t>(n, kAheadBytes / tab));
-  if (tab && n > 1) CK(cudaMallocAsync(&s->tabs, tab * n, s->stream));
+  if (tab && n > 1) {
+    void* more = nullptr;
+    const cudaError_t e = cudaMallocAsync(&more, tab * n, s->stream);
+    if (e == cudaErrorMemoryAllocation) {
+      (void)cudaGetLastError();
+      n = 1;
+    } else {
+      CK(e);
+      dfree(s->tab, s->stream);
+      s->tab = more;
+      if (s->batch) batch_member_changed(s->batch);  // its launches may hold the old table
+    }
+  }
   s->ahead = n;
   return LX_OK;
 }
@@ -1645,7 +1659,7 @@ static lx_status run_steps(lx_sim* s, int nsteps, KernelTimer* kt = nullptr) {
   lx::StepParams<T, C> sp = step_params<T, C>(s);
   sp.fault = s->d_fault;
   lx::PrologueParams pp = make_prologue(s);
-  C* const tabs = (C*)(s->tabs ? s->tabs : s->tab);
+  C* const tabs = (C*)s->tab;
   T* pf[6];  // the components after the current step (buffer (t+1) & 1 in ping-pong mode)
   auto post_step = [&](int t) {
     const bool b1 = s->pp && ((t + 1) & 1);
@@ -1724,7 +1738,7 @@ static lx_status run_steps(lx_sim* s, int nsteps, KernelTimer* kt = nullptr) {
       s->n_kernels++;
       behind = chain;
     }
-    sp.tab = tabs + (size_t)(s->tabs ? q : 0) * s->tab_total;
+    sp.tab = tabs + (size_t)q * s->tab_total;
     sp.max_slot = mon ? s->d_ring + q : nullptr;
     sp.etotal = (snap & (1u << LX_ETOTAL)) ? (C*)s->etotal : nullptr;
     bool swept = false;
@@ -1802,7 +1816,7 @@ static lx_status run_steps(lx_sim* s, int nsteps, KernelTimer* kt = nullptr) {
     return at;
   };
 
-  const int K = kt ? 0 : sequence_steps(s);
+  int K = kt ? 0 : sequence_steps(s);
   unsigned long long* last_slot = s->d_ring;
   for (int done = 0; done < nsteps;) {
     const int t = s->t, left = nsteps - done;
@@ -1829,6 +1843,13 @@ static lx_status run_steps(lx_sim* s, int nsteps, KernelTimer* kt = nullptr) {
         if (!st && e == cudaSuccess) e = cudaGraphInstantiate(&s->graph, g, 0);
         if (g) cudaGraphDestroy(g);
         if (st) return st;
+        if (e == cudaErrorMemoryAllocation) {  // none for the graph: launched one by one
+          (void)cudaGetLastError();
+          s->graph = nullptr;
+          s->alone_steps = 0;
+          K = 0;
+          continue;
+        }
         CK(e);
         s->graph_steps = K;
         s->graph_pp = s->pp;
@@ -2010,7 +2031,7 @@ extern "C" LX_API lx_status lx_sim_info(const lx_sim* s, lx_info* info) {
   }
   b += (s->sweep ? 2 : 1) * (info->psi_h_entries + info->psi_e_entries) * s->csize;
   if (s->etotal) b += s->ncell * s->csize;
-  b += s->xfer_cap * sizeof(double) + (size_t)s->tab_total * s->csize * (s->tabs ? 1 + s->ahead : 1);
+  b += s->xfer_cap * sizeof(double) + (size_t)s->tab_total * s->csize * std::max(s->ahead, 1);
   for (auto& sl : s->slots) b += sl.cap * sizeof(double);
   for (auto& d : s->dfts) b += d.n_acc * sizeof(double);
   b += (size_t)s->probe_cap * s->nprobes * 6 * sizeof(double);

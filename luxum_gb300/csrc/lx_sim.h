@@ -123,10 +123,9 @@ struct lx_sim {
   unsigned long long* d_ring = nullptr;
   double* d_srcv = nullptr;
   lx::StepCtl* d_ctl = nullptr;
-  // Stepped alone: TF/SF tables of `ahead` steps (the handle's own table when ahead is 1), formed
-  // by one launch.
+  // Steps whose TF/SF tables `tab` holds since the handle was first stepped alone (0 before: one
+  // step's), formed by one launch.
   int ahead = 0;
-  void* tabs = nullptr;
   // A captured sequence of graph_steps steps (short steps are bound by their launches); dropped
   // when anything its launches were given changes.  `ctl` is what d_ctl holds.
   cudaGraphExec_t graph = nullptr;
