@@ -2116,7 +2116,8 @@ struct lx_batch {
   lx::PrologueParams* d_pps = nullptr;
   int max_entries = 0;
   int* d_ts = nullptr;
-  // Steps formed ahead by one prologue launch, their tables, [row][member] slots and amplitudes.
+  // Steps formed ahead by one prologue launch, their tables (null: the members' own, one step),
+  // [row][member] slots and amplitudes.
   int ahead = 1;
   void* d_tabs = nullptr;
   unsigned long long* d_slots = nullptr;
@@ -2332,12 +2333,21 @@ static lx_status batch_rebuild(lx_batch* b) {
   b->graphable = true;
   b->sources = false;
   b->built_at = b->step;
-  // Steps ahead: as many as keep the members' tables within 32 MB.
+  // Steps ahead: as many as batch_table_steps gives, in tables of the batch's; one step at a time,
+  // in the members' own tables, where that is one or there is no memory for more.
   size_t entries = 0;
   for (auto* s : b->sims) entries += s->tfsf ? s->tab_total : 0;
-  constexpr size_t kTabBytes = 32 << 20;
-  b->ahead = entries ? (int)std::max<size_t>(1, std::min<size_t>(lx::kAhead, kTabBytes / (entries * sizeof(C)))) : lx::kAhead;
-  if (entries) BCK(cudaMallocAsync(&b->d_tabs, entries * b->ahead * sizeof(C), b->stream));
+  b->ahead = lx::batch_table_steps(entries * sizeof(C));
+  if (entries && b->ahead > 1) {
+    const cudaError_t e = cudaMallocAsync(&b->d_tabs, entries * b->ahead * sizeof(C), b->stream);
+    if (e == cudaErrorMemoryAllocation) {
+      (void)cudaGetLastError();
+      b->d_tabs = nullptr;
+      b->ahead = 1;
+    } else {
+      BCK(e);
+    }
+  }
   BCK(cudaMallocAsync(&b->d_slots, sizeof(unsigned long long) * lx::kAhead * (n > 0 ? n : 1), b->stream));
   BCK(cudaMallocAsync(&b->d_srcv, sizeof(double) * lx::kAhead * (n > 0 ? n : 1), b->stream));
   std::vector<std::vector<lx::DftParams>> dft_planes;
@@ -2369,7 +2379,7 @@ static lx_status batch_rebuild(lx_batch* b) {
     lx_sim* s = b->sims[q];
     pps[q] = make_prologue(s);
     if (s->tfsf) {
-      tabs[q] = (C*)b->d_tabs + at;
+      tabs[q] = b->d_tabs ? (C*)b->d_tabs + at : (C*)s->tab;
       pps[q].tab = tabs[q];
       at += (size_t)s->tab_total * b->ahead;
     }

@@ -27,6 +27,13 @@ constexpr int kMaxDftFreq = 256;
 // Steps whose field-independent values (TF/SF tables, source amplitude) one launch forms ahead
 // for a handle stepped alone.
 constexpr int kAhead = 16;
+// The same for a batch whose members' tables of one step take row_bytes: as many steps as stay
+// within 32 MB.
+constexpr size_t kBatchTableBytes = 32 << 20;
+inline int batch_table_steps(size_t row_bytes) {
+  const size_t n = row_bytes ? kBatchTableBytes / row_bytes : kAhead;
+  return n < 1 ? 1 : (n < (size_t)kAhead ? (int)n : kAhead);
+}
 
 // Where a handle's replayed step sequence stands (device memory; launches issued one by one take
 // the values from their parameters instead).

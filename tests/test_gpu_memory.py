@@ -1,6 +1,7 @@
-"""Device memory: a handle steps with what it holds when nothing more is to be had for tables formed
-ahead."""
+"""Device memory: handles and batches step with what they hold when nothing more is to be had for
+tables formed ahead, and a batch forms them beyond one step only within its allowance."""
 import ctypes as C
+from contextlib import ExitStack
 
 import numpy as np
 import pytest
@@ -102,3 +103,46 @@ def test_steps_alone_without_memory_for_tables_ahead(engine, precision):
         pool.empty()
         for a, b in zip(want, _fields(s)):
             assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("precision", [0, 1, 2])
+def test_batch_steps_without_memory_for_tables_ahead(engine, precision):
+    from luxum_gb300 import Batch, Sim
+
+    ps = [_oblique(n, precision) for n in (40, 33, 50)]
+    want = []
+    for p in ps:
+        with Sim(p) as s:
+            s.step(30)
+            want.append(_fields(s))
+    with _Pool(256 << 20) as pool, ExitStack() as held:
+        sims = [held.enter_context(Sim(p)) for p in ps]
+        batch = Batch(chunk=10)
+        held.callback(batch.close)
+        for s in sims:
+            batch.add(s)
+        pool.fill(1 << 18)  # a batch of three takes less than this besides its tables
+        batch.step(10)
+        batch.step(20)
+        pool.empty()
+        for w, s in zip(want, sims):
+            for a, b in zip(w, _fields(s)):
+                assert np.array_equal(a, b)
+
+
+def test_batch_tables_stay_within_their_allowance(engine):
+    """Members whose tables of one step take more than half the allowance: no second copy of them."""
+    from luxum_gb300 import Batch, Sim
+
+    n, count = 230, 4
+    face = (n - 12) ** 2
+    assert count * 24 * face * 8 > 17 << 20
+    with _Pool(8 << 30) as pool, ExitStack() as held:
+        sims = [held.enter_context(Sim(_oblique(n, 0))) for _ in range(count)]
+        batch = Batch()
+        held.callback(batch.close)
+        for s in sims:
+            batch.add(s)
+        before = pool.used()
+        batch.step(1)
+        assert pool.used() - before < 4 << 20
