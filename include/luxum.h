@@ -134,9 +134,12 @@ LX_API lx_status lx_params_from_yaml(const char* path, lx_params* p);
 LX_API lx_status lx_sim_create(const lx_params* p, lx_sim** out);
 LX_API void lx_sim_destroy(lx_sim* sim);
 /* Device memory lx_sim_create would hold for *p (fields, coefficients, CPML psi slabs and
- * profiles, TF/SF tables), computed on the host without a GPU; snapshot staging, probes,
- * DFT planes and transfer buffers come on top when used.  Serving loops admit requests
- * against an HBM budget with it. */
+ * profiles, the TF/SF tables of one step), computed on the host without a GPU.  On top come
+ * snapshot staging, probes, DFT planes and transfer buffers when used; for a handle that is
+ * stepped alone the TF/SF tables of up to 16 steps, at most 1 MB in all where one step's take
+ * less, and the driver's copy of a captured sequence of steps; for a batch the tables of up to
+ * 16 steps of all members, at most 32 MB, besides the members' own.  Serving loops admit
+ * requests against an HBM budget with it (the server counts its batch's tables too). */
 LX_API lx_status lx_params_device_bytes(const lx_params* p, size_t* bytes);
 /* Compulsory device-memory traffic of one time step for *p, computed on the host: every
  * field component read and written once, every Cb array read once and every stored CPML psi

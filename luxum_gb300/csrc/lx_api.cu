@@ -542,10 +542,8 @@ static lx_status create_typed(lx_sim* s) {
     build_sets(s);
     CK(cudaMallocAsync(&s->tab, (size_t)(s->tab_total > 0 ? s->tab_total : 1) * sizeof(C), s->own));
   }
-  const size_t words = 1 + 2 * lx::kAhead;
-  const size_t state = words * sizeof(unsigned long long) + sizeof(lx::StepCtl);
-  CK(cudaMallocAsync(&s->d_max, state, s->own));
-  CK(cudaMemsetAsync(s->d_max, 0, state, s->own));
+  CK(cudaMallocAsync(&s->d_max, lx::kStateBytes, s->own));
+  CK(cudaMemsetAsync(s->d_max, 0, lx::kStateBytes, s->own));
   s->d_fault = reinterpret_cast<unsigned*>(s->d_max);
   s->d_ring = s->d_max + 1;
   s->d_srcv = reinterpret_cast<double*>(s->d_ring + lx::kAhead);
@@ -718,8 +716,16 @@ extern "C" LX_API lx_status lx_params_device_bytes(const lx_params* p, size_t* b
     build_sets(&tmp);
     b += (size_t)tmp.tab_total * tmp.csize;
   }
-  *bytes = b + 64;
+  *bytes = b + lx::kStateBytes;
   return LX_OK;
+}
+
+size_t lx::table_bytes(const lx_params& p) {
+  lx_sim tmp;
+  setup_host(&tmp, &p);
+  if (!tmp.tfsf) return 0;
+  build_sets(&tmp);
+  return (size_t)tmp.tab_total * tmp.csize;
 }
 
 extern "C" LX_API lx_status lx_params_step_bytes(const lx_params* p, double* bytes) {

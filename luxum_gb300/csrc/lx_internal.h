@@ -34,6 +34,11 @@ inline int batch_table_steps(size_t row_bytes) {
   const size_t n = row_bytes ? kBatchTableBytes / row_bytes : kAhead;
   return n < 1 ? 1 : (n < (size_t)kAhead ? (int)n : kAhead);
 }
+// What it keeps for them beside its members' own tables.
+inline size_t batch_table_bytes(size_t row_bytes) {
+  const int n = batch_table_steps(row_bytes);
+  return n > 1 ? n * row_bytes : 0;
+}
 
 // Where a handle's replayed step sequence stands (device memory; launches issued one by one take
 // the values from their parameters instead).
@@ -42,6 +47,8 @@ struct StepCtl {
   int row;     // probe rows recorded
   int series;  // max|E|^2 series entries recorded
 };
+// A handle's fault word, the slots and source amplitudes of a sequence, and its counters.
+constexpr size_t kStateBytes = (1 + 2 * kAhead) * 8 + sizeof(StepCtl);
 // Default cells each thread of a batched update kernel walks through along x: planar rows 8
 // apart, and 3-D planes (the autotuner's picks on the lens and 3-D cube workloads);
 // lx_batch_autotune picks per batch among 1, 2, 4 and 8.

@@ -32,9 +32,11 @@
 #include <vector>
 
 #include "luxum.h"
+#include "lx_internal.h"
 
 namespace lx {
 lx_status set_thread_error(const char* msg, lx_status st);
+size_t table_bytes(const lx_params& p);
 }
 
 namespace {
@@ -52,6 +54,7 @@ struct Request {
   int dft_axis = 0, dft_index = 0, dft_every = 1;
   std::vector<double> omega;
   double bytes = 0.0;  // admission estimate
+  size_t table = 0;    // of it, the TF/SF tables of one step
   double cells = 0.0;
   int state = LX_REQ_QUEUED;
   bool cancel = false;
@@ -152,7 +155,10 @@ void prepare(lx_server* srv) {
     }
     const size_t live = srv->running.size() + srv->prepared.size();
     if (live > 0) {
-      if (srv->stats.bytes_running + r->bytes > srv->cfg.budget_bytes) return;
+      size_t table = r->table;  // the batch forms its members' tables of several steps ahead
+      for (auto& m : srv->running) table += m->table;
+      for (auto& m : srv->prepared) table += m->table;
+      if (srv->stats.bytes_running + r->bytes + lx::batch_table_bytes(table) > srv->cfg.budget_bytes) return;
       if (srv->cfg.max_running > 0 && (int)live >= srv->cfg.max_running) return;
     }
     srv->queue.pop_front();
@@ -456,6 +462,7 @@ extern "C" LX_API lx_status lx_server_submit(lx_server* srv, const lx_request* r
   // DFT accumulators: nfreq x 4 components x plane x (re, im)
   const double plane = req->dft_axis == 0 ? Ny * Nz : (req->dft_axis == 1 ? Nx * Nz : Nx * Ny);
   r->bytes = (double)bytes + 64.0 * req->nfreq * plane;
+  r->table = lx::table_bytes(req->params);
   for (int c = 0; c < 3; c++) r->bytes += 8.0 * r->material[c].size();  // transfer staging
   std::lock_guard<std::mutex> lk(srv->mu);
   r->id = srv->next_id++;

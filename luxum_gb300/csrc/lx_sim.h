@@ -177,4 +177,6 @@ namespace lx {
 // `other`, the buffer that does not.  Null when the handle keeps no such array.  Every reader
 // of a handle's fields takes its source from here.
 void* comp_ptr(lx_sim* s, int comp, bool other = false);
+// TF/SF tables of one step of the handle that *p, which is valid, would give.
+size_t table_bytes(const lx_params& p);
 }  // namespace lx

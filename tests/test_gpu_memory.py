@@ -1,5 +1,6 @@
 """Device memory: handles and batches step with what they hold when nothing more is to be had for
-tables formed ahead, and a batch forms them beyond one step only within its allowance."""
+tables formed ahead, a batch forms them beyond one step only within its allowance, and the server
+counts them."""
 import ctypes as C
 from contextlib import ExitStack
 
@@ -146,3 +147,16 @@ def test_batch_tables_stay_within_their_allowance(engine):
         before = pool.used()
         batch.step(1)
         assert pool.used() - before < 4 << 20
+
+
+def test_server_counts_the_tables_of_its_batch(engine):
+    """A budget for two requests, but not for the tables that a batch of the two forms ahead, runs
+    one at a time; with the batch's allowance on top of it, both."""
+    from luxum_gb300 import Server, device_bytes
+
+    p = _oblique(60, 1)
+    for extra, most in ((1 << 20, 1), (32 << 20, 2)):
+        with Server(chunk=20, budget_bytes=2 * device_bytes(p) + extra) as srv:
+            ids = [srv.submit(p, 2000) for _ in range(2)]
+            assert all(srv.wait(r, 120.0) == "done" for r in ids)
+            assert srv.stats()["peak_running"] == most
