@@ -98,12 +98,18 @@ static lx_status fail(lx_sim* s, lx_status st, const std::string& msg) {
   return st;
 }
 
+// The status of a failed call, which the runtime then no longer holds: the launches read their
+// errors with cudaGetLastError, and the next one would find this.
+static lx_status cuda_status(cudaError_t e) {
+  (void)cudaGetLastError();
+  return e == cudaErrorMemoryAllocation ? LX_ERR_OOM : LX_ERR_CUDA;
+}
+
 #define CK(...)                                                                                       \
   do {                                                                                                \
-    cudaError_t e_ = (__VA_ARGS__);                                                                        \
+    cudaError_t e_ = (__VA_ARGS__);                                                                   \
     if (e_ != cudaSuccess)                                                                            \
-      return fail(s, e_ == cudaErrorMemoryAllocation ? LX_ERR_OOM : LX_ERR_CUDA,                      \
-                  std::string(#__VA_ARGS__) + ": " + cudaGetErrorString(e_));                              \
+      return fail(s, cuda_status(e_), std::string(#__VA_ARGS__) + ": " + cudaGetErrorString(e_));     \
   } while (0)
 
 extern "C" LX_API const char* lx_version(void) { return "luxum-gb300 0.1 (sm_103a)"; }
@@ -2059,7 +2065,10 @@ extern "C" LX_API lx_status lx_sim_counters(const lx_sim* s, uint64_t* kernels, 
 extern "C" LX_API lx_status lx_host_alloc(size_t bytes, void** ptr) {
   if (!ptr) return fail(nullptr, LX_ERR_INVALID, "null argument");
   cudaError_t e = cudaHostAlloc(ptr, bytes ? bytes : 1, cudaHostAllocDefault);
-  if (e != cudaSuccess) return fail(nullptr, LX_ERR_OOM, std::string("cudaHostAlloc: ") + cudaGetErrorString(e));
+  if (e != cudaSuccess) {
+    cuda_status(e);
+    return fail(nullptr, LX_ERR_OOM, std::string("cudaHostAlloc: ") + cudaGetErrorString(e));
+  }
   return LX_OK;
 }
 
@@ -2239,8 +2248,8 @@ static lx_status bfail(lx_batch* b, lx_status st, const std::string& m) {
 #define BCK(...)                                                                                      \
   do {                                                                                                \
     cudaError_t e_ = (__VA_ARGS__);                                                                   \
-    if (e_ != cudaSuccess) return bfail(b, e_ == cudaErrorMemoryAllocation ? LX_ERR_OOM : LX_ERR_CUDA, \
-                                        std::string(#__VA_ARGS__) + ": " + cudaGetErrorString(e_));   \
+    if (e_ != cudaSuccess)                                                                            \
+      return bfail(b, cuda_status(e_), std::string(#__VA_ARGS__) + ": " + cudaGetErrorString(e_));    \
   } while (0)
 
 extern "C" LX_API lx_status lx_batch_create(lx_batch** out) {

@@ -1,6 +1,6 @@
 """Device memory: handles and batches step with what they hold when nothing more is to be had for
 tables formed ahead, a batch forms them beyond one step only within its allowance, and the server
-counts them."""
+counts them.  An allocation that fails is reported by its call and by no later one."""
 import ctypes as C
 from contextlib import ExitStack
 
@@ -160,3 +160,23 @@ def test_server_counts_the_tables_of_its_batch(engine):
             ids = [srv.submit(p, 2000) for _ in range(2)]
             assert all(srv.wait(r, 120.0) == "done" for r in ids)
             assert srv.stats()["peak_running"] == most
+
+
+def test_a_failed_allocation_is_reported_once(engine):
+    """A handle too large for the memory left fails to create; the next calls go on."""
+    from luxum_gb300 import Batch, LuxumError, Sim
+
+    with _Pool(64 << 20) as pool, ExitStack() as held:
+        for _ in range(2):
+            with pytest.raises(LuxumError):
+                Sim(_oblique(200, 0))
+            s = held.enter_context(Sim(_oblique(24, 0)))
+            s.step(5)
+            assert s.max_e2() > 0
+        batch = Batch()
+        held.callback(batch.close)
+        batch.add(s)
+        with pytest.raises(LuxumError):
+            Sim(_oblique(200, 0))
+        batch.step(5)
+        assert s.t == 10 and pool.used() > 0
