@@ -445,7 +445,7 @@ typedef struct lx_info {
 LX_API lx_status lx_sim_info(const lx_sim* sim, lx_info* info);
 
 /* Counters since creation: device kernels launched, bytes copied host->device and
- * device->host by the handle. */
+ * device->host by the handle.  A batched member counts the launches that it has part in. */
 LX_API lx_status lx_sim_counters(const lx_sim* sim, uint64_t* kernels, uint64_t* h2d, uint64_t* d2h);
 
 /* Page-locked host memory for fast transfers (cudaHostAlloc). */

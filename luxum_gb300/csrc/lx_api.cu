@@ -2667,8 +2667,12 @@ static lx_status batch_run_async(lx_batch* b, int nsteps) {
     b->chunks_since_rebuild = 0;
   }
   int done = 0;
+  // launches of the batch that every member has part in: tables formed ahead, the step counters
+  uint64_t common = 0;
+  auto part = [&](int k) { common += (uint64_t)(k + b->ahead - 1) / b->ahead + 1; };
   if (b->chunk > 0 && b->graphable) {
     while (nsteps - done >= b->chunk) {
+      part(b->chunk);
       // The first chunk after a change of members is launched directly: capturing and
       // instantiating a graph is host time before any of its work starts, while direct
       // launches run as they are issued.  A serving loop whose members change every chunk
@@ -2703,14 +2707,18 @@ static lx_status batch_run_async(lx_batch* b, int nsteps) {
     }
   }
   if (nsteps - done > 0) {
+    part(nsteps - done);
     if ((st = batch_enqueue<T, C>(b, b->step, nsteps - done))) return st;
     b->step += nsteps - done;
     b->chunks_since_rebuild++;
   }
   for (size_t q = 0; q < b->sims.size(); q++) {
-    b->sims[q]->t += nsteps;
-    b->host_ts[q] = b->sims[q]->t;
-    b->sims[q]->n_kernels += (uint64_t)nsteps * 4;
+    lx_sim* s = b->sims[q];
+    s->n_kernels += common + (uint64_t)nsteps * ((s->pp ? 1 : 2) + (s->src_kind >= 0 ? 1 : 0));
+    for (auto& d : s->dfts)  // samples at the multiples of d.every in [t, t + nsteps): phase factors, accumulation
+      s->n_kernels += 2 * (uint64_t)((s->t + nsteps + d.every - 1) / d.every - (s->t + d.every - 1) / d.every);
+    s->t += nsteps;
+    b->host_ts[q] = s->t;
   }
   b->pending += nsteps;
   return LX_OK;
