@@ -2114,7 +2114,6 @@ struct lx_batch {
     int* d_first = nullptr;
     int4* d_tiles = nullptr;
     int nblocks = 0;
-    std::vector<int> first;  // sweep groups: the members' first blocks
   };
   int march2d = lx::kMarch2, march3d = lx::kMarch3;  // per dimension (lx_batch_set_march / autotune)
   bool march_set = false;            // set by a caller or the tuner: not adapted to the batch's size
@@ -2512,7 +2511,7 @@ static lx_status batch_rebuild(lx_batch* b) {
           }
         g.host_params.assign((const char*)sw.data(), (const char*)(sw.data() + sw.size()));
         std::vector<int4> tiles;
-        lx::sweep_tiles(sw.data(), (int)ps.size(), g.march, g.first, tiles);
+        lx::sweep_tiles(sw.data(), (int)ps.size(), g.march, tiles);
         g.nblocks = (int)tiles.size();
         BCK(cudaMallocAsync(&g.d_tiles, sizeof(int4) * std::max<size_t>(tiles.size(), 1), b->stream));
         BCK(cudaMemcpyAsync(g.d_tiles, tiles.data(), sizeof(int4) * tiles.size(), cudaMemcpyHostToDevice, b->stream));
@@ -2635,7 +2634,7 @@ static lx_status batch_enqueue(lx_batch* b, long long step0, int nsteps) {
                 const auto* sw = (const lx::SweepParams<T, C>*)g.host_params.data();
                 if (half == 0)
                   BCK(lx::launch_batch_sweep<T, C>(sw + ((bs - b->built_at) & 1) * g.members.size(), (int)g.members.size(),
-                                                   g.first.data(), g.d_tiles, g.uniform, g.march, r, b->stream));
+                                                   g.d_tiles, g.nblocks, g.uniform, g.march, r, b->stream));
                 continue;
               }
             }

@@ -186,8 +186,9 @@ struct SweepParams {
   int planesH[3][2], planesE[3][2];
   PlaneSet setHx, setHz, setEz, setEx;  // Hx z part, Hz x part, Ey z and x parts
 };
-// Members of one batched sweep launch: as many as the parameter space of a launch takes.
-constexpr int kSweepMembers = 48;
+// Members of one batched sweep launch: as many as the parameter space of a launch takes beside its
+// other three parameters.
+constexpr int kSweepMembers = (32764 - 16) / sizeof(SweepParams<float, float>);
 template <class T, class C>
 struct SweepBatch {
   SweepParams<T, C> m[kSweepMembers];

@@ -2041,27 +2041,21 @@ cudaError_t launch_step_sweep2(const StepParams<T, C>& p, bool uniform, bool beh
 }
 
 template <class T, class C>
-cudaError_t launch_batch_sweep(const SweepParams<T, C>* m, int n, const int* first, const int4* tiles, bool uniform, int R,
+cudaError_t launch_batch_sweep(const SweepParams<T, C>* m, int n, const int4* tiles, int nblocks, bool uniform, int R,
                                int row, cudaStream_t s) {
+  if (n < 1 || n > kSweepMembers) return cudaErrorInvalidValue;
   SweepBatch<T, C> b;
   static_assert(sizeof(b) + 16 <= 32764, "a launch's parameter space");
+  std::memcpy(b.m, m, n * sizeof(SweepParams<T, C>));
   const dim3 block(32, 8);
-  for (int at = 0; at < n; at += kSweepMembers) {
-    const int k = n - at < kSweepMembers ? n - at : kSweepMembers;
-    std::memcpy(b.m, m + at, k * sizeof(SweepParams<T, C>));
-    const int nb = first[at + k] - first[at];
-    if (uniform) step_batch_2d<T, C, true><<<nb, block, 0, s>>>(b, tiles + first[at], R, row);
-    else step_batch_2d<T, C, false><<<nb, block, 0, s>>>(b, tiles + first[at], R, row);
-    const cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-  }
-  return cudaSuccess;
+  if (uniform) step_batch_2d<T, C, true><<<nblocks, block, 0, s>>>(b, tiles, R, row);
+  else step_batch_2d<T, C, false><<<nblocks, block, 0, s>>>(b, tiles, R, row);
+  return cudaGetLastError();
 }
 
-// {member of its launch, first row, interior, first column} of each block of the members' sweeps.
+// {member, first row, interior, first column} of each block of the members' sweeps.
 template <class T, class C>
-void sweep_tiles(const SweepParams<T, C>* m, int n, int R, std::vector<int>& first, std::vector<int4>& tiles) {
-  first.assign(1, 0);
+void sweep_tiles(const SweepParams<T, C>* m, int n, int R, std::vector<int4>& tiles) {
   tiles.clear();
   for (int q = 0; q < n; ++q) {
     const SweepParams<T, C>& p = m[q];
@@ -2072,9 +2066,8 @@ void sweep_tiles(const SweepParams<T, C>* m, int n, int R, std::vector<int>& fir
         const bool tf = p.tfsf && (tile_meets_planes(p.planesH, i - 1, i1 - i + 1, 0, 1, k - 1, 34) ||
                                    tile_meets_planes(p.planesE, i, i1 - i, 0, 1, k, 32));
         const bool in = !tf && tile_is_interior_2d(p.slab, p.pml, p.Nx, p.Nz, i - 1, i1 - i + 2, k - 1, 34);
-        tiles.push_back(make_int4(q % kSweepMembers, i, in ? 1 : 0, k));
+        tiles.push_back(make_int4(q, i, in ? 1 : 0, k));
       }
-    first.push_back((int)tiles.size());
   }
 }
 
@@ -2247,13 +2240,12 @@ template cudaError_t launch_prologue_ahead<float>(const PrologueParams&, int, co
                                                   unsigned long long*, cudaStream_t);
 template SweepParams<float, float> sweep_params<float, float>(const StepParams<float, float>&);
 template SweepParams<__half, float> sweep_params<__half, float>(const StepParams<__half, float>&);
-template cudaError_t launch_batch_sweep<float, float>(const SweepParams<float, float>*, int, const int*, const int4*, bool,
-                                                      int, int, cudaStream_t);
-template cudaError_t launch_batch_sweep<__half, float>(const SweepParams<__half, float>*, int, const int*, const int4*, bool,
-                                                       int, int, cudaStream_t);
-template void sweep_tiles<float, float>(const SweepParams<float, float>*, int, int, std::vector<int>&, std::vector<int4>&);
-template void sweep_tiles<__half, float>(const SweepParams<__half, float>*, int, int, std::vector<int>&,
-                                         std::vector<int4>&);
+template cudaError_t launch_batch_sweep<float, float>(const SweepParams<float, float>*, int, const int4*, int, bool, int, int,
+                                                      cudaStream_t);
+template cudaError_t launch_batch_sweep<__half, float>(const SweepParams<__half, float>*, int, const int4*, int, bool, int,
+                                                       int, cudaStream_t);
+template void sweep_tiles<float, float>(const SweepParams<float, float>*, int, int, std::vector<int4>&);
+template void sweep_tiles<__half, float>(const SweepParams<__half, float>*, int, int, std::vector<int4>&);
 template cudaError_t launch_prologue_batch<double>(const PrologueParams*, const int*, int, int, int, int, double*,
                                                    unsigned long long*, cudaStream_t);
 template cudaError_t launch_prologue_batch<float>(const PrologueParams*, const int*, int, int, int, int, double*,

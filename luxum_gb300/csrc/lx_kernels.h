@@ -57,15 +57,15 @@ cudaError_t launch_batch_tiles(const StepParams<T, C>* ps, const int* first, int
 template <class T, class C>
 cudaError_t launch_batch_step(const StepParams<T, C>* ps, const int4* tiles, int nblocks, bool planar, bool uniform,
                               int march, bool h_half, int row, cudaStream_t s);
-// Planar members in two buffers: H and E of a step, kSweepMembers members a launch, R rows a warp.
+// Planar members in two buffers: H and E of a step in one launch of at most kSweepMembers members.
 template <class T, class C>
 SweepParams<T, C> sweep_params(const StepParams<T, C>& p);
 template <class T, class C>
-cudaError_t launch_batch_sweep(const SweepParams<T, C>* m, int n, const int* first, const int4* tiles, bool uniform, int R,
+cudaError_t launch_batch_sweep(const SweepParams<T, C>* m, int n, const int4* tiles, int nblocks, bool uniform, int R,
                                int row, cudaStream_t s);
-// The members' first blocks (n + 1) and the blocks' tiles for it.
+// The blocks' tiles for it.
 template <class T, class C>
-void sweep_tiles(const SweepParams<T, C>* m, int n, int R, std::vector<int>& first, std::vector<int4>& tiles);
+void sweep_tiles(const SweepParams<T, C>* m, int n, int R, std::vector<int4>& tiles);
 // blocks one member occupies in a batched update launch; march = cells each thread walks
 // along x (planar: rows 8 apart; 3-D: planes), one of 1, 2, 4, 8
 int batch_blocks(int Nx, int Ny, int Nz, bool planar, int march);

@@ -1,0 +1,54 @@
+"""The forms in which a batch steps its planar float members, at the edges of the rules that choose
+among them.  Every member equals, bit for bit, its twin stepped alone."""
+import numpy as np
+import pytest
+
+import cases
+
+pytestmark = pytest.mark.gpu
+
+
+def _lens(n, m, precision, k=0):
+    kw = dict(isPlanar=1, Nx=n, Ny=1, Nz=m, precision=precision, cpml_mode=1)
+    if k % 4 == 1:
+        kw.update(usePS=1, source_kind=1, Nx_source=n // 2, Ny_source=0, Nz_source=m // 2, amp_source=1.0,
+                  omega_source=4e10, src_t0=9.0, src_tw=5.0)
+    else:
+        kw.update(cases.pw((0.6, 0, 0.8), (0, 1, 0), ((9, n - 10), (0, 0), (9, m - 10)), off=8.0))
+    return cases.make(**kw, **cases.pml(5 + k % 3))
+
+
+def _sim(p):
+    from luxum_gb300 import Sim
+
+    s = Sim(p)
+    s.set_eps_box((p.Nx // 3, 0, p.Nz // 3), (p.Nx // 2, 1, p.Nz // 2), 3.0)
+    return s
+
+
+def _compare(ps, runs=(17, 8, 8, 9), chunk=8):
+    from luxum_gb300 import Batch
+
+    sims = [_sim(p) for p in ps]
+    batch = Batch(chunk=chunk)
+    for s in sims:
+        batch.add(s)
+    for n in runs:
+        batch.step(n)
+    for p, s in zip(ps, sims):
+        twin = _sim(p)
+        twin.step(sum(runs))
+        for c in (1, 3, 5):
+            assert np.array_equal(s.field(c), twin.field(c)), (p.Nx, p.Nz, c)
+        assert s.max_e2() == twin.max_e2() > 0
+        twin.close()
+    batch.close()
+    for s in sims:
+        s.close()
+
+
+# 54 members fill the parameters of one batched sweep; one more takes the half steps
+@pytest.mark.parametrize("precision", [1, 2])
+@pytest.mark.parametrize("count", [1, 49, 54, 55])
+def test_members_of_one_sweep_launch(engine, precision, count):
+    _compare([_lens(24 + 3 * (k % 11), 30 + 7 * (k % 5), precision, k) for k in range(count)])
