@@ -292,9 +292,10 @@ LX_API lx_status lx_batch_step(lx_batch* b, int nsteps);
  * read-back, blow-up check).  Members must not be touched in between. */
 LX_API lx_status lx_batch_step_async(lx_batch* b, int nsteps);
 LX_API lx_status lx_batch_wait(lx_batch* b);
-/* Tile shape of the batched update kernels: cells each thread walks along x, for planar
+/* Tile shape of the batched half-step kernels: cells each thread walks along x, for planar
  * members (rows 8 apart) and for 3-D members below 2^18 cells (planes); each 1, 2, 4 or 8
- * (defaults 8, 8).  Results do not depend on it, only speed. */
+ * (defaults 8, 8).  Planar float members that a batch steps one by one, or few enough for
+ * one single-sweep launch, have none.  Results do not depend on it, only speed. */
 LX_API lx_status lx_batch_set_march(lx_batch* b, int planar_rows, int planes_3d);
 LX_API lx_status lx_batch_get_march(const lx_batch* b, int* planar_rows, int* planes_3d);
 /* Tile-shape table.  Members are classed by (dimension, size, precision, CPML slab depth);
@@ -313,10 +314,10 @@ LX_API lx_status lx_sim_tune_class(const lx_sim* sim, lx_tune_entry* key);
 LX_API lx_status lx_batch_set_tune_table(lx_batch* b, const lx_tune_entry* entries, int n);
 /* Copies up to cap entries to entries (may be NULL when cap is 0); *n = the table's length. */
 LX_API lx_status lx_batch_get_tune_table(const lx_batch* b, lx_tune_entry* entries, int cap, int* n);
-/* Tunes the class of every batched member (3-D members of 2^18 cells or more and planar
- * single-sweep members of 2^21 are launched one by one and have no tile shape).  Zero-field twins of
- * a sample of the members (up to 1.5e8 cells, at least one per class; created and freed here)
- * are stepped together, `steps` steps per timing: first with one march for every class, then
+/* Tunes the class of every member that may step in the half-step launches (3-D members of 2^18
+ * cells or more and planar float members of 2^19 never do).  Zero-field twins of a sample of the
+ * members (up to 1.5e8 cells, at least one per class; created and freed here) are stepped
+ * together in those launches, `steps` steps per timing: first with one march for every class, then
  * with each class in turn (largest first) moved to each other march, a move kept when the
  * whole sample runs 2 % faster, so that a class's pick pays for the launch it splits off.
  * Every class's pick is recorded in the table.  The members themselves are not stepped.  The

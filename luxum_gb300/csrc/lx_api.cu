@@ -2108,7 +2108,8 @@ struct lx_batch {
     bool sweep = false;             // planar members in two buffers
     std::vector<char> host_params;  // solo groups: the members' parameter blocks; sweep groups: their
                                     // SweepParams at their parity when built, then at the other
-    int march = lx::kMarch3;   // cells each thread walks along x (0 while it is still to be chosen)
+    int march = 0;             // cells each thread walks along x, of sweep groups the rows a warp (0
+                               // while it is still to be chosen)
     std::vector<int> members;  // batch-global indices
     void* d_params = nullptr;
     int* d_first = nullptr;
@@ -2117,6 +2118,7 @@ struct lx_batch {
   };
   int march2d = lx::kMarch2, march3d = lx::kMarch3;  // per dimension (lx_batch_set_march / autotune)
   bool march_set = false;            // set by a caller or the tuner: not adapted to the batch's size
+  bool half_steps = false;           // the tuner's twins: no batched sweep, which has no tile shape
   std::vector<lx_tune_entry> table;  // march per member class (lx_batch_set_tune_table / autotune)
   struct DftClass {  // DFT planes that sample at the same batch steps
     int every = 1, phase = 0;
@@ -2159,10 +2161,9 @@ static bool batch_alone(const lx_batch* b, const lx_sim* s) {
                    : (long long)s->Nx * s->Ny * s->Nz >= lx_batch::kSoloCells;
 }
 
-// A member the tuner takes no sample of: it never shares a launch.  (Smaller planar members
-// keep their entry in the table.)
+// A member the tuner takes no sample of: it never steps in the half-step launches.
 static bool batch_untuned(const lx_sim* s) {
-  return s->planar ? s->sweep && (long long)s->Nx * s->Nz >= 1LL << 21
+  return s->planar ? s->sweep && (long long)s->Nx * s->Nz >= lx_batch::kSoloCells2
                    : (long long)s->Nx * s->Ny * s->Nz >= lx_batch::kSoloCells;
 }
 
@@ -2380,7 +2381,7 @@ static lx_status batch_rebuild(lx_batch* b) {
       shared++;
       shared_cells += (long long)s->Nx * s->Nz;
     }
-  const bool few = shared <= lx::kSweepMembers && (sizeof(T) == 4 || shared_cells <= 1LL << 22);
+  const bool few = !b->half_steps && shared <= lx::kSweepMembers && (sizeof(T) == 4 || shared_cells <= 1LL << 22);
   for (int q = 0; q < n; q++) {
     lx_sim* s = b->sims[q];
     lx_status st;
@@ -2431,13 +2432,13 @@ static lx_status batch_rebuild(lx_batch* b) {
       dft_planes[ci].push_back(dp);
     }
     if (s->pp && b->chunk % 2) b->graphable = false;  // a captured chunk must keep each member's parity
-    // batched members share a launch only with members of the same march (their classes' picks; 0:
-    // chosen by the group's size)
-    const int march = solo ? lx::kMarch3 : batch_march(b, s);
+    // members share the half-step launches only with members of the same march (their classes' picks;
+    // 0: chosen by the group's size); the batched sweep is one launch with rows of its own choice
+    const int march = solo || s->pp ? 0 : batch_march(b, s);
     int gi = -1;
     for (size_t g = 0; g < b->groups.size(); g++)
       if (b->groups[g].planar == (bool)s->planar && b->groups[g].uniform == (bool)s->uniform &&
-          b->groups[g].solo == solo && b->groups[g].sweep == (bool)s->pp && (solo || b->groups[g].march == march))
+          b->groups[g].solo == solo && b->groups[g].sweep == (bool)s->pp && b->groups[g].march == march)
         gi = (int)g;
     if (gi < 0) {
       b->groups.emplace_back();
@@ -2484,6 +2485,24 @@ static lx_status batch_rebuild(lx_batch* b) {
       g.nblocks = 0;
       continue;
     }
+    if constexpr (sizeof(C) == 4) {
+      if (g.sweep) {  // passed by value: no device blocks or tile map
+        std::vector<lx::SweepParams<T, C>> sw;
+        for (int par = 0; par < 2; par++)
+          for (size_t m = 0; m < ps.size(); m++) {
+            lx::StepParams<T, C> sp = ps[m];
+            if ((b->sims[g.members[m]]->t + par) & 1) swap_buffers(sp);
+            sw.push_back(lx::sweep_params(sp));
+          }
+        g.host_params.assign((const char*)sw.data(), (const char*)(sw.data() + sw.size()));
+        std::vector<int4> tiles;
+        g.march = lx::sweep_tiles(sw.data(), (int)ps.size(), tiles);
+        g.nblocks = (int)tiles.size();
+        BCK(cudaMallocAsync(&g.d_tiles, sizeof(int4) * std::max<size_t>(tiles.size(), 1), b->stream));
+        BCK(cudaMemcpyAsync(g.d_tiles, tiles.data(), sizeof(int4) * tiles.size(), cudaMemcpyHostToDevice, b->stream));
+        continue;
+      }
+    }
     auto count = [&](int march) {
       long long nb = 0;
       for (int q : g.members) {
@@ -2499,24 +2518,6 @@ static lx_status batch_rebuild(lx_batch* b) {
       const long long nb = (long long)first.back() + lx::batch_blocks(s->Nx, s->Ny, s->Nz, s->planar, g.march);
       if (nb > 0x7fffffffLL) return bfail(b, LX_ERR_INVALID, "batch too large for one launch");
       first.push_back((int)nb);
-    }
-    if constexpr (sizeof(C) == 4) {
-      if (g.sweep) {  // passed by value: no device blocks or tile map
-        std::vector<lx::SweepParams<T, C>> sw;
-        for (int par = 0; par < 2; par++)
-          for (size_t m = 0; m < ps.size(); m++) {
-            lx::StepParams<T, C> sp = ps[m];
-            if ((b->sims[g.members[m]]->t + par) & 1) swap_buffers(sp);
-            sw.push_back(lx::sweep_params(sp));
-          }
-        g.host_params.assign((const char*)sw.data(), (const char*)(sw.data() + sw.size()));
-        std::vector<int4> tiles;
-        lx::sweep_tiles(sw.data(), (int)ps.size(), g.march, tiles);
-        g.nblocks = (int)tiles.size();
-        BCK(cudaMallocAsync(&g.d_tiles, sizeof(int4) * std::max<size_t>(tiles.size(), 1), b->stream));
-        BCK(cudaMemcpyAsync(g.d_tiles, tiles.data(), sizeof(int4) * tiles.size(), cudaMemcpyHostToDevice, b->stream));
-        continue;
-      }
     }
     g.nblocks = first.back();
     BCK(cudaMallocAsync(&g.d_params, sizeof(lx::StepParams<T, C>) * ps.size(), b->stream));
@@ -2796,9 +2797,11 @@ struct TuneTwins {
   }
 };
 
-// Twins of `sample`, each `copies` times, as members of one scratch batch (no graphs).
+// Twins of `sample`, each `copies` times, as members of one scratch batch (no graphs) in the
+// half-step launches, which the picks are for.
 static lx_status make_twins(const std::vector<const lx_sim*>& sample, int copies, TuneTwins* tw) {
   lx_status st = lx_batch_create(&tw->tb);
+  if (!st) tw->tb->half_steps = true;
   if (!st) st = lx_batch_set_chunk(tw->tb, 0);
   for (size_t q = 0; q < sample.size() * copies && !st; q++) {
     const lx_sim* src = sample[q % sample.size()];

@@ -1375,8 +1375,9 @@ __global__ void __launch_bounds__(256, kSweepMinBlocks) step_kernel_2d(const Swe
 // each) 48 lenses of side 128-1024 take 142 us a step, at 5 with spills 158; parameters copied to
 // shared memory took 168, and the half-step kernels h_batch_2d and e_batch_2d, which move 40
 // bytes a cell where this moves 28, 166.
+constexpr int kBatchSweepMinBlocks = 4;
 template <class T, class C, bool UNI>
-__global__ void __launch_bounds__(256, 4) step_batch_2d(const __grid_constant__ SweepBatch<T, C> b,
+__global__ void __launch_bounds__(256, kBatchSweepMinBlocks) step_batch_2d(const __grid_constant__ SweepBatch<T, C> b,
                                                                        const int4* __restrict__ tiles, const int R,
                                                                        const int row) {
   const int4 tl = __ldg(tiles + blockIdx.x);
@@ -2053,9 +2054,19 @@ cudaError_t launch_batch_sweep(const SweepParams<T, C>* m, int n, const int4* ti
   return cudaGetLastError();
 }
 
-// {member, first row, interior, first column} of each block of the members' sweeps.
+// {member, first row, interior, first column} of each block of the members' sweeps.  Rows a warp
+// (R) by the rows each resident warp has to do (U), as in sweep_rows: with few, short runs reach
+// more SMs; with many, long ones form the row above a run's first less often.  Us a step at 1, 2, 4, 6, 8
+// rows, FP32: 4 lenses of side 64-128 (U 0.3) 4.9, 6.2, 8.9, 11.6, 14.3; 16 (1.1) 10.0, 7.6, 9.5, 11.6,
+// 14.2; 16 of 128-256 (4.5) 31.5, 17.6, 13.9, 14.8, 16.3; 16 of 256-512 (18) 56.7, 38.4, 30.9, 30.3, 31.4;
+// 16 of 400-700 (36) 108.7, 75.6, 60.3, 57.7, 57.0; 48 of them (100) 306, 207, 161, 150, 145.  FP16, bound
+// by instructions rather than by memory, 4 and 6 rows: 8 of 256-512 22.7 and 23.6, 8 of 400-700 30.9 and 32.3.
 template <class T, class C>
-void sweep_tiles(const SweepParams<T, C>* m, int n, int R, std::vector<int4>& tiles) {
+int sweep_tiles(const SweepParams<T, C>* m, int n, std::vector<int4>& tiles) {
+  double U = 0;
+  for (int q = 0; q < n; ++q) U += (double)((m[q].Nz + 31) / 32) * m[q].Nx / (152.0 * 8 * kBatchSweepMinBlocks);
+  const bool half = sizeof(T) == 2;
+  const int R = U < 1 ? 1 : (U < 2 ? 2 : (U < 15 || half ? 4 : (U < 22 ? 6 : 8)));
   tiles.clear();
   for (int q = 0; q < n; ++q) {
     const SweepParams<T, C>& p = m[q];
@@ -2069,6 +2080,7 @@ void sweep_tiles(const SweepParams<T, C>* m, int n, int R, std::vector<int4>& ti
         tiles.push_back(make_int4(q, i, in ? 1 : 0, k));
       }
   }
+  return R;
 }
 
 template <class T>
@@ -2244,8 +2256,8 @@ template cudaError_t launch_batch_sweep<float, float>(const SweepParams<float, f
                                                       cudaStream_t);
 template cudaError_t launch_batch_sweep<__half, float>(const SweepParams<__half, float>*, int, const int4*, int, bool, int,
                                                        int, cudaStream_t);
-template void sweep_tiles<float, float>(const SweepParams<float, float>*, int, int, std::vector<int4>&);
-template void sweep_tiles<__half, float>(const SweepParams<__half, float>*, int, int, std::vector<int4>&);
+template int sweep_tiles<float, float>(const SweepParams<float, float>*, int, std::vector<int4>&);
+template int sweep_tiles<__half, float>(const SweepParams<__half, float>*, int, std::vector<int4>&);
 template cudaError_t launch_prologue_batch<double>(const PrologueParams*, const int*, int, int, int, int, double*,
                                                    unsigned long long*, cudaStream_t);
 template cudaError_t launch_prologue_batch<float>(const PrologueParams*, const int*, int, int, int, int, double*,

@@ -63,9 +63,9 @@ SweepParams<T, C> sweep_params(const StepParams<T, C>& p);
 template <class T, class C>
 cudaError_t launch_batch_sweep(const SweepParams<T, C>* m, int n, const int4* tiles, int nblocks, bool uniform, int R,
                                int row, cudaStream_t s);
-// The blocks' tiles for it.
+// The blocks' tiles for it; returns the rows a warp (R) that they are for.
 template <class T, class C>
-void sweep_tiles(const SweepParams<T, C>* m, int n, int R, std::vector<int4>& tiles);
+int sweep_tiles(const SweepParams<T, C>* m, int n, std::vector<int4>& tiles);
 // blocks one member occupies in a batched update launch; march = cells each thread walks
 // along x (planar: rows 8 apart; 3-D: planes), one of 1, 2, 4, 8
 int batch_blocks(int Nx, int Ny, int Nz, bool planar, int march);

@@ -52,3 +52,35 @@ def _compare(ps, runs=(17, 8, 8, 9), chunk=8):
 @pytest.mark.parametrize("count", [1, 49, 54, 55])
 def test_members_of_one_sweep_launch(engine, precision, count):
     _compare([_lens(24 + 3 * (k % 11), 30 + 7 * (k % 5), precision, k) for k in range(count)])
+
+
+def test_the_tuner_takes_members_of_the_half_steps(engine):
+    """Planar float members of 2^19 cells and more never step in the half-step launches: the tuner
+    has no pick for them, in a batch or for one handle."""
+    from luxum_gb300 import Batch
+
+    small, large = _sim(_lens(300, 311, 1)), _sim(_lens(725, 724, 1))
+    double = _sim(_lens(725, 724, 0))
+    batch = Batch()
+    batch.add(small)
+    batch.add(large)
+    assert batch.tune_member(large, 2) == 0 and batch.tune_table() == []
+    batch.autotune(2)
+    assert [dict(e, march=0) for e in batch.tune_table()] == [dict(small.tune_class(), march=0)]
+    assert batch.tune_member(small, 2) in (1, 2, 4, 8)
+    batch.close()
+    other = Batch()
+    other.add(double)
+    other.autotune(2)
+    assert len(other.tune_table()) == 1
+    other.close()
+    for s in (small, large, double):
+        s.close()
+
+
+# the sweep's rows a warp: 1, 2, 4, 6, 8 (4 at most in FP16), by the rows of all its members
+@pytest.mark.parametrize("precision", [1, 2])
+@pytest.mark.parametrize("count, n, m", [(1, 130, 127), (1, 300, 511), (1, 301, 513), (2, 450, 577), (3, 513, 640),
+                                         (8, 480, 700), (8, 640, 800)])
+def test_rows_of_the_batched_sweep(engine, precision, count, n, m):
+    _compare([_lens(n + k, m - 5 * k, precision, k) for k in range(count)])
