@@ -315,7 +315,7 @@ LX_API lx_status lx_batch_set_tune_table(lx_batch* b, const lx_tune_entry* entri
 /* Copies up to cap entries to entries (may be NULL when cap is 0); *n = the table's length. */
 LX_API lx_status lx_batch_get_tune_table(const lx_batch* b, lx_tune_entry* entries, int cap, int* n);
 /* Tunes the class of every member that may step in the half-step launches (3-D members of 2^18
- * cells or more and planar float members of 2^19 never do).  Zero-field twins of a sample of the
+ * cells or more, planar FP32 members of 2^19 and FP16 ones of 2^21 are left out).  Zero-field twins of a sample of the
  * members (up to 1.5e8 cells, at least one per class; created and freed here) are stepped
  * together in those launches, `steps` steps per timing: first with one march for every class, then
  * with each class in turn (largest first) moved to each other march, a move kept when the

@@ -1759,7 +1759,7 @@ static lx_status run_steps(lx_sim* s, int nsteps, KernelTimer* kt = nullptr) {
         lx::StepParams<T, C> sw = sp;
         if (t & 1) swap_buffers(sw);
         if ((st = tic())) return st;
-        if (s->planar) CK(lx::launch_step_sweep2<T, C>(sw, s->uniform, behind, s->stream));
+        if (s->planar) CK(lx::launch_step_sweep2<T, C>(sw, s->uniform, behind, false, s->stream));
         else CK(lx::launch_step_sweep3<T, C>(sw, s->uniform, s->stream));
         if ((st = toc(1))) return st;
         s->n_kernels += 1;
@@ -2088,16 +2088,11 @@ struct lx_batch {
   // 3-D members of at least kSoloCells cells take one kernel pair each, with their parameter
   // block passed by value (the constant bank, as for a handle stepped alone), spread over the
   // batch stream and kLanes - 1 more so that the members' kernels overlap.  Planar members with
-  // float compute step in their two buffers (ping-pong mode): of at least kSoloCells2 cells one
-  // by one like these, a few smaller ones together in the batched sweep (see batch_rebuild).  The
-  // others share the batched half-step launches in place.
+  // float compute step in their two buffers (ping-pong mode), of at least solo_cells2 cells one by
+  // one like these, smaller ones together in the batched sweep, or in place in the batched half-step
+  // launches (batch_rebuild chooses).  The others share the batched half-step launches.
   static constexpr long long kSoloCells = 1LL << 18;
-  // (us a step of 48 lenses of side 128-1024, 12 and 96 of them, 16 of side 1000, one by one from
-  // 2^21, 2^20 and 2^19 cells: 142, 138, 135; 43, 39, 38; 226, 222, 211; 140, 134, 143; 256 of them
-  // 107, 106 and 113 Gcell/s.  Launched directly a member's step costs the host 2 us: a served burst
-  // of 32 requests 91.1 and 96.3 ms from 2^20 and 2^19.)  Twice that in an FP32 batch whose planar
-  // members all fit one sweep launch.
-  static constexpr long long kSoloCells2 = 1LL << 19;
+  static constexpr long long kSoloCells2 = 1LL << 19;  // the least solo_cells2
   long long solo_cells2 = kSoloCells2;
   static constexpr int kLanes = 4;
   cudaStream_t lanes[kLanes - 1] = {};
@@ -2118,7 +2113,7 @@ struct lx_batch {
   };
   int march2d = lx::kMarch2, march3d = lx::kMarch3;  // per dimension (lx_batch_set_march / autotune)
   bool march_set = false;            // set by a caller or the tuner: not adapted to the batch's size
-  bool half_steps = false;           // the tuner's twins: no batched sweep, which has no tile shape
+  bool half_steps = false;           // the tuner's twins: planar members in the half-step launches only
   std::vector<lx_tune_entry> table;  // march per member class (lx_batch_set_tune_table / autotune)
   struct DftClass {  // DFT planes that sample at the same batch steps
     int every = 1, phase = 0;
@@ -2145,6 +2140,7 @@ struct lx_batch {
   cudaGraphExec_t exec = nullptr;
   int exec_steps = 0;
   long long chunks_since_rebuild = 0;  // a chunk is captured only when the one before had the same members
+  bool serving = false;                // a server's: members come and go between chunks
   long long exec_base_mod = -1;
   bool graphable = true;
   std::vector<int> host_ts;
@@ -2154,16 +2150,19 @@ struct lx_batch {
 
 static void batch_member_changed(lx_batch* b) { b->dirty = true; }
 
-// A member launched one by one: 3-D members of kSoloCells cells or more, planar single-sweep
-// members of solo_cells2 cells or more.
+void lx::batch_serves(lx_batch* b) { b->serving = true; }
+
+// A member launched one by one: 3-D members of kSoloCells cells or more, planar float members of
+// solo_cells2 cells or more.
 static bool batch_alone(const lx_batch* b, const lx_sim* s) {
   return s->planar ? s->sweep && (long long)s->Nx * s->Nz >= b->solo_cells2
                    : (long long)s->Nx * s->Ny * s->Nz >= lx_batch::kSoloCells;
 }
 
-// A member the tuner takes no sample of: it never steps in the half-step launches.
+// A member the tuner takes no sample of: it never steps in the half-step launches (or, FP16 members
+// of 2^21 cells or more, only beside many cells, where it runs best at the default).
 static bool batch_untuned(const lx_sim* s) {
-  return s->planar ? s->sweep && (long long)s->Nx * s->Nz >= lx_batch::kSoloCells2
+  return s->planar ? s->sweep && (long long)s->Nx * s->Nz >= lx_batch::kSoloCells2 << (s->prec == LX_PREC_FP16S ? 2 : 0)
                    : (long long)s->Nx * s->Ny * s->Nz >= lx_batch::kSoloCells;
 }
 
@@ -2366,22 +2365,42 @@ static lx_status batch_rebuild(lx_batch* b) {
   BCK(cudaMallocAsync(&b->d_slots, sizeof(unsigned long long) * lx::kAhead * (n > 0 ? n : 1), b->stream));
   BCK(cudaMallocAsync(&b->d_srcv, sizeof(double) * lx::kAhead * (n > 0 ? n : 1), b->stream));
   std::vector<std::vector<lx::DftParams>> dft_planes;
-  // Planar float members step in their two buffers, one by one or while those that share a launch
-  // are few, the others in place in buffer 0; a member whose mode changes at an odd step moves its
-  // state (one device copy).  The batched sweep has one launch a step and half the latency; many
-  // small members, whose rows are mostly CPML, run faster in the two half-step launches at twice the
-  // warps, FP16 storage sooner.  Gcell/s of the sweep and of those, FP32: 100 lenses of side 128-300
-  // 53 and 77, 256 of 128-400 69 and 85 (48 of 128-256 66 and 47, 128-700 96 and 75 before their
-  // tables were formed ahead); FP16: 48 of 128-700 79 and 107, 100 of 128-300 41 and 79.
-  long long shared = 0, shared_cells = 0, sweeps = 0;
-  for (auto* s : b->sims) sweeps += s->planar && s->sweep;
-  b->solo_cells2 = lx_batch::kSoloCells2 * (sizeof(T) == 4 && sweeps <= lx::kSweepMembers ? 2 : 1);
+  // Planar float members step in one of three forms: one by one in lanes, in their two buffers; those
+  // that share a launch in their two buffers too while one batched sweep holds them (one launch a
+  // step); else in place in buffer 0 in the two half-step launches.  A member whose mode changes at
+  // an odd step moves its state (one device copy).  Lenses of uneven side, us a step one by one, in
+  // the sweep, in half steps:
+  //   FP32, 8 and 48 of side 724-800       40 50 45, 220 238 247 (launched directly, 48: 250 241 253)
+  //         16 of 900-1024                 106 129 138
+  //         16 and 48 of 400-700           - 57 53, - 145 156 (half steps fit L2 longer, then move more)
+  //         32 and 64 of 128-256           - 21 22, - 44 39 (64: two sweep launches)
+  //   FP16, 8 and 32 of side 724-800       43 48 44, 170 181 149
+  //         16 of 800-850, 16 of 900-1024  81 - 94, 105 144 120
+  //         16 and 32 of 1024-1448         187 221 186, 362 408 330
+  //         8 and 16 of 400-700            - 31 35, - 64 49
+  //         16 and 48 of 128-256           - 16 16, - 33 29
+  // So FP32 members go one by one from 2^19 cells.  Only in a server's batch, whose chunks are mostly
+  // launched directly (2 us of host time a launch) or captured (3.5), those below 2^20 share the sweep
+  // if one launch holds them: a burst of 32 planar and 3-D requests 90.5 and 94.5 ms.
+  // FP16 is bound by instructions, which half steps have fewer of: they win by the cells of the
+  // batch, first over members that go two rows a warp in lanes (below 620 K cells, sweep_rows), then
+  // over all; and over the sweep in batches of 1.8 M cells, 4 M if their members have 2^18 or more.
+  const bool half = sizeof(T) == 2;
+  long long cells = 0, count = 0, small = 0;  // of the planar float members; those below 2^20 cells
   for (auto* s : b->sims)
-    if (s->planar && s->sweep && !batch_alone(b, s)) {
-      shared++;
-      shared_cells += (long long)s->Nx * s->Nz;
+    if (s->planar && s->sweep) {
+      cells += (long long)s->Nx * s->Nz;
+      count++;
+      small += (long long)s->Nx * s->Nz < 1LL << 20;
     }
-  const bool few = !b->half_steps && shared <= lx::kSweepMembers && (sizeof(T) == 4 || shared_cells <= 1LL << 22);
+  b->solo_cells2 = lx_batch::kSoloCells2;
+  if (!half && b->serving && small <= lx::kSweepMembers) b->solo_cells2 = 1LL << 20;
+  if (half && cells >= 6LL << 20) b->solo_cells2 = 620LL << 10;
+  if (half && (cells >= 27LL << 20 || b->half_steps)) b->solo_cells2 = 1LL << 62;
+  long long shared = 0;
+  for (auto* s : b->sims) shared += s->planar && s->sweep && !batch_alone(b, s);
+  const bool few = !b->half_steps && shared <= lx::kSweepMembers &&
+                   (!half || cells < (cells >= count << 18 ? 1LL << 22 : 7LL << 18));
   for (int q = 0; q < n; q++) {
     lx_sim* s = b->sims[q];
     lx_status st;
@@ -2532,9 +2551,10 @@ static lx_status batch_rebuild(lx_batch* b) {
   return LX_OK;
 }
 
-// Step q of a chunk for member m, launched by value on `st`; row: its place in the sequence.
+// Step q of a chunk for member m, launched by value on `st`; row: its place in the sequence; lanes:
+// the batch's other streams have work beside it.
 template <class T, class C>
-static lx_status solo_step(lx_batch* b, const lx_batch::Group& g, size_t m, int q, int row, cudaStream_t st) {
+static lx_status solo_step(lx_batch* b, const lx_batch::Group& g, size_t m, int q, int row, bool lanes, cudaStream_t st) {
   const int id = g.members[m];
   lx_sim* s = b->sims[id];
   const int t = b->host_ts[id] + q;
@@ -2545,7 +2565,7 @@ static lx_status solo_step(lx_batch* b, const lx_batch::Group& g, size_t m, int 
   if constexpr (sizeof(C) == 4) {
     if (g.sweep) {  // single sweep, state t & 1 -> (t+1) & 1
       if (t & 1) swap_buffers(sp);
-      BCK(lx::launch_step_sweep2<T, C>(sp, g.uniform, false, st));
+      BCK(lx::launch_step_sweep2<T, C>(sp, g.uniform, false, lanes, st));
       swept = true;
     }
   }
@@ -2590,6 +2610,7 @@ static lx_status batch_enqueue(lx_batch* b, long long step0, int nsteps) {
   std::vector<Solo> lane[lx_batch::kLanes];  // lane 0 is the batch stream: the grouped launches' when there are any
   double load[lx_batch::kLanes] = {};
   const int l0 = grouped ? 1 : 0;
+  const bool lanes = (int)solo.size() + l0 >= lx_batch::kLanes;
   for (const Solo& x : solo) {
     int best = l0;
     for (int l = l0; l < lx_batch::kLanes; l++)
@@ -2620,7 +2641,7 @@ static lx_status batch_enqueue(lx_batch* b, long long step0, int nsteps) {
         for (int r = r0; r < r0 + sub; r++)
           for (int l = l0; l < lx_batch::kLanes; l++)
             if (pos < lane[l].size()) {
-              const lx_status st = solo_step<T, C>(b, *lane[l][pos].g, lane[l][pos].m, q0 + r, r,
+              const lx_status st = solo_step<T, C>(b, *lane[l][pos].g, lane[l][pos].m, q0 + r, r, lanes,
                                                    l ? b->lanes[l - 1] : b->stream);
               if (st) return st;
             }

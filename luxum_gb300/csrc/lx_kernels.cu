@@ -1993,10 +1993,16 @@ cudaError_t launch_step(const StepParams<T, C>& p, bool planar, bool uniform, bo
 // spread a small grid over the SMs and even out the end of the launch; long ones form the row
 // above a run's first less often.  With CPML 16 and TF/SF, us a step at 2, 4, 6, 8 rows: 1024^2
 // (U 5.4) 20.0, 20.6, 22.6, 24.6; 2048^2 (21.6) 43.2, 41.1, 41.3, 42.6; 4096^2 (86) 127.2, 113.6,
-// 111.6, 112.8.
-static int sweep_rows(long long cols, int Nx) {
+// 111.6, 112.8.  Beside the launches of a batch's other lanes a launch has a quarter of the GPU, and
+// its end is filled by theirs: us a step of 32 members, 2, 4, 5, 6, 8 rows, FP32 of side 724-760 (U
+// 2.9) 146, 152, 162, 174, 197; of 800-850 (3.7) 190, 154, 145, 152, 169; of 900-1024 (4.9) 265, 217,
+// 213, 205, 202; of 1024-1200 (6.6) 346, 287, 274, 270, 263; FP16 of 900-1024 255, 213, 208, 207, 214,
+// 8 of 724-760 40, 36, 37, 41, 47.  (Four FP32 states of 800^2 and less stay in L2, where short runs
+// cost little.)
+static int sweep_rows(long long cols, int Nx, bool half, bool lanes) {
   const double U = (double)cols * Nx / (152.0 * 8 * kSweepMinBlocks);
-  const int R = U < 8 ? 2 : (U < 60 ? 4 : 6);
+  int R = U < 8 ? 2 : (U < 60 ? 4 : 6);
+  if (lanes) R = U < 4.3 ? (half ? 4 : (U < 3.27 ? 2 : 5)) : (U < 6 ? 6 : 8);
   const int least = (int)(((long long)Nx + 8 * 65535 - 1) / (8 * 65535));  // the grid is at most 65535 blocks high
   return R < least ? least : R;
 }
@@ -2031,9 +2037,9 @@ SweepParams<T, C> sweep_params(const StepParams<T, C>& p) {
 }
 
 template <class T, class C>
-cudaError_t launch_step_sweep2(const StepParams<T, C>& p, bool uniform, bool behind, cudaStream_t s) {
+cudaError_t launch_step_sweep2(const StepParams<T, C>& p, bool uniform, bool behind, bool lanes, cudaStream_t s) {
   const long long cols = (p.Nz + 31) / 32;
-  const int R = sweep_rows(cols, p.Nx);
+  const int R = sweep_rows(cols, p.Nx, sizeof(T) == 2, lanes);
   const dim3 block(32, 8), grid((unsigned)cols, (unsigned)((p.Nx + 8 * R - 1) / (8 * R)));
   const SweepParams<T, C> q = sweep_params(p);
   if (uniform) start(step_kernel_2d<T, C, true>, grid, block, behind, s, q, R);
@@ -2244,8 +2250,8 @@ cudaError_t launch_dft_flux(const double* acc, int nfreq, long long ncell, doubl
 LX_INST(double, double)
 LX_INST(float, float)
 LX_INST(__half, float)
-template cudaError_t launch_step_sweep2<float, float>(const StepParams<float, float>&, bool, bool, cudaStream_t);
-template cudaError_t launch_step_sweep2<__half, float>(const StepParams<__half, float>&, bool, bool, cudaStream_t);
+template cudaError_t launch_step_sweep2<float, float>(const StepParams<float, float>&, bool, bool, bool, cudaStream_t);
+template cudaError_t launch_step_sweep2<__half, float>(const StepParams<__half, float>&, bool, bool, bool, cudaStream_t);
 template cudaError_t launch_prologue_ahead<double>(const PrologueParams&, int, const StepCtl*, double*, double*,
                                                    unsigned long long*, cudaStream_t);
 template cudaError_t launch_prologue_ahead<float>(const PrologueParams&, int, const StepCtl*, float*, double*,

@@ -27,9 +27,10 @@ cudaError_t launch_set_ctl(StepCtl* ctl, StepCtl v, cudaStream_t s);
 template <class T, class C>
 cudaError_t launch_step(const StepParams<T, C>& p, bool planar, bool uniform, bool h_half, bool behind, cudaStream_t s);
 // Single-sweep planar step (float compute, two state buffers): reads the buffers named in
-// p.E, p.H, p.psiH, p.psiE and writes those in p.E1, p.H1, p.psiH1, p.psiE1.
+// p.E, p.H, p.psiH, p.psiE and writes those in p.E1, p.H1, p.psiH1, p.psiE1.  lanes: one of the
+// launches that fill a batch's streams.
 template <class T, class C>
-cudaError_t launch_step_sweep2(const StepParams<T, C>& p, bool uniform, bool behind, cudaStream_t s);
+cudaError_t launch_step_sweep2(const StepParams<T, C>& p, bool uniform, bool behind, bool lanes, cudaStream_t s);
 // Single-sweep 3-D step (float compute, two state buffers), lx_sweep3d.cu: the same buffer
 // convention as launch_step_sweep2.
 template <class T, class C>

@@ -37,6 +37,7 @@
 namespace lx {
 lx_status set_thread_error(const char* msg, lx_status st);
 size_t table_bytes(const lx_params& p);
+void batch_serves(lx_batch* b);
 }
 
 namespace {
@@ -391,6 +392,7 @@ extern "C" LX_API lx_status lx_server_create(const lx_server_config* cfg, lx_ser
   cudaGetDevice(&srv->device);
   std::memset(&srv->stats, 0, sizeof srv->stats);
   lx_status st = lx_batch_create(&srv->batch);
+  if (!st) lx::batch_serves(srv->batch);
   if (!st) st = lx_batch_set_chunk(srv->batch, c.chunk);
   if (!st && c.tune_entries > 0) {
     st = lx_batch_set_tune_table(srv->batch, c.tune_table, c.tune_entries);

@@ -103,8 +103,9 @@ struct lx_sim {
   void* psiE[3][2] = {};
   // Single-sweep handles (float compute) keep a second copy of the state.  Stepped
   // alone they run in ping-pong mode (pp): after t steps the state lives in buffer t & 1
-  // (buffer 0 = E, H, psiH, psiE above, buffer 1 here).  In a batch they are updated in place
-  // in buffer 0 (pp = 0); set_pp moves the state when the mode changes.
+  // (buffer 0 = E, H, psiH, psiE above, buffer 1 here).  A batch keeps them so or updates them in
+  // place in buffer 0 (pp = 0), by the form it steps them in; set_pp moves the state when the mode
+  // changes.
   int sweep = 0;
   int pp = 0;
   void* E1[3] = {};
@@ -179,4 +180,6 @@ namespace lx {
 void* comp_ptr(lx_sim* s, int comp, bool other = false);
 // TF/SF tables of one step of the handle that *p, which is valid, would give.
 size_t table_bytes(const lx_params& p);
+// Tells a new batch that it is a server's.
+void batch_serves(lx_batch* b);
 }  // namespace lx

@@ -26,18 +26,19 @@ def _sim(p):
     return s
 
 
-def _compare(ps, runs=(17, 8, 8, 9), chunk=8):
+def _compare(ps, runs=(17, 8, 8, 9), chunk=8, before=0):
     from luxum_gb300 import Batch
 
     sims = [_sim(p) for p in ps]
     batch = Batch(chunk=chunk)
-    for s in sims:
+    for k, s in enumerate(sims):
+        s.step(k % 3 if before else 0)
         batch.add(s)
     for n in runs:
         batch.step(n)
-    for p, s in zip(ps, sims):
+    for k, (p, s) in enumerate(zip(ps, sims)):
         twin = _sim(p)
-        twin.step(sum(runs))
+        twin.step(sum(runs) + (k % 3 if before else 0))
         for c in (1, 3, 5):
             assert np.array_equal(s.field(c), twin.field(c)), (p.Nx, p.Nz, c)
         assert s.max_e2() == twin.max_e2() > 0
@@ -84,3 +85,21 @@ def test_the_tuner_takes_members_of_the_half_steps(engine):
                                          (8, 480, 700), (8, 640, 800)])
 def test_rows_of_the_batched_sweep(engine, precision, count, n, m):
     _compare([_lens(n + k, m - 5 * k, precision, k) for k in range(count)])
+
+
+# members one by one in lanes, at 2, 5, 6 and 8 rows a warp (FP16 4, 6 and 8): FP32 from 2^19 cells beside more members
+# than one sweep holds, FP16 beside few cells
+SOLO = [(731, 740), (811, 835), (1001, 903), (1201, 1103)]
+
+
+@pytest.mark.parametrize("precision, small", [(1, 55), (2, 0)])
+def test_rows_of_members_in_lanes(engine, precision, small):
+    ps = [_lens(n, m, precision, k) for k, (n, m) in enumerate(SOLO + SOLO[::-1][:2])]
+    _compare(ps + [_lens(24 + k % 7, 40 + k % 9, precision, k) for k in range(small)], runs=(5, 8, 8, 4), before=1)
+
+
+# FP16: lanes for members of 620 K cells and more beside the half steps of the others, from 6 M cells
+# of the batch on; half steps for all from 27 M
+@pytest.mark.parametrize("sides", [[(1300, 1111)] * 4 + [(701, 803), (90, 77)], [(1901, 1853)] * 7 + [(2100, 1900), (300, 333)]])
+def test_fp16_members_by_the_cells_of_the_batch(engine, sides):
+    _compare([_lens(n + k, m - k, 2, k) for k, (n, m) in enumerate(sides)], runs=(5, 8, 8, 4), before=1)
