@@ -1972,11 +1972,10 @@ cudaError_t launch_step(const StepParams<T, C>& p, bool planar, bool uniform, bo
               p.Nz >= 48;
     // Float half steps beyond those give blocks in the slab of one axis their own path (h_slab_3d):
     // us a step of both with and without it, 512x512x128 FP32 (CPML 20) 592 and 654, 256^3 (CPML
-    // 16, TF/SF) 299 and 324, in FP16 storage 268 and 299; from 2^20 cells, as the longer code costs
-    // a short launch more than the path saves.  FP64 is bound by its pipe.
+    // 16, TF/SF) 299 and 324, in FP16 storage 268 and 299.  FP64 is bound by its pipe.
     bool slab = false;
     const bool reach = sizeof(T) != 2 || (long long)p.Nx * p.Ny * p.Nzp < (1LL << 30);  // e_slab_3d's offsets
-    if constexpr (sizeof(C) == 4) slab = p.pml && reach && (long long)p.Nx * p.Ny * p.Nz >= (1LL << 20);
+    if constexpr (sizeof(C) == 4) slab = p.pml && reach;
     if constexpr (sizeof(C) == 4)
       if (slab) {
         if (uniform) launch_step_3d<T, C, true, true>(q, mon, h_half, behind, s);
