@@ -39,3 +39,21 @@ def test_tall_planar_grids(engine, precision, rows):
     b, bm = _probes((333, 1, 35), precision, 5, 14, at)
     assert np.abs(a).max() > 0 and np.array_equal(a, b)
     assert am == bm > 0
+
+
+# 32-bit byte offsets reach FP32 arrays of 2^29 elements and FP16 ones of 2^30 (4-byte coefficients):
+# the largest grids below, in packed rows too, and the smallest beyond
+@pytest.mark.parametrize("precision, n", [(1, (1023, 1024, 509)), (1, (2047, 2048, 100)), (1, (1024, 1025, 510)),
+                                          (2, (1023, 2048, 509)), (2, (1025, 2048, 509))])
+def test_3d_grids_at_the_reach_of_offsets(engine, precision, n):
+    from luxum_gb300 import trim_device_memory
+
+    row = 128 // (4 if precision == 1 else 2)
+    padded = n[0] * n[1] * (-(-n[2] // row) * row)
+    assert abs(padded / (1 << (29 if precision == 1 else 30)) - 1) < 2e-3
+    at = [(i, j, k) for i in (0, 3, 6, 9) for j in (0, 4, 8, 10) for k in (0, 5, 9, 12)]
+    a, am = _probes(n, precision, 5, 14, at)
+    trim_device_memory()
+    b, bm = _probes((45, 46, 47), precision, 5, 14, at)
+    assert np.abs(a).max() > 0 and np.array_equal(a, b)
+    assert am == bm > 0
