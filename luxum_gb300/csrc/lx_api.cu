@@ -376,6 +376,7 @@ template <class C>
 static lx_status upload_vec(lx_sim* s, void** dst, const std::vector<double>& v) {
   std::vector<C> tmp(v.size());
   for (size_t q = 0; q < v.size(); q++) tmp[q] = (C)v[q];
+  // a cell on the far wall loads the entry past an H profile's end (of N - 1), and does not use it
   CK(cudaMallocAsync(dst, tmp.size() * sizeof(C) + 16, s->own));
   CK(cudaMemcpyAsync(*dst, tmp.data(), tmp.size() * sizeof(C), cudaMemcpyHostToDevice, s->own));
   s->n_h2d += tmp.size() * sizeof(C);

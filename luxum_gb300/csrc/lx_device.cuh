@@ -159,7 +159,8 @@ struct MaxBits<float> {
 // the FP64 pipe, which bounds these kernels (256^3 with CPML and TF/SF, monitored: E 509 us a
 // launch against 415 unmonitored); the bound takes about twenty of the idle integer and float
 // pipes.  The float of |v| is its high word one unit up, clamped to [2^-126, inf]: never below
-// |v|, inf for anything a float cannot hold and for NaN.
+// |v|, inf for anything a float cannot hold and for NaN.  (e_small_3d forms the squares of every
+// cell: its launches are not bound by that pipe.)
 template <class C>
 struct MaxScreen {
   __device__ __forceinline__ explicit MaxScreen(const unsigned long long*) {}

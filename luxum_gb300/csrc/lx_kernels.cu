@@ -470,7 +470,7 @@ __device__ __forceinline__ int slab_path(const StepParams<T, C>& p, unsigned tf,
 }
 
 // Resident blocks per SM asked of the compiler for the H kernel (a register cap): 8 for
-// float compute (32 registers, 12-16 bytes spilled; FP16 storage 14 % faster than at 40
+// float compute (32 registers, 0-28 bytes spilled; FP16 storage 14 % faster than at 40
 // registers), 5 for FP64 (its natural 48 registers; an explicit 1 lets the compiler take 54).
 template <class C>
 struct HMinBlocks {
@@ -748,9 +748,10 @@ __device__ __forceinline__ typename MaxBits<C>::type e_in_3d(const StepParams<T,
 
 // Resident blocks per SM asked of the compiler for the 3-D E kernel.  FP16 storage with the slab
 // paths' 32-bit offsets and FP32 run best at 40 registers (6 blocks; us an E launch of 201x187x259
-// FP16 104 against 108 with 8, 256^3 145 and 147, monitored 165 and 172), FP16 without CPML at 32
-// with a few spilled (256^3 0.3196 -> 0.3116 ms a step), and FP64 with its FMA forms at 6 blocks
-// (256^3 with CPML and TF/SF 0.431 -> 0.415 ms against the compiler's own 60 registers).
+// FP16 104 against 108 with 8, 256^3 145 and 147, monitored 165 and 172; the monitored forms spill
+// 4-36 bytes), FP16 without CPML at 32 with 12-44 bytes spilled (256^3 0.3196 -> 0.3116 ms a step),
+// and FP64 with its FMA forms at 6 blocks, although it spills 32-84 bytes there (256^3 with CPML and
+// TF/SF 0.431 -> 0.415 ms against the compiler's own 60 registers).
 template <class T, bool SLAB>
 struct EMinBlocks {
   static constexpr int v = sizeof(T) == 2 && !SLAB ? 8 : 6;
@@ -1352,8 +1353,8 @@ __device__ __forceinline__ typename MaxBits<C>::type step2_warp(const SweepParam
 }
 
 // Register cap of the single-sweep kernel: 5 blocks of 256 per SM (48 registers; the general path
-// spills 48 bytes).  With 6 it spills 120 (4096^2 with CPML and TF/SF 122.5 us a step against
-// 112.7), with 4 none (118.9).
+// spills 64 bytes, FP16 72).  4096^2 FP32 with CPML and TF/SF 112.7 us a step, with 6 blocks 122.5,
+// with 4 118.9.
 constexpr int kSweepMinBlocks = 5;
 
 // One simulation: a block is 32 z columns x 8 warps of R rows.
