@@ -1390,7 +1390,8 @@ __global__ void __launch_bounds__(256, kBatchSweepMinBlocks) step_batch_2d(const
   const int i1 = min(i0 + R, g.Nx);
   const C* tab = g.tab + (long long)row * g.tab_stride;
   const typename MaxBits<C>::type v =
-      warp_max(tl.z ? step2_rows<T, C, UNI, true>(g, i0, i1, k0, false, false, tab) : step2_warp<T, C, UNI>(g, i0, i1, k0, tab));
+      warp_max(tl.z ? step2_rows<T, C, UNI, true, true>(g, i0, i1, k0, false, false, tab)
+                    : step2_warp<T, C, UNI, true>(g, i0, i1, k0, tab));
   if (threadIdx.x == 0) {  // (a warp's maximum straight to the slot: a block's warps end at different times)
     unsigned long long* slot = g.max_slot + (long long)row * g.slot_stride;
     const unsigned long long bits = as_slot_bits(v);
@@ -1943,7 +1944,8 @@ static void launch_small_3d(const StepParams<T, C>& p, bool uniform, bool mon, b
 }
 
 template <class T, class C>
-cudaError_t launch_step(const StepParams<T, C>& p, bool planar, bool uniform, bool h_half, bool behind, cudaStream_t s) {
+cudaError_t launch_step(const StepParams<T, C>& p, bool planar, bool uniform, bool h_half, bool behind, bool lanes,
+                        cudaStream_t s) {
   // single simulations: one cell per thread (their parameters sit in the constant bank, and
   // walking several cells raises register use past what pays off)
   dim3 block(32, 8);
@@ -2045,8 +2047,13 @@ cudaError_t launch_step_sweep2(const StepParams<T, C>& p, bool uniform, bool beh
   const int R = sweep_rows(cols, p.Nx, sizeof(T) == 2, lanes);
   const dim3 block(32, 8), grid((unsigned)cols, (unsigned)((p.Nx + 8 * R - 1) / (8 * R)));
   const SweepParams<T, C> q = sweep_params(p);
-  if (uniform) start(step_kernel_2d<T, C, true>, grid, block, behind, s, q, R);
-  else start(step_kernel_2d<T, C, false>, grid, block, behind, s, q, R);
+  if (q.pml) {
+    if (uniform) start(step_kernel_2d<T, C, true, true>, grid, block, behind, s, q, R);
+    else start(step_kernel_2d<T, C, false, true>, grid, block, behind, s, q, R);
+  } else {
+    if (uniform) start(step_kernel_2d<T, C, true, false>, grid, block, behind, s, q, R);
+    else start(step_kernel_2d<T, C, false, false>, grid, block, behind, s, q, R);
+  }
   return cudaGetLastError();
 }
 
@@ -2238,7 +2245,7 @@ cudaError_t launch_dft_flux(const double* acc, int nfreq, long long ncell, doubl
 }
 
 #define LX_INST(T, C)                                                                                                  \
-  template cudaError_t launch_step<T, C>(const StepParams<T, C>&, bool, bool, bool, bool, cudaStream_t);                 \
+  template cudaError_t launch_step<T, C>(const StepParams<T, C>&, bool, bool, bool, bool, bool, cudaStream_t);           \
   template cudaError_t launch_gather<T>(const T*, double*, const int[3], int, int, double, cudaStream_t);                     \
   template cudaError_t launch_scatter<T>(const double*, T*, const int[3], int, int, int, double, double, double,      \
                                          double, cudaStream_t);                                                        \
