@@ -1204,7 +1204,7 @@ struct Row2 {
 
 // One warp's rows [i0, i1) of the 32 columns from k0; returns the bit pattern of its largest
 // Ey^2 (the max over the whole Ey array, two_dim_pml.cc:181).
-template <class T, class C, bool UNI, bool FAST>
+template <class T, class C, bool UNI, bool FAST, bool PML>
 __device__ __forceinline__ typename MaxBits<C>::type step2_rows(const SweepParams<T, C>& p, const int i0, const int i1,
                                                                 const int k0, const bool tfH, const bool tfE,
                                                                 const C* tab) {
@@ -1219,7 +1219,7 @@ __device__ __forceinline__ typename MaxBits<C>::type step2_rows(const SweepParam
   const long long si = p.si;
   // the z slab: psi index and profile values of this column, and (lane 0) of column k0-1
   const int zn = p.slab[2].n;
-  const bool pml = !FAST && p.pml;
+  const bool pml = !FAST && PML && p.pml;
   const int sz = pml ? slab_index(p.slab[2], k) : -1;
   const int szh = pml && halo ? slab_index(p.slab[2], k0 - 1) : -1;
   C bHz = C(0), cHz = C(0), rHz = C(0), bEz = C(0), cEz = C(0), rEz = C(0), bHh = C(0), cHh = C(0), rHh = C(0);
@@ -1342,30 +1342,32 @@ __device__ __forceinline__ typename MaxBits<C>::type step2_rows(const SweepParam
 
 // A warp's run with its TF/SF and interior tests: H is formed on rows [i0-1, i1) and columns
 // [k0-1, k0+32), E on rows [i0, i1) and columns [k0, k0+32).
-template <class T, class C, bool UNI>
+template <class T, class C, bool UNI, bool PML>
 __device__ __forceinline__ typename MaxBits<C>::type step2_warp(const SweepParams<T, C>& p, const int i0, const int i1,
                                                                 const int k0, const C* tab) {
   const bool tfH = p.tfsf && tile_meets_planes(p.planesH, i0 - 1, i1 - i0 + 1, 0, 1, k0 - 1, 34);
   const bool tfE = p.tfsf && tile_meets_planes(p.planesE, i0, i1 - i0, 0, 1, k0, 32);
   if (!tfH && !tfE && tile_is_interior_2d(p.slab, p.pml, p.Nx, p.Nz, i0 - 1, i1 - i0 + 2, k0 - 1, 34))
-    return step2_rows<T, C, UNI, true>(p, i0, i1, k0, false, false, tab);
-  return step2_rows<T, C, UNI, false>(p, i0, i1, k0, tfH, tfE, tab);
+    return step2_rows<T, C, UNI, true, PML>(p, i0, i1, k0, false, false, tab);
+  return step2_rows<T, C, UNI, false, PML>(p, i0, i1, k0, tfH, tfE, tab);
 }
 
 // Register cap of the single-sweep kernel: 5 blocks of 256 per SM (48 registers; the general path
-// spills 64 bytes, FP16 72).  4096^2 FP32 with CPML and TF/SF 112.7 us a step, with 6 blocks 122.5,
-// with 4 118.9.
+// spills 64 bytes, FP16 72, and without CPML none).  4096^2 FP32 with CPML and TF/SF 112.7 us a step,
+// with 6 blocks 122.5, with 4 118.9.
 constexpr int kSweepMinBlocks = 5;
 
-// One simulation: a block is 32 z columns x 8 warps of R rows.
-template <class T, class C, bool UNI>
+// One simulation: a block is 32 z columns x 8 warps of R rows.  Grids without CPML have their own
+// form: with the psi code in it, and its spills, 100000x64 FP32 takes 66.6 us a step instead of 44.6,
+// FP16 85.8 instead of 55.2, 512^2 FP32 5.4 instead of 3.9.
+template <class T, class C, bool UNI, bool PML>
 __global__ void __launch_bounds__(256, kSweepMinBlocks) step_kernel_2d(const SweepParams<T, C> p, const int R) {
   step_behind();
   step_open();
   const int k0 = blockIdx.x * 32;
   const int i0 = (blockIdx.y * 8 + threadIdx.y) * R;
   typename MaxBits<C>::type m = 0;
-  if (i0 < p.Nx) m = step2_warp<T, C, UNI>(p, i0, min(i0 + R, p.Nx), k0, p.tab);
+  if (i0 < p.Nx) m = step2_warp<T, C, UNI, PML>(p, i0, min(i0 + R, p.Nx), k0, p.tab);
   if (p.max_slot) block_max_atomic(m, p.max_slot);
 }
 
@@ -1388,7 +1390,8 @@ __global__ void __launch_bounds__(256, kBatchSweepMinBlocks) step_batch_2d(const
   const int i1 = min(i0 + R, g.Nx);
   const C* tab = g.tab + (long long)row * g.tab_stride;
   const typename MaxBits<C>::type v =
-      warp_max(tl.z ? step2_rows<T, C, UNI, true>(g, i0, i1, k0, false, false, tab) : step2_warp<T, C, UNI>(g, i0, i1, k0, tab));
+      warp_max(tl.z ? step2_rows<T, C, UNI, true, true>(g, i0, i1, k0, false, false, tab)
+                    : step2_warp<T, C, UNI, true>(g, i0, i1, k0, tab));
   if (threadIdx.x == 0) {  // (a warp's maximum straight to the slot: a block's warps end at different times)
     unsigned long long* slot = g.max_slot + (long long)row * g.slot_stride;
     const unsigned long long bits = as_slot_bits(v);
@@ -2042,8 +2045,13 @@ cudaError_t launch_step_sweep2(const StepParams<T, C>& p, bool uniform, bool beh
   const int R = sweep_rows(cols, p.Nx, sizeof(T) == 2, lanes);
   const dim3 block(32, 8), grid((unsigned)cols, (unsigned)((p.Nx + 8 * R - 1) / (8 * R)));
   const SweepParams<T, C> q = sweep_params(p);
-  if (uniform) start(step_kernel_2d<T, C, true>, grid, block, behind, s, q, R);
-  else start(step_kernel_2d<T, C, false>, grid, block, behind, s, q, R);
+  if (q.pml) {
+    if (uniform) start(step_kernel_2d<T, C, true, true>, grid, block, behind, s, q, R);
+    else start(step_kernel_2d<T, C, false, true>, grid, block, behind, s, q, R);
+  } else {
+    if (uniform) start(step_kernel_2d<T, C, true, false>, grid, block, behind, s, q, R);
+    else start(step_kernel_2d<T, C, false, false>, grid, block, behind, s, q, R);
+  }
   return cudaGetLastError();
 }
 
