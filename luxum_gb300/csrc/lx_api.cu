@@ -1769,10 +1769,10 @@ static lx_status run_steps(lx_sim* s, int nsteps, KernelTimer* kt = nullptr) {
     }
     if (!swept) {
       if ((st = tic())) return st;
-      CK(lx::launch_step<T, C>(sp, s->planar, s->uniform, true, behind, s->stream));
+      CK(lx::launch_step<T, C>(sp, s->planar, s->uniform, true, behind, false, s->stream));
       if ((st = toc(1))) return st;
       if ((st = tic())) return st;
-      CK(lx::launch_step<T, C>(sp, s->planar, s->uniform, false, chain, s->stream));
+      CK(lx::launch_step<T, C>(sp, s->planar, s->uniform, false, chain, false, s->stream));
       if ((st = toc(2))) return st;
       s->n_kernels += 2;
     }
@@ -2571,8 +2571,8 @@ static lx_status solo_step(lx_batch* b, const lx_batch::Group& g, size_t m, int 
     }
   }
   if (!swept) {
-    BCK(lx::launch_step<T, C>(sp, g.planar, g.uniform, true, false, st));
-    BCK(lx::launch_step<T, C>(sp, g.planar, g.uniform, false, true, st));
+    BCK(lx::launch_step<T, C>(sp, g.planar, g.uniform, true, false, lanes, st));
+    BCK(lx::launch_step<T, C>(sp, g.planar, g.uniform, false, true, lanes, st));
   }
   for (auto& d : s->dfts) {
     if (t % d.every != 0) continue;

@@ -1907,16 +1907,17 @@ static void launch_step_3d(const StepParams<T, C>& q, bool mon, bool h_half, boo
 //   size: 512x512x100 232 and 260, 800x800x40 249 and 320.
 // - FP16 storage with CPML: H 128^3 with CPML 6 and 12 21.4 and 22.2, 21.7 and 23.7, 150^3 44 and
 //   39; E 150^3 45.8 and 46.7 (with CPML 15 42.5 and 46.7), 200^3 113 and 77 (the slab paths there
-//   have 64 warps an SM).
+//   have 64 warps an SM).  Not beside the launches of a batch's other lanes, which fill the waits of
+//   either: 8 cubes of side 64-128 with CPML 5 and 10 208 and 185, 200 and 193.
 // - Float without CPML: 64^3 5.7 and 6.4, 73^3 7.7 and 8.5, 80^3 9.5 and 9.2.
 // 32-bit byte offsets: arrays below 2^31 bytes.
 template <class T, class C>
-static bool loads_ahead(const StepParams<T, C>& p, bool h_half, bool pack) {
+static bool loads_ahead(const StepParams<T, C>& p, bool h_half, bool pack, bool lanes) {
   const long long cells = (long long)p.Nx * p.Ny * p.Nz;
   if (sizeof(C) == 8) return cells <= 152LL * SmallCells<C>::v * (p.pml ? 10 : 5);
   if ((long long)p.Nx * p.Ny * p.Nzp >= 1LL << 29 || p.Ny > 4 * 65535) return false;
   if (!p.pml) return cells <= 3LL << 17;
-  if (sizeof(T) == 2) return cells <= (h_half ? 1LL << 21 : 1LL << 22);
+  if (sizeof(T) == 2) return !lanes && cells <= (h_half ? 1LL << 21 : 1LL << 22);
   return !h_half || pack || cells <= 5LL << 20;
 }
 
@@ -1943,7 +1944,8 @@ static void launch_small_3d(const StepParams<T, C>& p, bool uniform, bool mon, b
 }
 
 template <class T, class C>
-cudaError_t launch_step(const StepParams<T, C>& p, bool planar, bool uniform, bool h_half, bool behind, cudaStream_t s) {
+cudaError_t launch_step(const StepParams<T, C>& p, bool planar, bool uniform, bool h_half, bool behind, bool lanes,
+                        cudaStream_t s) {
   // single simulations: one cell per thread (their parameters sit in the constant bank, and
   // walking several cells raises register use past what pays off)
   dim3 block(32, 8);
@@ -1966,7 +1968,7 @@ cudaError_t launch_step(const StepParams<T, C>& p, bool planar, bool uniform, bo
     // 256^3 drop-in grid E 0.2035 -> 0.189 ms (FP32), 0.200 -> 0.187 (FP16 storage), from its
     // CPML and TF/SF tiles; the H kernel ran 0.015 ms slower with them, CPML or not.
     const bool pack = sizeof(C) == 8 || 5LL * p.Nz <= 4LL * ((p.Nz + 31) & ~31);
-    if (loads_ahead<T, C>(p, h_half, pack)) {
+    if (loads_ahead<T, C>(p, h_half, pack, lanes)) {
       if (pack) launch_small_3d<T, C, true>(p, uniform, mon, h_half, behind, s);
       else if constexpr (sizeof(C) == 4) launch_small_3d<T, C, false>(p, uniform, mon, h_half, behind, s);
       return cudaGetLastError();
@@ -2243,7 +2245,7 @@ cudaError_t launch_dft_flux(const double* acc, int nfreq, long long ncell, doubl
 }
 
 #define LX_INST(T, C)                                                                                                  \
-  template cudaError_t launch_step<T, C>(const StepParams<T, C>&, bool, bool, bool, bool, cudaStream_t);                 \
+  template cudaError_t launch_step<T, C>(const StepParams<T, C>&, bool, bool, bool, bool, bool, cudaStream_t);           \
   template cudaError_t launch_gather<T>(const T*, double*, const int[3], int, int, double, cudaStream_t);                     \
   template cudaError_t launch_scatter<T>(const double*, T*, const int[3], int, int, int, double, double, double,      \
                                          double, cudaStream_t);                                                        \

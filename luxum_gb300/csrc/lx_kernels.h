@@ -15,7 +15,7 @@ template <class C>
 cudaError_t launch_prologue_ahead(const PrologueParams& p, int steps, const StepCtl* ctl, C* tab, double* srcv,
                                   unsigned long long* ring, cudaStream_t s);
 // `behind`, of the launches of a step: the stream's last launch was one too, and this one may start
-// beside its end.
+// beside its end.  `lanes`: one of the launches that fill a batch's streams.
 // The point source of one step (its amplitude formed ahead), before the step's H update.
 template <class T>
 cudaError_t launch_source(T* field, long long idx, int kind, const double* v, bool behind, cudaStream_t s);
@@ -25,10 +25,10 @@ cudaError_t launch_finish(const unsigned long long* ring, unsigned mask, unsigne
                           StepCtl* ctl, int steps, int rows, cudaStream_t s);
 cudaError_t launch_set_ctl(StepCtl* ctl, StepCtl v, cudaStream_t s);
 template <class T, class C>
-cudaError_t launch_step(const StepParams<T, C>& p, bool planar, bool uniform, bool h_half, bool behind, cudaStream_t s);
+cudaError_t launch_step(const StepParams<T, C>& p, bool planar, bool uniform, bool h_half, bool behind, bool lanes,
+                        cudaStream_t s);
 // Single-sweep planar step (float compute, two state buffers): reads the buffers named in
-// p.E, p.H, p.psiH, p.psiE and writes those in p.E1, p.H1, p.psiH1, p.psiE1.  lanes: one of the
-// launches that fill a batch's streams.
+// p.E, p.H, p.psiH, p.psiE and writes those in p.E1, p.H1, p.psiH1, p.psiE1.
 template <class T, class C>
 cudaError_t launch_step_sweep2(const StepParams<T, C>& p, bool uniform, bool behind, bool lanes, cudaStream_t s);
 // Single-sweep 3-D step (float compute, two state buffers), lx_sweep3d.cu: the same buffer

@@ -103,3 +103,32 @@ def test_rows_of_members_in_lanes(engine, precision, small):
 @pytest.mark.parametrize("sides", [[(1300, 1111)] * 4 + [(701, 803), (90, 77)], [(1901, 1853)] * 7 + [(2100, 1900), (300, 333)]])
 def test_fp16_members_by_the_cells_of_the_batch(engine, sides):
     _compare([_lens(n + k, m - k, 2, k) for k, (n, m) in enumerate(sides)], runs=(5, 8, 8, 4), before=1)
+
+
+# FP16 cubes of 2^18 cells and more: lanes filled (the general kernels) and not (every load ahead)
+@pytest.mark.parametrize("count", [2, 4])
+def test_fp16_cubes_in_lanes(engine, count):
+    from luxum_gb300 import Batch, Sim
+
+    def cube(n, k):
+        kw = dict(isPlanar=0, Nx=n, Ny=n + 1, Nz=n + 3, precision=2, cpml_mode=1)
+        kw.update(cases.pw((1, 0, 0), (0, 0, 1), ((9, n - 10), (9, n - 9), (9, n - 7)), off=8.0))
+        return cases.make(**kw, **cases.pml(5 + k))
+
+    ps = [cube(n, k) for k, n in enumerate((64, 71, 90, 101)[:count])]
+    sims = [Sim(p) for p in ps]
+    batch = Batch(chunk=8)
+    for s in sims:
+        batch.add(s)
+    for n in (5, 8, 8, 4):
+        batch.step(n)
+    for p, s in zip(ps, sims):
+        twin = Sim(p)
+        twin.step(25)
+        for c in range(6):
+            assert np.array_equal(s.field(c), twin.field(c)), (p.Nx, c)
+        assert s.max_e2() == twin.max_e2() > 0
+        twin.close()
+    batch.close()
+    for s in sims:
+        s.close()
