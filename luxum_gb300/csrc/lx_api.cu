@@ -2134,7 +2134,7 @@ struct lx_batch {
   void* d_tabs = nullptr;
   unsigned long long* d_slots = nullptr;
   double* d_srcv = nullptr;
-  bool sources = false;
+  bool sources = false;    // of members that share launches (the others' go with their steps)
   int last_row = 0;        // row of the last step enqueued
   long long built_at = 0;  // batch step of the last rebuild (sweep groups' parity)
   long long step = 0;  // batch steps taken (DFT sampling classes are phases of it)
@@ -2418,10 +2418,11 @@ static lx_status batch_rebuild(lx_batch* b) {
       pps[q].tab = tabs[q];
       at += (size_t)s->tab_total * b->ahead;
     }
-    b->sources |= s->src_kind >= 0;
     b->max_entries = std::max(b->max_entries, pps[q].tab_total);
     b->host_ts[q] = s->t;
     const bool solo = batch_alone(b, s);
+    pps[q].own_source = solo;
+    b->sources |= s->src_kind >= 0 && !solo;
     T* pf[6] = {(T*)s->E[0], (T*)s->E[1], (T*)s->E[2], (T*)s->H[0], (T*)s->H[1], (T*)s->H[2]};
     for (auto& d : s->dfts) {
       if (b->chunk > 0 && b->chunk % d.every != 0) b->graphable = false;
@@ -2562,16 +2563,22 @@ static lx_status solo_step(lx_batch* b, const lx_batch::Group& g, size_t m, int 
   lx::StepParams<T, C> sp = ((const lx::StepParams<T, C>*)g.host_params.data())[m];
   sp.tab += (size_t)row * sp.tab_stride;
   sp.max_slot += (size_t)row * sp.slot_stride;
+  const bool source = s->src_kind >= 0;
+  if (source) {  // into the state that step t reads
+    void* const* e = g.sweep && (t & 1) ? s->E1 : s->E;
+    BCK(lx::launch_source<T>((T*)e[s->planar ? 1 : 2], s->src_idx, s->src_kind,
+                             b->d_srcv + (size_t)row * b->sims.size() + id, false, st));
+  }
   bool swept = false;
   if constexpr (sizeof(C) == 4) {
     if (g.sweep) {  // single sweep, state t & 1 -> (t+1) & 1
       if (t & 1) swap_buffers(sp);
-      BCK(lx::launch_step_sweep2<T, C>(sp, g.uniform, false, lanes, st));
+      BCK(lx::launch_step_sweep2<T, C>(sp, g.uniform, source, lanes, st));
       swept = true;
     }
   }
   if (!swept) {
-    BCK(lx::launch_step<T, C>(sp, g.planar, g.uniform, true, false, lanes, st));
+    BCK(lx::launch_step<T, C>(sp, g.planar, g.uniform, true, source, lanes, st));
     BCK(lx::launch_step<T, C>(sp, g.planar, g.uniform, false, true, lanes, st));
   }
   for (auto& d : s->dfts) {
@@ -2625,54 +2632,51 @@ static lx_status batch_enqueue(lx_batch* b, long long step0, int nsteps) {
     const int kn = std::min(b->ahead, nsteps - q0);
     BCK(lx::launch_prologue_batch<C>(b->d_pps, b->d_ts, q0, kn, n, b->max_entries, b->d_srcv, b->d_slots, b->stream));
     b->last_row = kn - 1;
-    const int sub = b->sources ? 1 : kn;  // steps between sources: the members' amplitudes go in together
-    for (int r0 = 0; r0 < kn; r0 += sub) {
-      if (b->sources) BCK(lx::launch_source_batch(b->d_pps, b->d_ts, q0 + r0, n, b->d_srcv + (size_t)r0 * n, b->stream));
-      bool fork = false;
-      for (int l = 1; l < lx_batch::kLanes; l++) fork |= !lane[l].empty();
-      if (fork) {
-        BCK(cudaEventRecord(b->lane_ev[0], b->stream));
-        for (int l = 1; l < lx_batch::kLanes; l++)
-          if (!lane[l].empty()) BCK(cudaStreamWaitEvent(b->lanes[l - 1], b->lane_ev[0], 0));
-      }
-      size_t deep = 0;
-      for (auto& v : lane) deep = std::max(deep, v.size());
-      // a lane takes its members in turn, each through the rows: a member's state stays in L2
-      for (size_t pos = 0; pos < deep; pos++)
-        for (int r = r0; r < r0 + sub; r++)
-          for (int l = l0; l < lx_batch::kLanes; l++)
-            if (pos < lane[l].size()) {
-              const lx_status st = solo_step<T, C>(b, *lane[l][pos].g, lane[l][pos].m, q0 + r, r, lanes,
-                                                   l ? b->lanes[l - 1] : b->stream);
-              if (st) return st;
-            }
-      for (int r = r0; grouped && r < r0 + sub; r++) {
-        const long long bs = step0 + q0 + r;
-        for (int half = 0; half < 2; half++)
-          for (auto& g : b->groups) {
-            if (g.solo) continue;
-            const auto* ps = (const lx::StepParams<T, C>*)g.d_params;
-            if constexpr (sizeof(C) == 4) {
-              if (g.sweep) {
-                const auto* sw = (const lx::SweepParams<T, C>*)g.host_params.data();
-                if (half == 0)
-                  BCK(lx::launch_batch_sweep<T, C>(sw + ((bs - b->built_at) & 1) * g.members.size(), (int)g.members.size(),
-                                                   g.d_tiles, g.nblocks, g.uniform, g.march, r, b->stream));
-                continue;
-              }
-            }
-            BCK(lx::launch_batch_step<T, C>(ps, g.d_tiles, g.nblocks, g.planar, g.uniform, g.march, half == 0, r, b->stream));
-          }
-        for (auto& cl : b->dft)
-          if (bs % cl.every == cl.phase)
-            BCK(lx::launch_dft_batch<T>(cl.d_planes, cl.d_map, cl.nplanes, cl.nblocks, b->d_ts, q0 + r, b->stream));
-      }
+    bool fork = false;
+    for (int l = 1; l < lx_batch::kLanes; l++) fork |= !lane[l].empty();
+    if (fork) {
+      BCK(cudaEventRecord(b->lane_ev[0], b->stream));
       for (int l = 1; l < lx_batch::kLanes; l++)
-        if (!lane[l].empty()) {
-          BCK(cudaEventRecord(b->lane_ev[l], b->lanes[l - 1]));
-          BCK(cudaStreamWaitEvent(b->stream, b->lane_ev[l], 0));
-        }
+        if (!lane[l].empty()) BCK(cudaStreamWaitEvent(b->lanes[l - 1], b->lane_ev[0], 0));
     }
+    size_t deep = 0;
+    for (auto& v : lane) deep = std::max(deep, v.size());
+    // a lane takes its members in turn, each through the rows: a member's state stays in L2
+    for (size_t pos = 0; pos < deep; pos++)
+      for (int r = 0; r < kn; r++)
+        for (int l = l0; l < lx_batch::kLanes; l++)
+          if (pos < lane[l].size()) {
+            const lx_status st = solo_step<T, C>(b, *lane[l][pos].g, lane[l][pos].m, q0 + r, r, lanes,
+                                                 l ? b->lanes[l - 1] : b->stream);
+            if (st) return st;
+          }
+    for (int r = 0; grouped && r < kn; r++) {
+      const long long bs = step0 + q0 + r;
+      if (b->sources) BCK(lx::launch_source_batch(b->d_pps, b->d_ts, q0 + r, n, b->d_srcv + (size_t)r * n, b->stream));
+      for (int half = 0; half < 2; half++)
+        for (auto& g : b->groups) {
+          if (g.solo) continue;
+          const auto* ps = (const lx::StepParams<T, C>*)g.d_params;
+          if constexpr (sizeof(C) == 4) {
+            if (g.sweep) {
+              const auto* sw = (const lx::SweepParams<T, C>*)g.host_params.data();
+              if (half == 0)
+                BCK(lx::launch_batch_sweep<T, C>(sw + ((bs - b->built_at) & 1) * g.members.size(), (int)g.members.size(),
+                                                 g.d_tiles, g.nblocks, g.uniform, g.march, r, b->stream));
+              continue;
+            }
+          }
+          BCK(lx::launch_batch_step<T, C>(ps, g.d_tiles, g.nblocks, g.planar, g.uniform, g.march, half == 0, r, b->stream));
+        }
+      for (auto& cl : b->dft)
+        if (bs % cl.every == cl.phase)
+          BCK(lx::launch_dft_batch<T>(cl.d_planes, cl.d_map, cl.nplanes, cl.nblocks, b->d_ts, q0 + r, b->stream));
+    }
+    for (int l = 1; l < lx_batch::kLanes; l++)
+      if (!lane[l].empty()) {
+        BCK(cudaEventRecord(b->lane_ev[l], b->lanes[l - 1]));
+        BCK(cudaStreamWaitEvent(b->stream, b->lane_ev[l], 0));
+      }
   }
   if (nsteps > 0) BCK(lx::launch_tick(b->d_ts, n, nsteps, b->stream));
   return LX_OK;

@@ -113,6 +113,7 @@ struct PrologueParams {
   int src_amp_i, src_omega_i;
   double src_amp, src_omega, src_t0, src_tw;
   int prec;           // storage precision of src_field
+  int own_source;     // batched: applied with the member's own launches
 };
 
 // Device pointers and constants of one 3-D or planar simulation, passed by value.

@@ -184,7 +184,7 @@ __global__ void source_batch_kernel(const PrologueParams* __restrict__ pps, cons
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= nsims) return;
   const PrologueParams& p = pps[s];
-  if (p.src_kind < 0) return;
+  if (p.src_kind < 0 || p.own_source) return;
   void* const f = (((ts[s] + k) & 1) && p.src_field1) ? p.src_field1 : p.src_field;  // the state the step reads
   if (p.prec == 0) source_apply((double*)f + p.src_idx, p.src_kind, v[s]);
   else if (p.prec == 1) source_apply((float*)f + p.src_idx, p.src_kind, v[s]);

@@ -77,7 +77,8 @@ cudaError_t launch_block_map(const int* first, int n, int nblocks, int2* map, cu
 template <class C>
 cudaError_t launch_prologue_batch(const PrologueParams* pps, const int* ts, int k, int steps, int nsims, int max_entries,
                                   double* srcv, unsigned long long* slots, cudaStream_t s);
-// The members' point sources of step k, before its H updates (amplitudes v[sim]).
+// The point sources of step k of the members without own_source, before its H updates (amplitudes
+// v[sim]).
 cudaError_t launch_source_batch(const PrologueParams* pps, const int* ts, int k, int nsims, const double* v, cudaStream_t s);
 cudaError_t launch_tick(int* ts, int n, int steps, cudaStream_t s);
 template <class T>

@@ -132,3 +132,40 @@ def test_fp16_cubes_in_lanes(engine, count):
     batch.close()
     for s in sims:
         s.close()
+
+
+# members one by one with point sources (each in its lane), beside grouped members with and without
+@pytest.mark.parametrize("precision", [0, 1, 2])
+@pytest.mark.parametrize("hard", [0, 1])
+def test_sources_of_members_in_lanes(engine, precision, hard):
+    from luxum_gb300 import Batch, Sim
+
+    def cube(n, k):
+        kw = dict(isPlanar=0, Nx=n, Ny=n + 1, Nz=n + 3, precision=precision, cpml_mode=1)
+        if k != 1:
+            kw.update(usePS=1, source_kind=0 if hard else 1, Nx_source=n // 2, Ny_source=n // 2, Nz_source=n // 2,
+                      amp_source=5.0, omega_source=2e9 if hard else 4e10, src_t0=9.0, src_tw=5.0)
+        else:
+            kw.update(cases.pw((1, 0, 0), (0, 0, 1), ((9, n - 10), (9, n - 9), (9, n - 7)), off=8.0))
+        return cases.make(**kw, **(cases.pml(5) if k % 2 else {}))
+
+    ps = [cube(n, k) for k, n in enumerate((64, 70, 67, 81, 30, 41))]
+    ps += [_lens(1101, 1013, precision, 1), _lens(40, 50, precision, 1)]
+    sims = [Sim(p) for p in ps]
+    batch = Batch(chunk=8)
+    for k, s in enumerate(sims):
+        s.step(k % 2)
+        batch.add(s)
+    for n in (5, 8, 8, 18):
+        batch.step(n)
+    for k, (p, s) in enumerate(zip(ps, sims)):
+        twin = Sim(p)
+        twin.step(39 + k % 2)
+        for c in range(6):
+            if np.prod(s.shape(c)):
+                assert np.array_equal(s.field(c), twin.field(c)), (p.Nx, c)
+        assert s.max_e2() == twin.max_e2() > 0
+        twin.close()
+    batch.close()
+    for s in sims:
+        s.close()
