@@ -2380,28 +2380,42 @@ static lx_status batch_rebuild(lx_batch* b) {
   //         16 and 32 of 1024-1448         187 221 186, 362 408 330
   //         8 and 16 of 400-700            - 31 35, - 64 49
   //         16 and 48 of 128-256           - 16 16, - 33 29
+  // and without CPML (one by one: the sweep's form without psi):
+  //   FP32, 16, 32 and 54 of 256-512       - 25 21, - 47 37, - 71 73; 32 of 128-256 - 20 17
+  //   FP16, 32 of 724-900 and of 900-1200  117 186 143, 176 290 218; 16 of 128-256 - 14 13
   // So FP32 members go one by one from 2^19 cells.  Only in a server's batch, whose chunks are mostly
   // launched directly (2 us of host time a launch) or captured (3.5), those below 2^20 share the sweep
-  // if one launch holds them: a burst of 32 planar and 3-D requests 90.5 and 94.5 ms.
-  // FP16 is bound by instructions, which half steps have fewer of: they win by the cells of the
-  // batch, first over members that go two rows a warp in lanes (below 620 K cells, sweep_rows), then
-  // over all; and over the sweep in batches of 1.8 M cells, 4 M if their members have 2^18 or more.
+  // if one launch holds them: a burst of 32 planar and 3-D requests 90.5 and 94.5 ms.  Smaller ones
+  // share the sweep, except while their state in place stays in L2 and the two buffers of it do not
+  // (half steps are then 5-25 % faster, from fewer cells on without CPML).
+  // FP16 with CPML is bound by instructions, which half steps have fewer of: they win by the cells of
+  // the batch, first over members that go two rows a warp in lanes (below 620 K cells, sweep_rows),
+  // then over all; and over the sweep in batches of 1.8 M cells, 4 M if their members have 2^18 or
+  // more, without CPML 0.4 M.
   const bool half = sizeof(T) == 2;
-  long long cells = 0, count = 0, small = 0;  // of the planar float members; those below 2^20 cells
+  long long cells = 0, plain_cells = 0, count = 0, small = 0;  // of the planar float members; those below 2^20 cells
   for (auto* s : b->sims)
     if (s->planar && s->sweep) {
-      cells += (long long)s->Nx * s->Nz;
+      const long long c = (long long)s->Nx * s->Nz;
+      cells += c;
+      plain_cells += s->pml ? 0 : c;
       count++;
-      small += (long long)s->Nx * s->Nz < 1LL << 20;
+      small += c < 1LL << 20;
     }
+  const bool plain = 2 * plain_cells >= cells;
   b->solo_cells2 = lx_batch::kSoloCells2;
   if (!half && b->serving && small <= lx::kSweepMembers) b->solo_cells2 = 1LL << 20;
-  if (half && cells >= 6LL << 20) b->solo_cells2 = 620LL << 10;
-  if (half && (cells >= 27LL << 20 || b->half_steps)) b->solo_cells2 = 1LL << 62;
-  long long shared = 0;
-  for (auto* s : b->sims) shared += s->planar && s->sweep && !batch_alone(b, s);
-  const bool few = !b->half_steps && shared <= lx::kSweepMembers &&
-                   (!half || cells < (cells >= count << 18 ? 1LL << 22 : 7LL << 18));
+  if (half && !plain && cells >= 6LL << 20) b->solo_cells2 = 620LL << 10;
+  if (half && ((!plain && cells >= 27LL << 20) || b->half_steps)) b->solo_cells2 = 1LL << 62;
+  long long shared = 0, shared_cells = 0;
+  for (auto* s : b->sims)
+    if (s->planar && s->sweep && !batch_alone(b, s)) {
+      shared++;
+      shared_cells += (long long)s->Nx * s->Nz;
+    }
+  bool few = !b->half_steps && shared <= lx::kSweepMembers;
+  if (half) few = few && cells < (plain ? 3LL << 17 : cells >= count << 18 ? 1LL << 22 : 7LL << 18);
+  else few = few && (shared_cells < (plain ? 1LL << 20 : 3LL << 20) || shared_cells > 3LL << 21);
   for (int q = 0; q < n; q++) {
     lx_sim* s = b->sims[q];
     lx_status st;
