@@ -2071,18 +2071,25 @@ cudaError_t launch_batch_sweep(const SweepParams<T, C>* m, int n, const int4* ti
 }
 
 // {member, first row, interior, first column} of each block of the members' sweeps.  Rows a warp
-// (R) by the rows each resident warp has to do (U), as in sweep_rows: with few, short runs reach
-// more SMs; with many, long ones form the row above a run's first less often.  Us a step at 1, 2, 4, 6, 8
-// rows, FP32: 4 lenses of side 64-128 (U 0.3) 4.9, 6.2, 8.9, 11.6, 14.3; 16 (1.1) 10.0, 7.6, 9.5, 11.6,
-// 14.2; 16 of 128-256 (4.5) 31.5, 17.6, 13.9, 14.8, 16.3; 16 of 256-512 (18) 56.7, 38.4, 30.9, 30.3, 31.4;
-// 16 of 400-700 (36) 108.7, 75.6, 60.3, 57.7, 57.0; 48 of them (100) 306, 207, 161, 150, 145.  FP16, bound
-// by instructions rather than by memory, 4 and 6 rows: 8 of 256-512 22.7 and 23.6, 8 of 400-700 30.9 and 32.3.
+// (R): the fewest, up to 4, at which all blocks are resident at once, since short runs reach more
+// SMs; beyond, by the rows each resident warp has to do (U), as in sweep_rows, long ones form the row
+// above a run's first less often.  Us a step at 1, 2, 3, 4, 6, 8 rows, FP32: 4 lenses of side 64-128 (U
+// 0.3) 4.9, 6.2, 7.5, 8.9, 11.6, 14.3; 16 (1.1) 10.0, 7.6, 8.1, 9.5, 11.6, 14.2; 8 of 128-256 (2.4) 16.5,
+// 11.9, 9.6, 10.1, 12.6, 14.9; 16 of 128-256 (4.5) 31.5, 17.6, 14.9, 13.9, 14.8, 16.3; 16 of 256-512 (18)
+// 56.7, 38.4, 33.1, 30.9, 30.3, 31.4; 16 of 400-700 (36) 108.7, 75.6, 65.9, 60.3, 57.7, 57.0; 48 of them
+// (100) 306, 207, 176, 161, 150, 145.  FP16, bound by instructions rather than by memory, 4 and 6 rows: 8
+// of 256-512 22.7 and 23.6, 8 of 400-700 30.9 and 32.3.
 template <class T, class C>
 int sweep_tiles(const SweepParams<T, C>* m, int n, std::vector<int4>& tiles) {
+  constexpr double kResident = 152.0 * kBatchSweepMinBlocks;
   double U = 0;
-  for (int q = 0; q < n; ++q) U += (double)((m[q].Nz + 31) / 32) * m[q].Nx / (152.0 * 8 * kBatchSweepMinBlocks);
-  const bool half = sizeof(T) == 2;
-  const int R = U < 1 ? 1 : (U < 2 ? 2 : (U < 15 || half ? 4 : (U < 22 ? 6 : 8)));
+  for (int q = 0; q < n; ++q) U += (double)((m[q].Nz + 31) / 32) * m[q].Nx / (8 * kResident);
+  int R = U < 15 || sizeof(T) == 2 ? 4 : (U < 22 ? 6 : 8);
+  for (int r = 3; r >= 1; --r) {
+    double blocks = 0;
+    for (int q = 0; q < n; ++q) blocks += (double)((m[q].Nz + 31) / 32) * ((m[q].Nx + 8 * r - 1) / (8 * r));
+    if (blocks <= kResident) R = r;
+  }
   tiles.clear();
   for (int q = 0; q < n; ++q) {
     const SweepParams<T, C>& p = m[q];

@@ -79,9 +79,9 @@ def test_the_tuner_takes_members_of_the_half_steps(engine):
         s.close()
 
 
-# the sweep's rows a warp: 1, 2, 4, 6, 8 (4 at most in FP16), by the rows of all its members
+# the sweep's rows a warp: 1 to 4, 6, 8 (4 at most in FP16), by the rows of all its members
 @pytest.mark.parametrize("precision", [1, 2])
-@pytest.mark.parametrize("count, n, m", [(1, 130, 127), (1, 300, 511), (1, 301, 513), (2, 450, 577), (3, 513, 640),
+@pytest.mark.parametrize("count, n, m", [(1, 130, 127), (1, 300, 511), (1, 301, 513), (1, 520, 700), (2, 450, 577), (3, 513, 640),
                                          (8, 480, 700), (8, 640, 800)])
 def test_rows_of_the_batched_sweep(engine, precision, count, n, m):
     _compare([_lens(n + k, m - 5 * k, precision, k) for k in range(count)])
